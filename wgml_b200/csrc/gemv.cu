@@ -23,8 +23,8 @@
 //     are issued before the wait, so they overlap the consumers' work on the stage.
 //   * Group g belongs to block g % gridDim.x, so every SM gets the same number of groups to within
 //     one; rs and the row split are chosen per launch (see plan()).
-// Every mbarrier wait is bounded: after ~2^22 polls a waiter records an error code in the launch's
-// status word and carries on with whatever is in shared memory, so the kernel always terminates.
+// Every wait is bounded in time: a waiter that runs out records an error code in the launch's status word and
+// carries on with whatever is in shared memory, so the kernel always terminates.
 #include "async_copy.cuh"
 #include "gemv_core.cuh"
 #include "kernels.h"
@@ -64,6 +64,34 @@ __device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t *p)
     uint32_t v;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
+}
+
+// Ring slots are told apart by a count of their releases, not by the parity of an mbarrier.  The lanes of the producer
+// and epilogue warps progress independently, consumer warps take every ncl-th task, and copies land in any order, so a
+// waiter can come to a slot while the slot's previous use is unfinished; a parity is then that of the use before and
+// reads as "done" (a slot taken early is armed twice, which the hardware reports as a launch failure).  Waiting for the
+// exact number of releases first makes the parities of `full` and `done` unambiguous.
+__device__ __forceinline__ void count_set(uint32_t addr, uint32_t v)
+{
+    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ bool count_wait(uint32_t addr, uint32_t want, uint32_t *err, uint32_t code, unsigned long long limit_ns)
+{
+    if (want == 0) return true;
+    unsigned long long t0 = 0;
+#pragma unroll 1
+    for (uint32_t i = 1;; i++) {
+        uint32_t v;
+        asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+        if (v >= want) return true;
+        if ((i & 1023u) == 0) {
+            const unsigned long long t = global_ns();
+            if (!t0) t0 = t;
+            if (t - t0 > limit_ns) break;
+        }
+    }
+    if (err) atomicCAS(err, 0u, code);
+    return false;
 }
 
 __device__ __forceinline__ void cons_sync() { asm volatile("bar.sync 1, %0;" ::"n"(GEMV_CONS_THREADS) : "memory"); }
@@ -327,7 +355,8 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
     __shared__ float red[32];
     __shared__ float part[GEMV_MAX_STAGES][GEMV_NCONS][GEMV_MAX_RS];    // [stage][column part][stage row]
     __shared__ __align__(16) float lane_part[GEMV_NCONS][GEMV_TASK_ROWS][32];   // [consumer warp][task row][lane]
-    __shared__ __align__(8) unsigned long long bars[3 * GEMV_MAX_STAGES];
+    __shared__ __align__(8) unsigned long long bars[2 * GEMV_MAX_STAGES];
+    __shared__ uint32_t freed[GEMV_MAX_STAGES];    // per ring slot: how often the epilogue warp has released it
     __shared__ float2 rope_tab[GEMV_ROPE_TAB];     // (cos, sin) per pair index of a head (EPI_QKV_ROPE)
 
     const uint32_t K = a.mat[0].ncols;
@@ -335,14 +364,14 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
     const uint32_t nstage = a.nstage;
     uint8_t *smem = reinterpret_cast<uint8_t *>(smem4);
     const uint32_t ring = smem_addr(smem + a.ring_offset);
-    const uint32_t full0 = smem_addr(&bars[0]), empty0 = smem_addr(&bars[GEMV_MAX_STAGES]),
-                   done0 = smem_addr(&bars[2 * GEMV_MAX_STAGES]);
+    const uint32_t full0 = smem_addr(&bars[0]), done0 = smem_addr(&bars[GEMV_MAX_STAGES]), freed0 = smem_addr(&freed[0]);
     const uint32_t kp = a.kparts, rparts = a.rparts;
 
     // one thread per barrier: initialising them one after the other would cost a microsecond
-    if (threadIdx.x < 3 * nstage) {
+    if (threadIdx.x < 2 * nstage) {
         const uint32_t kind = threadIdx.x / nstage, s = threadIdx.x - kind * nstage;
-        mbar_init((kind == 0 ? full0 : (kind == 1 ? empty0 : done0)) + 8 * s, kind == 2 ? kp * rparts : 1);
+        mbar_init((kind == 0 ? full0 : done0) + 8 * s, kind == 1 ? kp * rparts : 1);
+        if (kind == 0) freed[s] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -370,7 +399,7 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
             uint32_t n = 0;
             const int nparts = group_parts(a, EPI, blockIdx.x + it * gridDim.x, parts, n);
             if (ci == 0) {
-                if (round) mbar_wait(empty0 + 8 * s, (round - 1) & 1, a.err, 2, a.wait_ns);
+                count_wait(freed0 + 4 * s, round, a.err, 2, a.wait_ns);
                 mbar_expect_tx(full0 + 8 * s, nparts * n * row_bytes);
             }
             __syncwarp(gmask);
@@ -409,13 +438,13 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
         const uint32_t nb = epilogue_batch(nstage);
         const uint32_t sub = (uint32_t)lane >> 3, ul = (uint32_t)lane & 7;
         const uint32_t gmask = 0xffu << (8 * sub);
-        uint32_t s = sub % nstage, phase = (sub / nstage) & 1;   // ring slot and parity of stage it0 + sub
+        uint32_t s = sub % nstage, round = sub / nstage;   // ring slot and use of stage it0 + sub
         float rms_scale = 1.0f;
         bool have_scale = false;
         for (uint32_t it0 = 0; it0 < nst; it0 += nb, s += nb) {
             while (s >= nstage) {
                 s -= nstage;
-                phase ^= 1;
+                round++;
             }
             const uint32_t it = it0 + sub;
             if (sub >= nb || it >= nst) continue;
@@ -426,7 +455,8 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
             const EpiCtx c = epi_prepare(a, EPI, parts, nparts, n, ul, nunits, rope_tab);
             uint32_t ra = 0, rb = 0;
             if (c.on) unit_rows(EPI, parts, nparts, n, ul, ra, rb);
-            mbar_wait(done0 + 8 * s, phase, a.err, 3, a.wait_ns);
+            count_wait(freed0 + 4 * s, round, a.err, 3, a.wait_ns);
+            mbar_wait(done0 + 8 * s, round & 1, a.err, 3, a.wait_ns);
             if (PRO == PRO_RMS && !have_scale) {
                 // every consumer warp wrote its sum of squares before its first arrival on a `done` barrier
                 float ss = 0.0f;
@@ -447,7 +477,7 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
                 }
             }
             __syncwarp(gmask);
-            if (ul == 0) mbar_arrive(empty0 + 8 * s);   // stage and partial sums may be overwritten
+            if (ul == 0) count_set(freed0 + 4 * s, round + 1);   // stage and partial sums may be overwritten
             epi_finish(a, EPI, parts, c, ya, yb);
         }
         if ((EPI == EPI_STORE || EPI == EPI_RESIDUAL) && a.peer_out.n) {
@@ -664,14 +694,14 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
     float *my_part = &lane_part[warp][0][0];
     uint32_t held = ~0u;   // column step whose part of the input is in `x`
     int lane_d = lane;
-    uint32_t s = 0, phase = 0, it_prev = 0;
+    uint32_t s = 0, round = 0, it_prev = 0;
     for (uint32_t t = cl; t < nst * rparts; t += ncl) {
         const uint32_t it = t >> a.rparts_log2, rp = t & (rparts - 1);
         s += it - it_prev;
         it_prev = it;
         while (s >= nstage) {
             s -= nstage;
-            phase ^= 1;
+            round++;
         }
         uint32_t nrows = a.rs;   // rows in this stage: fewer only in the last group of a matrix
         if (EPI != EPI_QKV_ROPE) {
@@ -683,7 +713,8 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
         const uint32_t j0 = rp * Rn;
         const uint32_t jn = min(Rn, nrows > j0 ? nrows - j0 : 0u);
         const uint32_t stage = ring + s * a.stage_bytes;
-        mbar_wait(full0 + 8 * s, phase, a.err, 1, a.wait_ns);
+        count_wait(freed0 + 4 * s, round, a.err, 1, a.wait_ns);
+        mbar_wait(full0 + 8 * s, round & 1, a.err, 1, a.wait_ns);
         for (uint32_t ks = kw; ks < nsteps; ks += kp) {
             const uint32_t col0 = ks * step_cols<QT>();
             if (held != ks) {
