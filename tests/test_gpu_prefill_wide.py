@@ -1,0 +1,99 @@
+"""Wide prompt passes (tens to hundreds of positions per pass): products, attention and the passes as a whole against
+float64 and against the position-by-position loop, at the edges of the tiles of positions, rows and passes."""
+import numpy as np
+import pytest
+
+import oracle
+from conftest import ATOL, RTOL, assert_close
+from helpers import SMALL_GPT2, SMALL_LLAMA, gpt2_pair, llama_pair
+from wgml_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def value_rows(fmt, dim, kv_heads, heads, n, seed):
+    """Values of layer 0 for n prompt positions (cache rows) and the same in float64: one product of the normed embedding."""
+    cfg = dict(SMALL_LLAMA, dim=dim, hidden_dim=256, n_layers=1, n_q_heads=heads, n_kv_heads=kv_heads, vocab_size=700, seq_len=n + 8)
+    t = synth.llama_tensors(cfg, seed, scale=0.002)
+    kv = dim * kv_heads // heads
+    t["blk.0.attn_v.weight"] = synth.matrix(fmt, kv, dim, seed, "v", 0.002)
+    t["token_embd.weight"] = (synth.F32, np.random.default_rng(seed).standard_normal(700 * dim).astype(np.float32) *
+                              np.repeat(10.0 ** np.random.default_rng(1).uniform(-3, 3, 700), dim).astype(np.float32))
+    gpu, _, _ = llama_pair(cfg, tensors=t)
+    prompt = synth.prompt(n + 1, 700, seed)
+    emb = t["token_embd.weight"][1].reshape(700, dim)[prompt[:n]].astype(np.float64)
+    xn = emb / np.sqrt((emb ** 2).mean(1, keepdims=True) + cfg["rms_norm_eps"]) * t["blk.0.attn_norm.weight"][1].astype(np.float64)
+    w = oracle.dequantize(fmt, t["blk.0.attn_v.weight"][1]).reshape(kv, dim).astype(np.float64)
+    return gpu, prompt, xn @ w.T
+
+
+@pytest.mark.parametrize("fmt", [synth.Q4_K, synth.Q6_K, synth.Q8_0])
+@pytest.mark.parametrize("shape", [(256, 2, 4, 16), (768, 12, 12, 97), (4096, 32, 32, 193), (1024, 16, 16, 520), (11008 // 43 * 8, 16, 16, 95)])
+def test_wide_product_vs_f64(fmt, shape):
+    """As exact as the position-by-position product: the sums of both are good to a few units of 2^-22 of the row's
+    terms, so the error of each row of outputs stays below 2e-6 of its norm and no element is off by more than 1e-5 of
+    the row's RMS (f32 sums of up to 4096 products)."""
+    dim, kvh, heads, n = shape
+    gpu, prompt, ref = value_rows(fmt, dim, kvh, heads, n, 5)
+    gpu.set_prefill(True)
+    gpu.decode(prompt, 1)
+    assert gpu.prefill_positions() == n - (n % 8 if n % 8 < 4 else 0)
+    n = gpu.prefill_positions()
+    got = gpu.value_cache(0)[:n].cpu().numpy().astype(np.float64)
+    err = np.linalg.norm(got - ref[:n], axis=1) / np.linalg.norm(ref[:n], axis=1)
+    worst = np.abs(got - ref[:n]).max(1) / np.sqrt((ref[:n] ** 2).mean(1))
+    assert err.max() < 2e-6 and worst.max() < 1e-5, (err.max(), worst.max())
+
+
+def _caches(gpu, n):
+    return [(gpu.key_cache(l)[:n].cpu().numpy(), gpu.value_cache(l)[:n].cpu().numpy()) for l in range(gpu.config.n_layers)]
+
+
+@pytest.mark.parametrize("case", [
+    dict(n_prompt=17, heads=8, kv=8, qwen=False, mixed=False),              # the smallest wide pass
+    dict(n_prompt=72, heads=8, kv=2, qwen=True, mixed=False),               # 71: 64-position attention tile + 7; biases, Neox RoPE, grouped heads
+    dict(n_prompt=90, heads=4, kv=4, qwen=False, mixed=True),               # head size 128; three formats in one layer's products
+    dict(n_prompt=620, heads=4, kv=2, qwen=False, mixed=False, seq_len=640),   # two equal passes: the second attends to the first's rows
+    dict(n_prompt=530, heads=8, kv=4, qwen=False, mixed=True, seq_len=700, start=150, n_layers=1),   # a pass that starts at a later position
+])
+def test_wide_passes_match_sequential_loop(case):
+    cfg = dict(SMALL_LLAMA, n_layers=case.get("n_layers", 3), n_q_heads=case["heads"], n_kv_heads=case["kv"], seq_len=case.get("seq_len", 128))
+    t = synth.llama_tensors(cfg, 21, biases=case["qwen"], scale=0.002)
+    if case["mixed"]:
+        kv = 512 * case["kv"] // case["heads"]
+        t["blk.0.attn_v.weight"] = synth.matrix(synth.Q6_K, kv, 512, 3, "v6", 0.002)
+        t["blk.0.ffn_down.weight"] = synth.matrix(synth.Q6_K, 512, 1024, 3, "d6", 0.002)
+        t["blk.0.ffn_up.weight"] = synth.matrix(synth.Q8_0, 1024, 512, 3, "up8", 0.002)
+        t["blk.0.attn_k.weight"] = synth.matrix(synth.Q8_0, kv, 512, 3, "k8", 0.002)
+    seq, _, _ = llama_pair(cfg, qwen=case["qwen"], tensors=t)
+    bat, _, _ = llama_pair(cfg, qwen=case["qwen"], tensors=t)
+    bat.set_prefill(True)
+    start = case.get("start", 0)
+    before = synth.prompt(start + 1, cfg["vocab_size"], seed=4)
+    prompt = synth.prompt(case["n_prompt"], cfg["vocab_size"], seed=5)
+    toks = []
+    for m in (seq, bat):
+        if start:
+            m.decode(before, 0)
+        toks.append(m.decode(prompt, 6, start_pos=start))
+    assert np.array_equal(*toks), "greedy tokens differ between wide and sequential prompt"
+    n = start + case["n_prompt"] - 1 + 6
+    for l, ((kb, vb), (ks, vs)) in enumerate(zip(_caches(bat, n), _caches(seq, n))):
+        assert_close(kb, ks, RTOL, ATOL * max(1.0, float(np.abs(ks).max())), f"key cache {l}")
+        assert_close(vb, vs, RTOL, ATOL * max(1.0, float(np.abs(vs).max())), f"value cache {l}")
+    lb, ls = bat.logits().cpu().numpy(), seq.logits().cpu().numpy()
+    assert_close(lb, ls, RTOL, ATOL * max(1.0, float(np.abs(ls).max())), "final logits")
+
+
+@pytest.mark.parametrize("qtype,n_prompt", [(synth.Q8_0, 65), (synth.Q4_K, 121)])
+def test_wide_gpt2_passes_match_sequential_loop(qtype, n_prompt):
+    cfg = dict(SMALL_GPT2, default_qtype=qtype)
+    seq, _, _ = gpt2_pair(cfg, seed=31, scale=0.002)
+    bat, _, _ = gpt2_pair(cfg, seed=31, scale=0.002)
+    bat.set_prefill(True)
+    prompt = synth.prompt(n_prompt, cfg["n_vocab"], seed=7)
+    assert np.array_equal(bat.decode(prompt, 6), seq.decode(prompt, 6))
+    for l in range(cfg["n_layer"]):
+        for a, b in ((bat.key_cache(l), seq.key_cache(l)), (bat.value_cache(l), seq.value_cache(l))):
+            a, b = a[:n_prompt].cpu().numpy(), b[:n_prompt].cpu().numpy()
+            assert_close(a, b, RTOL, ATOL * max(1.0, float(np.abs(b).max())), f"cache {l}")

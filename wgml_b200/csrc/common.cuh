@@ -51,6 +51,8 @@ struct DeviceState {
     bool prefill_attrs = false;           // the same for the batched tensor-memory kernel
     bool prefill6_attrs = false;          // the same for its Q6_K counterpart
     bool prefill8_attrs = false;          // and its Q8_0 counterpart
+    bool wide_attrs[3] = {};              // wide prompt passes: Q4_K, Q6_K, Q8_0 product
+    bool wide_attn_attrs[2] = {};         //   and attention (head size 64, 128)
     float *attn_scratch = nullptr;        // scratch of the stand-alone attention op, grown on demand
     size_t attn_scratch_floats = 0;
     uint32_t *attn_counters = nullptr;

@@ -56,6 +56,12 @@ struct wgb_gpt2 {
         float *attn_scratch = nullptr;
         uint32_t *attn_counters = nullptr, *pos = nullptr;   // pos: the PF_TOK positions of a pass
         size_t positions = 0;
+        // wide passes (all matrices have tile-major copies, head size 64 or 128): positions per pass, 0 = off
+        uint32_t wide_cap = 0;
+        uint8_t *wimg_e = nullptr, *wimg_h = nullptr;
+        float *wx = nullptr, *wq = nullptr, *wxb = nullptr;   // [wide_cap][n_embd]
+        float *wpart[2] = {};                // product slices of a wide pass
+        size_t wpart_floats = 0;
     } pf;
 };
 
@@ -257,6 +263,10 @@ void prefill_free(wgb_gpt2 *m)
     for (float *b : bufs) if (b) cudaFree(b);
     if (m->pf.attn_counters) cudaFree(m->pf.attn_counters);
     if (m->pf.pos) cudaFree(m->pf.pos);
+    if (m->pf.wimg_e) cudaFree(m->pf.wimg_e);
+    if (m->pf.wimg_h) cudaFree(m->pf.wimg_h);
+    float *wbufs[] = { m->pf.wx, m->pf.wq, m->pf.wxb, m->pf.wpart[0], m->pf.wpart[1] };
+    for (float *b : wbufs) if (b) cudaFree(b);
     m->pf = wgb_gpt2::Prefill();
 }
 
@@ -309,7 +319,7 @@ int prefill_pass(wgb_gpt2 *m, cudaStream_t s, const uint32_t *d_tokens, uint32_t
                                           n, s)))
             return rc;
         if ((rc = prefill_product(m, l, WGB_G_ATTN_QKV, pf.img_e, pf.xn, n, ntok, pf.part[0], 3 * n, &nq, s))) return rc;
-        if ((rc = launch_prefill_qkv_split(pf.part[0], nq, w.v[WGB_G_ATTN_QKV_B], pf.q, kc, vc, n, pos0, ntok, s))) return rc;
+        if ((rc = launch_prefill_qkv_split(pf.part[0], nq, PF_TOK, w.v[WGB_G_ATTN_QKV_B], pf.q, kc, vc, n, pos0, ntok, s))) return rc;
         if ((rc = launch_prefill_attention(pf.q, kc, vc, pf.xb, p.n_head, hs, 1, n, hs, pos0, ntok, attn_image ? pf.img_a : nullptr, pf.attn_scratch,
                                            pf.attn_counters, s)))
             return rc;
@@ -327,6 +337,50 @@ int prefill_pass(wgb_gpt2 *m, cudaStream_t s, const uint32_t *d_tokens, uint32_t
     }
     // leave the residual stream of the pass complete
     if ((rc = launch_prefill_ln_image(pf.x, n, pending, pending_split, n, pending_bias, nullptr, nullptr, n, ntok, nullptr, nullptr, 0, s))) return rc;
+    pf.positions += ntok;
+    return WGB_OK;
+}
+
+int wide_product(wgb_gpt2 *m, uint32_t layer, int which, const uint8_t *image, uint32_t ntok, const WideTiling &t, float *out, uint32_t *nsplit, cudaStream_t s)
+{
+    const QMat &w = m->layers[layer].m[which]->view;
+    const uint8_t *tiles = m->pf.tiles[(size_t)layer * 4 + which];
+    *nsplit = prefill_wide_splits(w.nrows, w.ncols, t, (uint32_t)(m->pf.wpart_floats / ((size_t)ntok * w.nrows)));
+    return launch_gemm_wide(w.qtype, 1, &tiles, &w.nrows, w.ncols, image, ntok, t, &out, &w.nrows, *nsplit, s);
+}
+
+// As prefill_pass, for up to wide_cap positions at a time (prefill_wide.cu).  The residual stream ends with the last
+// layer's product unfolded: nothing reads it.
+int wide_pass(wgb_gpt2 *m, cudaStream_t s, const uint32_t *d_tokens, uint32_t pos0, uint32_t ntok)
+{
+    const wgb_gpt2_params &p = m->p;
+    wgb_gpt2::Prefill &pf = m->pf;
+    const uint32_t n = p.n_embd, ff = p.ff_len, hs = n / p.n_head;
+    const WideTiling t = prefill_wide_tiling(ntok);
+    const size_t cache_stride = (size_t)p.n_seq * n;
+    int rc;
+    if ((rc = launch_embed_rows(m->wte->view, &m->wpe->view, d_tokens, pos0, ntok, pf.wx, s))) return rc;
+    const float *pending = nullptr, *pending_bias = nullptr;
+    uint32_t ns = 0, pending_split = 0;
+    for (uint32_t l = 0; l < p.n_layer; l++) {
+        const wgb_gpt2::Layer &w = m->layers[l];
+        float *kc = m->key_cache + l * cache_stride, *vc = m->value_cache + l * cache_stride;
+        if ((rc = launch_wide_norm_image(pf.wx, pending, pending_split, pending_bias, w.v[WGB_G_LN_1_G], w.v[WGB_G_LN_1_B], 1.0e-5f, n, ntok, t, pf.wimg_e, s)))
+            return rc;
+        if ((rc = wide_product(m, l, WGB_G_ATTN_QKV, pf.wimg_e, ntok, t, pf.wpart[0], &ns, s))) return rc;
+        if ((rc = launch_prefill_qkv_split(pf.wpart[0], ns, ntok, w.v[WGB_G_ATTN_QKV_B], pf.wq, kc, vc, n, pos0, ntok, s))) return rc;
+        if ((rc = launch_wide_attention(pf.wq, kc, vc, pf.wxb, p.n_head, hs, 1, n, hs, pos0, ntok, s))) return rc;
+        if ((rc = launch_wide_norm_image(pf.wxb, nullptr, 0, nullptr, nullptr, nullptr, 0.0f, n, ntok, t, pf.wimg_e, s))) return rc;
+        if ((rc = wide_product(m, l, WGB_G_ATTN_PROJ, pf.wimg_e, ntok, t, pf.wpart[1], &ns, s))) return rc;
+        if ((rc = launch_wide_norm_image(pf.wx, pf.wpart[1], ns, w.v[WGB_G_ATTN_PROJ_B], w.v[WGB_G_LN_2_G], w.v[WGB_G_LN_2_B], 1.0e-5f, n, ntok, t, pf.wimg_e, s)))
+            return rc;
+        if ((rc = wide_product(m, l, WGB_G_MLP_FC, pf.wimg_e, ntok, t, pf.wpart[0], &ns, s))) return rc;
+        if ((rc = launch_wide_gelu_image(pf.wpart[0], ns, w.v[WGB_G_MLP_FC_B], ff, ntok, t, pf.wimg_h, s))) return rc;
+        if ((rc = wide_product(m, l, WGB_G_MLP_PROJ, pf.wimg_h, ntok, t, pf.wpart[1], &ns, s))) return rc;
+        pending = pf.wpart[1];
+        pending_bias = w.v[WGB_G_MLP_PROJ_B];
+        pending_split = ns;
+    }
     pf.positions += ntok;
     return WGB_OK;
 }
@@ -612,11 +666,11 @@ WGB_EXPORT int wgb_gpt2_decode(wgb_gpt2 *m, const uint32_t *h_prompt, size_t n_p
     if (m->pf.enabled && n_prompt - 1 >= PF_TOK) {
         const size_t rem = (n_prompt - 1) % PF_TOK;
         const size_t batched = n_prompt - 1 - (rem >= PF_TOK / 2 ? 0 : rem);
-        for (; done < batched; done += PF_TOK) {
-            const uint32_t nt = (uint32_t)(batched - done < PF_TOK ? batched - done : PF_TOK);
-            if ((rc = prefill_pass(m, s, m->d_prompt + done, start_pos + (uint32_t)done, nt))) return rc;
+        while (done < batched) {
+            const uint32_t nt = prefill_next_pass(batched - done, m->pf.wide_cap), pos = start_pos + (uint32_t)done;
+            if ((rc = nt > PF_TOK ? wide_pass(m, s, m->d_prompt + done, pos, nt) : prefill_pass(m, s, m->d_prompt + done, pos, nt))) return rc;
+            done += nt;
         }
-        done = batched;
         WGB_CUDA(cudaMemcpyAsync(m->d_out, m->d_prompt + 1, done * 4, cudaMemcpyDeviceToDevice, s));   // step i reports prompt[i + 1]
     }
     set_scalars_kernel<<<1, 1, 0, s>>>(m->scalars, h_prompt[done], start_pos + (uint32_t)done, (uint32_t)done);
@@ -716,6 +770,18 @@ WGB_EXPORT int wgb_gpt2_set_prefill(wgb_gpt2 *m, int enable)
         if (e == cudaSuccess) e = cudaMemset(pf.attn_counters, 0, nc * 4);
         if (e == cudaSuccess) e = cudaMalloc((void **)&pf.pos, PF_TOK * 4);
         if (e != cudaSuccess) { prefill_free(m); return cuda_fail(e, "cudaMalloc(prompt pass state)"); }
+    }
+    bool wide = prefill_wide_attention_supported(hs);
+    for (const uint8_t *t : pf.tiles) wide = wide && t;
+    if (wide) {
+        const size_t cap = std::min<size_t>(PW_CAP, p.n_seq);
+        pf.wpart_floats = cap * std::max<size_t>(4 * (size_t)n, ff);
+        if (cudaMalloc((void **)&pf.wimg_e, prefill_wide_image_bytes(n)) != cudaSuccess || cudaMalloc((void **)&pf.wimg_h, prefill_wide_image_bytes(ff)) != cudaSuccess)
+            return bail(fail(WGB_ERR_CUDA, "cudaMalloc(images of a wide prompt pass)"));
+        if ((rc = dalloc(&pf.wx, cap * n)) || (rc = dalloc(&pf.wq, cap * n)) || (rc = dalloc(&pf.wxb, cap * n)) || (rc = dalloc(&pf.wpart[0], pf.wpart_floats)) ||
+            (rc = dalloc(&pf.wpart[1], pf.wpart_floats)))
+            return bail(rc);
+        pf.wide_cap = (uint32_t)cap;
     }
     WGB_CUDA(cudaDeviceSynchronize());
     pf.enabled = true;

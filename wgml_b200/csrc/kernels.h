@@ -205,13 +205,14 @@ int launch_gemm_q80_tiles(const uint8_t *w_tiles, uint32_t nrows, uint32_t K, co
 int launch_prefill_ln_image(float *x, uint32_t x_stride, const float *part, uint32_t nsplit, uint32_t part_stride, const float *fold_bias,
                             const float *gain, const float *bias, uint32_t K, uint32_t ntok, uint8_t *image, float *xn, uint32_t xn_stride,
                             cudaStream_t stream);
-int launch_prefill_qkv_split(const float *qkv, uint32_t nsplit, const float *bias, float *q_out, float *k_cache, float *v_cache, uint32_t n,
+int launch_prefill_qkv_split(const float *qkv, uint32_t nsplit, uint32_t slice_tok, const float *bias, float *q_out, float *k_cache, float *v_cache, uint32_t n,
                              uint32_t pos0, uint32_t ntok, cudaStream_t stream);
 int launch_prefill_gelu_image(const float *part, uint32_t nsplit, uint32_t stride, const float *bias, uint32_t K, uint32_t ntok, uint8_t *image,
                               float *h, uint32_t h_stride, cudaStream_t stream);
 int launch_prefill_positions(uint32_t *positions, uint32_t pos0, cudaStream_t stream);
 struct PrefillQkv {
-    const float *q, *k, *v;            // product slices: [split][PF_TOK][stride]
+    const float *q, *k, *v;            // product slices: [split][slice_tok][stride]
+    uint32_t slice_tok;                // positions per slice
     uint32_t q_split, k_split, v_split, q_stride, kv_stride;
     const float *bq, *bk, *bv;         // optional biases
     float *q_out;                      // [ntok][q_dim]
@@ -232,5 +233,40 @@ size_t prefill_attention_counters(uint32_t n_heads);
 int launch_prefill_attention(const float *q, const float *k_cache, const float *v_cache, float *out, uint32_t n_heads, uint32_t head_size,
                              uint32_t kv_mul, uint32_t row_stride, uint32_t head_stride, uint32_t pos0, uint32_t ntok, uint8_t *image,
                              float *scratch, uint32_t *counters, cudaStream_t stream);
+
+
+// ---- wide prompt passes (prefill_wide.cu) ---------------------------------------------------------------
+constexpr uint32_t PW_CAP = 512;   // prompt positions per wide pass, most
+constexpr uint32_t PW_MIN = 16;    // fewer than this go through the passes of PF_TOK positions
+// Tiles of positions of a pass: npt tiles of np positions each.
+struct WideTiling { uint32_t np, npt; };
+WideTiling prefill_wide_tiling(uint32_t ntok);
+size_t prefill_wide_image_bytes(uint32_t K);
+uint32_t prefill_wide_splits(uint32_t nrows, uint32_t K, const WideTiling &t, uint32_t max_split);
+// out[i][slice][ntok][out_stride[i]] = slices of the products of up to three tile-major matrices (all of format `qtype`:
+// Q4_K, Q6_K or Q8_0) with the vectors of a wide image.
+int launch_gemm_wide(int qtype, uint32_t nmat, const uint8_t *const *w_tiles, const uint32_t *nrows, uint32_t K, const uint8_t *image, uint32_t ntok,
+                     const WideTiling &t, float *const *out, const uint32_t *out_stride, uint32_t nsplit, cudaStream_t stream);
+// x [ntok][K] (+= slices and bias, written back); RMSNorm with `gain`, LayerNorm with `gain` and `bias`, or nothing; the image.
+int launch_wide_norm_image(float *x, const float *part, uint32_t nsplit, const float *fold_bias, const float *gain, const float *bias, float eps, uint32_t K,
+                           uint32_t ntok, const WideTiling &t, uint8_t *image, cudaStream_t stream);
+int launch_wide_silu_image(const float *gate, uint32_t gsplit, const float *up, uint32_t usplit, uint32_t K, uint32_t ntok, const WideTiling &t, uint8_t *image,
+                           cudaStream_t stream);
+int launch_wide_gelu_image(const float *part, uint32_t nsplit, const float *bias, uint32_t K, uint32_t ntok, const WideTiling &t, uint8_t *image, cudaStream_t stream);
+bool prefill_wide_attention_supported(uint32_t head_size);
+int launch_wide_attention(const float *q, const float *k_cache, const float *v_cache, float *out, uint32_t n_heads, uint32_t head_size, uint32_t kv_mul,
+                          uint32_t row_stride, uint32_t head_stride, uint32_t pos0, uint32_t ntok, cudaStream_t stream);
+// x[t] = row d_tokens[t] of the embedding (+ row pos0 + t of `pos_embd`).
+int launch_embed_rows(const QMat &embd, const QMat *pos_embd, const uint32_t *d_tokens, uint32_t pos0, uint32_t ntok, float *x, cudaStream_t stream);
+
+// Positions of the next prompt pass when `left` are still to go: equal wide passes, or passes of PF_TOK.
+inline uint32_t prefill_next_pass(size_t left, uint32_t wide_cap)
+{
+    if (wide_cap && left >= PW_MIN) {
+        const size_t passes = (left + wide_cap - 1) / wide_cap;
+        return (uint32_t)((left + passes - 1) / passes);
+    }
+    return (uint32_t)(left < PF_TOK ? left : PF_TOK);
+}
 
 }  // namespace wgb

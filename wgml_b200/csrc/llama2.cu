@@ -95,6 +95,12 @@ struct wgb_llama2 {
         uint32_t *attn_counters = nullptr;   //   and arrival counters
         float *red = nullptr;                // tensor parallel: [PF_TOK][dim], a rank's partial product summed over the group
         size_t positions = 0;                // prompt positions that went through it, over all decode calls
+        // wide passes (all matrices have tile-major copies, one rank, head size 64 or 128): positions per pass, 0 = off
+        uint32_t wide_cap = 0;
+        uint8_t *wimg_dim = nullptr, *wimg_q = nullptr, *wimg_hidden = nullptr;
+        float *wx = nullptr, *wq = nullptr, *wxb = nullptr;   // [wide_cap][dim | q_dim]
+        float *wpart[3] = {};                // product slices of a wide pass
+        size_t wpart_floats = 0;             //   floats of each
     } pf;
 };
 
@@ -428,6 +434,10 @@ void prefill_free(wgb_llama2 *m)
     float *bufs[] = { m->pf.x, m->pf.xn, m->pf.q, m->pf.xb, m->pf.h, m->pf.part[0], m->pf.part[1], m->pf.part[2], m->pf.red, m->pf.attn_scratch };
     if (m->pf.attn_counters) cudaFree(m->pf.attn_counters);
     for (float *b : bufs) if (b) cudaFree(b);
+    uint8_t *wimgs[] = { m->pf.wimg_dim, m->pf.wimg_q, m->pf.wimg_hidden };
+    for (uint8_t *b : wimgs) if (b) cudaFree(b);
+    float *wbufs[] = { m->pf.wx, m->pf.wq, m->pf.wxb, m->pf.wpart[0], m->pf.wpart[1], m->pf.wpart[2] };
+    for (float *b : wbufs) if (b) cudaFree(b);
     m->pf = wgb_llama2::Prefill();
 }
 
@@ -539,6 +549,7 @@ int prefill_pass(wgb_llama2 *m, cudaStream_t s, const uint32_t *d_tokens, uint32
         qa.q_split = nq; qa.k_split = nk; qa.v_split = nv;
         qa.q_stride = q_dim; qa.kv_stride = kv_dim;
         qa.bq = w.v[WGB_L_ATTN_Q_BIAS]; qa.bk = w.v[WGB_L_ATTN_K_BIAS]; qa.bv = w.v[WGB_L_ATTN_V_BIAS];
+        qa.slice_tok = PF_TOK;
         qa.q_out = pf.q;
         qa.k_cache = m->key_cache + l * cache_stride;
         qa.v_cache = m->value_cache + l * cache_stride;
@@ -572,6 +583,81 @@ int prefill_pass(wgb_llama2 *m, cudaStream_t s, const uint32_t *d_tokens, uint32
     }
     // leave the residual stream of the pass complete (nothing reads it; it keeps wgb_llama2_x meaningful for tests)
     if ((rc = launch_prefill_norm_image(pf.x, dim, pending, pending_split, dim, nullptr, 0.0f, dim, ntok, nullptr, nullptr, 0, s))) return rc;
+    pf.positions += ntok;
+    return WGB_OK;
+}
+
+// Products of `n` matrices of a layer with the same input in a wide pass, product i as slices [slice][ntok][rows] in
+// out[i]: one launch per run of matrices of one format.
+int wide_products(wgb_llama2 *m, uint32_t layer, const int *which, uint32_t n, const uint8_t *image, uint32_t ntok, const WideTiling &t, float *const *out,
+                  uint32_t *nsplit, cudaStream_t s)
+{
+    const wgb_llama2::Prefill &pf = m->pf;
+    for (uint32_t i = 0; i < n;) {
+        const QMat &w0 = m->layers[layer].m[which[i]]->view;
+        const uint8_t *tiles[3];
+        uint32_t rows[3], total = 0, widest = 0, cnt = 0;
+        for (; i + cnt < n; cnt++) {
+            const QMat &w = m->layers[layer].m[which[i + cnt]]->view;
+            if (w.qtype != w0.qtype) break;
+            tiles[cnt] = pf.tiles[(size_t)layer * 7 + which[i + cnt]];
+            rows[cnt] = w.nrows;
+            total += w.nrows;
+            widest = std::max(widest, w.nrows);
+        }
+        const uint32_t ns = prefill_wide_splits(total, w0.ncols, t, (uint32_t)(pf.wpart_floats / ((size_t)ntok * widest)));
+        for (uint32_t k = 0; k < cnt; k++) nsplit[i + k] = ns;
+        int rc = launch_gemm_wide(w0.qtype, cnt, tiles, rows, w0.ncols, image, ntok, t, out + i, rows, ns, s);
+        if (rc) return rc;
+        i += cnt;
+    }
+    return WGB_OK;
+}
+
+// As prefill_pass, for up to wide_cap positions at a time (prefill_wide.cu).  The residual stream ends with the last
+// layer's products unfolded: nothing reads it.
+int wide_pass(wgb_llama2 *m, cudaStream_t s, const uint32_t *d_tokens, uint32_t pos0, uint32_t ntok)
+{
+    const wgb_llama2_config &c = m->cfg;
+    wgb_llama2::Prefill &pf = m->pf;
+    const uint32_t dim = c.dim, q_dim = m->q_dim, kv_dim = m->kv_dim, hidden = m->hidden;
+    const WideTiling t = prefill_wide_tiling(ntok);
+    const size_t cache_stride = (size_t)c.seq_len * kv_dim;
+    int rc;
+    if ((rc = launch_embed_rows(m->token_embd->view, nullptr, d_tokens, pos0, ntok, pf.wx, s))) return rc;
+    const float *pending = nullptr;
+    uint32_t ns[3] = {}, pending_split = 0;
+    for (uint32_t l = 0; l < c.n_layers; l++) {
+        const wgb_llama2::Layer &w = m->layers[l];
+        const int qkv[3] = { WGB_L_ATTN_Q, WGB_L_ATTN_K, WGB_L_ATTN_V }, gu[2] = { WGB_L_FFN_GATE, WGB_L_FFN_UP };
+        const int wo = WGB_L_ATTN_OUTPUT, wd = WGB_L_FFN_DOWN;
+        if ((rc = launch_wide_norm_image(pf.wx, pending, pending_split, nullptr, w.v[WGB_L_ATTN_NORM], nullptr, c.rms_norm_eps, dim, ntok, t, pf.wimg_dim, s))) return rc;
+        if ((rc = wide_products(m, l, qkv, 3, pf.wimg_dim, ntok, t, pf.wpart, ns, s))) return rc;
+        PrefillQkv qa = {};
+        qa.q = pf.wpart[0]; qa.k = pf.wpart[1]; qa.v = pf.wpart[2];
+        qa.q_split = ns[0]; qa.k_split = ns[1]; qa.v_split = ns[2];
+        qa.slice_tok = ntok;
+        qa.q_stride = q_dim; qa.kv_stride = kv_dim;
+        qa.bq = w.v[WGB_L_ATTN_Q_BIAS]; qa.bk = w.v[WGB_L_ATTN_K_BIAS]; qa.bv = w.v[WGB_L_ATTN_V_BIAS];
+        qa.q_out = pf.wq;
+        qa.k_cache = m->key_cache + l * cache_stride;
+        qa.v_cache = m->value_cache + l * cache_stride;
+        qa.q_dim = q_dim; qa.kv_dim = kv_dim; qa.head_size = m->head_size; qa.seq_len = c.seq_len; qa.pos0 = pos0;
+        qa.variant = m->model_type == WGB_QWEN2 ? WGB_ROPE_NEOX : WGB_ROPE_ORIGINAL;
+        qa.freq = m->rope_freq;
+        if ((rc = launch_prefill_rope_append(qa, ntok, s))) return rc;
+        if ((rc = launch_wide_attention(pf.wq, qa.k_cache, qa.v_cache, pf.wxb, m->n_q_local, m->head_size, m->kv_mul, m->head_size, c.seq_len * m->head_size, pos0,
+                                        ntok, s)))
+            return rc;
+        if ((rc = launch_wide_norm_image(pf.wxb, nullptr, 0, nullptr, nullptr, nullptr, 0.0f, q_dim, ntok, t, pf.wimg_q, s))) return rc;
+        if ((rc = wide_products(m, l, &wo, 1, pf.wimg_q, ntok, t, pf.wpart, ns, s))) return rc;
+        if ((rc = launch_wide_norm_image(pf.wx, pf.wpart[0], ns[0], nullptr, w.v[WGB_L_FFN_NORM], nullptr, c.rms_norm_eps, dim, ntok, t, pf.wimg_dim, s))) return rc;
+        if ((rc = wide_products(m, l, gu, 2, pf.wimg_dim, ntok, t, pf.wpart, ns, s))) return rc;
+        if ((rc = launch_wide_silu_image(pf.wpart[0], ns[0], pf.wpart[1], ns[1], hidden, ntok, t, pf.wimg_hidden, s))) return rc;
+        if ((rc = wide_products(m, l, &wd, 1, pf.wimg_hidden, ntok, t, pf.wpart + 2, ns, s))) return rc;
+        pending = pf.wpart[2];
+        pending_split = ns[0];
+    }
     pf.positions += ntok;
     return WGB_OK;
 }
@@ -1172,11 +1258,11 @@ WGB_EXPORT int wgb_llama2_decode(wgb_llama2 *m, const uint32_t *h_prompt, size_t
     if (m->pf.enabled && n_prompt - 1 >= PF_TOK) {
         const size_t rem = (n_prompt - 1) % PF_TOK;
         const size_t batched = n_prompt - 1 - (rem >= PF_TOK / 2 ? 0 : rem);
-        for (; done < batched; done += PF_TOK) {
-            const uint32_t nt = (uint32_t)(batched - done < PF_TOK ? batched - done : PF_TOK);
-            if ((rc = prefill_pass(m, s, m->d_prompt + done, start_pos + (uint32_t)done, nt))) return rc;
+        while (done < batched) {
+            const uint32_t nt = prefill_next_pass(batched - done, m->pf.wide_cap), pos = start_pos + (uint32_t)done;
+            if ((rc = nt > PF_TOK ? wide_pass(m, s, m->d_prompt + done, pos, nt) : prefill_pass(m, s, m->d_prompt + done, pos, nt))) return rc;
+            done += nt;
         }
-        done = batched;
         // the token loop reports prompt[i + 1] for step i < n_prompt - 1
         WGB_CUDA(cudaMemcpyAsync(m->d_out, m->d_prompt + 1, done * 4, cudaMemcpyDeviceToDevice, s));
     }
@@ -1296,6 +1382,22 @@ WGB_EXPORT int wgb_llama2_set_prefill(wgb_llama2 *m, int enable)
         cudaError_t e = cudaMalloc((void **)&pf.attn_counters, nc * 4);
         if (e == cudaSuccess) e = cudaMemset(pf.attn_counters, 0, nc * 4);
         if (e != cudaSuccess) { prefill_free(m); return cuda_fail(e, "cudaMalloc(prompt attention counters)"); }
+    }
+    bool wide = m->tp_size == 1 && prefill_wide_attention_supported(m->head_size);
+    for (const uint8_t *t : pf.tiles) wide = wide && t;
+    if (wide) {
+        const size_t cap = std::min<size_t>(PW_CAP, c.seq_len);
+        pf.wpart_floats = cap * std::max<size_t>(m->hidden, 4 * std::max<size_t>(c.dim, m->q_dim));
+        auto wimage = [&](uint8_t **p, uint32_t K) -> int {
+            WGB_CUDA(cudaMalloc((void **)p, prefill_wide_image_bytes(K)));
+            return WGB_OK;
+        };
+        if ((rc = wimage(&pf.wimg_dim, c.dim)) || (rc = wimage(&pf.wimg_q, m->q_dim)) || (rc = wimage(&pf.wimg_hidden, m->hidden)) ||
+            (rc = dalloc(&pf.wx, cap * c.dim)) || (rc = dalloc(&pf.wq, cap * m->q_dim)) || (rc = dalloc(&pf.wxb, cap * m->q_dim)))
+            return bail(rc);
+        for (int i = 0; i < 3; i++)
+            if ((rc = dalloc(&pf.wpart[i], pf.wpart_floats))) return bail(rc);
+        pf.wide_cap = (uint32_t)cap;
     }
     WGB_CUDA(cudaDeviceSynchronize());
     pf.enabled = true;

@@ -239,6 +239,27 @@ int launch_embed(const QMat &embd, const QMat *pos_embd, const uint32_t *d_token
     return WGB_OK;
 }
 
+// The same for the positions of a prompt pass, one grid row each.
+__global__ void embed_rows_kernel(const __grid_constant__ QMat embd, const __grid_constant__ QMat pos_embd, int have_pos,
+                                  const uint32_t *__restrict__ d_tokens, uint32_t pos0, float *__restrict__ x)
+{
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t t = blockIdx.y, tok = d_tokens[t], pos = pos0 + t;
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= embd.ncols) return;
+    float v = tok < embd.nrows ? qmat_weight_any(embd, tok, c) : 0.0f;
+    if (have_pos && pos < pos_embd.nrows) v += qmat_weight_any(pos_embd, pos, c);
+    x[(size_t)t * embd.ncols + c] = v;
+}
+
+int launch_embed_rows(const QMat &embd, const QMat *pos_embd, const uint32_t *d_tokens, uint32_t pos0, uint32_t ntok, float *x, cudaStream_t stream)
+{
+    embed_rows_kernel<<<dim3((embd.ncols + 127) / 128, ntok), 128, 0, stream>>>(embd, pos_embd ? *pos_embd : embd, pos_embd ? 1 : 0, d_tokens, pos0, x);
+    WGB_LAUNCH_CHECK("embed_rows_kernel");
+    return WGB_OK;
+}
+
 // scratch: ARGMAX_BLOCKS 64-bit words
 int launch_argmax_advance(const float *logits, uint32_t n, const LoopState &ls, uint32_t *scratch, cudaStream_t stream)
 {

@@ -592,7 +592,7 @@ int launch_prefill_ln_image(float *x, uint32_t x_stride, const float *part, uint
 
 // The three Copy dispatches of models/gpt2/transformer.rs:329-353 for a batch of positions, with the bias of the fused
 // qkv product: rows [0, n) -> q_out[t], [n, 2n) -> key cache row pos0 + t, [2n, 3n) -> value cache row ([seq][n] caches).
-__global__ void __launch_bounds__(256) prefill_qkv_split_kernel(const float *__restrict__ qkv, uint32_t nsplit, const float *__restrict__ bias,
+__global__ void __launch_bounds__(256) prefill_qkv_split_kernel(const float *__restrict__ qkv, uint32_t nsplit, uint32_t slice_tok, const float *__restrict__ bias,
                                                                 float *__restrict__ q_out, float *__restrict__ k_cache,
                                                                 float *__restrict__ v_cache, uint32_t n, uint32_t pos0)
 {
@@ -601,17 +601,17 @@ __global__ void __launch_bounds__(256) prefill_qkv_split_kernel(const float *__r
     const uint32_t i = blockIdx.x * 256 + threadIdx.x, t = blockIdx.y;
     if (i >= 3 * n) return;
     float v = 0.0f;
-    for (uint32_t s = 0; s < nsplit; s++) v += qkv[((size_t)s * PF_TOK + t) * (3 * n) + i];
+    for (uint32_t s = 0; s < nsplit; s++) v += qkv[((size_t)s * slice_tok + t) * (3 * n) + i];
     if (bias) v += bias[i];
     if (i < n) q_out[(size_t)t * n + i] = v;
     else if (i < 2 * n) k_cache[(size_t)(pos0 + t) * n + (i - n)] = v;
     else v_cache[(size_t)(pos0 + t) * n + (i - 2 * n)] = v;
 }
 
-int launch_prefill_qkv_split(const float *qkv, uint32_t nsplit, const float *bias, float *q_out, float *k_cache, float *v_cache, uint32_t n,
+int launch_prefill_qkv_split(const float *qkv, uint32_t nsplit, uint32_t slice_tok, const float *bias, float *q_out, float *k_cache, float *v_cache, uint32_t n,
                              uint32_t pos0, uint32_t ntok, cudaStream_t stream)
 {
-    WGB_CUDA(launch_pdl(prefill_qkv_split_kernel, dim3((3 * n + 255) / 256, ntok), dim3(256), 0, stream, qkv, nsplit, bias, q_out, k_cache, v_cache, n,
+    WGB_CUDA(launch_pdl(prefill_qkv_split_kernel, dim3((3 * n + 255) / 256, ntok), dim3(256), 0, stream, qkv, nsplit, slice_tok, bias, q_out, k_cache, v_cache, n,
                         pos0));
     return WGB_OK;
 }
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(128) prefill_rope_append_kernel(PrefillQkv a)
     else { ia = i + ((2 * i) / a.head_size) * half; ib = ia + half; }
     auto gather = [&](const float *p, uint32_t nsplit, uint32_t stride, const float *bias, uint32_t idx) {
         float v = 0.0f;
-        for (uint32_t s = 0; s < nsplit; s++) v += p[((size_t)s * PF_TOK + t) * stride + idx];
+        for (uint32_t s = 0; s < nsplit; s++) v += p[((size_t)s * a.slice_tok + t) * stride + idx];
         return v + (bias ? bias[idx] : 0.0f);
     };
     float x = gather(a.q, a.q_split, a.q_stride, a.bq, ia), y = gather(a.q, a.q_split, a.q_stride, a.bq, ib);

@@ -1,0 +1,901 @@
+// Wide prompt passes: up to PW_CAP prompt positions per pass through the layer stack.
+//
+// The passes of eight positions (prefill.cu) read every weight once per eight positions and spend their time on the
+// chain unpack -> MMA -> read-back of each 256-column unit, whose tensor work is 4 % of it.  With a long prompt the
+// same unpacked weights can serve up to 96 positions at a time, and the pass becomes a contraction proper: this file
+// holds its matrix product on the tensor cores (tcgen05.mma kind::f16 with f32 accumulators in tensor memory), the
+// activation image it reads, the element-wise kernels between the products and a causal attention over tiles of 64
+// positions.  Operators as in the narrow passes: GemvQuant::dispatch (crates/wgml/src/ops/gemv_quant.rs:241-348),
+// RmsNorm / LayerNorm / Silu / GELU / BatchedMultiqueryAttention of one position, for many.
+//
+// Arithmetic.  A unit is 256 columns.  Activations: x = X * 2^e with one exponent per position and unit, |X| <= 2^22,
+// written as two f16 digits X = 2048 hi + lo (hi an integer, |hi| <= 2048; |lo| <= 1024 rounded to eleven bits, so X is
+// good to a quarter on average: finer than the integer X of the other products, which makes up for the exponent being
+// shared by 256 columns instead of 32).  Weights: the
+// part of a weight that varies inside a unit, as one or two f16 integers,
+//   Q4_K  scale * code           <= 945: one plane;  d per row and unit, mins through a product of their own
+//   Q6_K  scale * (code - 32)    <= 4096 in magnitude: 16 a1 + a2, two planes;  d per row and unit
+//   Q8_0  code * d_group / 2^E   18 bits: a1 + a2 (a1 an integer <= 512), two planes;  2^E the row's power of two
+// so every product is an integer below 2^22 (a few bits more for a2) and the sums of a unit stay within or near the
+// 24 bits of the f32 accumulator; the small planes go first, while the accumulator is small.  After a unit
+// the two digit sums are joined and scaled in f32, as in the other products.
+#include "kernels.h"
+#include "tc_common.cuh"
+
+#include <algorithm>
+
+namespace wgb {
+
+constexpr uint32_t PW_MAXN = 96;                                   // positions per tile (two digits each: N = 192)
+constexpr uint32_t PW_UNPACK_WARPS = 8;                            // build the weight operand
+constexpr uint32_t PW_FINISH_WARPS = 8;                            // read the sums, apply scales
+constexpr uint32_t PW_NT = 32 * (2 + PW_UNPACK_WARPS + PW_FINISH_WARPS);
+constexpr uint32_t PW_A_STEP = TC_TILE_ROWS * 128;                 // weight operand of a step: 64 columns in f16
+constexpr uint32_t PW_B_STEP = 2 * PW_MAXN * 128;                  // activation operand of a step, largest
+constexpr uint32_t PW_STAGE = PW_A_STEP + PW_B_STEP;
+constexpr uint32_t PW_AUX = 36 * PW_MAXN;                          // per unit: sums of the mins' product, exponents
+constexpr uint32_t PW_AMIN = 2 * TC_TILE_ROWS * 16;                // mins as f16, [two K-cores][row]
+constexpr uint32_t PW_TMEM_COLS = 512;                             // two sets of 2 x 96 sums, one of 96 min sums
+constexpr uint32_t PW_TMEM_MIN = 4 * PW_MAXN;
+
+// Per format: raw bytes of a unit of 128 rows (tile-major copies of prefill.cu, prefill_q6k.cu, prefill_q80.cu).
+template <int FMT> struct PwFmt;
+template <> struct PwFmt<WGB_Q4_K> { static constexpr uint32_t RAW = TC_UNIT_BYTES, STAGES = 4, PLANES = 1, AMIN = PW_AMIN; };
+template <> struct PwFmt<WGB_Q6_K> { static constexpr uint32_t RAW = TC_TILE_ROWS * 210, STAGES = 4, PLANES = 2, AMIN = 0; };
+template <> struct PwFmt<WGB_Q8_0> { static constexpr uint32_t RAW = TC_TILE_ROWS * 272, STAGES = 3, PLANES = 2, AMIN = 0; };
+template <int FMT> constexpr uint32_t pw_unit_slot() { return (PwFmt<FMT>::AMIN + PwFmt<FMT>::RAW + PW_AUX + 127) / 128 * 128; }
+template <int FMT> constexpr uint32_t pw_smem() { return PwFmt<FMT>::STAGES * PW_STAGE + 2 * pw_unit_slot<FMT>(); }
+static_assert(pw_smem<WGB_Q4_K>() + 1024 + 512 <= 227 * 1024 && pw_smem<WGB_Q6_K>() + 1024 + 512 <= 227 * 1024 && pw_smem<WGB_Q8_0>() + 1024 + 512 <= 227 * 1024,
+              "shared memory budget");
+static_assert(PW_STAGE % 1024 == 0 && PW_A_STEP % 1024 == 0, "swizzled operands start on 1 KB boundaries");
+static_assert(PW_TMEM_MIN + PW_MAXN <= PW_TMEM_COLS, "tensor memory");
+
+// Activation image of a pass: [tile of np positions][unit]: four steps of 64 columns, each [hi rows | lo rows] x 128
+// bytes in the 128-byte swizzle; then the sums of the eight 32-column groups as two f16 digits
+// ([digit][position][group]); then one exponent (a power of two) per position.
+__host__ __device__ constexpr uint32_t pw_image_unit(uint32_t np) { return (1024 + 36) * np; }
+
+size_t prefill_wide_image_bytes(uint32_t K)
+{
+    // any split of PW_CAP positions into tiles of a multiple of 8 pads by less than one such multiple per tile
+    return (size_t)(K / 256) * pw_image_unit(PW_CAP + 8 * ((PW_CAP + PW_MAXN - 1) / PW_MAXN + 1));
+}
+
+struct PwArgs {
+    const uint8_t *w[3];
+    float *out[3];            // [nsplit][slice_tok][out_stride]
+    uint32_t tile0[3];
+    uint32_t out_stride[3];
+    uint32_t nmat, ntiles;
+    const uint8_t *img;
+    uint32_t nkb, nsplit, ntok, np, npt, slice_tok;
+    uint32_t *err;
+};
+
+// Items of a block: blockIdx.x, blockIdx.x + gridDim.x, ...; item = ((tile, slice of the units), tile of positions),
+// positions fastest, so that blocks running side by side read the same weights.
+struct PwWalk {
+    uint32_t tile, sp, pt, kb, kb_end;
+    __device__ __forceinline__ void set(const PwArgs &a, uint32_t item)
+    {
+        pt = item % a.npt;
+        const uint32_t r = item / a.npt;
+        sp = r % a.nsplit;
+        tile = r / a.nsplit;
+        kb = sp * a.nkb / a.nsplit;
+        kb_end = (sp + 1) * a.nkb / a.nsplit;
+    }
+};
+__device__ __forceinline__ uint32_t pw_matrix_of(const PwArgs &a, uint32_t tile)
+{
+    return (a.nmat > 2 && tile >= a.tile0[2]) ? 2u : (a.nmat > 1 && tile >= a.tile0[1]) ? 1u : 0u;
+}
+
+__device__ __forceinline__ void pw_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.u32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// kind::f16 instruction descriptor: D f32, A and B f16, both K-major, M = 128, N = n.
+__device__ __forceinline__ uint32_t pw_idesc(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24); }
+
+__device__ __forceinline__ __half2 u2h(uint32_t v) { return *reinterpret_cast<__half2 *>(&v); }
+__device__ __forceinline__ uint32_t h2u(__half2 v) { return *reinterpret_cast<uint32_t *>(&v); }
+
+// Two f32 at a time (the packed FMA of this architecture).
+__device__ __forceinline__ uint64_t f2pack(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2unpack(uint64_t v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t f2fma(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2mul(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// Exponent field of the power of two above the largest of a row's eight Q8_0 scales (clamped above zero).
+__device__ __forceinline__ uint32_t pw_q80_exp(uint4 sc)
+{
+    uint32_t m = 0;
+    const uint32_t w[4] = { sc.x, sc.y, sc.z, sc.w };
+#pragma unroll
+    for (int i = 0; i < 4; i++) m = max(m, max(w[i] & 0x7fffu, (w[i] >> 16) & 0x7fffu));
+    const uint32_t ex = __float_as_uint(__half2float(__ushort_as_half((unsigned short)m))) >> 23;
+    return ex < 100u ? 100u : (ex > 142u ? 142u : ex);
+}
+
+// Weight operand of one step for (row r, half h): `raw` = the unit's raw bytes, step chunk c (64 columns), plane 0 = the
+// small one of a two-plane format.  Writes 32 f16 values into the row at `arow` (16-byte chunks swizzled by the row).
+template <int FMT>
+__device__ __forceinline__ void pw_unpack(uint32_t raw, uint32_t arow, uint32_t r, uint32_t h, uint32_t c, bool small_plane)
+{
+    const uint32_t sw = r & 7;
+    if constexpr (FMT == WGB_Q4_K) {
+        const uint4 hdr = lds128(raw + r * 144);
+        const uint32_t j0 = 2 * c;
+        const uint32_t sc_lo = hdr.y & 0x3f3f3f3fu, sc_hi = (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u);
+        const uint32_t scw = ((j0 & 4) ? sc_hi : sc_lo) >> (8 * (j0 & 3));
+        const uint4 q = lds128(raw + r * 144 + 16 + 32 * c + 16 * h);
+        // 1024 + code and 1024 + 16 code as f16, times the scale (a sixteenth of it), minus 1024 (64) times the scale:
+        // every intermediate is exact
+        const __half2 s0 = __half2half2(__ushort2half_rn((unsigned short)(scw & 0xffu)));
+        const __half2 s1 = __half2half2(__ushort2half_rn((unsigned short)((scw >> 8) & 0xffu)));
+        const __half2 o0 = __hmul2(s0, __float2half2_rn(-1024.0f)), o1 = __hmul2(s1, __float2half2_rn(-64.0f));
+        const __half2 s1s = __hmul2(s1, __float2half2_rn(0.0625f));
+        const uint32_t qw[4] = { q.x, q.y, q.z, q.w };
+        uint32_t lo[8], hi[8];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+#pragma unroll
+            for (int p = 0; p < 2; p++) {
+                const uint32_t t = __byte_perm(qw[k], 0u, p ? 0x4342 : 0x4140);
+                lo[2 * k + p] = h2u(__hfma2(u2h((t & 0x000f000fu) | 0x64006400u), s0, o0));
+                hi[2 * k + p] = h2u(__hfma2(u2h((t & 0x00f000f0u) | 0x64006400u), s1s, o1));
+            }
+        }
+        sts128(arow + (((2 * h) ^ sw) << 4), lo[0], lo[1], lo[2], lo[3]);
+        sts128(arow + (((2 * h + 1) ^ sw) << 4), lo[4], lo[5], lo[6], lo[7]);
+        sts128(arow + (((4 + 2 * h) ^ sw) << 4), hi[0], hi[1], hi[2], hi[3]);
+        sts128(arow + (((5 + 2 * h) ^ sw) << 4), hi[4], hi[5], hi[6], hi[7]);
+    } else if constexpr (FMT == WGB_Q6_K) {
+        const uint32_t H = c >> 1, s = 2 * (c & 1) + h;   // 128-column half, 32-column group of it
+        const uint4 scq = lds128(raw + TC_TILE_ROWS * 192 + r * 16);
+        const uint32_t scw = (s >> 1) ? (H ? scq.w : scq.y) : (H ? scq.z : scq.x);
+        const __half2 c1056 = __float2half2_rn(1056.0f), magic = __float2half2_rn(24576.0f);
+#pragma unroll
+        for (uint32_t cc = 0; cc < 2; cc++) {
+            const uint4 qlq = lds128(raw + r * 128 + (((4 * H + 2 * (s & 1) + cc) ^ sw) << 4));
+            const uint4 qhq = lds128(raw + TC_TILE_ROWS * 128 + (r >> 1) * 128 + (((4 * (r & 1) + 2 * H + cc) ^ ((r >> 1) & 7)) << 4));
+            const __half2 sc = __half2half2(__short2half_rn((short)(signed char)((scw >> (8 * (2 * (s & 1) + cc))) & 0xffu)));
+            const uint32_t qlw[4] = { qlq.x, qlq.y, qlq.z, qlq.w }, qhw[4] = { qhq.x, qhq.y, qhq.z, qhq.w };
+            uint32_t v[8];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint32_t q = ((qlw[k] >> (4 * (s >> 1))) & 0x0f0f0f0fu) | (((qhw[k] >> (2 * s)) & 0x03030303u) << 4);
+#pragma unroll
+                for (int p = 0; p < 2; p++) {
+                    const __half2 qv = __hsub2(u2h(__byte_perm(q, 0x64646464u, p ? 0x4342 : 0x4140)), c1056);
+                    const __half2 a1 = __hsub2(__hfma2(qv, sc, magic), magic);   // multiple of 16
+                    v[2 * k + p] = small_plane ? h2u(__hfma2(qv, sc, __hneg2(a1))) : h2u(a1);
+                }
+            }
+            sts128(arow + (((4 * h + 2 * cc) ^ sw) << 4), v[0], v[1], v[2], v[3]);
+            sts128(arow + (((4 * h + 2 * cc + 1) ^ sw) << 4), v[4], v[5], v[6], v[7]);
+        }
+    } else {
+        const uint4 scs = lds128(raw + TC_TILE_ROWS * 256 + r * 16);
+        const uint32_t ex = pw_q80_exp(scs), g = 2 * c + h;
+        const uint32_t scw = (g >> 1) == 0 ? scs.x : (g >> 1) == 1 ? scs.y : (g >> 1) == 2 ? scs.z : scs.w;
+        const float d = __half2float(__ushort_as_half((unsigned short)((g & 1) ? (scw >> 16) : (scw & 0xffffu))));
+        const __half2 ds = __float2half2_rn(d * __uint_as_float((255u - ex) << 23));   // d 2^(2 - E) < 4
+        const __half2 c1152 = __float2half2_rn(1152.0f), magic = __float2half2_rn(1536.0f);
+        const uint32_t row = raw + (c >> 1) * 16384 + r * 128;
+#pragma unroll
+        for (uint32_t cc = 0; cc < 2; cc++) {
+            const uint4 qq = lds128(row + (((4 * (c & 1) + 2 * h + cc) ^ sw) << 4));
+            const uint32_t qw[4] = { qq.x, qq.y, qq.z, qq.w };
+            uint32_t v[8];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint32_t u = qw[k] ^ 0x80808080u;
+#pragma unroll
+                for (int p = 0; p < 2; p++) {
+                    const __half2 qv = __hsub2(u2h(__byte_perm(u, 0x64646464u, p ? 0x4342 : 0x4140)), c1152);
+                    const __half2 a1 = __hsub2(__hfma2(qv, ds, magic), magic);   // an integer
+                    v[2 * k + p] = small_plane ? h2u(__hfma2(qv, ds, __hneg2(a1))) : h2u(a1);
+                }
+            }
+            sts128(arow + (((4 * h + 2 * cc) ^ sw) << 4), v[0], v[1], v[2], v[3]);
+            sts128(arow + (((4 * h + 2 * cc + 1) ^ sw) << 4), v[4], v[5], v[6], v[7]);
+        }
+    }
+}
+
+template <int FMT>
+__global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_constant__ PwArgs a)
+{
+    using F = PwFmt<FMT>;
+    constexpr uint32_t S = F::STAGES, STEPS = 4 * F::PLANES, SLOT = pw_unit_slot<FMT>();
+    extern __shared__ uint8_t pw_smem_raw[];
+    __shared__ __align__(8) unsigned long long bars[3 * S + 9];
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ uint32_t dead_flag;
+    uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)pw_smem_raw + 1023) & ~(uintptr_t)1023);
+    volatile uint32_t *dead = &dead_flag;
+
+    pdl_launch_dependents();
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t nitems = a.ntiles * a.nsplit * a.npt, np = a.np;
+    auto bar = [&](uint32_t i) { return smem_addr(&bars[i]); };
+    auto bar_b = [&](uint32_t s) { return bar(s); };                 // activation operand of a stage has landed
+    auto bar_a = [&](uint32_t s) { return bar(S + s); };             // weight operand of a stage is built
+    auto bar_e = [&](uint32_t s) { return bar(2 * S + s); };         // the MMAs that read the stage are done
+    auto bar_u = [&](uint32_t u) { return bar(3 * S + u); };         // raw unit has landed
+    auto bar_ue = [&](uint32_t u) { return bar(3 * S + 2 + u); };    //   and is no longer needed
+    auto bar_d = [&](uint32_t u) { return bar(3 * S + 4 + u); };     // the unit's sums are complete
+    auto bar_t = [&](uint32_t u) { return bar(3 * S + 6 + u); };     //   and have been read
+    const uint32_t bar_m = bar(3 * S + 8);                           // the min sums have been read
+    const uint32_t stage0 = smem_addr(smem), slot0 = stage0 + S * PW_STAGE;   // slot: [mins operand][raw][aux]
+
+    if (threadIdx.x == 0) {
+        dead_flag = 0;
+        for (uint32_t s = 0; s < S; s++) {
+            mbar_init(bar_b(s), 1);
+            mbar_init(bar_a(s), PW_UNPACK_WARPS);
+            mbar_init(bar_e(s), 1);
+        }
+        for (uint32_t u = 0; u < 2; u++) {
+            mbar_init(bar_u(u), 1);
+            mbar_init(bar_ue(u), PW_UNPACK_WARPS + PW_FINISH_WARPS);
+            mbar_init(bar_d(u), 1);
+            mbar_init(bar_t(u), PW_FINISH_WARPS);
+        }
+        mbar_init(bar_m, PW_FINISH_WARPS);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_slot)), "r"(PW_TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = tmem_base_slot;
+    pdl_wait();   // barriers and tensor memory are set up while the preceding launch (which writes the image) still runs
+
+    // Every role walks the same items, units m and steps n (both numbered through over the block's life) and waits on
+    // every phase of the barriers it uses, so a parity is never two phases off.  A role whose wait has expired
+    // leaves its loop; the others see the flag and follow.
+    if (warp == 0) {
+        // ------------------------------ producer ------------------------------
+        if (lane == 0) {
+            uint32_t m = 0, n = 0;
+            bool ok = true;
+            const uint32_t unit_bytes = pw_image_unit(np), bstep = 256 * np, aux = 36 * np;
+            for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+                PwWalk w;
+                w.set(a, item);
+                const uint32_t mi = pw_matrix_of(a, w.tile);
+                const uint8_t *wt = a.w[mi] + (size_t)(w.tile - a.tile0[mi]) * a.nkb * F::RAW;
+                for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++, m++) {
+                    const uint32_t u = m & 1, slot = slot0 + u * SLOT;
+                    const uint8_t *img = a.img + ((size_t)w.pt * a.nkb + kb) * unit_bytes;
+                    if (m >= 2) ok = tc_wait(bar_ue(u), ((m >> 1) - 1) & 1, dead, a.err, 41);
+                    if (!ok) break;
+                    mbar_expect_tx(bar_u(u), F::RAW + aux);
+                    bulk_copy_g2s(slot + F::AMIN, wt + (size_t)kb * F::RAW, F::RAW, bar_u(u));
+                    bulk_copy_g2s(slot + F::AMIN + F::RAW, img + 4 * bstep, aux, bar_u(u));
+                    for (uint32_t st = 0; st < STEPS; st++, n++) {
+                        const uint32_t s = n % S;
+                        if (n >= S) ok = tc_wait(bar_e(s), (n / S - 1) & 1, dead, a.err, 42);
+                        if (!ok) break;
+                        mbar_expect_tx(bar_b(s), bstep);
+                        bulk_copy_g2s(stage0 + s * PW_STAGE + PW_A_STEP, img + (st & 3) * bstep, bstep, bar_b(s));
+                    }
+                }
+            }
+            if (!ok) {
+                // the copies in flight land before the block gives its shared memory back
+                for (uint32_t k = n > S ? n - S : 0; k < n; k++) mbar_wait(bar_b(k % S), (k / S) & 1, nullptr, 0, 1000000000ull);
+                for (uint32_t k = m > 2 ? m - 2 : 0; k < m; k++) mbar_wait(bar_u(k & 1), (k >> 1) & 1, nullptr, 0, 1000000000ull);
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------ MMA issue ------------------------------
+        if (lane == 0) {
+            uint32_t m = 0, n = 0;
+            bool ok = true;
+            const uint32_t idesc = pw_idesc(2 * np), idesc_min = pw_idesc((np + 15) & ~15u);
+            for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+                PwWalk w;
+                w.set(a, item);
+                for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++, m++) {
+                    const uint32_t u = m & 1, dcol = tmem_base + u * 2 * PW_MAXN;
+                    ok = tc_wait(bar_u(u), (m >> 1) & 1, dead, a.err, 43);
+                    if (ok && m >= 2) ok = tc_wait(bar_t(u), ((m >> 1) - 1) & 1, dead, a.err, 44);
+                    for (uint32_t st = 0; st < STEPS && ok; st++, n++) {
+                        const uint32_t s = n % S;
+                        ok = tc_wait(bar_b(s), (n / S) & 1, dead, a.err, 45) && tc_wait(bar_a(s), (n / S) & 1, dead, a.err, 46);
+                        if (!ok) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint64_t ad = tc_smem_desc_sw128(stage0 + s * PW_STAGE, 1024);
+                        const uint64_t bd = tc_smem_desc_sw128(stage0 + s * PW_STAGE + PW_A_STEP, 1024);
+#pragma unroll
+                        for (uint32_t k = 0; k < 4; k++) pw_mma(dcol, ad + 2 * k, bd + 2 * k, idesc, (st | k) ? 1u : 0u);
+                        tc_commit(bar_e(s));
+                    }
+                    if (FMT == WGB_Q4_K && ok) {
+                        // sum over the eight groups of min x (sum of the group's X), both digits of the sums in one MMA
+                        if (m >= 1) ok = tc_wait(bar_m, (m - 1) & 1, dead, a.err, 47);
+                        if (ok) {
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                            const uint32_t slot = slot0 + u * SLOT;
+                            pw_mma(tmem_base + PW_TMEM_MIN, tc_smem_desc(slot, TC_TILE_ROWS * 16, 128), tc_smem_desc(slot + F::AMIN + F::RAW, np * 16, 128),
+                                   idesc_min, 0u);
+                        }
+                    }
+                    if (ok) tc_commit(bar_d(u));
+                }
+            }
+        }
+    } else if (warp < 2 + PW_UNPACK_WARPS) {
+        // ------------------------------ weight operand ------------------------------
+        const uint32_t h = (warp - 2) >> 2, r = (warp & 3) * 32 + lane;
+        const uint32_t arow0 = stage0 + (r >> 3) * 1024 + (r & 7) * 128;
+        uint32_t m = 0, n = 0;
+        bool ok = true;
+        for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+            PwWalk w;
+            w.set(a, item);
+            for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++, m++) {
+                const uint32_t u = m & 1, slot = slot0 + u * SLOT, raw = slot + F::AMIN;
+                ok = __all_sync(0xffffffffu, tc_wait(bar_u(u), (m >> 1) & 1, dead, a.err, 48));
+                if (!ok) break;
+                if (FMT == WGB_Q4_K) {
+                    // the row's eight mins, once per K-core (this thread's half writes one of the two)
+                    const uint4 hdr = lds128(raw + r * 144);
+                    const uint32_t m_lo = hdr.z & 0x3f3f3f3fu, m_hi = ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u);
+                    const __half2 k1024 = __float2half2_rn(1024.0f);
+                    sts128(slot + h * TC_TILE_ROWS * 16 + r * 16, h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4140)), k1024)),
+                           h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4342)), k1024)), h2u(__hsub2(u2h(__byte_perm(m_hi, 0x64646464u, 0x4140)), k1024)),
+                           h2u(__hsub2(u2h(__byte_perm(m_hi, 0x64646464u, 0x4342)), k1024)));
+                }
+                for (uint32_t st = 0; st < STEPS; st++, n++) {
+                    const uint32_t s = n % S;
+                    if (n >= S) ok = __all_sync(0xffffffffu, tc_wait(bar_e(s), (n / S - 1) & 1, dead, a.err, 49));
+                    if (!ok) break;
+                    pw_unpack<FMT>(raw, arow0 + s * PW_STAGE, r, h, st & 3, F::PLANES == 2 && st < 4);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_a(s));
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_ue(u));
+            }
+        }
+    } else {
+        // ------------------------------ finishing ------------------------------
+        // Thread (quarter, lane, half): row r of the tile, groups of eight positions half, half + 2, ...
+        constexpr uint32_t NG = PW_MAXN / 16;
+        const uint32_t half = (warp - 2 - PW_UNPACK_WARPS) >> 2, quarter = warp & 3, r = quarter * 32 + lane, ng = np / 8;
+        const uint32_t trow = tmem_base + ((quarter * 32u) << 16);
+        const uint64_t k2048 = f2pack(2048.0f, 2048.0f);
+        uint64_t acc[NG][4];
+        uint32_t m = 0;
+        bool ok = true;
+        for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+            PwWalk w;
+            w.set(a, item);
+#pragma unroll
+            for (uint32_t g = 0; g < NG; g++)
+#pragma unroll
+                for (uint32_t j = 0; j < 4; j++) acc[g][j] = 0ull;
+            for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++, m++) {
+                const uint32_t u = m & 1, raw = slot0 + u * SLOT + F::AMIN, ebase = raw + F::RAW + 32 * np;
+                ok = __all_sync(0xffffffffu, tc_wait(bar_u(u), (m >> 1) & 1, dead, a.err, 50));
+                if (!ok) break;
+                float d, dmin = 0.0f;
+                if constexpr (FMT == WGB_Q4_K) {
+                    uint32_t dm;
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(dm) : "r"(raw + r * 144));
+                    const float2 f = __half22float2(u2h(dm));
+                    d = f.x;
+                    dmin = f.y * -4096.0f;
+                } else if constexpr (FMT == WGB_Q6_K) {
+                    uint32_t db;
+                    asm volatile("ld.shared.u16 %0, [%1];" : "=r"(db) : "r"(raw + TC_TILE_ROWS * 208 + r * 2));
+                    d = __half2float(__ushort_as_half((unsigned short)db));
+                } else {
+                    d = __uint_as_float((pw_q80_exp(lds128(raw + TC_TILE_ROWS * 256 + r * 16)) - 1u) << 23);   // 2^(E - 2)
+                }
+                const uint64_t d2 = f2pack(d, d), dm2 = f2pack(dmin, dmin);
+                ok = __all_sync(0xffffffffu, tc_wait(bar_d(u), (m >> 1) & 1, dead, a.err, 51));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t tb = trow + u * 2 * PW_MAXN;
+#pragma unroll
+                for (uint32_t gi = 0; gi < NG; gi++) {
+                    const uint32_t g = 2 * gi + half;
+                    if (g < ng) {
+                        int hi[8], lo[8], mn[8];
+                        tc_ld8(tb + 8 * g, hi);
+                        tc_ld8(tb + np + 8 * g, lo);
+                        if (FMT == WGB_Q4_K) tc_ld8(trow + PW_TMEM_MIN + 8 * g, mn);
+                        const uint4 e0 = lds128(ebase + 32 * g), e1 = lds128(ebase + 32 * g + 16);
+                        const uint32_t ev[8] = { e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w };
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (uint32_t j = 0; j < 4; j++) {
+                            uint64_t t = f2fma(f2pack(__int_as_float(hi[2 * j]), __int_as_float(hi[2 * j + 1])), k2048,
+                                               f2pack(__int_as_float(lo[2 * j]), __int_as_float(lo[2 * j + 1])));
+                            t = f2mul(t, d2);
+                            if (FMT == WGB_Q4_K) t = f2fma(f2pack(__int_as_float(mn[2 * j]), __int_as_float(mn[2 * j + 1])), dm2, t);
+                            acc[gi][j] = f2fma(t, f2pack(__uint_as_float(ev[2 * j]), __uint_as_float(ev[2 * j + 1])), acc[gi][j]);
+                        }
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(bar_t(u));
+                    mbar_arrive(bar_m);
+                    mbar_arrive(bar_ue(u));
+                }
+            }
+            if (!ok) break;
+            const uint32_t mi = pw_matrix_of(a, w.tile), stride = a.out_stride[mi];
+            const uint32_t t0 = w.pt * np;
+            float *outp = a.out[mi] + ((size_t)w.sp * a.slice_tok + t0) * stride + (size_t)(w.tile - a.tile0[mi]) * TC_TILE_ROWS + r;
+#pragma unroll
+            for (uint32_t gi = 0; gi < NG; gi++) {
+                const uint32_t g = 2 * gi + half;
+#pragma unroll
+                for (uint32_t j = 0; j < 4; j++) {
+                    float v0, v1;
+                    f2unpack(acc[gi][j], v0, v1);
+                    const uint32_t p = 8 * g + 2 * j;
+                    if (p < np && t0 + p < a.ntok) outp[(size_t)p * stride] = v0;
+                    if (p + 1 < np && t0 + p + 1 < a.ntok) outp[(size_t)(p + 1) * stride] = v1;
+                }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(PW_TMEM_COLS) : "memory");
+    }
+}
+
+// Tiles of positions: as few as fit, of equal size (a multiple of eight).
+WideTiling prefill_wide_tiling(uint32_t ntok)
+{
+    WideTiling t;
+    t.npt = (ntok + PW_MAXN - 1) / PW_MAXN;
+    t.np = ((ntok + t.npt - 1) / t.npt + 7) & ~7u;
+    return t;
+}
+
+// Slices of the units: items are (row tile, tile of positions, slice); an item costs its units plus about one for
+// filling the pipeline and writing its rows, and the last wave should be full.  `max_split` bounds the slices by the
+// room for them.
+uint32_t prefill_wide_splits(uint32_t nrows, uint32_t K, const WideTiling &t, uint32_t max_split)
+{
+    const uint32_t tiles = nrows / TC_TILE_ROWS * t.npt, nkb = K / 256, sms = (uint32_t)sm_count();
+    uint32_t best = 1;
+    float best_cost = 1e30f;
+    for (uint32_t s = 1; s <= max_split && s <= PF_MAX_SPLIT && s <= nkb; s++) {
+        const uint32_t waves = (tiles * s + sms - 1) / sms;
+        const float cost = (float)waves * ((float)((nkb + s - 1) / s) + 1.0f) + 0.5f * (float)s;
+        if (cost < best_cost - 1e-3f) { best_cost = cost; best = s; }
+    }
+    return best;
+}
+
+template <int FMT>
+static int launch_wide(const PwArgs &a, bool *attrs, cudaStream_t stream)
+{
+    if (!*attrs) {
+        WGB_CUDA(cudaFuncSetAttribute(gemm_wide_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(pw_smem<FMT>() + 1024)));
+        *attrs = true;
+    }
+    const uint32_t items = a.ntiles * a.nsplit * a.npt, sms = (uint32_t)sm_count();
+    WGB_CUDA(launch_pdl(gemm_wide_kernel<FMT>, dim3(items < sms ? items : sms), dim3(PW_NT), pw_smem<FMT>() + 1024, stream, a));
+    return WGB_OK;
+}
+
+int launch_gemm_wide(int qtype, uint32_t nmat, const uint8_t *const *w_tiles, const uint32_t *nrows, uint32_t K, const uint8_t *image, uint32_t ntok,
+                     const WideTiling &t, float *const *out, const uint32_t *out_stride, uint32_t nsplit, cudaStream_t stream)
+{
+    WGB_REQUIRE(nmat >= 1 && nmat <= 3 && K % 256 == 0 && ntok >= 1 && ntok <= PW_CAP && nsplit >= 1 && nsplit <= K / 256 && t.np % 8 == 0 && t.np <= PW_MAXN &&
+                    t.np * t.npt >= ntok,
+                "wide product: %u matrices, %u columns, %u positions, %u slices", nmat, K, ntok, nsplit);
+    DeviceState *ds = device_state();
+    if (!ds) return WGB_ERR_CUDA;
+    PwArgs a = {};
+    for (uint32_t i = 0; i < nmat; i++) {
+        WGB_REQUIRE(nrows[i] > 0 && nrows[i] % TC_TILE_ROWS == 0, "wide product: %u rows", nrows[i]);
+        a.w[i] = w_tiles[i];
+        a.out[i] = out[i];
+        a.out_stride[i] = out_stride[i];
+        a.tile0[i] = a.ntiles;
+        a.ntiles += nrows[i] / TC_TILE_ROWS;
+    }
+    a.nmat = nmat;
+    a.img = image;
+    a.nkb = K / 256;
+    a.nsplit = nsplit;
+    a.ntok = ntok;
+    a.np = t.np;
+    a.npt = t.npt;
+    a.slice_tok = ntok;
+    a.err = gemv_status_word();
+    if (qtype == WGB_Q4_K) return launch_wide<WGB_Q4_K>(a, &ds->wide_attrs[0], stream);
+    if (qtype == WGB_Q6_K) return launch_wide<WGB_Q6_K>(a, &ds->wide_attrs[1], stream);
+    if (qtype == WGB_Q8_0) return launch_wide<WGB_Q8_0>(a, &ds->wide_attrs[2], stream);
+    return fail(WGB_ERR_INVALID, "wide product of type %d", qtype);
+}
+
+// ---- activation image ---------------------------------------------------------------------------------
+
+// One warp writes the image of 256 values of position t (lane: columns 8 lane .. 8 lane + 7 of the unit).
+__device__ __forceinline__ void wide_image_unit(uint8_t *__restrict__ image, uint32_t nkb, uint32_t np, uint32_t t, uint32_t unit, uint32_t lane, const float (&v)[8])
+{
+    float mx = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) mx = fmaxf(mx, fabsf(v[i]));
+    mx = warp_max(mx);
+    // |v| < 2^(ex - 126), so X = v * 2^(148 - ex) lies within +-2^22
+    uint32_t ex = (__float_as_uint(mx) >> 23) & 0xffu;
+    ex = ex < 24u ? 24u : (ex > 253u ? 253u : ex);
+    const float up = __uint_as_float((275u - ex) << 23), down = __uint_as_float((ex - 21u) << 23);
+    uint32_t hw[4], lw[4];
+    float hsum = 0.0f, lsum = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        float hi[2], lo[2];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const float X = v[2 * i + j] * up;
+            hi[j] = rintf(X * (1.0f / 2048.0f));
+            lo[j] = __half2float(__float2half_rn(fmaf(hi[j], -2048.0f, X)));
+            hsum += hi[j];
+            lsum += lo[j];
+        }
+        hw[i] = h2u(__floats2half2_rn(hi[0], hi[1]));
+        lw[i] = h2u(__floats2half2_rn(lo[0], lo[1]));
+    }
+    hsum += __shfl_xor_sync(0xffffffffu, hsum, 1);
+    lsum += __shfl_xor_sync(0xffffffffu, lsum, 1);
+    hsum += __shfl_xor_sync(0xffffffffu, hsum, 2);
+    lsum += __shfl_xor_sync(0xffffffffu, lsum, 2);
+    const uint32_t pt = t / np, p = t - pt * np;
+    uint8_t *base = image + ((size_t)pt * nkb + unit) * pw_image_unit(np);
+    uint8_t *row = base + (lane >> 3) * (256 * np) + p * 128 + (((lane & 7) ^ (p & 7)) << 4);
+    *reinterpret_cast<uint4 *>(row) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+    *reinterpret_cast<uint4 *>(row + np * 128) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+    uint8_t *aux = base + 1024 * np;
+    if ((lane & 3) == 0) {
+        // the group's sum over 4096 (at most 2^15), as two f16 digits
+        const float l = lsum * (1.0f / 4096.0f);
+        const __half s1 = __float2half_rn(fmaf(hsum, 0.5f, l));
+        __half *s = reinterpret_cast<__half *>(aux) + p * 8 + (lane >> 2);
+        s[0] = s1;
+        s[8 * np] = __float2half_rn(fmaf(hsum, 0.5f, -__half2float(s1)) + l);
+    }
+    if (lane == 0) *reinterpret_cast<float *>(aux + 32 * np + 4 * p) = down;
+}
+
+__device__ __forceinline__ void wide_load8(float (&v)[8], const float *__restrict__ p)
+{
+    const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + 4);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void wide_add8(float (&v)[8], const float *__restrict__ p)
+{
+    float q[8];
+    wide_load8(q, p);
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] += q[i];
+}
+__device__ __forceinline__ void wide_store8(float *__restrict__ p, const float (&v)[8])
+{
+    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4 *>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+
+// x (+= slices of a product and its bias, written back), then nothing, RMSNorm or LayerNorm (gain and bias), then the
+// image.  One block per position; a thread owns the same eight columns of every eighth unit throughout.
+constexpr uint32_t PW_NORM_NT = 256;
+__global__ void __launch_bounds__(PW_NORM_NT) wide_norm_image_kernel(float *__restrict__ x, const float *__restrict__ part, uint32_t nsplit, uint32_t ntok,
+                                                                     const float *__restrict__ fold_bias, const float *__restrict__ gain,
+                                                                     const float *__restrict__ bias, float eps, uint32_t K, uint32_t np, uint8_t *__restrict__ image)
+{
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nkb = K / 256;
+    __shared__ float red[32];
+    float *xr = x + (size_t)t * K;
+    float s = 0.0f;
+    if (part || gain) {
+        for (uint32_t u = warp; u < nkb; u += PW_NORM_NT / 32) {
+            const uint32_t i = u * 256 + lane * 8;
+            float v[8];
+            wide_load8(v, xr + i);
+            if (part) {
+                for (uint32_t k = 0; k < nsplit; k++) wide_add8(v, part + ((size_t)k * ntok + t) * K + i);
+                if (fold_bias) wide_add8(v, fold_bias + i);
+                wide_store8(xr + i, v);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) s += bias ? v[k] : v[k] * v[k];
+        }
+    }
+    if (!image) return;
+    float mean = 0.0f, scale = 1.0f;
+    if (gain) {
+        s = block_sum<PW_NORM_NT>(s, red);
+        if (bias) {
+            mean = s / (float)K;
+            float ss = 0.0f;
+            for (uint32_t u = warp; u < nkb; u += PW_NORM_NT / 32) {
+                float v[8];
+                wide_load8(v, xr + u * 256 + lane * 8);
+#pragma unroll
+                for (int k = 0; k < 8; k++) ss = fmaf(v[k] - mean, v[k] - mean, ss);
+            }
+            s = block_sum<PW_NORM_NT>(ss, red);
+        }
+        scale = 1.0f / sqrtf(s / (float)K + eps);
+    }
+    for (uint32_t u = warp; u < nkb; u += PW_NORM_NT / 32) {
+        const uint32_t i = u * 256 + lane * 8;
+        float v[8];
+        wide_load8(v, xr + i);
+        if (gain) {
+            float g[8];
+            wide_load8(g, gain + i);
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = ((v[k] - mean) * scale) * g[k];
+            if (bias) wide_add8(v, bias + i);
+        }
+        wide_image_unit(image, nkb, np, t, u, lane, v);
+    }
+}
+
+int launch_wide_norm_image(float *x, const float *part, uint32_t nsplit, const float *fold_bias, const float *gain, const float *bias, float eps, uint32_t K,
+                           uint32_t ntok, const WideTiling &t, uint8_t *image, cudaStream_t stream)
+{
+    WGB_REQUIRE(K % 256 == 0, "wide image of %u columns", K);
+    WGB_CUDA(launch_pdl(wide_norm_image_kernel, dim3(ntok), dim3(PW_NORM_NT), 0, stream, x, part, nsplit, ntok, fold_bias, gain, bias, eps, K, t.np, image));
+    return WGB_OK;
+}
+
+// act(slices of one or two products) and its image: SiLU(gate) * up (ops/silu.wgsl:19-27) or GELU(product + bias)
+// (ops/unary.wgsl:50-52).  One warp per unit and position.
+template <bool GELU>
+__global__ void __launch_bounds__(256) wide_act_image_kernel(const float *__restrict__ gate, uint32_t gsplit, const float *__restrict__ upv, uint32_t usplit,
+                                                             const float *__restrict__ bias, uint32_t K, uint32_t ntok, uint32_t np, uint8_t *__restrict__ image)
+{
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t t = blockIdx.y, lane = threadIdx.x & 31, u = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (u >= K / 256) return;
+    const size_t i = (size_t)t * K + u * 256 + lane * 8;
+    float v[8];
+    wide_load8(v, gate + i);
+    for (uint32_t k = 1; k < gsplit; k++) wide_add8(v, gate + (size_t)k * ntok * K + i);
+    if constexpr (GELU) {
+        if (bias) wide_add8(v, bias + u * 256 + lane * 8);
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = 0.5f * v[k] * (1.0f + tanhf(0.7978846f * v[k] * (1.0f + 0.044715f * v[k] * v[k])));
+    } else {
+        float b[8];
+        wide_load8(b, upv + i);
+        for (uint32_t k = 1; k < usplit; k++) wide_add8(b, upv + (size_t)k * ntok * K + i);
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = b[k] * (v[k] / (1.0f + expf(-v[k])));
+    }
+    wide_image_unit(image, K / 256, np, t, u, lane, v);
+}
+
+int launch_wide_silu_image(const float *gate, uint32_t gsplit, const float *up, uint32_t usplit, uint32_t K, uint32_t ntok, const WideTiling &t, uint8_t *image,
+                           cudaStream_t stream)
+{
+    WGB_CUDA(launch_pdl(wide_act_image_kernel<false>, dim3((K / 256 + 7) / 8, ntok), dim3(256), 0, stream, gate, gsplit, up, usplit, nullptr, K, ntok, t.np, image));
+    return WGB_OK;
+}
+int launch_wide_gelu_image(const float *part, uint32_t nsplit, const float *bias, uint32_t K, uint32_t ntok, const WideTiling &t, uint8_t *image, cudaStream_t stream)
+{
+    WGB_CUDA(launch_pdl(wide_act_image_kernel<true>, dim3((K / 256 + 7) / 8, ntok), dim3(256), 0, stream, part, nsplit, nullptr, 0u, bias, K, ntok, t.np, image));
+    return WGB_OK;
+}
+
+// ---- causal attention of a wide pass --------------------------------------------------------------------
+
+// BatchedMultiqueryAttention (ops/batched_multiquery_attention.wgsl:38-99) for positions pos0 + t, t < ntok, each
+// attending to cache rows 0 .. pos0 + t.  One block per (query head, tile of 64 positions), cache rows in tiles of 64
+// with a running softmax; everything in f32 on the CUDA cores.  256 threads: thread (ty, tx) owns positions 4 ty .. + 3,
+// scores of rows tx + 16 j, and value columns 4 tx + 64 j.  Rows of the K and Q tiles are padded by four floats so
+// that the sixteen rows a half-warp reads sit in different banks.  Longest tiles first.
+template <uint32_t HD>
+__global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__restrict__ q, const float *__restrict__ k_cache, const float *__restrict__ v_cache,
+                                                                float *__restrict__ out, uint32_t q_dim, uint32_t kv_mul, uint32_t row_stride,
+                                                                uint32_t head_stride, uint32_t pos0, uint32_t ntok)
+{
+    constexpr uint32_t LD = HD + 4, LP = 64 + 4, NC = HD / 64, NP = HD / 16;
+    extern __shared__ float wa_smem[];
+    float *qs = wa_smem, *ks = qs + 64 * LD, *vs = ks, *ps = ks + 64 * LD;   // K and V tiles take turns in one buffer
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t h = blockIdx.x, t0 = (gridDim.y - 1 - blockIdx.y) * 64, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const uint32_t nq = ntok - t0 < 64 ? ntok - t0 : 64;
+    const float *kh = k_cache + (size_t)(h / kv_mul) * head_stride, *vh = v_cache + (size_t)(h / kv_mul) * head_stride;
+    const float inv_sqrt = 1.0f / sqrtf((float)HD);
+    for (uint32_t i = tid; i < 64 * HD / 4; i += 256) {
+        const uint32_t r = i / (HD / 4), e = 4 * (i % (HD / 4));
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < nq) v = *reinterpret_cast<const float4 *>(q + (size_t)(t0 + r) * q_dim + h * HD + e);
+        *reinterpret_cast<float4 *>(qs + r * LD + e) = v;
+    }
+    float mrun[4], lrun[4];
+    float4 acc[4][NC];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        mrun[i] = -INFINITY;
+        lrun[i] = 0.0f;
+#pragma unroll
+        for (uint32_t c = 0; c < NC; c++) acc[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const uint32_t last = pos0 + t0 + nq - 1;
+    // a tile travels through registers, requested one phase before it is needed
+    float4 pre[NP];
+    auto fetch = [&](const float *base, uint32_t c0) {
+#pragma unroll
+        for (uint32_t k = 0; k < NP; k++) {
+            const uint32_t i = tid + 256 * k, r = i / (HD / 4), e = 4 * (i % (HD / 4));
+            pre[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c0 + r <= last) pre[k] = *reinterpret_cast<const float4 *>(base + (size_t)(c0 + r) * row_stride + e);
+        }
+    };
+    auto place = [&]() {
+        __syncthreads();   // the tile before has been read
+#pragma unroll
+        for (uint32_t k = 0; k < NP; k++) {
+            const uint32_t i = tid + 256 * k, r = i / (HD / 4), e = 4 * (i % (HD / 4));
+            *reinterpret_cast<float4 *>(ks + r * LD + e) = pre[k];
+        }
+        __syncthreads();
+    };
+    fetch(kh, 0);
+    for (uint32_t c0 = 0; c0 <= last; c0 += 64) {
+        place();
+        fetch(vh, c0);
+        float s[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) s[i][j] = 0.0f;
+#pragma unroll 4
+        for (uint32_t e = 0; e < HD; e += 4) {
+            float4 qv[4], kv[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) qv[i] = *reinterpret_cast<const float4 *>(qs + (4 * ty + i) * LD + e);
+#pragma unroll
+            for (int j = 0; j < 4; j++) kv[j] = *reinterpret_cast<const float4 *>(ks + (tx + 16 * j) * LD + e);
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    s[i][j] = fmaf(qv[i].x, kv[j].x, s[i][j]);
+                    s[i][j] = fmaf(qv[i].y, kv[j].y, s[i][j]);
+                    s[i][j] = fmaf(qv[i].z, kv[j].z, s[i][j]);
+                    s[i][j] = fmaf(qv[i].w, kv[j].w, s[i][j]);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint32_t p = pos0 + t0 + 4 * ty + i;   // positions past the pass (zero queries) follow the same rule
+            float mx = mrun[i];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const uint32_t row = c0 + tx + 16 * j;
+                s[i][j] = (row <= p && row <= last) ? s[i][j] * inv_sqrt : -INFINITY;
+                mx = fmaxf(mx, s[i][j]);
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            // row 0 is always attended to, so from the first tile on the maximum is finite (or the scores are not)
+            const float rs = mx == -INFINITY ? 1.0f : expf(mrun[i] - mx);
+            mrun[i] = mx;
+            float sum = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float w = s[i][j] == -INFINITY ? 0.0f : expf(s[i][j] - mx);
+                ps[(4 * ty + i) * LP + tx + 16 * j] = w;
+                sum += w;
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            lrun[i] = lrun[i] * rs + sum;
+#pragma unroll
+            for (uint32_t c = 0; c < NC; c++) { acc[i][c].x *= rs; acc[i][c].y *= rs; acc[i][c].z *= rs; acc[i][c].w *= rs; }
+        }
+        place();
+        if (c0 + 64 <= last) fetch(kh, c0 + 64);
+#pragma unroll 2
+        for (uint32_t j = 0; j < 64; j += 4) {
+            float4 pv[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) pv[i] = *reinterpret_cast<const float4 *>(ps + (4 * ty + i) * LP + j);
+#pragma unroll
+            for (int jj = 0; jj < 4; jj++) {
+#pragma unroll
+                for (uint32_t c = 0; c < NC; c++) {
+                    const float4 vv = *reinterpret_cast<const float4 *>(vs + (j + jj) * LD + 64 * c + 4 * tx);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const float w = jj == 0 ? pv[i].x : jj == 1 ? pv[i].y : jj == 2 ? pv[i].z : pv[i].w;
+                        acc[i][c].x = fmaf(w, vv.x, acc[i][c].x);
+                        acc[i][c].y = fmaf(w, vv.y, acc[i][c].y);
+                        acc[i][c].z = fmaf(w, vv.z, acc[i][c].z);
+                        acc[i][c].w = fmaf(w, vv.w, acc[i][c].w);
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        if (4 * ty + i < nq) {
+#pragma unroll
+            for (uint32_t c = 0; c < NC; c++) {
+                const float4 v = make_float4(acc[i][c].x / lrun[i], acc[i][c].y / lrun[i], acc[i][c].z / lrun[i], acc[i][c].w / lrun[i]);
+                *reinterpret_cast<float4 *>(out + (size_t)(t0 + 4 * ty + i) * q_dim + h * HD + 64 * c + 4 * tx) = v;
+            }
+        }
+    }
+}
+
+template <uint32_t HD>
+static int launch_wide_attention_hd(const float *q, const float *k_cache, const float *v_cache, float *out, uint32_t n_heads, uint32_t kv_mul, uint32_t row_stride,
+                                    uint32_t head_stride, uint32_t pos0, uint32_t ntok, bool *attrs, cudaStream_t stream)
+{
+    const size_t smem = (size_t)(2 * 64 * (HD + 4) + 64 * 68) * sizeof(float);
+    if (!*attrs) {
+        WGB_CUDA(cudaFuncSetAttribute(wide_attention_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        *attrs = true;
+    }
+    WGB_CUDA(launch_pdl(wide_attention_kernel<HD>, dim3(n_heads, (ntok + 63) / 64), dim3(256), smem, stream, q, k_cache, v_cache, out, n_heads * HD, kv_mul,
+                        row_stride, head_stride, pos0, ntok));
+    return WGB_OK;
+}
+
+bool prefill_wide_attention_supported(uint32_t head_size) { return head_size == 64 || head_size == 128; }
+
+int launch_wide_attention(const float *q, const float *k_cache, const float *v_cache, float *out, uint32_t n_heads, uint32_t head_size, uint32_t kv_mul,
+                          uint32_t row_stride, uint32_t head_stride, uint32_t pos0, uint32_t ntok, cudaStream_t stream)
+{
+    DeviceState *ds = device_state();
+    if (!ds) return WGB_ERR_CUDA;
+    if (head_size == 64)
+        return launch_wide_attention_hd<64>(q, k_cache, v_cache, out, n_heads, kv_mul, row_stride, head_stride, pos0, ntok, &ds->wide_attn_attrs[0], stream);
+    WGB_REQUIRE(head_size == 128, "wide prompt attention: head size %u", head_size);
+    return launch_wide_attention_hd<128>(q, k_cache, v_cache, out, n_heads, kv_mul, row_stride, head_stride, pos0, ntok, &ds->wide_attn_attrs[1], stream);
+}
+
+}  // namespace wgb
