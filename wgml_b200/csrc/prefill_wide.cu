@@ -26,29 +26,36 @@
 
 namespace wgb {
 
-constexpr uint32_t PW_MAXN = 96;                                   // positions per tile (two digits each: N = 192)
-constexpr uint32_t PW_UNPACK_WARPS = 8;                            // build the weight operand
+constexpr uint32_t PW_MAXN = 88;                                   // positions per tile (two digits each: N = 176)
+constexpr uint32_t PW_UNPACK_WARPS = 8;                            // build the weight operand, two groups of four
 constexpr uint32_t PW_FINISH_WARPS = 8;                            // read the sums, apply scales
-constexpr uint32_t PW_NT = 32 * (2 + PW_UNPACK_WARPS + PW_FINISH_WARPS);
+constexpr uint32_t PW_NT = 32 * (3 + PW_UNPACK_WARPS + PW_FINISH_WARPS);
 constexpr uint32_t PW_A_STEP = TC_TILE_ROWS * 128;                 // weight operand of a step: 64 columns in f16
 constexpr uint32_t PW_B_STEP = 2 * PW_MAXN * 128;                  // activation operand of a step, largest
-constexpr uint32_t PW_STAGE = PW_A_STEP + PW_B_STEP;
+constexpr uint32_t PW_A_RING = 3;                                  // odd: consecutive uses of a buffer are different groups'
+constexpr uint32_t PW_E_RING = 2 * PW_A_RING;                      // steps have a barrier pair each, six in turn
 constexpr uint32_t PW_AUX = 36 * PW_MAXN;                          // per unit: sums of the mins' product, exponents
+constexpr uint32_t PW_X_RING = 3;
 constexpr uint32_t PW_AMIN = 2 * TC_TILE_ROWS * 16;                // mins as f16, [two K-cores][row]
-constexpr uint32_t PW_TMEM_COLS = 512;                             // two sets of 2 x 96 sums, one of 96 min sums
+constexpr uint32_t PW_TMEM_COLS = 512;                             // two sets of 2 x 88 sums, one of 88 (96 written) min sums
 constexpr uint32_t PW_TMEM_MIN = 4 * PW_MAXN;
 
-// Per format: raw bytes of a unit of 128 rows (tile-major copies of prefill.cu, prefill_q6k.cu, prefill_q80.cu).
+// Per format: raw bytes of a unit of 128 rows (tile-major copies of prefill.cu, prefill_q6k.cu, prefill_q80.cu); steps of
+// the activation operand in flight (a request takes about a microsecond, a step a quarter of one: five, or what fits).
 template <int FMT> struct PwFmt;
-template <> struct PwFmt<WGB_Q4_K> { static constexpr uint32_t RAW = TC_UNIT_BYTES, STAGES = 4, PLANES = 1, AMIN = PW_AMIN; };
-template <> struct PwFmt<WGB_Q6_K> { static constexpr uint32_t RAW = TC_TILE_ROWS * 210, STAGES = 4, PLANES = 2, AMIN = 0; };
-template <> struct PwFmt<WGB_Q8_0> { static constexpr uint32_t RAW = TC_TILE_ROWS * 272, STAGES = 3, PLANES = 2, AMIN = 0; };
-template <int FMT> constexpr uint32_t pw_unit_slot() { return (PwFmt<FMT>::AMIN + PwFmt<FMT>::RAW + PW_AUX + 127) / 128 * 128; }
-template <int FMT> constexpr uint32_t pw_smem() { return PwFmt<FMT>::STAGES * PW_STAGE + 2 * pw_unit_slot<FMT>(); }
-static_assert(pw_smem<WGB_Q4_K>() + 1024 + 512 <= 227 * 1024 && pw_smem<WGB_Q6_K>() + 1024 + 512 <= 227 * 1024 && pw_smem<WGB_Q8_0>() + 1024 + 512 <= 227 * 1024,
+template <> struct PwFmt<WGB_Q4_K> { static constexpr uint32_t RAW = TC_UNIT_BYTES, B_RING = 5, PLANES = 1, AMIN = PW_AMIN; };
+template <> struct PwFmt<WGB_Q6_K> { static constexpr uint32_t RAW = TC_TILE_ROWS * 210, B_RING = 5, PLANES = 2, AMIN = 0; };
+template <> struct PwFmt<WGB_Q8_0> { static constexpr uint32_t RAW = TC_TILE_ROWS * 272, B_RING = 4, PLANES = 2, AMIN = 0; };
+template <int FMT> constexpr uint32_t pw_smem()
+{
+    return PW_A_RING * PW_A_STEP + PwFmt<FMT>::B_RING * PW_B_STEP + 2 * (PwFmt<FMT>::RAW + PwFmt<FMT>::AMIN) + PW_X_RING * PW_AUX;
+}
+constexpr uint32_t PW_STATIC = 4 * TC_TILE_ROWS * 8 + 512;         // row scales, barriers
+static_assert(pw_smem<WGB_Q4_K>() + 1024 + PW_STATIC <= 227 * 1024 && pw_smem<WGB_Q6_K>() + 1024 + PW_STATIC <= 227 * 1024 &&
+                  pw_smem<WGB_Q8_0>() + 1024 + PW_STATIC <= 227 * 1024,
               "shared memory budget");
-static_assert(PW_STAGE % 1024 == 0 && PW_A_STEP % 1024 == 0, "swizzled operands start on 1 KB boundaries");
-static_assert(PW_TMEM_MIN + PW_MAXN <= PW_TMEM_COLS, "tensor memory");
+static_assert(PW_A_STEP % 1024 == 0 && PW_B_STEP % 1024 == 0 && PW_AUX % 16 == 0, "swizzled operands start on 1 KB boundaries");
+static_assert(PW_TMEM_MIN + (PW_MAXN + 15) / 16 * 16 <= PW_TMEM_COLS, "tensor memory");
 
 // Activation image of a pass: [tile of np positions][unit]: four steps of 64 columns, each [hi rows | lo rows] x 128
 // bytes in the 128-byte swizzle; then the sums of the eight 32-column groups as two f16 digits
@@ -224,13 +231,19 @@ __device__ __forceinline__ void pw_unpack(uint32_t raw, uint32_t arow, uint32_t 
     }
 }
 
+// Roles: two producer threads (raw weights and per-unit extras; activation operand), one thread issuing MMAs, two groups
+// of four warps building the weight operand (alternate steps), eight warps finishing units.  Raw weights are free again
+// as soon as they are unpacked, a unit ahead of its MMAs; the rows' scales travel in a small ring of their own.
+// (With the raw unit held until its sums were finished, and its successor requested by the thread that feeds the
+// activation operand, a unit cost 1.4 us on top of its MMAs.)
 template <int FMT>
 __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_constant__ PwArgs a)
 {
     using F = PwFmt<FMT>;
-    constexpr uint32_t S = F::STAGES, STEPS = 4 * F::PLANES, SLOT = pw_unit_slot<FMT>();
+    constexpr uint32_t NA = PW_A_RING, NB = F::B_RING, NX = PW_X_RING, NE = PW_E_RING, STEPS = 4 * F::PLANES;
     extern __shared__ uint8_t pw_smem_raw[];
-    __shared__ __align__(8) unsigned long long bars[3 * S + 9];
+    __shared__ __align__(8) unsigned long long bars[2 * NE + 2 * NX + 13];
+    __shared__ float2 rowscale[4][TC_TILE_ROWS];
     __shared__ uint32_t tmem_base_slot;
     __shared__ uint32_t dead_flag;
     uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)pw_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -240,26 +253,34 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t nitems = a.ntiles * a.nsplit * a.npt, np = a.np;
     auto bar = [&](uint32_t i) { return smem_addr(&bars[i]); };
-    auto bar_b = [&](uint32_t s) { return bar(s); };                 // activation operand of a stage has landed
-    auto bar_a = [&](uint32_t s) { return bar(S + s); };             // weight operand of a stage is built
-    auto bar_e = [&](uint32_t s) { return bar(2 * S + s); };         // the MMAs that read the stage are done
-    auto bar_u = [&](uint32_t u) { return bar(3 * S + u); };         // raw unit has landed
-    auto bar_ue = [&](uint32_t u) { return bar(3 * S + 2 + u); };    //   and is no longer needed
-    auto bar_d = [&](uint32_t u) { return bar(3 * S + 4 + u); };     // the unit's sums are complete
-    auto bar_t = [&](uint32_t u) { return bar(3 * S + 6 + u); };     //   and have been read
-    const uint32_t bar_m = bar(3 * S + 8);                           // the min sums have been read
-    const uint32_t stage0 = smem_addr(smem), slot0 = stage0 + S * PW_STAGE;   // slot: [mins operand][raw][aux]
+    auto bar_f = [&](uint32_t n) { return bar(n % NE); };                  // both operands of step n are there
+    auto bar_e = [&](uint32_t n) { return bar(NE + n % NE); };             //   and have been read by its MMAs
+    auto bar_x = [&](uint32_t s) { return bar(2 * NE + s); };              // group sums and exponents of a unit have landed
+    auto bar_xe = [&](uint32_t s) { return bar(2 * NE + NX + s); };
+    constexpr uint32_t B0 = 2 * NE + 2 * NX;
+    auto bar_u = [&](uint32_t u) { return bar(B0 + u); };                  // raw unit has landed
+    auto bar_ue = [&](uint32_t u) { return bar(B0 + 2 + u); };             //   and is unpacked
+    auto bar_d = [&](uint32_t u) { return bar(B0 + 4 + u); };              // the unit's sums are complete
+    auto bar_t = [&](uint32_t u) { return bar(B0 + 6 + u); };              //   and have been read
+    auto bar_r = [&](uint32_t i) { return bar(B0 + 8 + i); };              // its rows' scales are written (i = m % 4)
+    const uint32_t bar_m = bar(B0 + 12);                                   // the min sums have been read
+    const uint32_t sm_a = smem_addr(smem), sm_b = sm_a + NA * PW_A_STEP, sm_raw = sm_b + NB * PW_B_STEP, sm_min = sm_raw + 2 * F::RAW,
+                   sm_aux = sm_min + 2 * F::AMIN;
 
     if (threadIdx.x == 0) {
         dead_flag = 0;
-        for (uint32_t s = 0; s < S; s++) {
-            mbar_init(bar_b(s), 1);
-            mbar_init(bar_a(s), PW_UNPACK_WARPS);
-            mbar_init(bar_e(s), 1);
+        for (uint32_t n = 0; n < NE; n++) {
+            mbar_init(bar_f(n), PW_UNPACK_WARPS / 2 + 1);
+            mbar_init(bar_e(n), 1);
+        }
+        for (uint32_t s = 0; s < 4; s++) mbar_init(bar_r(s), PW_UNPACK_WARPS / 2);
+        for (uint32_t s = 0; s < NX; s++) {
+            mbar_init(bar_x(s), 1);
+            mbar_init(bar_xe(s), PW_FINISH_WARPS);
         }
         for (uint32_t u = 0; u < 2; u++) {
             mbar_init(bar_u(u), 1);
-            mbar_init(bar_ue(u), PW_UNPACK_WARPS + PW_FINISH_WARPS);
+            mbar_init(bar_ue(u), PW_UNPACK_WARPS);
             mbar_init(bar_d(u), 1);
             mbar_init(bar_t(u), PW_FINISH_WARPS);
         }
@@ -276,46 +297,69 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
     const uint32_t tmem_base = tmem_base_slot;
     pdl_wait();   // barriers and tensor memory are set up while the preceding launch (which writes the image) still runs
 
-    // Every role walks the same items, units m and steps n (both numbered through over the block's life) and waits on
-    // every phase of the barriers it uses, so a parity is never two phases off.  A role whose wait has expired
-    // leaves its loop; the others see the flag and follow.
+    // Every role walks the same items, units m and steps n (both numbered through over the block's life).  A parity tells
+    // two phases apart, so each waiter waits on every phase of a barrier, in order, and a barrier cannot run a phase
+    // ahead of any of its waiters: a buffer's next use needs the waiter's own arrival, directly (rings) or through the
+    // MMA order (the barriers of step n come round at step n + 6; the operand group that waits for step n before it
+    // builds n + 3 is always the same one, and step n + 6 needs the buffer of its step n + 3; scales of unit m + 4
+    // are written when MMAs of unit m + 3 are through, which takes the sums of unit m + 1 read).  A role whose wait has
+    // expired leaves its loop; the others see the flag and follow.
+    constexpr unsigned long long DRAIN_NS = 1000000000ull;
     if (warp == 0) {
-        // ------------------------------ producer ------------------------------
+        // ------------------------------ raw weights, group sums, exponents ------------------------------
         if (lane == 0) {
-            uint32_t m = 0, n = 0;
+            uint32_t m = 0;
             bool ok = true;
-            const uint32_t unit_bytes = pw_image_unit(np), bstep = 256 * np, aux = 36 * np;
+            const uint32_t unit_bytes = pw_image_unit(np), aux = 36 * np;
             for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
                 PwWalk w;
                 w.set(a, item);
                 const uint32_t mi = pw_matrix_of(a, w.tile);
                 const uint8_t *wt = a.w[mi] + (size_t)(w.tile - a.tile0[mi]) * a.nkb * F::RAW;
-                for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++, m++) {
-                    const uint32_t u = m & 1, slot = slot0 + u * SLOT;
-                    const uint8_t *img = a.img + ((size_t)w.pt * a.nkb + kb) * unit_bytes;
+                for (uint32_t kb = w.kb; kb < w.kb_end; kb++, m++) {
+                    const uint32_t u = m & 1, x = m % NX;
                     if (m >= 2) ok = tc_wait(bar_ue(u), ((m >> 1) - 1) & 1, dead, a.err, 41);
+                    if (ok && m >= NX) ok = tc_wait(bar_xe(x), (m / NX - 1) & 1, dead, a.err, 42);
                     if (!ok) break;
-                    mbar_expect_tx(bar_u(u), F::RAW + aux);
-                    bulk_copy_g2s(slot + F::AMIN, wt + (size_t)kb * F::RAW, F::RAW, bar_u(u));
-                    bulk_copy_g2s(slot + F::AMIN + F::RAW, img + 4 * bstep, aux, bar_u(u));
+                    mbar_expect_tx(bar_u(u), F::RAW);
+                    bulk_copy_g2s(sm_raw + u * F::RAW, wt + (size_t)kb * F::RAW, F::RAW, bar_u(u));
+                    mbar_expect_tx(bar_x(x), aux);
+                    bulk_copy_g2s(sm_aux + x * PW_AUX, a.img + ((size_t)w.pt * a.nkb + kb) * unit_bytes + 1024 * np, aux, bar_x(x));
+                }
+            }
+            if (!ok) {   // the copies in flight land before the block gives its shared memory back
+                for (uint32_t k = m > 2 ? m - 2 : 0; k < m; k++) mbar_wait(bar_u(k & 1), (k >> 1) & 1, nullptr, 0, DRAIN_NS);
+                for (uint32_t k = m > NX ? m - NX : 0; k < m; k++) mbar_wait(bar_x(k % NX), (k / NX) & 1, nullptr, 0, DRAIN_NS);
+            }
+        }
+    } else if (warp == 2 + PW_UNPACK_WARPS + PW_FINISH_WARPS) {
+        // ------------------------------ activation operand ------------------------------
+        if (lane == 0) {
+            uint32_t n = 0;
+            bool ok = true;
+            const uint32_t unit_bytes = pw_image_unit(np), bstep = 256 * np;
+            for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+                PwWalk w;
+                w.set(a, item);
+                for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++) {
+                    const uint8_t *img = a.img + ((size_t)w.pt * a.nkb + kb) * unit_bytes;
                     for (uint32_t st = 0; st < STEPS; st++, n++) {
-                        const uint32_t s = n % S;
-                        if (n >= S) ok = tc_wait(bar_e(s), (n / S - 1) & 1, dead, a.err, 42);
+                        const uint32_t s = n % NB;
+                        if (n >= NB) ok = tc_wait(bar_e(n - NB), ((n - NB) / NE) & 1, dead, a.err, 43);
                         if (!ok) break;
-                        mbar_expect_tx(bar_b(s), bstep);
-                        bulk_copy_g2s(stage0 + s * PW_STAGE + PW_A_STEP, img + (st & 3) * bstep, bstep, bar_b(s));
+                        mbar_expect_tx(bar_f(n), bstep);
+                        bulk_copy_g2s(sm_b + s * PW_B_STEP, img + (st & 3) * bstep, bstep, bar_f(n));
                     }
                 }
             }
-            if (!ok) {
-                // the copies in flight land before the block gives its shared memory back
-                for (uint32_t k = n > S ? n - S : 0; k < n; k++) mbar_wait(bar_b(k % S), (k / S) & 1, nullptr, 0, 1000000000ull);
-                for (uint32_t k = m > 2 ? m - 2 : 0; k < m; k++) mbar_wait(bar_u(k & 1), (k >> 1) & 1, nullptr, 0, 1000000000ull);
-            }
+            // After an expired wait the operand's copies cannot be told from the barrier alone (it also counts the
+            // unpacking warps): give them the time any copy takes.
+            if (!ok)
+                for (const unsigned long long t0 = global_ns(); global_ns() - t0 < DRAIN_NS / 100;) {}
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issue ------------------------------
-        if (lane == 0) {
+        if (tc_elect()) {
             uint32_t m = 0, n = 0;
             bool ok = true;
             const uint32_t idesc = pw_idesc(2 * np), idesc_min = pw_idesc((np + 15) & ~15u);
@@ -324,27 +368,26 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                 w.set(a, item);
                 for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++, m++) {
                     const uint32_t u = m & 1, dcol = tmem_base + u * 2 * PW_MAXN;
-                    ok = tc_wait(bar_u(u), (m >> 1) & 1, dead, a.err, 43);
-                    if (ok && m >= 2) ok = tc_wait(bar_t(u), ((m >> 1) - 1) & 1, dead, a.err, 44);
+                    if (m >= 2) ok = tc_wait(bar_t(u), ((m >> 1) - 1) & 1, dead, a.err, 44);
                     for (uint32_t st = 0; st < STEPS && ok; st++, n++) {
-                        const uint32_t s = n % S;
-                        ok = tc_wait(bar_b(s), (n / S) & 1, dead, a.err, 45) && tc_wait(bar_a(s), (n / S) & 1, dead, a.err, 46);
+                        const uint32_t sa = n % NA, sb = n % NB;
+                        ok = tc_wait(bar_f(n), (n / NE) & 1, dead, a.err, 45);
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        const uint64_t ad = tc_smem_desc_sw128(stage0 + s * PW_STAGE, 1024);
-                        const uint64_t bd = tc_smem_desc_sw128(stage0 + s * PW_STAGE + PW_A_STEP, 1024);
+                        const uint64_t ad = tc_smem_desc_sw128(sm_a + sa * PW_A_STEP, 1024);
+                        const uint64_t bd = tc_smem_desc_sw128(sm_b + sb * PW_B_STEP, 1024);
 #pragma unroll
                         for (uint32_t k = 0; k < 4; k++) pw_mma(dcol, ad + 2 * k, bd + 2 * k, idesc, (st | k) ? 1u : 0u);
-                        tc_commit(bar_e(s));
+                        tc_commit(bar_e(n));
                     }
                     if (FMT == WGB_Q4_K && ok) {
                         // sum over the eight groups of min x (sum of the group's X), both digits of the sums in one MMA
-                        if (m >= 1) ok = tc_wait(bar_m, (m - 1) & 1, dead, a.err, 47);
+                        const uint32_t x = m % NX;
+                        if (m >= 1) ok = tc_wait(bar_m, (m - 1) & 1, dead, a.err, 48);
                         if (ok) {
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            const uint32_t slot = slot0 + u * SLOT;
-                            pw_mma(tmem_base + PW_TMEM_MIN, tc_smem_desc(slot, TC_TILE_ROWS * 16, 128), tc_smem_desc(slot + F::AMIN + F::RAW, np * 16, 128),
-                                   idesc_min, 0u);
+                            pw_mma(tmem_base + PW_TMEM_MIN, tc_smem_desc(sm_min + u * F::AMIN, TC_TILE_ROWS * 16, 128),
+                                   tc_smem_desc(sm_aux + x * PW_AUX, np * 16, 128), idesc_min, 0u);
                         }
                     }
                     if (ok) tc_commit(bar_d(u));
@@ -353,34 +396,63 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
         }
     } else if (warp < 2 + PW_UNPACK_WARPS) {
         // ------------------------------ weight operand ------------------------------
-        const uint32_t h = (warp - 2) >> 2, r = (warp & 3) * 32 + lane;
-        const uint32_t arow0 = stage0 + (r >> 3) * 1024 + (r & 7) * 128;
-        uint32_t m = 0, n = 0;
+        // Group `grp` builds steps grp, grp + 2, ...; a thread builds one row of 64 columns.
+        const uint32_t grp = (warp - 2) >> 2, r = (warp & 3) * 32 + lane;
+        const uint32_t arow0 = sm_a + (r >> 3) * 1024 + (r & 7) * 128;
+        uint32_t m = 0;
         bool ok = true;
         for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
             PwWalk w;
             w.set(a, item);
             for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++, m++) {
-                const uint32_t u = m & 1, slot = slot0 + u * SLOT, raw = slot + F::AMIN;
-                ok = __all_sync(0xffffffffu, tc_wait(bar_u(u), (m >> 1) & 1, dead, a.err, 48));
+                const uint32_t u = m & 1, raw = sm_raw + u * F::RAW;
+                ok = tc_wait(bar_u(u), (m >> 1) & 1, dead, a.err, 49);
+                // (on behalf of the MMA of the mins, which reads the group sums)
+                if (FMT == WGB_Q4_K && grp == 1 && ok) ok = tc_wait(bar_x(m % NX), (m / NX) & 1, dead, a.err, 47);
+                ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                if (FMT == WGB_Q4_K) {
-                    // the row's eight mins, once per K-core (this thread's half writes one of the two)
-                    const uint4 hdr = lds128(raw + r * 144);
-                    const uint32_t m_lo = hdr.z & 0x3f3f3f3fu, m_hi = ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u);
-                    const __half2 k1024 = __float2half2_rn(1024.0f);
-                    sts128(slot + h * TC_TILE_ROWS * 16 + r * 16, h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4140)), k1024)),
-                           h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4342)), k1024)), h2u(__hsub2(u2h(__byte_perm(m_hi, 0x64646464u, 0x4140)), k1024)),
-                           h2u(__hsub2(u2h(__byte_perm(m_hi, 0x64646464u, 0x4342)), k1024)));
-                }
-                for (uint32_t st = 0; st < STEPS; st++, n++) {
-                    const uint32_t s = n % S;
-                    if (n >= S) ok = __all_sync(0xffffffffu, tc_wait(bar_e(s), (n / S - 1) & 1, dead, a.err, 49));
+#pragma unroll 1
+                for (uint32_t st = grp; st < STEPS; st += 2) {
+                    const uint32_t n = m * STEPS + st, s = n % NA;
+                    if (n >= NA) ok = __all_sync(0xffffffffu, tc_wait(bar_e(n - NA), ((n - NA) / NE) & 1, dead, a.err, 50));
                     if (!ok) break;
-                    pw_unpack<FMT>(raw, arow0 + s * PW_STAGE, r, h, st & 3, F::PLANES == 2 && st < 4);
+                    if (st == grp) {
+                        // Once per unit (the MMAs of two units back are through: a later step's buffer was just free).
+                        if (grp == 0) {
+                            float d, dmin = 0.0f;
+                            if constexpr (FMT == WGB_Q4_K) {
+                                uint32_t dm;
+                                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(dm) : "r"(raw + r * 144));
+                                const float2 f = __half22float2(u2h(dm));
+                                d = f.x;
+                                dmin = f.y * -4096.0f;
+                            } else if constexpr (FMT == WGB_Q6_K) {
+                                uint32_t db;
+                                asm volatile("ld.shared.u16 %0, [%1];" : "=r"(db) : "r"(raw + TC_TILE_ROWS * 208 + r * 2));
+                                d = __half2float(__ushort_as_half((unsigned short)db));
+                            } else {
+                                d = __uint_as_float((pw_q80_exp(lds128(raw + TC_TILE_ROWS * 256 + r * 16)) - 1u) << 23);   // 2^(E - 2)
+                            }
+                            rowscale[m & 3][r] = make_float2(d, dmin);
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(bar_r(m & 3));
+                        }
+                        if (FMT == WGB_Q4_K) {
+                            // the row's eight mins, once per K-core: each group writes one of the two
+                            const uint4 hdr = lds128(raw + r * 144);
+                            const uint32_t m_lo = hdr.z & 0x3f3f3f3fu, m_hi = ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u);
+                            const __half2 k1024 = __float2half2_rn(1024.0f);
+                            sts128(sm_min + u * F::AMIN + grp * TC_TILE_ROWS * 16 + r * 16, h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4140)), k1024)),
+                                   h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4342)), k1024)),
+                                   h2u(__hsub2(u2h(__byte_perm(m_hi, 0x64646464u, 0x4140)), k1024)),
+                                   h2u(__hsub2(u2h(__byte_perm(m_hi, 0x64646464u, 0x4342)), k1024)));
+                        }
+                    }
+#pragma unroll
+                    for (uint32_t h = 0; h < 2; h++) pw_unpack<FMT>(raw, arow0 + s * PW_A_STEP, r, h, st & 3, F::PLANES == 2 && st < 4);
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_a(s));
+                    if (lane == 0) mbar_arrive(bar_f(n));
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_ue(u));
@@ -389,7 +461,7 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
     } else {
         // ------------------------------ finishing ------------------------------
         // Thread (quarter, lane, half): row r of the tile, groups of eight positions half, half + 2, ...
-        constexpr uint32_t NG = PW_MAXN / 16;
+        constexpr uint32_t NG = (PW_MAXN / 8 + 1) / 2;
         const uint32_t half = (warp - 2 - PW_UNPACK_WARPS) >> 2, quarter = warp & 3, r = quarter * 32 + lane, ng = np / 8;
         const uint32_t trow = tmem_base + ((quarter * 32u) << 16);
         const uint64_t k2048 = f2pack(2048.0f, 2048.0f);
@@ -404,26 +476,13 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
 #pragma unroll
                 for (uint32_t j = 0; j < 4; j++) acc[g][j] = 0ull;
             for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++, m++) {
-                const uint32_t u = m & 1, raw = slot0 + u * SLOT + F::AMIN, ebase = raw + F::RAW + 32 * np;
-                ok = __all_sync(0xffffffffu, tc_wait(bar_u(u), (m >> 1) & 1, dead, a.err, 50));
+                const uint32_t u = m & 1, x = m % NX, ebase = sm_aux + x * PW_AUX + 32 * np;
+                ok = tc_wait(bar_x(x), (m / NX) & 1, dead, a.err, 52) && tc_wait(bar_r(m & 3), (m >> 2) & 1, dead, a.err, 53) &&
+                     tc_wait(bar_d(u), (m >> 1) & 1, dead, a.err, 54);
+                ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                float d, dmin = 0.0f;
-                if constexpr (FMT == WGB_Q4_K) {
-                    uint32_t dm;
-                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(dm) : "r"(raw + r * 144));
-                    const float2 f = __half22float2(u2h(dm));
-                    d = f.x;
-                    dmin = f.y * -4096.0f;
-                } else if constexpr (FMT == WGB_Q6_K) {
-                    uint32_t db;
-                    asm volatile("ld.shared.u16 %0, [%1];" : "=r"(db) : "r"(raw + TC_TILE_ROWS * 208 + r * 2));
-                    d = __half2float(__ushort_as_half((unsigned short)db));
-                } else {
-                    d = __uint_as_float((pw_q80_exp(lds128(raw + TC_TILE_ROWS * 256 + r * 16)) - 1u) << 23);   // 2^(E - 2)
-                }
-                const uint64_t d2 = f2pack(d, d), dm2 = f2pack(dmin, dmin);
-                ok = __all_sync(0xffffffffu, tc_wait(bar_d(u), (m >> 1) & 1, dead, a.err, 51));
-                if (!ok) break;
+                const float2 sc = rowscale[m & 3][r];
+                const uint64_t d2 = f2pack(sc.x, sc.x), dm2 = f2pack(sc.y, sc.y);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t tb = trow + u * 2 * PW_MAXN;
 #pragma unroll
@@ -452,7 +511,7 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                 if (lane == 0) {
                     mbar_arrive(bar_t(u));
                     mbar_arrive(bar_m);
-                    mbar_arrive(bar_ue(u));
+                    mbar_arrive(bar_xe(x));
                 }
             }
             if (!ok) break;
