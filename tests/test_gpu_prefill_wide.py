@@ -28,7 +28,7 @@ def value_rows(fmt, dim, kv_heads, heads, n, seed):
 
 
 @pytest.mark.parametrize("fmt", [synth.Q4_K, synth.Q6_K, synth.Q8_0])
-@pytest.mark.parametrize("shape", [(256, 2, 4, 16), (768, 12, 12, 92), (4096, 32, 32, 181), (1024, 16, 16, 520), (2048, 16, 16, 88)])
+@pytest.mark.parametrize("shape", [(256, 2, 4, 16), (768, 12, 12, 92), (4096, 32, 32, 181), (1024, 16, 16, 520), (2048, 16, 16, 80)])
 def test_wide_product_vs_f64(fmt, shape):
     """As exact as the position-by-position product: the sums of both are good to a few units of 2^-22 of the row's
     terms, so the error of each row of outputs stays below 2e-6 of its norm and no element is off by more than 1e-5 of
@@ -53,7 +53,7 @@ def _caches(gpu, n):
     dict(n_prompt=17, heads=8, kv=8, qwen=False, mixed=False),              # the smallest wide pass
     dict(n_prompt=72, heads=8, kv=2, qwen=True, mixed=False),               # 71: 64-position attention tile + 7; biases, Neox RoPE, grouped heads
     dict(n_prompt=90, heads=4, kv=4, qwen=False, mixed=True),               # head size 128; three formats in one layer's products
-    dict(n_prompt=620, heads=4, kv=2, qwen=False, mixed=False, seq_len=640),   # two equal passes: the second attends to the first's rows
+    dict(n_prompt=700, heads=4, kv=2, qwen=False, mixed=False, seq_len=720),   # two passes: the second attends to the first's rows
     dict(n_prompt=530, heads=8, kv=4, qwen=False, mixed=True, seq_len=700, start=150, n_layers=1),   # a pass that starts at a later position
 ])
 def test_wide_passes_match_sequential_loop(case):

@@ -236,8 +236,9 @@ int launch_prefill_attention(const float *q, const float *k_cache, const float *
 
 
 // ---- wide prompt passes (prefill_wide.cu) ---------------------------------------------------------------
-constexpr uint32_t PW_CAP = 512;   // prompt positions per wide pass, most
-constexpr uint32_t PW_MIN = 16;    // fewer than this go through the passes of PF_TOK positions
+constexpr uint32_t PW_TILE = 80;             // prompt positions per tile of a wide product, most
+constexpr uint32_t PW_CAP = 8 * PW_TILE;     // prompt positions per wide pass, most
+constexpr uint32_t PW_MIN = 16;              // fewer than this go through the passes of PF_TOK positions
 // Tiles of positions of a pass: npt tiles of np positions each.
 struct WideTiling { uint32_t np, npt; };
 WideTiling prefill_wide_tiling(uint32_t ntok);
@@ -259,12 +260,15 @@ int launch_wide_attention(const float *q, const float *k_cache, const float *v_c
 // x[t] = row d_tokens[t] of the embedding (+ row pos0 + t of `pos_embd`).
 int launch_embed_rows(const QMat &embd, const QMat *pos_embd, const uint32_t *d_tokens, uint32_t pos0, uint32_t ntok, float *x, cudaStream_t stream);
 
-// Positions of the next prompt pass when `left` are still to go: equal wide passes, or passes of PF_TOK.
+// Positions of the next prompt pass when `left` are still to go: wide passes of about equal size, whole tiles but for
+// the last, or passes of PF_TOK.
 inline uint32_t prefill_next_pass(size_t left, uint32_t wide_cap)
 {
     if (wide_cap && left >= PW_MIN) {
-        const size_t passes = (left + wide_cap - 1) / wide_cap;
-        return (uint32_t)((left + passes - 1) / passes);
+        if (left <= wide_cap) return (uint32_t)left;
+        const size_t passes = (left + wide_cap - 1) / wide_cap, each = (left + passes - 1) / passes;
+        const size_t tiles = (each + PW_TILE - 1) / PW_TILE * PW_TILE;
+        return (uint32_t)(tiles < wide_cap ? tiles : wide_cap);
     }
     return (uint32_t)(left < PF_TOK ? left : PF_TOK);
 }

@@ -2,7 +2,7 @@
 //
 // The passes of eight positions (prefill.cu) read every weight once per eight positions and spend their time on the
 // chain unpack -> MMA -> read-back of each 256-column unit, whose tensor work is 4 % of it.  With a long prompt the
-// same unpacked weights can serve up to 96 positions at a time, and the pass becomes a contraction proper: this file
+// same unpacked weights can serve up to 80 positions at a time, and the pass becomes a contraction proper: this file
 // holds its matrix product on the tensor cores (tcgen05.mma kind::f16 with f32 accumulators in tensor memory), the
 // activation image it reads, the element-wise kernels between the products and a causal attention over tiles of 64
 // positions.  Operators as in the narrow passes: GemvQuant::dispatch (crates/wgml/src/ops/gemv_quant.rs:241-348),
@@ -26,36 +26,37 @@
 
 namespace wgb {
 
-constexpr uint32_t PW_MAXN = 88;                                   // positions per tile (two digits each: N = 176)
+constexpr uint32_t PW_MAXN = PW_TILE;                              // positions per tile (two digits each: N = 160)
 constexpr uint32_t PW_UNPACK_WARPS = 8;                            // build the weight operand, two groups of four
 constexpr uint32_t PW_FINISH_WARPS = 8;                            // read the sums, apply scales
 constexpr uint32_t PW_NT = 32 * (3 + PW_UNPACK_WARPS + PW_FINISH_WARPS);
-constexpr uint32_t PW_A_STEP = TC_TILE_ROWS * 128;                 // weight operand of a step: 64 columns in f16
-constexpr uint32_t PW_B_STEP = 2 * PW_MAXN * 128;                  // activation operand of a step, largest
+constexpr uint32_t PW_A_COLS = 32;                                 // weight operand of a step: 64 columns in f16, in tensor memory
 constexpr uint32_t PW_A_RING = 3;                                  // odd: consecutive uses of a buffer are different groups'
+constexpr uint32_t PW_B_STEP = 2 * PW_MAXN * 128;                  // activation operand of a step, largest, in shared memory
+constexpr uint32_t PW_B_RING = 6;
 constexpr uint32_t PW_E_RING = 2 * PW_A_RING;                      // steps have a barrier pair each, six in turn
 constexpr uint32_t PW_AUX = 36 * PW_MAXN;                          // per unit: sums of the mins' product, exponents
 constexpr uint32_t PW_X_RING = 3;
-constexpr uint32_t PW_AMIN = 2 * TC_TILE_ROWS * 16;                // mins as f16, [two K-cores][row]
-constexpr uint32_t PW_TMEM_COLS = 512;                             // two sets of 2 x 88 sums, one of 88 (96 written) min sums
+// Tensor memory: two sets of sums (2 x 80 columns), the min sums (80), three weight operands (32), two of mins (8).
+constexpr uint32_t PW_TMEM_COLS = 512;
 constexpr uint32_t PW_TMEM_MIN = 4 * PW_MAXN;
+constexpr uint32_t PW_TMEM_A = PW_TMEM_MIN + PW_MAXN;
+constexpr uint32_t PW_TMEM_AMIN = PW_TMEM_A + PW_A_RING * PW_A_COLS;
+static_assert(PW_MAXN % 16 == 0 && PW_TMEM_AMIN + 2 * 8 <= PW_TMEM_COLS, "tensor memory");
+static_assert(PW_B_RING <= PW_E_RING, "a step's barriers outlive its buffer");
 
-// Per format: raw bytes of a unit of 128 rows (tile-major copies of prefill.cu, prefill_q6k.cu, prefill_q80.cu); steps of
-// the activation operand in flight (a request takes about a microsecond, a step a quarter of one: five, or what fits).
+// Per format: raw bytes of a unit of 128 rows (tile-major copies of prefill.cu, prefill_q6k.cu, prefill_q80.cu) and how
+// many units fit.
 template <int FMT> struct PwFmt;
-template <> struct PwFmt<WGB_Q4_K> { static constexpr uint32_t RAW = TC_UNIT_BYTES, B_RING = 5, PLANES = 1, AMIN = PW_AMIN; };
-template <> struct PwFmt<WGB_Q6_K> { static constexpr uint32_t RAW = TC_TILE_ROWS * 210, B_RING = 5, PLANES = 2, AMIN = 0; };
-template <> struct PwFmt<WGB_Q8_0> { static constexpr uint32_t RAW = TC_TILE_ROWS * 272, B_RING = 4, PLANES = 2, AMIN = 0; };
-template <int FMT> constexpr uint32_t pw_smem()
-{
-    return PW_A_RING * PW_A_STEP + PwFmt<FMT>::B_RING * PW_B_STEP + 2 * (PwFmt<FMT>::RAW + PwFmt<FMT>::AMIN) + PW_X_RING * PW_AUX;
-}
+template <> struct PwFmt<WGB_Q4_K> { static constexpr uint32_t RAW = TC_UNIT_BYTES, RAW_RING = 3, PLANES = 1; };
+template <> struct PwFmt<WGB_Q6_K> { static constexpr uint32_t RAW = TC_TILE_ROWS * 210, RAW_RING = 3, PLANES = 2; };
+template <> struct PwFmt<WGB_Q8_0> { static constexpr uint32_t RAW = TC_TILE_ROWS * 272, RAW_RING = 2, PLANES = 2; };
+template <int FMT> constexpr uint32_t pw_smem() { return PW_B_RING * PW_B_STEP + PwFmt<FMT>::RAW_RING * PwFmt<FMT>::RAW + PW_X_RING * PW_AUX; }
 constexpr uint32_t PW_STATIC = 4 * TC_TILE_ROWS * 8 + 512;         // row scales, barriers
 static_assert(pw_smem<WGB_Q4_K>() + 1024 + PW_STATIC <= 227 * 1024 && pw_smem<WGB_Q6_K>() + 1024 + PW_STATIC <= 227 * 1024 &&
                   pw_smem<WGB_Q8_0>() + 1024 + PW_STATIC <= 227 * 1024,
               "shared memory budget");
-static_assert(PW_A_STEP % 1024 == 0 && PW_B_STEP % 1024 == 0 && PW_AUX % 16 == 0, "swizzled operands start on 1 KB boundaries");
-static_assert(PW_TMEM_MIN + (PW_MAXN + 15) / 16 * 16 <= PW_TMEM_COLS, "tensor memory");
+static_assert(PW_B_STEP % 1024 == 0 && PW_AUX % 16 == 0, "swizzled operands start on 1 KB boundaries");
 
 // Activation image of a pass: [tile of np positions][unit]: four steps of 64 columns, each [hi rows | lo rows] x 128
 // bytes in the 128-byte swizzle; then the sums of the eight 32-column groups as two f16 digits
@@ -98,12 +99,13 @@ __device__ __forceinline__ uint32_t pw_matrix_of(const PwArgs &a, uint32_t tile)
     return (a.nmat > 2 && tile >= a.tile0[2]) ? 2u : (a.nmat > 1 && tile >= a.tile0[1]) ? 1u : 0u;
 }
 
-__device__ __forceinline__ void pw_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+// D (+)= A B with A in tensor memory: lane = row, a column of 32 bits = two consecutive f16 along K.
+__device__ __forceinline__ void pw_mma(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
 {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.u32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // kind::f16 instruction descriptor: D f32, A and B f16, both K-major, M = 128, N = n.
@@ -111,6 +113,22 @@ __device__ __forceinline__ uint32_t pw_idesc(uint32_t n) { return (1u << 4) | ((
 
 __device__ __forceinline__ __half2 u2h(uint32_t v) { return *reinterpret_cast<__half2 *>(&v); }
 __device__ __forceinline__ uint32_t h2u(__half2 v) { return *reinterpret_cast<uint32_t *>(&v); }
+
+// A thread's 32 (8) words into 32 (8) columns of its lane.
+__device__ __forceinline__ void pw_st32(uint32_t taddr, const uint32_t (&v)[32])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,"
+        "%28,%29,%30,%31,%32};" ::"r"(taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]),
+        "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]),
+        "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
+__device__ __forceinline__ void pw_st8(uint32_t taddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d)   // the four words twice
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%1,%2,%3,%4};" ::"r"(taddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 
 // Two f32 at a time (the packed FMA of this architecture).
 __device__ __forceinline__ uint64_t f2pack(float a, float b)
@@ -144,10 +162,10 @@ __device__ __forceinline__ uint32_t pw_q80_exp(uint4 sc)
     return ex < 100u ? 100u : (ex > 142u ? 142u : ex);
 }
 
-// Weight operand of one step for (row r, half h): `raw` = the unit's raw bytes, step chunk c (64 columns), plane 0 = the
-// small one of a two-plane format.  Writes 32 f16 values into the row at `arow` (16-byte chunks swizzled by the row).
+// Weight operand of one step for row r: the 64 columns of chunk c of the unit at `raw`, plane 0 = the small one of a
+// two-plane format, as 32 words of two f16.
 template <int FMT>
-__device__ __forceinline__ void pw_unpack(uint32_t raw, uint32_t arow, uint32_t r, uint32_t h, uint32_t c, bool small_plane)
+__device__ __forceinline__ void pw_unpack(uint32_t (&v)[32], uint32_t raw, uint32_t r, uint32_t c, bool small_plane)
 {
     const uint32_t sw = r & 7;
     if constexpr (FMT == WGB_Q4_K) {
@@ -155,78 +173,76 @@ __device__ __forceinline__ void pw_unpack(uint32_t raw, uint32_t arow, uint32_t 
         const uint32_t j0 = 2 * c;
         const uint32_t sc_lo = hdr.y & 0x3f3f3f3fu, sc_hi = (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u);
         const uint32_t scw = ((j0 & 4) ? sc_hi : sc_lo) >> (8 * (j0 & 3));
-        const uint4 q = lds128(raw + r * 144 + 16 + 32 * c + 16 * h);
         // 1024 + code and 1024 + 16 code as f16, times the scale (a sixteenth of it), minus 1024 (64) times the scale:
         // every intermediate is exact
         const __half2 s0 = __half2half2(__ushort2half_rn((unsigned short)(scw & 0xffu)));
         const __half2 s1 = __half2half2(__ushort2half_rn((unsigned short)((scw >> 8) & 0xffu)));
         const __half2 o0 = __hmul2(s0, __float2half2_rn(-1024.0f)), o1 = __hmul2(s1, __float2half2_rn(-64.0f));
         const __half2 s1s = __hmul2(s1, __float2half2_rn(0.0625f));
-        const uint32_t qw[4] = { q.x, q.y, q.z, q.w };
-        uint32_t lo[8], hi[8];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
+        for (int h = 0; h < 2; h++) {
+            const uint4 q = lds128(raw + r * 144 + 16 + 32 * c + 16 * h);
+            const uint32_t qw[4] = { q.x, q.y, q.z, q.w };
 #pragma unroll
-            for (int p = 0; p < 2; p++) {
-                const uint32_t t = __byte_perm(qw[k], 0u, p ? 0x4342 : 0x4140);
-                lo[2 * k + p] = h2u(__hfma2(u2h((t & 0x000f000fu) | 0x64006400u), s0, o0));
-                hi[2 * k + p] = h2u(__hfma2(u2h((t & 0x00f000f0u) | 0x64006400u), s1s, o1));
+            for (int k = 0; k < 4; k++) {
+#pragma unroll
+                for (int p = 0; p < 2; p++) {
+                    const uint32_t t = __byte_perm(qw[k], 0u, p ? 0x4342 : 0x4140);
+                    v[8 * h + 2 * k + p] = h2u(__hfma2(u2h((t & 0x000f000fu) | 0x64006400u), s0, o0));
+                    v[16 + 8 * h + 2 * k + p] = h2u(__hfma2(u2h((t & 0x00f000f0u) | 0x64006400u), s1s, o1));
+                }
             }
         }
-        sts128(arow + (((2 * h) ^ sw) << 4), lo[0], lo[1], lo[2], lo[3]);
-        sts128(arow + (((2 * h + 1) ^ sw) << 4), lo[4], lo[5], lo[6], lo[7]);
-        sts128(arow + (((4 + 2 * h) ^ sw) << 4), hi[0], hi[1], hi[2], hi[3]);
-        sts128(arow + (((5 + 2 * h) ^ sw) << 4), hi[4], hi[5], hi[6], hi[7]);
     } else if constexpr (FMT == WGB_Q6_K) {
-        const uint32_t H = c >> 1, s = 2 * (c & 1) + h;   // 128-column half, 32-column group of it
+        const uint32_t H = c >> 1;   // 128-column half; 32-column groups s of it
         const uint4 scq = lds128(raw + TC_TILE_ROWS * 192 + r * 16);
-        const uint32_t scw = (s >> 1) ? (H ? scq.w : scq.y) : (H ? scq.z : scq.x);
+        const uint32_t scw = (c & 1) ? (H ? scq.w : scq.y) : (H ? scq.z : scq.x);
         const __half2 c1056 = __float2half2_rn(1056.0f), magic = __float2half2_rn(24576.0f);
 #pragma unroll
         for (uint32_t cc = 0; cc < 2; cc++) {
-            const uint4 qlq = lds128(raw + r * 128 + (((4 * H + 2 * (s & 1) + cc) ^ sw) << 4));
             const uint4 qhq = lds128(raw + TC_TILE_ROWS * 128 + (r >> 1) * 128 + (((4 * (r & 1) + 2 * H + cc) ^ ((r >> 1) & 7)) << 4));
-            const __half2 sc = __half2half2(__short2half_rn((short)(signed char)((scw >> (8 * (2 * (s & 1) + cc))) & 0xffu)));
-            const uint32_t qlw[4] = { qlq.x, qlq.y, qlq.z, qlq.w }, qhw[4] = { qhq.x, qhq.y, qhq.z, qhq.w };
-            uint32_t v[8];
+            const uint32_t qhw[4] = { qhq.x >> (4 * (c & 1)), qhq.y >> (4 * (c & 1)), qhq.z >> (4 * (c & 1)), qhq.w >> (4 * (c & 1)) };
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const uint32_t q = ((qlw[k] >> (4 * (s >> 1))) & 0x0f0f0f0fu) | (((qhw[k] >> (2 * s)) & 0x03030303u) << 4);
+            for (uint32_t h = 0; h < 2; h++) {   // s = 2 (c & 1) + h
+                const uint4 qlq = lds128(raw + r * 128 + (((4 * H + 2 * h + cc) ^ sw) << 4));
+                const __half2 sc = __half2half2(__short2half_rn((short)(signed char)((scw >> (8 * (2 * h + cc))) & 0xffu)));
+                const uint32_t qlw[4] = { qlq.x, qlq.y, qlq.z, qlq.w };
 #pragma unroll
-                for (int p = 0; p < 2; p++) {
-                    const __half2 qv = __hsub2(u2h(__byte_perm(q, 0x64646464u, p ? 0x4342 : 0x4140)), c1056);
-                    const __half2 a1 = __hsub2(__hfma2(qv, sc, magic), magic);   // multiple of 16
-                    v[2 * k + p] = small_plane ? h2u(__hfma2(qv, sc, __hneg2(a1))) : h2u(a1);
+                for (int k = 0; k < 4; k++) {
+                    const uint32_t q = ((qlw[k] >> (4 * (c & 1))) & 0x0f0f0f0fu) | (((qhw[k] >> (2 * h)) & 0x03030303u) << 4);
+#pragma unroll
+                    for (int p = 0; p < 2; p++) {
+                        const __half2 qv = __hsub2(u2h(__byte_perm(q, 0x64646464u, p ? 0x4342 : 0x4140)), c1056);
+                        const __half2 a1 = __hsub2(__hfma2(qv, sc, magic), magic);   // multiple of 16
+                        v[16 * h + 8 * cc + 2 * k + p] = small_plane ? h2u(__hfma2(qv, sc, __hneg2(a1))) : h2u(a1);
+                    }
                 }
             }
-            sts128(arow + (((4 * h + 2 * cc) ^ sw) << 4), v[0], v[1], v[2], v[3]);
-            sts128(arow + (((4 * h + 2 * cc + 1) ^ sw) << 4), v[4], v[5], v[6], v[7]);
         }
     } else {
         const uint4 scs = lds128(raw + TC_TILE_ROWS * 256 + r * 16);
-        const uint32_t ex = pw_q80_exp(scs), g = 2 * c + h;
-        const uint32_t scw = (g >> 1) == 0 ? scs.x : (g >> 1) == 1 ? scs.y : (g >> 1) == 2 ? scs.z : scs.w;
-        const float d = __half2float(__ushort_as_half((unsigned short)((g & 1) ? (scw >> 16) : (scw & 0xffffu))));
-        const __half2 ds = __float2half2_rn(d * __uint_as_float((255u - ex) << 23));   // d 2^(2 - E) < 4
+        const float norm = __uint_as_float((255u - pw_q80_exp(scs)) << 23);   // 2^(2 - E): d norm < 4
+        const uint32_t scw = c == 0 ? scs.x : c == 1 ? scs.y : c == 2 ? scs.z : scs.w;
         const __half2 c1152 = __float2half2_rn(1152.0f), magic = __float2half2_rn(1536.0f);
         const uint32_t row = raw + (c >> 1) * 16384 + r * 128;
 #pragma unroll
-        for (uint32_t cc = 0; cc < 2; cc++) {
-            const uint4 qq = lds128(row + (((4 * (c & 1) + 2 * h + cc) ^ sw) << 4));
-            const uint32_t qw[4] = { qq.x, qq.y, qq.z, qq.w };
-            uint32_t v[8];
+        for (uint32_t h = 0; h < 2; h++) {
+            const __half2 ds = __float2half2_rn(__half2float(__ushort_as_half((unsigned short)(h ? (scw >> 16) : (scw & 0xffffu)))) * norm);
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const uint32_t u = qw[k] ^ 0x80808080u;
+            for (uint32_t cc = 0; cc < 2; cc++) {
+                const uint4 qq = lds128(row + (((4 * (c & 1) + 2 * h + cc) ^ sw) << 4));
+                const uint32_t qw[4] = { qq.x, qq.y, qq.z, qq.w };
 #pragma unroll
-                for (int p = 0; p < 2; p++) {
-                    const __half2 qv = __hsub2(u2h(__byte_perm(u, 0x64646464u, p ? 0x4342 : 0x4140)), c1152);
-                    const __half2 a1 = __hsub2(__hfma2(qv, ds, magic), magic);   // an integer
-                    v[2 * k + p] = small_plane ? h2u(__hfma2(qv, ds, __hneg2(a1))) : h2u(a1);
+                for (int k = 0; k < 4; k++) {
+                    const uint32_t u = qw[k] ^ 0x80808080u;
+#pragma unroll
+                    for (int p = 0; p < 2; p++) {
+                        const __half2 qv = __hsub2(u2h(__byte_perm(u, 0x64646464u, p ? 0x4342 : 0x4140)), c1152);
+                        const __half2 a1 = __hsub2(__hfma2(qv, ds, magic), magic);   // an integer
+                        v[16 * h + 8 * cc + 2 * k + p] = small_plane ? h2u(__hfma2(qv, ds, __hneg2(a1))) : h2u(a1);
+                    }
                 }
             }
-            sts128(arow + (((4 * h + 2 * cc) ^ sw) << 4), v[0], v[1], v[2], v[3]);
-            sts128(arow + (((4 * h + 2 * cc + 1) ^ sw) << 4), v[4], v[5], v[6], v[7]);
         }
     }
 }
@@ -234,15 +250,16 @@ __device__ __forceinline__ void pw_unpack(uint32_t raw, uint32_t arow, uint32_t 
 // Roles: two producer threads (raw weights and per-unit extras; activation operand), one thread issuing MMAs, two groups
 // of four warps building the weight operand (alternate steps), eight warps finishing units.  Raw weights are free again
 // as soon as they are unpacked, a unit ahead of its MMAs; the rows' scales travel in a small ring of their own.
-// (With the raw unit held until its sums were finished, and its successor requested by the thread that feeds the
-// activation operand, a unit cost 1.4 us on top of its MMAs.)
+// The weight operand goes from registers to tensor memory: written to and read from shared memory it
+// cost as much of that memory's 128 bytes a clock as everything else together (per step of 64 columns and 88 positions
+// 710 clocks, against 350 of MMA; now 400 against 320).
 template <int FMT>
 __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_constant__ PwArgs a)
 {
     using F = PwFmt<FMT>;
-    constexpr uint32_t NA = PW_A_RING, NB = F::B_RING, NX = PW_X_RING, NE = PW_E_RING, STEPS = 4 * F::PLANES;
+    constexpr uint32_t NA = PW_A_RING, NB = PW_B_RING, NX = PW_X_RING, NE = PW_E_RING, NR = F::RAW_RING, STEPS = 4 * F::PLANES;
     extern __shared__ uint8_t pw_smem_raw[];
-    __shared__ __align__(8) unsigned long long bars[2 * NE + 2 * NX + 13];
+    __shared__ __align__(8) unsigned long long bars[2 * NE + 2 * NX + 2 * NR + 9];
     __shared__ float2 rowscale[4][TC_TILE_ROWS];
     __shared__ uint32_t tmem_base_slot;
     __shared__ uint32_t dead_flag;
@@ -258,14 +275,13 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
     auto bar_x = [&](uint32_t s) { return bar(2 * NE + s); };              // group sums and exponents of a unit have landed
     auto bar_xe = [&](uint32_t s) { return bar(2 * NE + NX + s); };
     constexpr uint32_t B0 = 2 * NE + 2 * NX;
-    auto bar_u = [&](uint32_t u) { return bar(B0 + u); };                  // raw unit has landed
-    auto bar_ue = [&](uint32_t u) { return bar(B0 + 2 + u); };             //   and is unpacked
-    auto bar_d = [&](uint32_t u) { return bar(B0 + 4 + u); };              // the unit's sums are complete
-    auto bar_t = [&](uint32_t u) { return bar(B0 + 6 + u); };              //   and have been read
-    auto bar_r = [&](uint32_t i) { return bar(B0 + 8 + i); };              // its rows' scales are written (i = m % 4)
-    const uint32_t bar_m = bar(B0 + 12);                                   // the min sums have been read
-    const uint32_t sm_a = smem_addr(smem), sm_b = sm_a + NA * PW_A_STEP, sm_raw = sm_b + NB * PW_B_STEP, sm_min = sm_raw + 2 * F::RAW,
-                   sm_aux = sm_min + 2 * F::AMIN;
+    auto bar_u = [&](uint32_t i) { return bar(B0 + i); };                  // raw unit has landed
+    auto bar_ue = [&](uint32_t i) { return bar(B0 + NR + i); };            //   and is unpacked
+    auto bar_d = [&](uint32_t u) { return bar(B0 + 2 * NR + u); };         // the unit's sums are complete
+    auto bar_t = [&](uint32_t u) { return bar(B0 + 2 * NR + 2 + u); };     //   and have been read
+    auto bar_r = [&](uint32_t i) { return bar(B0 + 2 * NR + 4 + i); };     // its rows' scales are written (i = m % 4)
+    const uint32_t bar_m = bar(B0 + 2 * NR + 8);                           // the min sums have been read
+    const uint32_t sm_b = smem_addr(smem), sm_raw = sm_b + NB * PW_B_STEP, sm_aux = sm_raw + NR * F::RAW;
 
     if (threadIdx.x == 0) {
         dead_flag = 0;
@@ -273,14 +289,16 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
             mbar_init(bar_f(n), PW_UNPACK_WARPS / 2 + 1);
             mbar_init(bar_e(n), 1);
         }
+        for (uint32_t s = 0; s < NR; s++) {
+            mbar_init(bar_u(s), 1);
+            mbar_init(bar_ue(s), PW_UNPACK_WARPS);
+        }
         for (uint32_t s = 0; s < 4; s++) mbar_init(bar_r(s), PW_UNPACK_WARPS / 2);
         for (uint32_t s = 0; s < NX; s++) {
             mbar_init(bar_x(s), 1);
             mbar_init(bar_xe(s), PW_FINISH_WARPS);
         }
         for (uint32_t u = 0; u < 2; u++) {
-            mbar_init(bar_u(u), 1);
-            mbar_init(bar_ue(u), PW_UNPACK_WARPS);
             mbar_init(bar_d(u), 1);
             mbar_init(bar_t(u), PW_FINISH_WARPS);
         }
@@ -317,8 +335,8 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                 const uint32_t mi = pw_matrix_of(a, w.tile);
                 const uint8_t *wt = a.w[mi] + (size_t)(w.tile - a.tile0[mi]) * a.nkb * F::RAW;
                 for (uint32_t kb = w.kb; kb < w.kb_end; kb++, m++) {
-                    const uint32_t u = m & 1, x = m % NX;
-                    if (m >= 2) ok = tc_wait(bar_ue(u), ((m >> 1) - 1) & 1, dead, a.err, 41);
+                    const uint32_t u = m % NR, x = m % NX;
+                    if (m >= NR) ok = tc_wait(bar_ue(u), (m / NR - 1) & 1, dead, a.err, 41);
                     if (ok && m >= NX) ok = tc_wait(bar_xe(x), (m / NX - 1) & 1, dead, a.err, 42);
                     if (!ok) break;
                     mbar_expect_tx(bar_u(u), F::RAW);
@@ -328,7 +346,7 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                 }
             }
             if (!ok) {   // the copies in flight land before the block gives its shared memory back
-                for (uint32_t k = m > 2 ? m - 2 : 0; k < m; k++) mbar_wait(bar_u(k & 1), (k >> 1) & 1, nullptr, 0, DRAIN_NS);
+                for (uint32_t k = m > NR ? m - NR : 0; k < m; k++) mbar_wait(bar_u(k % NR), (k / NR) & 1, nullptr, 0, DRAIN_NS);
                 for (uint32_t k = m > NX ? m - NX : 0; k < m; k++) mbar_wait(bar_x(k % NX), (k / NX) & 1, nullptr, 0, DRAIN_NS);
             }
         }
@@ -370,14 +388,13 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                     const uint32_t u = m & 1, dcol = tmem_base + u * 2 * PW_MAXN;
                     if (m >= 2) ok = tc_wait(bar_t(u), ((m >> 1) - 1) & 1, dead, a.err, 44);
                     for (uint32_t st = 0; st < STEPS && ok; st++, n++) {
-                        const uint32_t sa = n % NA, sb = n % NB;
+                        const uint32_t at = tmem_base + PW_TMEM_A + (n % NA) * PW_A_COLS;
                         ok = tc_wait(bar_f(n), (n / NE) & 1, dead, a.err, 45);
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        const uint64_t ad = tc_smem_desc_sw128(sm_a + sa * PW_A_STEP, 1024);
-                        const uint64_t bd = tc_smem_desc_sw128(sm_b + sb * PW_B_STEP, 1024);
+                        const uint64_t bd = tc_smem_desc_sw128(sm_b + (n % NB) * PW_B_STEP, 1024);
 #pragma unroll
-                        for (uint32_t k = 0; k < 4; k++) pw_mma(dcol, ad + 2 * k, bd + 2 * k, idesc, (st | k) ? 1u : 0u);
+                        for (uint32_t k = 0; k < 4; k++) pw_mma(dcol, at + 8 * k, bd + 2 * k, idesc, (st | k) ? 1u : 0u);
                         tc_commit(bar_e(n));
                     }
                     if (FMT == WGB_Q4_K && ok) {
@@ -386,8 +403,7 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                         if (m >= 1) ok = tc_wait(bar_m, (m - 1) & 1, dead, a.err, 48);
                         if (ok) {
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            pw_mma(tmem_base + PW_TMEM_MIN, tc_smem_desc(sm_min + u * F::AMIN, TC_TILE_ROWS * 16, 128),
-                                   tc_smem_desc(sm_aux + x * PW_AUX, np * 16, 128), idesc_min, 0u);
+                            pw_mma(tmem_base + PW_TMEM_MIN, tmem_base + PW_TMEM_AMIN + 8 * u, tc_smem_desc(sm_aux + x * PW_AUX, np * 16, 128), idesc_min, 0u);
                         }
                     }
                     if (ok) tc_commit(bar_d(u));
@@ -398,24 +414,25 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
         // ------------------------------ weight operand ------------------------------
         // Group `grp` builds steps grp, grp + 2, ...; a thread builds one row of 64 columns.
         const uint32_t grp = (warp - 2) >> 2, r = (warp & 3) * 32 + lane;
-        const uint32_t arow0 = sm_a + (r >> 3) * 1024 + (r & 7) * 128;
+        const uint32_t trow = tmem_base + (((warp & 3) * 32u) << 16);   // the quarter of tensor memory the warp may touch
         uint32_t m = 0;
         bool ok = true;
         for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
             PwWalk w;
             w.set(a, item);
             for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++, m++) {
-                const uint32_t u = m & 1, raw = sm_raw + u * F::RAW;
-                ok = tc_wait(bar_u(u), (m >> 1) & 1, dead, a.err, 49);
+                const uint32_t ur = m % NR, raw = sm_raw + ur * F::RAW;
+                ok = tc_wait(bar_u(ur), (m / NR) & 1, dead, a.err, 49);
                 // (on behalf of the MMA of the mins, which reads the group sums)
                 if (FMT == WGB_Q4_K && grp == 1 && ok) ok = tc_wait(bar_x(m % NX), (m / NX) & 1, dead, a.err, 47);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
 #pragma unroll 1
                 for (uint32_t st = grp; st < STEPS; st += 2) {
-                    const uint32_t n = m * STEPS + st, s = n % NA;
+                    const uint32_t n = m * STEPS + st;
                     if (n >= NA) ok = __all_sync(0xffffffffu, tc_wait(bar_e(n - NA), ((n - NA) / NE) & 1, dead, a.err, 50));
                     if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (st == grp) {
                         // Once per unit (the MMAs of two units back are through: a later step's buffer was just free).
                         if (grp == 0) {
@@ -437,25 +454,27 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                             __syncwarp();
                             if (lane == 0) mbar_arrive(bar_r(m & 3));
                         }
-                        if (FMT == WGB_Q4_K) {
-                            // the row's eight mins, once per K-core: each group writes one of the two
+                        if (FMT == WGB_Q4_K && grp == 1) {
+                            // the row's eight mins, for either digit of the group sums
                             const uint4 hdr = lds128(raw + r * 144);
                             const uint32_t m_lo = hdr.z & 0x3f3f3f3fu, m_hi = ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u);
                             const __half2 k1024 = __float2half2_rn(1024.0f);
-                            sts128(sm_min + u * F::AMIN + grp * TC_TILE_ROWS * 16 + r * 16, h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4140)), k1024)),
+                            pw_st8(trow + PW_TMEM_AMIN + 8 * (m & 1), h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4140)), k1024)),
                                    h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4342)), k1024)),
                                    h2u(__hsub2(u2h(__byte_perm(m_hi, 0x64646464u, 0x4140)), k1024)),
                                    h2u(__hsub2(u2h(__byte_perm(m_hi, 0x64646464u, 0x4342)), k1024)));
                         }
                     }
-#pragma unroll
-                    for (uint32_t h = 0; h < 2; h++) pw_unpack<FMT>(raw, arow0 + s * PW_A_STEP, r, h, st & 3, F::PLANES == 2 && st < 4);
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    uint32_t v[32];
+                    pw_unpack<FMT>(v, raw, r, st & 3, F::PLANES == 2 && st < 4);
+                    pw_st32(trow + PW_TMEM_A + (n % NA) * PW_A_COLS, v);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar_f(n));
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar_ue(u));
+                if (lane == 0) mbar_arrive(bar_ue(ur));
             }
         }
     } else {
