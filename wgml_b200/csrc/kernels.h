@@ -236,8 +236,8 @@ int launch_prefill_attention(const float *q, const float *k_cache, const float *
 
 
 // ---- wide prompt passes (prefill_wide.cu) ---------------------------------------------------------------
-constexpr uint32_t PW_TILE = 80;             // prompt positions per tile of a wide product, most
-constexpr uint32_t PW_CAP = 8 * PW_TILE;     // prompt positions per wide pass, most
+constexpr uint32_t PW_TILE = 128;            // prompt positions per tile of a wide product, most
+constexpr uint32_t PW_CAP = 5 * PW_TILE;     // prompt positions per wide pass, most
 constexpr uint32_t PW_MIN = 16;              // fewer than this go through the passes of PF_TOK positions
 // Tiles of positions of a pass: npt tiles of np positions each.
 struct WideTiling { uint32_t np, npt; };

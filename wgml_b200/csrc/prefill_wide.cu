@@ -2,23 +2,23 @@
 //
 // The passes of eight positions (prefill.cu) read every weight once per eight positions and spend their time on the
 // chain unpack -> MMA -> read-back of each 256-column unit, whose tensor work is 4 % of it.  With a long prompt the
-// same unpacked weights can serve up to 80 positions at a time, and the pass becomes a contraction proper: this file
+// same unpacked weights can serve up to 128 positions at a time, and the pass becomes a contraction proper: this file
 // holds its matrix product on the tensor cores (tcgen05.mma kind::f16 with f32 accumulators in tensor memory), the
 // activation image it reads, the element-wise kernels between the products and a causal attention over tiles of 64
 // positions.  Operators as in the narrow passes: GemvQuant::dispatch (crates/wgml/src/ops/gemv_quant.rs:241-348),
 // RmsNorm / LayerNorm / Silu / GELU / BatchedMultiqueryAttention of one position, for many.
 //
-// Arithmetic.  A unit is 256 columns.  Activations: x = X * 2^e with one exponent per position and unit, |X| <= 2^22,
-// written as two f16 digits X = 2048 hi + lo (hi an integer, |hi| <= 2048; |lo| <= 1024 rounded to eleven bits, so X is
-// good to a quarter on average: finer than the integer X of the other products, which makes up for the exponent being
-// shared by 256 columns instead of 32).  Weights: the
-// part of a weight that varies inside a unit, as one or two f16 integers,
+// Arithmetic.  A unit is 256 columns.  Activations: x = X * 2^e with one exponent per position and unit, |X| <= 2048,
+// written as two f16 digits X = hi + lo (hi an integer; |lo| <= 1/2 rounded to eleven bits, so X is good to 2^-13
+// on average: finer than the integers of 2^22 of the other products, which makes up for the exponent being
+// shared by 256 columns instead of 32).  Weights: the part of a weight that varies inside a unit, as one or two f16
+// numbers,
 //   Q4_K  scale * code           <= 945: one plane;  d per row and unit, mins through a product of their own
 //   Q6_K  scale * (code - 32)    <= 4096 in magnitude: 16 a1 + a2, two planes;  d per row and unit
 //   Q8_0  code * d_group / 2^E   18 bits: a1 + a2 (a1 an integer <= 512), two planes;  2^E the row's power of two
-// so every product is an integer below 2^22 (a few bits more for a2) and the sums of a unit stay within or near the
-// 24 bits of the f32 accumulator; the small planes go first, while the accumulator is small.  After a unit
-// the two digit sums are joined and scaled in f32, as in the other products.
+// The products of the large digits are integers below 2^22 and their sum over a unit stays within or near the 24 bits of
+// the f32 accumulator.  One accumulator takes all of a unit's products, the small ones (a2, lo) first: what they add
+// below the final sum's last bit is dropped once, not per product.
 #include "kernels.h"
 #include "tc_common.cuh"
 
@@ -26,47 +26,48 @@
 
 namespace wgb {
 
-constexpr uint32_t PW_MAXN = PW_TILE;                              // positions per tile (two digits each: N = 160)
+constexpr uint32_t PW_MAXN = PW_TILE;                              // positions per tile
 constexpr uint32_t PW_UNPACK_WARPS = 8;                            // build the weight operand, two groups of four
 constexpr uint32_t PW_FINISH_WARPS = 8;                            // read the sums, apply scales
 constexpr uint32_t PW_NT = 32 * (3 + PW_UNPACK_WARPS + PW_FINISH_WARPS);
-constexpr uint32_t PW_A_COLS = 32;                                 // weight operand of a step: 64 columns in f16, in tensor memory
-constexpr uint32_t PW_A_RING = 3;                                  // odd: consecutive uses of a buffer are different groups'
-constexpr uint32_t PW_B_STEP = 2 * PW_MAXN * 128;                  // activation operand of a step, largest, in shared memory
-constexpr uint32_t PW_B_RING = 6;
-constexpr uint32_t PW_E_RING = 2 * PW_A_RING;                      // steps have a barrier pair each, six in turn
+constexpr uint32_t PW_A_COLS = 32;                                 // weight operand of 64 columns in f16, in tensor memory
+constexpr uint32_t PW_A_RING = 4;                                  // one plane of a unit, in two pairs
+constexpr uint32_t PW_B_STEP = 2 * PW_MAXN * 128;                  // one digit of 128 columns, largest, in shared memory
+constexpr uint32_t PW_B_RING = 4;
 constexpr uint32_t PW_AUX = 36 * PW_MAXN;                          // per unit: sums of the mins' product, exponents
 constexpr uint32_t PW_X_RING = 3;
-// Tensor memory: two sets of sums (2 x 80 columns), the min sums (80), three weight operands (32), two of mins (8).
+constexpr uint32_t PW_AMIN = 2 * TC_TILE_ROWS * 16;                // mins as f16, [two K-cores][row], in shared memory
+// Tensor memory: two sets of sums (128 columns), the min sums (128), four weight operands (32).
 constexpr uint32_t PW_TMEM_COLS = 512;
-constexpr uint32_t PW_TMEM_MIN = 4 * PW_MAXN;
+constexpr uint32_t PW_TMEM_MIN = 2 * PW_MAXN;
 constexpr uint32_t PW_TMEM_A = PW_TMEM_MIN + PW_MAXN;
-constexpr uint32_t PW_TMEM_AMIN = PW_TMEM_A + PW_A_RING * PW_A_COLS;
-static_assert(PW_MAXN % 16 == 0 && PW_TMEM_AMIN + 2 * 8 <= PW_TMEM_COLS, "tensor memory");
-static_assert(PW_B_RING <= PW_E_RING, "a step's barriers outlive its buffer");
+static_assert(PW_MAXN % 16 == 0 && PW_TMEM_A + PW_A_RING * PW_A_COLS <= PW_TMEM_COLS, "tensor memory");
 
 // Per format: raw bytes of a unit of 128 rows (tile-major copies of prefill.cu, prefill_q6k.cu, prefill_q80.cu) and how
 // many units fit.
 template <int FMT> struct PwFmt;
-template <> struct PwFmt<WGB_Q4_K> { static constexpr uint32_t RAW = TC_UNIT_BYTES, RAW_RING = 3, PLANES = 1; };
-template <> struct PwFmt<WGB_Q6_K> { static constexpr uint32_t RAW = TC_TILE_ROWS * 210, RAW_RING = 3, PLANES = 2; };
-template <> struct PwFmt<WGB_Q8_0> { static constexpr uint32_t RAW = TC_TILE_ROWS * 272, RAW_RING = 2, PLANES = 2; };
-template <int FMT> constexpr uint32_t pw_smem() { return PW_B_RING * PW_B_STEP + PwFmt<FMT>::RAW_RING * PwFmt<FMT>::RAW + PW_X_RING * PW_AUX; }
+template <> struct PwFmt<WGB_Q4_K> { static constexpr uint32_t RAW = TC_UNIT_BYTES, RAW_RING = 3, PLANES = 1, AMIN = PW_AMIN; };
+template <> struct PwFmt<WGB_Q6_K> { static constexpr uint32_t RAW = TC_TILE_ROWS * 210, RAW_RING = 3, PLANES = 2, AMIN = 0; };
+template <> struct PwFmt<WGB_Q8_0> { static constexpr uint32_t RAW = TC_TILE_ROWS * 272, RAW_RING = 2, PLANES = 2, AMIN = 0; };
+template <int FMT> constexpr uint32_t pw_smem()
+{
+    return PW_B_RING * PW_B_STEP + PwFmt<FMT>::RAW_RING * PwFmt<FMT>::RAW + 2 * PwFmt<FMT>::AMIN + PW_X_RING * PW_AUX;
+}
 constexpr uint32_t PW_STATIC = 4 * TC_TILE_ROWS * 8 + 512;         // row scales, barriers
 static_assert(pw_smem<WGB_Q4_K>() + 1024 + PW_STATIC <= 227 * 1024 && pw_smem<WGB_Q6_K>() + 1024 + PW_STATIC <= 227 * 1024 &&
                   pw_smem<WGB_Q8_0>() + 1024 + PW_STATIC <= 227 * 1024,
               "shared memory budget");
 static_assert(PW_B_STEP % 1024 == 0 && PW_AUX % 16 == 0, "swizzled operands start on 1 KB boundaries");
 
-// Activation image of a pass: [tile of np positions][unit]: four steps of 64 columns, each [hi rows | lo rows] x 128
-// bytes in the 128-byte swizzle; then the sums of the eight 32-column groups as two f16 digits
+// Activation image of a pass: [tile of np positions][unit]: the low digits of four times 64 columns, then the high ones,
+// each [np rows] x 128 bytes in the 128-byte swizzle; then the sums of the eight 32-column groups as two f16 digits
 // ([digit][position][group]); then one exponent (a power of two) per position.
 __host__ __device__ constexpr uint32_t pw_image_unit(uint32_t np) { return (1024 + 36) * np; }
 
 size_t prefill_wide_image_bytes(uint32_t K)
 {
-    // any split of PW_CAP positions into tiles of a multiple of 8 pads by less than one such multiple per tile
-    return (size_t)(K / 256) * pw_image_unit(PW_CAP + 8 * ((PW_CAP + PW_MAXN - 1) / PW_MAXN + 1));
+    // any split of PW_CAP positions into tiles of a multiple of 16 pads by less than one such multiple per tile
+    return (size_t)(K / 256) * pw_image_unit(PW_CAP + 16 * ((PW_CAP + PW_MAXN - 1) / PW_MAXN + 1));
 }
 
 struct PwArgs {
@@ -108,13 +109,22 @@ __device__ __forceinline__ void pw_mma(uint32_t d_tmem, uint32_t a_tmem, uint64_
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// The same with A in shared memory.
+__device__ __forceinline__ void pw_mma_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.u32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 // kind::f16 instruction descriptor: D f32, A and B f16, both K-major, M = 128, N = n.
 __device__ __forceinline__ uint32_t pw_idesc(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24); }
 
 __device__ __forceinline__ __half2 u2h(uint32_t v) { return *reinterpret_cast<__half2 *>(&v); }
 __device__ __forceinline__ uint32_t h2u(__half2 v) { return *reinterpret_cast<uint32_t *>(&v); }
 
-// A thread's 32 (8) words into 32 (8) columns of its lane.
+// A thread's 32 words into 32 columns of its lane.
 __device__ __forceinline__ void pw_st32(uint32_t taddr, const uint32_t (&v)[32])
 {
     asm volatile(
@@ -125,11 +135,6 @@ __device__ __forceinline__ void pw_st32(uint32_t taddr, const uint32_t (&v)[32])
         "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
         : "memory");
 }
-__device__ __forceinline__ void pw_st8(uint32_t taddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d)   // the four words twice
-{
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%1,%2,%3,%4};" ::"r"(taddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-
 // Two f32 at a time (the packed FMA of this architecture).
 __device__ __forceinline__ uint64_t f2pack(float a, float b)
 {
@@ -248,18 +253,21 @@ __device__ __forceinline__ void pw_unpack(uint32_t (&v)[32], uint32_t raw, uint3
 }
 
 // Roles: two producer threads (raw weights and per-unit extras; activation operand), one thread issuing MMAs, two groups
-// of four warps building the weight operand (alternate steps), eight warps finishing units.  Raw weights are free again
-// as soon as they are unpacked, a unit ahead of its MMAs; the rows' scales travel in a small ring of their own.
-// The weight operand goes from registers to tensor memory: written to and read from shared memory it
-// cost as much of that memory's 128 bytes a clock as everything else together (per step of 64 columns and 88 positions
-// 710 clocks, against 350 of MMA; now 400 against 320).
+// of four warps building the weight operand (alternate chunks of 64 columns), eight warps finishing units.
+// What bounds it: unpacking, per weight about 1.3 instructions on top of what the tensor pipe does.  A chunk of
+// weights therefore serves as many positions as tensor memory has room for: the accumulator holds both digits (low
+// digits of the four chunks first, then the high ones over the same weight operands, which stay in tensor memory), so
+// a tile is 128 positions; with an accumulator per digit it was 80 and 400 ns per chunk.  The operand goes from
+// registers to tensor memory: written to and read from shared memory it cost as much of that memory's 128 bytes a
+// clock as everything else together.  Raw weights are free again as soon as they are unpacked, ahead of their MMAs;
+// the rows' scales travel in a small ring of their own.
 template <int FMT>
 __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_constant__ PwArgs a)
 {
     using F = PwFmt<FMT>;
-    constexpr uint32_t NA = PW_A_RING, NB = PW_B_RING, NX = PW_X_RING, NE = PW_E_RING, NR = F::RAW_RING, STEPS = 4 * F::PLANES;
+    constexpr uint32_t NA = PW_A_RING / 2, NB = PW_B_RING, NX = PW_X_RING, NR = F::RAW_RING, P = F::PLANES;
     extern __shared__ uint8_t pw_smem_raw[];
-    __shared__ __align__(8) unsigned long long bars[2 * NE + 2 * NX + 2 * NR + 9];
+    __shared__ __align__(8) unsigned long long bars[2 * NA + 2 * NB + 2 * NX + 2 * NR + 9];
     __shared__ float2 rowscale[4][TC_TILE_ROWS];
     __shared__ uint32_t tmem_base_slot;
     __shared__ uint32_t dead_flag;
@@ -267,37 +275,44 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
     volatile uint32_t *dead = &dead_flag;
 
     pdl_launch_dependents();
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = tc_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const uint32_t nitems = a.ntiles * a.nsplit * a.npt, np = a.np;
-    auto bar = [&](uint32_t i) { return smem_addr(&bars[i]); };
-    auto bar_f = [&](uint32_t n) { return bar(n % NE); };                  // both operands of step n are there
-    auto bar_e = [&](uint32_t n) { return bar(NE + n % NE); };             //   and have been read by its MMAs
-    auto bar_x = [&](uint32_t s) { return bar(2 * NE + s); };              // group sums and exponents of a unit have landed
-    auto bar_xe = [&](uint32_t s) { return bar(2 * NE + NX + s); };
-    constexpr uint32_t B0 = 2 * NE + 2 * NX;
+    const uint32_t bar0 = tc_uniform(smem_addr(bars));
+    auto bar = [&](uint32_t i) { return bar0 + 8 * i; };
+    auto bar_a = [&](uint32_t j) { return bar(j); };                       // weight operand of chunks 2 j and 2 j + 1 is built
+    auto bar_ae = [&](uint32_t j) { return bar(NA + j); };                 //   and has been read by the MMAs of both digits
+    auto bar_b = [&](uint32_t s) { return bar(2 * NA + s); };              // activation operand of a step has landed
+    auto bar_be = [&](uint32_t s) { return bar(2 * NA + NB + s); };        //   and has been read
+    auto bar_x = [&](uint32_t s) { return bar(2 * NA + 2 * NB + s); };     // group sums and exponents of a unit have landed
+    auto bar_xe = [&](uint32_t s) { return bar(2 * NA + 2 * NB + NX + s); };
+    constexpr uint32_t B0 = 2 * NA + 2 * NB + 2 * NX;
     auto bar_u = [&](uint32_t i) { return bar(B0 + i); };                  // raw unit has landed
     auto bar_ue = [&](uint32_t i) { return bar(B0 + NR + i); };            //   and is unpacked
     auto bar_d = [&](uint32_t u) { return bar(B0 + 2 * NR + u); };         // the unit's sums are complete
     auto bar_t = [&](uint32_t u) { return bar(B0 + 2 * NR + 2 + u); };     //   and have been read
     auto bar_r = [&](uint32_t i) { return bar(B0 + 2 * NR + 4 + i); };     // its rows' scales are written (i = m % 4)
     const uint32_t bar_m = bar(B0 + 2 * NR + 8);                           // the min sums have been read
-    const uint32_t sm_b = smem_addr(smem), sm_raw = sm_b + NB * PW_B_STEP, sm_aux = sm_raw + NR * F::RAW;
+    const uint32_t sm_b = tc_uniform(smem_addr(smem)), sm_raw = sm_b + NB * PW_B_STEP, sm_min = sm_raw + NR * F::RAW, sm_aux = sm_min + 2 * F::AMIN;
 
     if (threadIdx.x == 0) {
         dead_flag = 0;
-        for (uint32_t n = 0; n < NE; n++) {
-            mbar_init(bar_f(n), PW_UNPACK_WARPS / 2 + 1);
-            mbar_init(bar_e(n), 1);
+        for (uint32_t c = 0; c < NA; c++) {
+            mbar_init(bar_a(c), PW_UNPACK_WARPS);
+            mbar_init(bar_ae(c), 1);
+        }
+        for (uint32_t s = 0; s < NB; s++) {
+            mbar_init(bar_b(s), 1);
+            mbar_init(bar_be(s), 1);
+        }
+        for (uint32_t s = 0; s < NX; s++) {
+            mbar_init(bar_x(s), 1);
+            mbar_init(bar_xe(s), PW_FINISH_WARPS);
         }
         for (uint32_t s = 0; s < NR; s++) {
             mbar_init(bar_u(s), 1);
             mbar_init(bar_ue(s), PW_UNPACK_WARPS);
         }
         for (uint32_t s = 0; s < 4; s++) mbar_init(bar_r(s), PW_UNPACK_WARPS / 2);
-        for (uint32_t s = 0; s < NX; s++) {
-            mbar_init(bar_x(s), 1);
-            mbar_init(bar_xe(s), PW_FINISH_WARPS);
-        }
         for (uint32_t u = 0; u < 2; u++) {
             mbar_init(bar_d(u), 1);
             mbar_init(bar_t(u), PW_FINISH_WARPS);
@@ -312,16 +327,15 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = tmem_base_slot;
+    const uint32_t tmem_base = tc_uniform(tmem_base_slot);
     pdl_wait();   // barriers and tensor memory are set up while the preceding launch (which writes the image) still runs
 
-    // Every role walks the same items, units m and steps n (both numbered through over the block's life).  A parity tells
-    // two phases apart, so each waiter waits on every phase of a barrier, in order, and a barrier cannot run a phase
-    // ahead of any of its waiters: a buffer's next use needs the waiter's own arrival, directly (rings) or through the
-    // MMA order (the barriers of step n come round at step n + 6; the operand group that waits for step n before it
-    // builds n + 3 is always the same one, and step n + 6 needs the buffer of its step n + 3; scales of unit m + 4
-    // are written when MMAs of unit m + 3 are through, which takes the sums of unit m + 1 read).  A role whose wait has
-    // expired leaves its loop; the others see the flag and follow.
+    // Every role walks the same items, units m, operand chunks q and steps n (numbered through over the block's life).  A
+    // parity tells two phases apart, so each waiter waits on every phase of a barrier, in order, and a barrier cannot
+    // run a phase ahead of any of its waiters: the next use of what it guards needs the waiter's own arrival, directly
+    // (rings) or through the MMA order (scales of unit m + 4 are written when MMAs of unit m + 3 are through, which
+    // takes the sums of unit m + 1 read).  A role whose wait has expired leaves its loop; the others see the flag and
+    // follow.
     constexpr unsigned long long DRAIN_NS = 1000000000ull;
     if (warp == 0) {
         // ------------------------------ raw weights, group sums, exponents ------------------------------
@@ -361,61 +375,72 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                 w.set(a, item);
                 for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++) {
                     const uint8_t *img = a.img + ((size_t)w.pt * a.nkb + kb) * unit_bytes;
-                    for (uint32_t st = 0; st < STEPS; st++, n++) {
+                    for (uint32_t st = 0; st < 4 * P; st++, n++) {
                         const uint32_t s = n % NB;
-                        if (n >= NB) ok = tc_wait(bar_e(n - NB), ((n - NB) / NE) & 1, dead, a.err, 43);
+                        if (n >= NB) ok = tc_wait(bar_be(s), (n / NB - 1) & 1, dead, a.err, 43);
                         if (!ok) break;
-                        mbar_expect_tx(bar_f(n), bstep);
-                        bulk_copy_g2s(sm_b + s * PW_B_STEP, img + (st & 3) * bstep, bstep, bar_f(n));
+                        mbar_expect_tx(bar_b(s), bstep);
+                        bulk_copy_g2s(sm_b + s * PW_B_STEP, img + (st & 3) * bstep, bstep, bar_b(s));
                     }
                 }
             }
-            // After an expired wait the operand's copies cannot be told from the barrier alone (it also counts the
-            // unpacking warps): give them the time any copy takes.
             if (!ok)
-                for (const unsigned long long t0 = global_ns(); global_ns() - t0 < DRAIN_NS / 100;) {}
+                for (uint32_t k = n > NB ? n - NB : 0; k < n; k++) mbar_wait(bar_b(k % NB), (k / NB) & 1, nullptr, 0, DRAIN_NS);
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issue ------------------------------
-        if (tc_elect()) {
-            uint32_t m = 0, n = 0;
-            bool ok = true;
-            const uint32_t idesc = pw_idesc(2 * np), idesc_min = pw_idesc((np + 15) & ~15u);
-            for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
-                PwWalk w;
-                w.set(a, item);
-                for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++, m++) {
-                    const uint32_t u = m & 1, dcol = tmem_base + u * 2 * PW_MAXN;
-                    if (m >= 2) ok = tc_wait(bar_t(u), ((m >> 1) - 1) & 1, dead, a.err, 44);
-                    for (uint32_t st = 0; st < STEPS && ok; st++, n++) {
-                        const uint32_t at = tmem_base + PW_TMEM_A + (n % NA) * PW_A_COLS;
-                        ok = tc_wait(bar_f(n), (n / NE) & 1, dead, a.err, 45);
+        // The whole warp walks the loop and waits, with votes, so that control flow stays uniform for the compiler.
+        uint32_t m = 0, n = 0, q = 0;   // q: planes so far
+        bool ok = true;
+        const uint32_t idesc = pw_idesc(np);
+        auto wait = [&](uint32_t b, uint32_t parity, uint32_t code) { return __all_sync(0xffffffffu, tc_wait(b, parity, dead, a.err, code)) != 0; };
+        for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+            PwWalk w;
+            w.set(a, item);
+            for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++, m++) {
+                const uint32_t u = m & 1, dcol = tmem_base + u * PW_MAXN;
+                // (with mins, the wait for the min sums of unit m - 2 covers this one)
+                if (FMT != WGB_Q4_K && m >= 2) ok = wait(bar_t(u), ((m >> 1) - 1) & 1, 44);
+                for (uint32_t pl = 0; pl < P && ok; pl++, q++) {
+#pragma unroll 1
+                    for (uint32_t st = 0; st < 4; st++, n++) {
+                        const uint32_t j = st & 1, s = n % NB;   // low digits of the two pairs of chunks, then the high ones
+                        if (st < 2) ok = wait(bar_a(j), q & 1, 46);
+                        if (ok) ok = wait(bar_b(s), (n / NB) & 1, 45);
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        const uint64_t bd = tc_smem_desc_sw128(sm_b + (n % NB) * PW_B_STEP, 1024);
+                        const uint32_t at = tmem_base + PW_TMEM_A + 2 * j * PW_A_COLS;
+                        const uint64_t bd0 = tc_smem_desc_sw128(sm_b + s * PW_B_STEP, 1024), bd1 = tc_smem_desc_sw128(sm_b + s * PW_B_STEP + 128 * np, 1024);
+                        if (tc_elect()) {
 #pragma unroll
-                        for (uint32_t k = 0; k < 4; k++) pw_mma(dcol, at + 8 * k, bd + 2 * k, idesc, (st | k) ? 1u : 0u);
-                        tc_commit(bar_e(n));
-                    }
-                    if (FMT == WGB_Q4_K && ok) {
-                        // sum over the eight groups of min x (sum of the group's X), both digits of the sums in one MMA
-                        const uint32_t x = m % NX;
-                        if (m >= 1) ok = tc_wait(bar_m, (m - 1) & 1, dead, a.err, 48);
-                        if (ok) {
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            pw_mma(tmem_base + PW_TMEM_MIN, tmem_base + PW_TMEM_AMIN + 8 * u, tc_smem_desc(sm_aux + x * PW_AUX, np * 16, 128), idesc_min, 0u);
+                            for (uint32_t k = 0; k < 4; k++) pw_mma(dcol, at + 8 * k, bd0 + 2 * k, idesc, (pl | st | k) ? 1u : 0u);
+#pragma unroll
+                            for (uint32_t k = 0; k < 4; k++) pw_mma(dcol, at + PW_A_COLS + 8 * k, bd1 + 2 * k, idesc, 1u);
+                            tc_commit(bar_be(s));
+                            if (st >= 2) tc_commit(bar_ae(j));
                         }
+                        __syncwarp();
                     }
-                    if (ok) tc_commit(bar_d(u));
                 }
+                if (FMT == WGB_Q4_K && ok && m >= 1) ok = wait(bar_m, (m - 1) & 1, 48);
+                if (!ok) break;
+                if (FMT == WGB_Q4_K) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (tc_elect()) {
+                    // sum over the eight groups of min x (sum of the group's X), both digits of the sums in one MMA
+                    if (FMT == WGB_Q4_K)
+                        pw_mma_ss(tmem_base + PW_TMEM_MIN, tc_smem_desc(sm_min + u * F::AMIN, TC_TILE_ROWS * 16, 128),
+                                  tc_smem_desc(sm_aux + (m % NX) * PW_AUX, np * 16, 128), idesc, 0u);
+                    tc_commit(bar_d(u));
+                }
+                __syncwarp();
             }
         }
     } else if (warp < 2 + PW_UNPACK_WARPS) {
         // ------------------------------ weight operand ------------------------------
-        // Group `grp` builds steps grp, grp + 2, ...; a thread builds one row of 64 columns.
+        // Group `grp` builds chunks grp and grp + 2 of a plane; a thread builds one row of 64 columns.
         const uint32_t grp = (warp - 2) >> 2, r = (warp & 3) * 32 + lane;
         const uint32_t trow = tmem_base + (((warp & 3) * 32u) << 16);   // the quarter of tensor memory the warp may touch
-        uint32_t m = 0;
+        uint32_t m = 0, q = 0;
         bool ok = true;
         for (uint32_t item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
             PwWalk w;
@@ -426,15 +451,24 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                 // (on behalf of the MMA of the mins, which reads the group sums)
                 if (FMT == WGB_Q4_K && grp == 1 && ok) ok = tc_wait(bar_x(m % NX), (m / NX) & 1, dead, a.err, 47);
                 ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
 #pragma unroll 1
-                for (uint32_t st = grp; st < STEPS; st += 2) {
-                    const uint32_t n = m * STEPS + st;
-                    if (n >= NA) ok = __all_sync(0xffffffffu, tc_wait(bar_e(n - NA), ((n - NA) / NE) & 1, dead, a.err, 50));
+                for (uint32_t i = 0; i < 2 * P && ok; i++) {
+                    const uint32_t j = i & 1, c = 2 * j + grp;
+                    // the row is built in registers before its buffer is free: only the store waits for the MMAs
+                    uint32_t v[32];
+                    pw_unpack<FMT>(v, raw, r, c, P == 2 && i < 2);
+                    if (q) ok = __all_sync(0xffffffffu, tc_wait(bar_ae(j), (q - 1) & 1, dead, a.err, 50));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (st == grp) {
-                        // Once per unit (the MMAs of two units back are through: a later step's buffer was just free).
+                    pw_st32(trow + PW_TMEM_A + c * PW_A_COLS, v);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_a(j));
+                    if (i & 1) q++;
+                    if (i == 0) {
+                        // Once per unit, off the path of its first MMAs.  (The MMAs of two units back are through: a chunk of
+                        // the unit before has just been read.)
                         if (grp == 0) {
                             float d, dmin = 0.0f;
                             if constexpr (FMT == WGB_Q4_K) {
@@ -442,7 +476,7 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                                 asm volatile("ld.shared.u32 %0, [%1];" : "=r"(dm) : "r"(raw + r * 144));
                                 const float2 f = __half22float2(u2h(dm));
                                 d = f.x;
-                                dmin = f.y * -4096.0f;
+                                dmin = f.y * -2.0f;
                             } else if constexpr (FMT == WGB_Q6_K) {
                                 uint32_t db;
                                 asm volatile("ld.shared.u16 %0, [%1];" : "=r"(db) : "r"(raw + TC_TILE_ROWS * 208 + r * 2));
@@ -453,25 +487,21 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                             rowscale[m & 3][r] = make_float2(d, dmin);
                             __syncwarp();
                             if (lane == 0) mbar_arrive(bar_r(m & 3));
-                        }
-                        if (FMT == WGB_Q4_K && grp == 1) {
-                            // the row's eight mins, for either digit of the group sums
+                        } else if (FMT == WGB_Q4_K) {
+                            // the row's eight mins, once per K-core: for either digit of the group sums
                             const uint4 hdr = lds128(raw + r * 144);
                             const uint32_t m_lo = hdr.z & 0x3f3f3f3fu, m_hi = ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u);
                             const __half2 k1024 = __float2half2_rn(1024.0f);
-                            pw_st8(trow + PW_TMEM_AMIN + 8 * (m & 1), h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4140)), k1024)),
-                                   h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4342)), k1024)),
-                                   h2u(__hsub2(u2h(__byte_perm(m_hi, 0x64646464u, 0x4140)), k1024)),
-                                   h2u(__hsub2(u2h(__byte_perm(m_hi, 0x64646464u, 0x4342)), k1024)));
+                            const uint32_t v0 = h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4140)), k1024)),
+                                           v1 = h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4342)), k1024)),
+                                           v2 = h2u(__hsub2(u2h(__byte_perm(m_hi, 0x64646464u, 0x4140)), k1024)),
+                                           v3 = h2u(__hsub2(u2h(__byte_perm(m_hi, 0x64646464u, 0x4342)), k1024));
+                            const uint32_t at = sm_min + (m & 1) * F::AMIN + r * 16;
+                            sts128(at, v0, v1, v2, v3);
+                            sts128(at + TC_TILE_ROWS * 16, v0, v1, v2, v3);
+                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                         }
                     }
-                    uint32_t v[32];
-                    pw_unpack<FMT>(v, raw, r, st & 3, F::PLANES == 2 && st < 4);
-                    pw_st32(trow + PW_TMEM_A + (n % NA) * PW_A_COLS, v);
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_f(n));
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_ue(ur));
@@ -480,10 +510,9 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
     } else {
         // ------------------------------ finishing ------------------------------
         // Thread (quarter, lane, half): row r of the tile, groups of eight positions half, half + 2, ...
-        constexpr uint32_t NG = (PW_MAXN / 8 + 1) / 2;
+        constexpr uint32_t NG = PW_MAXN / 16;
         const uint32_t half = (warp - 2 - PW_UNPACK_WARPS) >> 2, quarter = warp & 3, r = quarter * 32 + lane, ng = np / 8;
         const uint32_t trow = tmem_base + ((quarter * 32u) << 16);
-        const uint64_t k2048 = f2pack(2048.0f, 2048.0f);
         uint64_t acc[NG][4];
         uint32_t m = 0;
         bool ok = true;
@@ -503,23 +532,20 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                 const float2 sc = rowscale[m & 3][r];
                 const uint64_t d2 = f2pack(sc.x, sc.x), dm2 = f2pack(sc.y, sc.y);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t tb = trow + u * 2 * PW_MAXN;
+                const uint32_t tb = trow + u * PW_MAXN;
 #pragma unroll
                 for (uint32_t gi = 0; gi < NG; gi++) {
                     const uint32_t g = 2 * gi + half;
                     if (g < ng) {
-                        int hi[8], lo[8], mn[8];
-                        tc_ld8(tb + 8 * g, hi);
-                        tc_ld8(tb + np + 8 * g, lo);
+                        int dv[8], mn[8];
+                        tc_ld8(tb + 8 * g, dv);
                         if (FMT == WGB_Q4_K) tc_ld8(trow + PW_TMEM_MIN + 8 * g, mn);
                         const uint4 e0 = lds128(ebase + 32 * g), e1 = lds128(ebase + 32 * g + 16);
                         const uint32_t ev[8] = { e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w };
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                         for (uint32_t j = 0; j < 4; j++) {
-                            uint64_t t = f2fma(f2pack(__int_as_float(hi[2 * j]), __int_as_float(hi[2 * j + 1])), k2048,
-                                               f2pack(__int_as_float(lo[2 * j]), __int_as_float(lo[2 * j + 1])));
-                            t = f2mul(t, d2);
+                            uint64_t t = f2mul(f2pack(__int_as_float(dv[2 * j]), __int_as_float(dv[2 * j + 1])), d2);
                             if (FMT == WGB_Q4_K) t = f2fma(f2pack(__int_as_float(mn[2 * j]), __int_as_float(mn[2 * j + 1])), dm2, t);
                             acc[gi][j] = f2fma(t, f2pack(__uint_as_float(ev[2 * j]), __uint_as_float(ev[2 * j + 1])), acc[gi][j]);
                         }
@@ -559,12 +585,12 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
     }
 }
 
-// Tiles of positions: as few as fit, of equal size (a multiple of eight).
+// Tiles of positions: as few as fit, of equal size (a multiple of sixteen, the step of an MMA's N).
 WideTiling prefill_wide_tiling(uint32_t ntok)
 {
     WideTiling t;
     t.npt = (ntok + PW_MAXN - 1) / PW_MAXN;
-    t.np = ((ntok + t.npt - 1) / t.npt + 7) & ~7u;
+    t.np = ((ntok + t.npt - 1) / t.npt + 15) & ~15u;
     return t;
 }
 
@@ -599,7 +625,7 @@ static int launch_wide(const PwArgs &a, bool *attrs, cudaStream_t stream)
 int launch_gemm_wide(int qtype, uint32_t nmat, const uint8_t *const *w_tiles, const uint32_t *nrows, uint32_t K, const uint8_t *image, uint32_t ntok,
                      const WideTiling &t, float *const *out, const uint32_t *out_stride, uint32_t nsplit, cudaStream_t stream)
 {
-    WGB_REQUIRE(nmat >= 1 && nmat <= 3 && K % 256 == 0 && ntok >= 1 && ntok <= PW_CAP && nsplit >= 1 && nsplit <= K / 256 && t.np % 8 == 0 && t.np <= PW_MAXN &&
+    WGB_REQUIRE(nmat >= 1 && nmat <= 3 && K % 256 == 0 && ntok >= 1 && ntok <= PW_CAP && nsplit >= 1 && nsplit <= K / 256 && t.np % 16 == 0 && t.np <= PW_MAXN &&
                     t.np * t.npt >= ntok,
                 "wide product: %u matrices, %u columns, %u positions, %u slices", nmat, K, ntok, nsplit);
     DeviceState *ds = device_state();
@@ -637,10 +663,10 @@ __device__ __forceinline__ void wide_image_unit(uint8_t *__restrict__ image, uin
 #pragma unroll
     for (int i = 0; i < 8; i++) mx = fmaxf(mx, fabsf(v[i]));
     mx = warp_max(mx);
-    // |v| < 2^(ex - 126), so X = v * 2^(148 - ex) lies within +-2^22
+    // |v| < 2^(ex - 126), so X = v * 2^(137 - ex) lies within +-2048
     uint32_t ex = (__float_as_uint(mx) >> 23) & 0xffu;
     ex = ex < 24u ? 24u : (ex > 253u ? 253u : ex);
-    const float up = __uint_as_float((275u - ex) << 23), down = __uint_as_float((ex - 21u) << 23);
+    const float up = __uint_as_float((264u - ex) << 23), down = __uint_as_float((ex - 10u) << 23);
     uint32_t hw[4], lw[4];
     float hsum = 0.0f, lsum = 0.0f;
 #pragma unroll
@@ -649,8 +675,8 @@ __device__ __forceinline__ void wide_image_unit(uint8_t *__restrict__ image, uin
 #pragma unroll
         for (int j = 0; j < 2; j++) {
             const float X = v[2 * i + j] * up;
-            hi[j] = rintf(X * (1.0f / 2048.0f));
-            lo[j] = __half2float(__float2half_rn(fmaf(hi[j], -2048.0f, X)));
+            hi[j] = rintf(X);
+            lo[j] = __half2float(__float2half_rn(X - hi[j]));
             hsum += hi[j];
             lsum += lo[j];
         }
@@ -663,13 +689,13 @@ __device__ __forceinline__ void wide_image_unit(uint8_t *__restrict__ image, uin
     lsum += __shfl_xor_sync(0xffffffffu, lsum, 2);
     const uint32_t pt = t / np, p = t - pt * np;
     uint8_t *base = image + ((size_t)pt * nkb + unit) * pw_image_unit(np);
-    uint8_t *row = base + (lane >> 3) * (256 * np) + p * 128 + (((lane & 7) ^ (p & 7)) << 4);
-    *reinterpret_cast<uint4 *>(row) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-    *reinterpret_cast<uint4 *>(row + np * 128) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+    uint8_t *row = base + (lane >> 3) * (128 * np) + p * 128 + (((lane & 7) ^ (p & 7)) << 4);
+    *reinterpret_cast<uint4 *>(row) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+    *reinterpret_cast<uint4 *>(row + 512 * np) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
     uint8_t *aux = base + 1024 * np;
     if ((lane & 3) == 0) {
-        // the group's sum over 4096 (at most 2^15), as two f16 digits
-        const float l = lsum * (1.0f / 4096.0f);
+        // half the group's sum (at most 2^15), as two f16 digits
+        const float l = 0.5f * lsum;
         const __half s1 = __float2half_rn(fmaf(hsum, 0.5f, l));
         __half *s = reinterpret_cast<__half *>(aux) + p * 8 + (lane >> 2);
         s[0] = s1;

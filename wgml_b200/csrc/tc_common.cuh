@@ -45,10 +45,13 @@ __device__ __forceinline__ uint32_t tc_idesc(uint32_t n, uint32_t a_signed = 0)
     return (2u << 4) | (a_signed << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
-// One lane of a converged warp, chosen by elect.sync.  MMAs are issued under this predicate and not under `lane == 0`:
-// the compiler then knows that a single thread runs the region and issues each MMA once from uniform registers;
-// under a lane comparison an issue took 70 ns whatever its shape, under this one 46 ns or the tensor pipe's time (four
-// MMAs of N = 176, K = 16: 284 -> 215 ns).
+// MMAs and commits are issued by one lane of a converged warp, chosen by elect.sync (and not by `lane == 0`: the
+// compiler then knows that a single thread runs the region), from operands it can tell to be the same for the whole
+// warp: the instruction takes them from uniform registers, and a value read from shared memory or derived from the
+// thread index is moved there, and waited for, at every issue.  Four MMAs of K = 16, N = 176 took 284 ns under a lane
+// comparison, 215 ns under elect.sync; with uniform operands four of N = 128 (64, 32) take 140 (73, 54) ns, the
+// tensor pipe's own time, and a commit costs nothing on top.
+__device__ __forceinline__ uint32_t tc_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ bool tc_elect()
 {
     uint32_t p;
