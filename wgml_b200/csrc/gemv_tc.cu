@@ -104,11 +104,12 @@ __global__ void __launch_bounds__(TC_NT, 1) gemv_q4k_tc_kernel(const __grid_cons
     uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
     volatile uint32_t *dead = &dead_flag;
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = tc_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const uint32_t nkb = a.K / 256, ntiles = a.nrows / TC_TILE_ROWS;
-    auto bar_full = [&](uint32_t s) { return smem_addr(&bars[s]); };
-    auto bar_empty = [&](uint32_t s) { return smem_addr(&bars[TC_RING + s]); };
-    auto bar_done = [&](uint32_t u) { return smem_addr(&bars[2 * TC_RING + u]); };
+    const uint32_t bar0 = tc_uniform(smem_addr(bars));
+    auto bar_full = [&](uint32_t s) { return bar0 + 8 * s; };
+    auto bar_empty = [&](uint32_t s) { return bar0 + 8 * (TC_RING + s); };
+    auto bar_done = [&](uint32_t u) { return bar0 + 8 * (2 * TC_RING + u); };
     // tiles of this block: blockIdx.x, blockIdx.x + gridDim.x, ...; unit n = column n % nkb of tile n / nkb
     const uint32_t my_tiles = blockIdx.x < ntiles ? (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
     const uint32_t total = my_tiles * nkb;
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(TC_NT, 1) gemv_q4k_tc_kernel(const __grid_cons
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = tmem_base_slot;
+    const uint32_t tmem_base = tc_uniform(tmem_base_slot);
 
     if (warp == 0) {
         // ------------------------------ producer ------------------------------
@@ -151,28 +152,29 @@ __global__ void __launch_bounds__(TC_NT, 1) gemv_q4k_tc_kernel(const __grid_cons
     } else if (warp == 1) {
         // ------------------------------ MMA issue ------------------------------
         // Unit n is complete in its operand buffer once all worker threads have arrived at hardware barrier
-        // 3 + n % 2 (they do not wait there); this warp does wait there, then one thread issues the unit's
+        // 3 + n % 2 (they do not wait there); this warp does wait there, then its elected lane issues the unit's
         // eight MMAs into accumulator columns 128 (n % 2) ... and commits them to the unit's barrier.
-        // The descriptors are worked out once: a single thread issues, and its own instruction stream is what
-        // bounds the rate.  The start-address field is the low 14 bits in units of 16 bytes; the offsets added
+        // The descriptors are worked out once.  The start-address field is the low 14 bits in units of 16 bytes; the offsets added
         // below stay inside it (shared memory ends below 2^18).
         const uint32_t idesc = tc_idesc(16);
-        const uint64_t adesc0 = tc_smem_desc_sw128(smem_addr(smem + TC_OFF_A), 1024);
-        const uint64_t bdesc0 = tc_smem_desc(smem_addr(smem + TC_OFF_B), 128, 0);
+        const uint64_t adesc0 = tc_smem_desc_sw128(tc_uniform(smem_addr(smem + TC_OFF_A)), 1024);
+        const uint64_t bdesc0 = tc_smem_desc(tc_uniform(smem_addr(smem + TC_OFF_B)), 128, 0);
         uint32_t kb = 0;
         for (uint32_t n = 0; n < total; n++) {
             const uint32_t u = n & 1;
             if (u) asm volatile("bar.sync 4, %0;" ::"n"(32 * TC_WORKER_WARPS + 32) : "memory");
             else asm volatile("bar.sync 3, %0;" ::"n"(32 * TC_WORKER_WARPS + 32) : "memory");
-            if (lane == 0 && !*dead) {
+            if (__all_sync(0xffffffffu, !*dead)) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t ad = adesc0 + (uint64_t)(u * (TC_A_BYTES >> 4));
                 const uint64_t bd = bdesc0 + (uint64_t)(kb * ((256 / 16) * 128 >> 4));
                 const uint32_t dcol = tmem_base + u * 128;
+                if (tc_elect()) {
 #pragma unroll
-                for (uint32_t j = 0; j < 8; j++)
-                    tc_mma(dcol + 16 * j, ad + (uint64_t)(((j >> 2) * 16384 + (j & 3) * 32) >> 4), bd + (uint64_t)((j * 256) >> 4), idesc);
-                tc_commit(bar_done(u));
+                    for (uint32_t j = 0; j < 8; j++)
+                        tc_mma(dcol + 16 * j, ad + (uint64_t)(((j >> 2) * 16384 + (j & 3) * 32) >> 4), bd + (uint64_t)((j * 256) >> 4), idesc);
+                    tc_commit(bar_done(u));
+                }
             }
             __syncwarp();
             kb = kb + 1 == nkb ? 0 : kb + 1;

@@ -85,13 +85,14 @@ __global__ void __launch_bounds__(TB_NT, 1) gemm_q4k_tc_kernel(const __grid_cons
     volatile uint32_t *dead = &dead_flag;
 
     pdl_launch_dependents();
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = tc_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const uint32_t nkb = a.nkb, nsplit = a.nsplit, nitems = a.ntiles * nsplit;
-    auto bar_full = [&](uint32_t s) { return smem_addr(&bars[s]); };
-    auto bar_empty = [&](uint32_t s) { return smem_addr(&bars[TB_RING + s]); };
-    auto bar_done = [&](uint32_t u) { return smem_addr(&bars[2 * TB_RING + u]); };        // the unit's MMAs have completed
-    auto bar_tfree = [&](uint32_t u) { return smem_addr(&bars[2 * TB_RING + 2 + u]); };   // its accumulators have been read
-    auto stage = [&](uint32_t s) { return smem_addr(smem + TB_OFF_RING) + s * TB_STAGE; };
+    const uint32_t bar0 = tc_uniform(smem_addr(bars)), ring0 = tc_uniform(smem_addr(smem + TB_OFF_RING));
+    auto bar_full = [&](uint32_t s) { return bar0 + 8 * s; };
+    auto bar_empty = [&](uint32_t s) { return bar0 + 8 * (TB_RING + s); };
+    auto bar_done = [&](uint32_t u) { return bar0 + 8 * (2 * TB_RING + u); };        // the unit's MMAs have completed
+    auto bar_tfree = [&](uint32_t u) { return bar0 + 8 * (2 * TB_RING + 2 + u); };   // its accumulators have been read
+    auto stage = [&](uint32_t s) { return ring0 + s * TB_STAGE; };
     uint32_t total = 0;
     for (uint32_t i = blockIdx.x; i < nitems; i += gridDim.x) {
         const uint32_t sp = i % nsplit;
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(TB_NT, 1) gemm_q4k_tc_kernel(const __grid_cons
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = tmem_base_slot;
+    const uint32_t tmem_base = tc_uniform(tmem_base_slot);
     // barriers and tensor memory are set up while the preceding launch (which writes the image) still runs
     pdl_wait();
 
@@ -142,26 +143,26 @@ __global__ void __launch_bounds__(TB_NT, 1) gemm_q4k_tc_kernel(const __grid_cons
     } else if (warp == 1) {
         // ------------------------------ MMA issue ------------------------------
         // Unit n is complete in operand buffer n % 2 once all unpacking threads have arrived at hardware barrier
-        // 3 + n % 2 (they do not wait there); this warp waits there, then one thread -- once the accumulators of
+        // 3 + n % 2 (they do not wait there); this warp waits there, then its elected lane -- once the accumulators of
         // unit n - 2 have been read -- issues the unit's eight MMAs into accumulator columns 256 (n % 2) ... and
         // commits them to the unit's barrier.  The B operand is read in place from the unit's stage (K-major, no
         // swizzle: core matrices of eight positions x 16 columns, the four row groups of a K-core 128 bytes apart,
         // K-cores 512 bytes apart).
         const uint32_t idesc = tc_idesc(32);
-        const uint64_t adesc0 = tc_smem_desc_sw128(smem_addr(smem + TB_OFF_A), 1024);
+        const uint64_t adesc0 = tc_smem_desc_sw128(tc_uniform(smem_addr(smem + TB_OFF_A)), 1024);
         bool ok = true;
         for (uint32_t n = 0; n < total; n++) {
             const uint32_t u = n & 1, s = n % TB_RING;
             if (u) asm volatile("bar.sync 4, %0;" ::"n"(32 * TB_UNPACK_WARPS + 32) : "memory");
             else asm volatile("bar.sync 3, %0;" ::"n"(32 * TB_UNPACK_WARPS + 32) : "memory");
-            if (lane == 0 && ok && !*dead) {
-                ok = tc_wait(bar_full(s), (n / TB_RING) & 1, dead, a.err, 22);
-                if (ok && n >= 2) ok = tc_wait(bar_tfree(u), ((n - 2) >> 1) & 1, dead, a.err, 25);
-                if (ok) {
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t ad = adesc0 + (uint64_t)(u * (TC_A_BYTES >> 4));
-                    const uint64_t bd = tc_smem_desc(stage(s), 512, 128);
-                    const uint32_t dcol = tmem_base + u * 256;
+            if (ok) ok = __all_sync(0xffffffffu, !*dead && tc_wait(bar_full(s), (n / TB_RING) & 1, dead, a.err, 22) &&
+                                                     (n < 2 || tc_wait(bar_tfree(u), ((n - 2) >> 1) & 1, dead, a.err, 25)));
+            if (ok) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t ad = adesc0 + (uint64_t)(u * (TC_A_BYTES >> 4));
+                const uint64_t bd = tc_smem_desc(stage(s), 512, 128);
+                const uint32_t dcol = tmem_base + u * 256;
+                if (tc_elect()) {
 #pragma unroll
                     for (uint32_t j = 0; j < 8; j++)
                         tc_mma(dcol + 32 * j, ad + (uint64_t)(((j >> 2) * 16384 + (j & 3) * 32) >> 4), bd + (uint64_t)((j * 1024) >> 4), idesc);

@@ -64,13 +64,14 @@ __global__ void __launch_bounds__(T6_NT, 1) gemm_q6k_tc_kernel(const __grid_cons
     volatile uint32_t *dead = &dead_flag;
 
     pdl_launch_dependents();
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = tc_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const uint32_t nkb = a.nkb, nsplit = a.nsplit, nitems = (a.nrows / TC_TILE_ROWS) * nsplit;
-    auto bar_full = [&](uint32_t s) { return smem_addr(&bars[s]); };
-    auto bar_empty = [&](uint32_t s) { return smem_addr(&bars[T6_RING + s]); };
-    auto bar_done = [&](uint32_t u) { return smem_addr(&bars[2 * T6_RING + u]); };        // the unit's MMAs have completed
-    auto bar_tfree = [&](uint32_t u) { return smem_addr(&bars[2 * T6_RING + 2 + u]); };   // its accumulators have been read
-    auto stage = [&](uint32_t s) { return smem_addr(smem + T6_OFF_RING) + s * T6_STAGE; };
+    const uint32_t bar0 = tc_uniform(smem_addr(bars)), ring0 = tc_uniform(smem_addr(smem + T6_OFF_RING));
+    auto bar_full = [&](uint32_t s) { return bar0 + 8 * s; };
+    auto bar_empty = [&](uint32_t s) { return bar0 + 8 * (T6_RING + s); };
+    auto bar_done = [&](uint32_t u) { return bar0 + 8 * (2 * T6_RING + u); };        // the unit's MMAs have completed
+    auto bar_tfree = [&](uint32_t u) { return bar0 + 8 * (2 * T6_RING + 2 + u); };   // its accumulators have been read
+    auto stage = [&](uint32_t s) { return ring0 + s * T6_STAGE; };
     uint32_t total = 0;
     for (uint32_t i = blockIdx.x; i < nitems; i += gridDim.x) {
         const uint32_t sp = i % nsplit;
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(T6_NT, 1) gemm_q6k_tc_kernel(const __grid_cons
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = tmem_base_slot;
+    const uint32_t tmem_base = tc_uniform(tmem_base_slot);
     // barriers and tensor memory are set up while the preceding launch (which writes the image) still runs
     pdl_wait();
 
@@ -124,25 +125,29 @@ __global__ void __launch_bounds__(T6_NT, 1) gemm_q6k_tc_kernel(const __grid_cons
         // place from the stage: K-major, no swizzle, core matrices of eight vectors x 16 columns, K-cores 128 bytes
         // apart, the digits (row groups) 2 KB apart.
         const uint32_t idesc_lo = tc_idesc(32, 0), idesc_hi = tc_idesc(32, 1);
-        const uint64_t adesc0 = tc_smem_desc_sw128(smem_addr(smem), 1024);
+        const uint64_t adesc0 = tc_smem_desc_sw128(tc_uniform(smem_addr(smem)), 1024);
+        bool ok = true;
         for (uint32_t n = 0; n < total; n++) {
             const uint32_t u = n & 1, s = n % T6_RING;
             if (u) asm volatile("bar.sync 4, %0;" ::"n"(32 * T6_WORKER_WARPS + 32) : "memory");
             else asm volatile("bar.sync 3, %0;" ::"n"(32 * T6_WORKER_WARPS + 32) : "memory");
-            if (lane == 0 && !*dead && tc_wait(bar_full(s), (n / T6_RING) & 1, dead, a.err, 32) &&
-                (n < 2 || tc_wait(bar_tfree(u), ((n - 2) >> 1) & 1, dead, a.err, 35))) {   // the accumulators of unit n - 2 have been read
+            if (ok) ok = __all_sync(0xffffffffu, !*dead && tc_wait(bar_full(s), (n / T6_RING) & 1, dead, a.err, 32) &&
+                                                     (n < 2 || tc_wait(bar_tfree(u), ((n - 2) >> 1) & 1, dead, a.err, 35)));   // the accumulators of unit n - 2 have been read
+            if (ok) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t bd = tc_smem_desc(stage(s), 128, 2048);
                 const uint32_t dcol = tmem_base + u * 64;
+                if (tc_elect()) {
 #pragma unroll
-                for (uint32_t plane = 0; plane < 2; plane++) {
-                    const uint64_t ad = adesc0 + (uint64_t)((u * T6_A_BYTES + plane * TC_A_BYTES) >> 4);
+                    for (uint32_t plane = 0; plane < 2; plane++) {
+                        const uint64_t ad = adesc0 + (uint64_t)((u * T6_A_BYTES + plane * TC_A_BYTES) >> 4);
 #pragma unroll
-                    for (uint32_t j = 0; j < 8; j++)
-                        tc_mma_acc(dcol + 32 * plane, ad + (uint64_t)(((j >> 2) * 16384 + (j & 3) * 32) >> 4), bd + (uint64_t)((j * 256) >> 4),
-                                   plane ? idesc_hi : idesc_lo, j ? 1u : 0u);
+                        for (uint32_t j = 0; j < 8; j++)
+                            tc_mma_acc(dcol + 32 * plane, ad + (uint64_t)(((j >> 2) * 16384 + (j & 3) * 32) >> 4), bd + (uint64_t)((j * 256) >> 4),
+                                       plane ? idesc_hi : idesc_lo, j ? 1u : 0u);
+                    }
+                    tc_commit(bar_done(u));
                 }
-                tc_commit(bar_done(u));
             }
             __syncwarp();
         }

@@ -49,13 +49,14 @@ __global__ void __launch_bounds__(T8_NT, 1) gemm_q80_tc_kernel(const __grid_cons
     volatile uint32_t *dead = &dead_flag;
 
     pdl_launch_dependents();
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = tc_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const uint32_t nkb = a.nkb, nsplit = a.nsplit, nitems = (a.nrows / TC_TILE_ROWS) * nsplit;
-    auto bar_full = [&](uint32_t s) { return smem_addr(&bars[s]); };
-    auto bar_empty = [&](uint32_t s) { return smem_addr(&bars[T8_RING + s]); };
-    auto bar_done = [&](uint32_t u) { return smem_addr(&bars[2 * T8_RING + u]); };        // the unit's MMAs have completed
-    auto bar_tfree = [&](uint32_t u) { return smem_addr(&bars[2 * T8_RING + 2 + u]); };   // its accumulators have been read
-    auto stage = [&](uint32_t s) { return smem_addr(smem) + s * T8_STAGE; };
+    const uint32_t bar0 = tc_uniform(smem_addr(bars)), ring0 = tc_uniform(smem_addr(smem));
+    auto bar_full = [&](uint32_t s) { return bar0 + 8 * s; };
+    auto bar_empty = [&](uint32_t s) { return bar0 + 8 * (T8_RING + s); };
+    auto bar_done = [&](uint32_t u) { return bar0 + 8 * (2 * T8_RING + u); };        // the unit's MMAs have completed
+    auto bar_tfree = [&](uint32_t u) { return bar0 + 8 * (2 * T8_RING + 2 + u); };   // its accumulators have been read
+    auto stage = [&](uint32_t s) { return ring0 + s * T8_STAGE; };
     uint32_t total = 0;
     for (uint32_t i = blockIdx.x; i < nitems; i += gridDim.x) {
         const uint32_t sp = i % nsplit;
@@ -81,7 +82,7 @@ __global__ void __launch_bounds__(T8_NT, 1) gemm_q80_tc_kernel(const __grid_cons
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = tmem_base_slot;
+    const uint32_t tmem_base = tc_uniform(tmem_base_slot);
     // barriers and tensor memory are set up while the preceding launch (which writes the image) still runs
     pdl_wait();
 
@@ -103,29 +104,29 @@ __global__ void __launch_bounds__(T8_NT, 1) gemm_q80_tc_kernel(const __grid_cons
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issue ------------------------------
-        // One thread: as soon as unit n's stage is full and the accumulators of unit n - 2 have been read, eight
+        // As soon as unit n's stage is full and the accumulators of unit n - 2 have been read, eight
         // MMAs (A: the stage's codes, 128-byte swizzle; B: the stage's slice of the image, K-major without swizzle,
         // the four row groups of a K-core 128 bytes apart, K-cores 512 bytes apart) into columns 256 (n % 2) ...,
         // committed to the unit's barrier.
-        if (lane == 0) {
-            const uint32_t idesc = tc_idesc(32, 1);
-            bool ok = true;
-            for (uint32_t n = 0; n < total && ok; n++) {
-                const uint32_t u = n & 1, s = n % T8_RING;
-                ok = tc_wait(bar_full(s), (n / T8_RING) & 1, dead, a.err, 42);
-                if (ok && n >= 2) ok = tc_wait(bar_tfree(u), ((n - 2) >> 1) & 1, dead, a.err, 45);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t ad = tc_smem_desc_sw128(stage(s), 1024);
-                const uint64_t bd = tc_smem_desc(stage(s) + T8_UNIT_BYTES, 512, 128);
-                const uint32_t dcol = tmem_base + u * 256;
+        const uint32_t idesc = tc_idesc(32, 1);
+        bool ok = true;
+        for (uint32_t n = 0; n < total && ok; n++) {
+            const uint32_t u = n & 1, s = n % T8_RING;
+            ok = __all_sync(0xffffffffu, tc_wait(bar_full(s), (n / T8_RING) & 1, dead, a.err, 42) &&
+                                             (n < 2 || tc_wait(bar_tfree(u), ((n - 2) >> 1) & 1, dead, a.err, 45)));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t ad = tc_smem_desc_sw128(stage(s), 1024);
+            const uint64_t bd = tc_smem_desc(stage(s) + T8_UNIT_BYTES, 512, 128);
+            const uint32_t dcol = tmem_base + u * 256;
+            if (tc_elect()) {
 #pragma unroll
                 for (uint32_t j = 0; j < 8; j++)
                     tc_mma(dcol + 32 * j, ad + (uint64_t)(((j >> 2) * 16384 + (j & 3) * 32) >> 4), bd + (uint64_t)((j * 1024) >> 4), idesc);
                 tc_commit(bar_done(u));
             }
+            __syncwarp();
         }
-        __syncwarp();
     } else {
         // ------------------------------ finishing ------------------------------
         // Thread (quarter, lane, half): row r = 32 quarter + lane (the quarter of tensor memory its warp may read),
