@@ -399,12 +399,11 @@ WGB_EXPORT int wgb_gemm_q4k_tiles(wgb_q4k_tiles *m, const float *d_v, size_t n_v
         m->image = image;
         m->part = part;
     }
-    WGB_CUDA(cudaMemsetAsync(d_out, 0, n_vec * m->nrows * sizeof(float), st));
     // image of the inputs (they are not written: no slices are folded into them)
     int rc = launch_prefill_norm_image(const_cast<float *>(d_v), m->ncols, nullptr, 0, 0, nullptr, 0.0f, m->ncols, (uint32_t)n_vec, m->image, nullptr, 0, st);
-    if (!rc) rc = launch_gemm_q4k_tiles(m->w, m->nrows, m->ncols, m->image, (uint32_t)n_vec, m->part, m->nrows, ns, st);
-    // d_out (zero) += the slices
-    if (!rc) rc = launch_prefill_norm_image(d_out, m->nrows, m->part, ns, m->nrows, nullptr, 0.0f, m->nrows, (uint32_t)n_vec, nullptr, nullptr, 0, st);
+    // a product in one slice is written in place
+    if (!rc) rc = launch_gemm_q4k_tiles(m->w, m->nrows, m->ncols, m->image, (uint32_t)n_vec, ns == 1 ? d_out : m->part, m->nrows, ns, st);
+    if (!rc && ns > 1) rc = launch_prefill_fold(m->part, ns, m->nrows, (uint32_t)n_vec, d_out, st);
     return rc;
 }
 

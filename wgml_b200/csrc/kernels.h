@@ -183,6 +183,8 @@ int launch_gemm_q4k_tiles_multi(uint32_t nmat, const uint8_t *const *w_tiles, co
 // of the result and, with xn, the values.  With neither image nor xn only x is updated.
 int launch_prefill_norm_image(float *x, uint32_t x_stride, const float *part, uint32_t nsplit, uint32_t part_stride, const float *norm_w,
                               float eps, uint32_t K, uint32_t ntok, uint8_t *image, float *xn, uint32_t xn_stride, cudaStream_t stream);
+// out[t][row] = the slices [slice][PF_TOK][nrows] of a product added up.
+int launch_prefill_fold(const float *part, uint32_t nsplit, uint32_t nrows, uint32_t ntok, float *out, cudaStream_t stream);
 int launch_prefill_silu_image(const float *gate, uint32_t gsplit, const float *up, uint32_t usplit, uint32_t stride, uint32_t K,
                               uint32_t ntok, uint8_t *image, float *h, uint32_t h_stride, cudaStream_t stream);
 // The Q6_K counterparts (prefill_q6k.cu): the scale is folded into a two-plane weight operand and a super-block's

@@ -953,6 +953,23 @@ int launch_prefill_attention(const float *q, const float *k_cache, const float *
     return launch_prefill_attention_tq<2>(q, k_cache, v_cache, out, n_heads, head_size, kv_mul, row_stride, head_stride, pos0, ntok, image, scratch, counters, chunks, stream);
 }
 
+// out[t][i] = the slices of a product added up (the stand-alone products' last step; out has no alignment to rely on).
+__global__ void __launch_bounds__(256) prefill_fold_kernel(const float *__restrict__ part, uint32_t nsplit, uint32_t nrows, float *__restrict__ out)
+{
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x, t = blockIdx.y;
+    if (i >= nrows) return;
+    float v = part[(size_t)t * nrows + i];
+    for (uint32_t s = 1; s < nsplit; s++) v += part[((size_t)s * PF_TOK + t) * nrows + i];
+    out[(size_t)t * nrows + i] = v;
+}
+int launch_prefill_fold(const float *part, uint32_t nsplit, uint32_t nrows, uint32_t ntok, float *out, cudaStream_t stream)
+{
+    WGB_CUDA(launch_pdl(prefill_fold_kernel, dim3((nrows + 255) / 256, ntok), dim3(256), 0, stream, part, nsplit, nrows, out));
+    return WGB_OK;
+}
+
 // Raw row-major Q4_K blocks -> [tile][column][row in tile][144 bytes].  One thread per 16 bytes.
 __global__ void prefill_tile_major_kernel(const uint4 *__restrict__ raw, uint4 *__restrict__ tiled, uint32_t nrows, uint32_t nkb)
 {

@@ -467,10 +467,9 @@ WGB_EXPORT int wgb_gemm_q6k_tiles(wgb_q6k_tiles *m, const float *d_v, size_t n_v
         m->image = image;
         m->part = part;
     }
-    WGB_CUDA(cudaMemsetAsync(d_out, 0, n_vec * m->nrows * sizeof(float), st));
     int rc = launch_prefill_image6(d_v, m->ncols, m->ncols, (uint32_t)n_vec, m->image, st);
-    if (!rc) rc = launch_gemm_q6k_tiles(m->w, m->nrows, m->ncols, m->image, (uint32_t)n_vec, m->part, m->nrows, ns, st);
-    // d_out (zero) += the slices
-    if (!rc) rc = launch_prefill_norm_image(d_out, m->nrows, m->part, ns, m->nrows, nullptr, 0.0f, m->nrows, (uint32_t)n_vec, nullptr, nullptr, 0, st);
+    // a product in one slice is written in place
+    if (!rc) rc = launch_gemm_q6k_tiles(m->w, m->nrows, m->ncols, m->image, (uint32_t)n_vec, ns == 1 ? d_out : m->part, m->nrows, ns, st);
+    if (!rc && ns > 1) rc = launch_prefill_fold(m->part, ns, m->nrows, (uint32_t)n_vec, d_out, st);
     return rc;
 }

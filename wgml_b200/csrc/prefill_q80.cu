@@ -351,9 +351,9 @@ WGB_EXPORT int wgb_gemm_q80_tiles(wgb_q80_tiles *m, const float *d_v, size_t n_v
         m->image = image;
         m->part = part;
     }
-    WGB_CUDA(cudaMemsetAsync(d_out, 0, n_vec * m->nrows * sizeof(float), st));
     int rc = launch_prefill_norm_image(const_cast<float *>(d_v), m->ncols, nullptr, 0, 0, nullptr, 0.0f, m->ncols, (uint32_t)n_vec, m->image, nullptr, 0, st);
-    if (!rc) rc = launch_gemm_q80_tiles(m->w, m->nrows, m->ncols, m->image, (uint32_t)n_vec, m->part, m->nrows, ns, st);
-    if (!rc) rc = launch_prefill_norm_image(d_out, m->nrows, m->part, ns, m->nrows, nullptr, 0.0f, m->nrows, (uint32_t)n_vec, nullptr, nullptr, 0, st);
+    // a product in one slice is written in place
+    if (!rc) rc = launch_gemm_q80_tiles(m->w, m->nrows, m->ncols, m->image, (uint32_t)n_vec, ns == 1 ? d_out : m->part, m->nrows, ns, st);
+    if (!rc && ns > 1) rc = launch_prefill_fold(m->part, ns, m->nrows, (uint32_t)n_vec, d_out, st);
     return rc;
 }
