@@ -52,6 +52,9 @@ def test_split_kernel_shapes(case):
     (4224, 96, 128, 12, 1500),   # twelve: two groups of eight (tail masked)
     (8256, 64, 64, 8, 8200),     # head size 64: half of the lanes idle
     (8256, 24, 96, 1, 5000),     # head size 96
+    (4224, 64, 128, 8, 2047), (4224, 64, 128, 8, 2048),   # grouped streaming kernel: last chunk full, one position in it
+    (4224, 64, 128, 8, 1300),    # a little more than a chunk per block: runs of one and two chunks
+    (8256, 32, 96, 4, 7001),     # four heads per KV head, a quarter of the lanes idle
     (4224, 64, 128, 8, 0),       # only the first chunk holds anything, and only one position
     (4224, 64, 128, 8, 63), (4224, 64, 128, 8, 64), (4224, 64, 128, 8, 130),
 ])

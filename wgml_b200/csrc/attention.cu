@@ -10,8 +10,8 @@
 // finishes last for a KV head (an atomic ticket, nobody waits) merges the chunks.  K and V rows
 // are read once for all kv_mul query heads.
 //
-// Long contexts (more chunks than blocks fit in one wave) take the streaming kernel further down: one block
-// per SM walks a run of chunks with a producer warp feeding K / V tiles through shared memory.
+// Streaming kernel and row-streaming kernel, further down: one block per SM walks a run of the cache rows and keeps the
+// running softmax per warp; launch_split says which launch takes which.
 //
 // Full kernel (API path that returns the attention weights): one block per query head, the
 // probabilities are materialised in the caller's [n_heads][seq_len] buffer.
@@ -500,10 +500,10 @@ __global__ void __launch_bounds__(ATT_NT) attn_full_kernel(const __grid_constant
 }
 
 // ---------------------------------------------------------------------------------------------
-// Streaming kernel (long contexts; head sizes up to 128).  Grid (splits, KV heads, query-head groups) with
+// Streaming kernel (long contexts; head sizes up to 128; cache rows of a head contiguous).  Grid (splits, KV heads, query-head groups) with
 // one block per SM; a block owns a run of 64-position chunks of one KV head and all QH query heads that
 // share it.  A producer warp streams the K and V rows of chunk after chunk into a two-stage ring of shared
-// memory with bulk asynchronous copies (one per cache row, completion on an mbarrier), so the DRAM round
+// memory with bulk asynchronous copies (one per tile, completion on an mbarrier), so the DRAM round
 // trip of the next chunk overlaps the arithmetic of the current one; eight consumer warps score the chunk
 // (8 positions per warp); each warp keeps its own running softmax and weighted value sum over its positions,
 // so nothing inside the loop synchronises the warps, and the eight are merged once at the end.  The block's
@@ -564,16 +564,9 @@ __global__ void __launch_bounds__(ATS_NT, 1) attn_stream_kernel(const __grid_con
             const float *kbase = a.k_cache + (size_t)t0 * rstr + (size_t)kvh * hstr;
             const float *vbase = a.v_cache + (size_t)t0 * rstr + (size_t)kvh * hstr;
             const uint32_t dst = ring + s * stage_bytes;
-            if (rstr == hs) {
-                // head-major cache: the rows of the chunk are one contiguous run, one copy per tile
-                if (lane == 0) bulk_copy_g2s(dst, kbase, nt * row_bytes, full0 + 8 * s);
-                if (lane == 1) bulk_copy_g2s(dst + tile_bytes, vbase, nt * row_bytes, full0 + 8 * s);
-            } else {
-                for (uint32_t r = lane; r < nt; r += 32) {
-                    bulk_copy_g2s(dst + r * row_bytes, kbase + (size_t)r * rstr, row_bytes, full0 + 8 * s);
-                    bulk_copy_g2s(dst + tile_bytes + r * row_bytes, vbase + (size_t)r * rstr, row_bytes, full0 + 8 * s);
-                }
-            }
+            // the rows of the chunk are one contiguous run, one copy per tile
+            if (lane == 0) bulk_copy_g2s(dst, kbase, nt * row_bytes, full0 + 8 * s);
+            if (lane == 1) bulk_copy_g2s(dst + tile_bytes, vbase, nt * row_bytes, full0 + 8 * s);
         }
         return;
     }
@@ -791,6 +784,269 @@ __global__ void __launch_bounds__(ATS_NT, 1) attn_stream_kernel(const __grid_con
     if (threadIdx.x == 0) stamp_end(a.stamp);
 }
 
+// Row-streaming kernel (head sizes up to 128; one, two, four or eight query heads per KV head).  Grid (splits, KV heads),
+// one block of eight warps per SM; a block owns a run of the KV head's cache rows in groups of eight, a warp every
+// eighth group of the run.  A warp requests its groups itself (asynchronous 16-byte copies, ATR_STAGES groups in
+// flight per warp, 192 KB per SM), scores them for all query heads that share the KV head and keeps its own running
+// softmax and value sums, so nothing inside the loop synchronises warps or touches a barrier.
+// Bound by the cache with few query heads (32 heads on 32, 4000 positions: 131 MB in 29 us, 4.5 TB/s), by instructions
+// with eight (64 on 8: 22 us for 33 MB).  Rows may lie anywhere: with the reference layout ([seq_len][kv_dim])
+// a row of one head is 512 bytes, and a producer warp with one bulk copy per row was bound by the rate at which those are
+// issued (68 us; with eight heads, the cache read by two blocks per KV head of the split kernel, 29 us).
+constexpr int ATR_STAGES = 3;
+__device__ __forceinline__ void atr_copy16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+
+template <int QH>
+__global__ void __launch_bounds__(ATT_NT, 1) attn_rows_kernel(const __grid_constant__ AttnArgs a)
+{
+    extern __shared__ uint4 ring4[];   // [warp][stage][K | V][ATT_TPW rows][hs floats]
+    __shared__ float s_sc[ATT_WARPS][QH][ATT_TPW];
+    __shared__ float s_red[QH][ATT_WARPS], s_sum[QH][ATT_WARPS];
+    __shared__ uint32_t s_last;
+
+    const uint32_t pos = a.pos ? *a.pos : a.p.pos;   // written by an earlier step: readable before the wait
+    const uint32_t hs = a.p.head_size, kv_mul = a.p.kv_mul;
+    const uint32_t rstr = a.row_stride ? a.row_stride : a.p.kv_dim, hstr = a.row_stride ? a.head_stride : hs;
+    const uint32_t split = blockIdx.x, kvh = blockIdx.y, max_splits = gridDim.x;
+    const uint32_t ngroups = pos / ATT_TPW + 1, nsplit_active = min(ngroups, max_splits);   // runs as equal as they can be
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    pdl_launch_dependents();
+    if (split >= nsplit_active) {
+        if (threadIdx.x == 0) stamp_end(a.stamp);
+        return;
+    }
+    const uint32_t g_begin = (uint32_t)((uint64_t)split * ngroups / nsplit_active), g_end = (uint32_t)((uint64_t)(split + 1) * ngroups / nsplit_active);
+    const uint32_t nchunk = hs / 4;   // float4 chunks per head (at most 32: one per lane)
+    const bool on = (uint32_t)lane < nchunk;
+    const uint32_t row_bytes = hs * 4, half = ATT_TPW * row_bytes, stage_bytes = 2 * half;
+    const uint32_t ring = smem_addr(ring4) + warp * ATR_STAGES * stage_bytes;
+    const float *kh = a.k_cache + (size_t)kvh * hstr + 4 * lane, *vh = a.v_cache + (size_t)kvh * hstr + 4 * lane;
+    auto request = [&](uint32_t g, uint32_t st) {
+        if (g < g_end && on) {
+            const uint32_t dst = ring + st * stage_bytes + 16 * lane, t0 = g * ATT_TPW;
+#pragma unroll
+            for (int i = 0; i < ATT_TPW; i++) {
+                if (t0 + i <= pos) {
+                    atr_copy16(dst + i * row_bytes, kh + (size_t)(t0 + i) * rstr);
+                    atr_copy16(dst + half + i * row_bytes, vh + (size_t)(t0 + i) * rstr);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");   // one group per stage and lane, empty or not
+    };
+    // Every row before `pos` was written by an earlier step and is requested before the wait for the preceding launch,
+    // which writes the row of `pos`.
+    const uint32_t g0 = g_begin + warp;
+    const bool early = (g0 + (ATR_STAGES - 1) * ATT_WARPS) < ngroups - 1;
+    if (!early) pdl_wait();
+#pragma unroll
+    for (int st = 0; st < ATR_STAGES; st++) request(g0 + st * ATT_WARPS, st);
+    if (early) pdl_wait();
+
+    const float inv_sqrt = sqrtf((float)hs);
+    float4 q[QH], acc[QH];
+    float M[QH], L[QH];
+#pragma unroll
+    for (int j = 0; j < QH; j++) {
+        q[j] = on ? __ldcg(reinterpret_cast<const float4 *>(a.q + (size_t)(kvh * kv_mul + j) * hs) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+        M[j] = -INFINITY;
+        L[j] = 0.0f;
+        acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float *my_sc = &s_sc[warp][0][0];
+    uint32_t st = 0;
+    for (uint32_t g = g0; g < g_end; g += ATT_WARPS) {
+        const uint32_t t0 = g * ATT_TPW, nt = min((uint32_t)ATT_TPW, pos + 1 - t0), src = ring + st * stage_bytes + 16 * lane;
+        asm volatile("cp.async.wait_group %0;" ::"n"(ATR_STAGES - 1) : "memory");   // a lane reads back only what it copied
+        float4 rows[ATT_TPW];
+        auto fetch = [&](uint32_t base) {
+#pragma unroll
+            for (int i = 0; i < ATT_TPW; i++) {
+                rows[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (on && (uint32_t)i < nt)
+                    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
+                                 : "=f"(rows[i].x), "=f"(rows[i].y), "=f"(rows[i].z), "=f"(rows[i].w)
+                                 : "r"(base + i * row_bytes)
+                                 : "memory");
+            }
+        };
+        fetch(src);
+#pragma unroll
+        for (int j = 0; j < QH; j++) {
+            float part[ATT_TPW];
+#pragma unroll
+            for (int i = 0; i < ATT_TPW; i++) part[i] = q[j].x * rows[i].x + q[j].y * rows[i].y + q[j].z * rows[i].z + q[j].w * rows[i].w;
+            // 8 sums over the warp at once (8 -> 4 -> 2 -> 1 values per lane, then two plain steps)
+#pragma unroll
+            for (int s = 16; s > 2; s >>= 1) {
+                const bool up = lane & s;
+#pragma unroll
+                for (int i = 0; i < s / 4; i++) {
+                    const float keep = up ? part[2 * i + 1] : part[2 * i], give = up ? part[2 * i] : part[2 * i + 1];
+                    part[i] = keep + __shfl_xor_sync(0xffffffffu, give, s);
+                }
+            }
+            float f1 = part[0];
+            f1 += __shfl_xor_sync(0xffffffffu, f1, 2);
+            f1 += __shfl_xor_sync(0xffffffffu, f1, 1);
+            if ((lane & 3) == 0) {
+                const uint32_t i = ((lane >> 4) & 1) | (((lane >> 3) & 1) << 1) | (((lane >> 2) & 1) << 2);
+                my_sc[j * ATT_TPW + i] = i < nt ? f1 / inv_sqrt : -INFINITY;
+            }
+        }
+        __syncwarp();
+        fetch(src + half);   // the value rows take the registers of the key rows
+#pragma unroll
+        for (int j = 0; j < QH; j++) {
+            const float sv = my_sc[j * ATT_TPW + (lane & 7)];   // lane l looks after position l % 8
+            float m = sv;
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+            const float mn = fmaxf(M[j], m);          // finite: position 0 of the group is valid
+            const float rs = expf(M[j] - mn);         // 0 at the warp's first group (M = -inf)
+            const float e = expf(sv - mn);            // 0 for positions past the end
+            M[j] = mn;
+            float psum = 0.0f;
+            acc[j].x *= rs;
+            acc[j].y *= rs;
+            acc[j].z *= rs;
+            acc[j].w *= rs;
+#pragma unroll
+            for (int i = 0; i < ATT_TPW; i++) {
+                const float p = __shfl_sync(0xffffffffu, e, i);
+                psum += p;
+                acc[j].x = fmaf(p, rows[i].x, acc[j].x);
+                acc[j].y = fmaf(p, rows[i].y, acc[j].y);
+                acc[j].z = fmaf(p, rows[i].z, acc[j].z);
+                acc[j].w = fmaf(p, rows[i].w, acc[j].w);
+            }
+            L[j] = fmaf(L[j], rs, psum);
+        }
+        __syncwarp();   // the scores are rewritten by the next group
+        request(g + ATR_STAGES * ATT_WARPS, st);
+        st = st + 1 == ATR_STAGES ? 0 : st + 1;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+
+    // Merge of the eight warps: all copies have landed and been consumed, the ring now holds their vectors.
+    float *s_acc = reinterpret_cast<float *>(ring4);   // [ATT_WARPS][QH][hs + 4]
+    const uint32_t astr = hs + 4;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < QH; j++) {
+        if (on) reinterpret_cast<float4 *>(s_acc + ((size_t)warp * QH + j) * astr)[lane] = acc[j];
+        if (lane == 0) {
+            s_red[j][warp] = M[j];
+            s_sum[j][warp] = L[j];
+        }
+    }
+    __syncthreads();
+    for (uint32_t e = threadIdx.x; e < QH * hs; e += ATT_NT) {
+        const uint32_t j = e / hs, i = e % hs;
+        float mb = s_red[j][0];
+#pragma unroll
+        for (int w = 1; w < ATT_WARPS; w++) mb = fmaxf(mb, s_red[j][w]);
+        float sv = 0.0f, lb = 0.0f;
+#pragma unroll
+        for (int w = 0; w < ATT_WARPS; w++) {
+            const float f = expf(s_red[j][w] - mb);   // 0 for a warp that had no positions
+            sv = fmaf(s_acc[((size_t)w * QH + j) * astr + i], f, sv);
+            lb = fmaf(s_sum[j][w], f, lb);
+        }
+        float *dst = a.scratch + ((size_t)(kvh * kv_mul + j) * max_splits + split) * astr;
+        dst[i] = sv;
+        if (i == 0) {
+            dst[hs] = mb;
+            dst[hs + 1] = lb;
+        }
+    }
+
+    // Ticket: the last block of this KV head merges the splits, in their order, a head per warp (fewer heads than warps:
+    // the splits of a head dealt to 8 / QH warps).
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const uint32_t ticket = atomicAdd(a.counters + kvh, 1u);
+        s_last = (ticket == nsplit_active - 1);
+        if (s_last) a.counters[kvh] = 0;  // ready for the next launch
+    }
+    __syncthreads();
+    if (!s_last) {
+        if (threadIdx.x == 0) stamp_end(a.stamp);
+        return;
+    }
+    __threadfence();
+    constexpr uint32_t WPH = ATT_WARPS / QH;
+    const uint32_t j = warp % QH, part = warp / QH;
+    const float *base = a.scratch + (size_t)(kvh * kv_mul + j) * max_splits * astr;
+    float Mj = -INFINITY;
+    for (uint32_t sp = lane; sp < nsplit_active; sp += 32) Mj = fmaxf(Mj, __ldcg(base + (size_t)sp * astr + hs));
+    Mj = warp_max(Mj);
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    float Lt = 0.0f;
+#pragma unroll 8
+    for (uint32_t sp = part; sp < nsplit_active; sp += WPH) {
+        const float *row = base + (size_t)sp * astr;
+        const float4 v = on ? __ldcg(reinterpret_cast<const float4 *>(row) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float wgt = expf(__ldcg(row + hs) - Mj);
+        Lt = fmaf(__ldcg(row + hs + 1), wgt, Lt);
+        o.x = fmaf(v.x, wgt, o.x);
+        o.y = fmaf(v.y, wgt, o.y);
+        o.z = fmaf(v.z, wgt, o.z);
+        o.w = fmaf(v.w, wgt, o.w);
+    }
+    if constexpr (WPH > 1) {
+        if (on) reinterpret_cast<float4 *>(s_acc + ((size_t)warp) * astr)[lane] = o;
+        if (lane == 0) s_sum[j][part] = Lt;
+        __syncthreads();
+        if (part) return;
+        o = make_float4(0.f, 0.f, 0.f, 0.f);
+        Lt = 0.0f;
+#pragma unroll
+        for (uint32_t p = 0; p < WPH; p++) {
+            Lt += s_sum[j][p];
+            if (on) {
+                const float4 v = reinterpret_cast<const float4 *>(s_acc + ((size_t)(p * QH + j)) * astr)[lane];
+                o.x += v.x; o.y += v.y; o.z += v.z; o.w += v.w;
+            }
+        }
+    }
+    if (on) reinterpret_cast<float4 *>(a.xb + (size_t)(kvh * kv_mul + j) * hs)[lane] = make_float4(o.x / Lt, o.y / Lt, o.z / Lt, o.w / Lt);
+    if (threadIdx.x == 0) stamp_end(a.stamp);
+}
+
+template <int QH>
+static int launch_rows(const AttnArgs &a, uint32_t nchunks, cudaStream_t stream, bool pdl)
+{
+    const size_t smem = (size_t)ATT_WARPS * ATR_STAGES * 2 * ATT_TPW * a.p.head_size * sizeof(float);
+    static bool ready[MAX_DEVICES] = {};   // per instantiation and device
+    const int dev = current_device();
+    if (dev < 0) return WGB_ERR_CUDA;
+    if (!ready[dev]) {
+        WGB_CUDA(cudaFuncSetAttribute(attn_rows_kernel<QH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(ATT_WARPS * ATR_STAGES * 2 * ATT_TPW * 128 * sizeof(float))));
+        ready[dev] = true;
+    }
+    const uint32_t n_kv = a.p.n_heads / a.p.kv_mul;
+    uint32_t splits = (uint32_t)sm_count() / n_kv;   // one block per SM
+    if (splits < 1) splits = 1;
+    if (splits > nchunks) splits = nchunks;          // the scratch has room for one per 64 positions
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(splits, n_kv);
+    cfg.blockDim = dim3(ATT_NT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    if (pdl) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    WGB_CUDA(cudaLaunchKernelEx(&cfg, attn_rows_kernel<QH>, a));
+    return WGB_OK;
+}
+
 template <int QH>
 static int launch_stream(const AttnArgs &a, uint32_t nchunks, uint32_t n_kv, uint32_t zgroups, cudaStream_t stream, bool pdl)
 {
@@ -821,7 +1077,7 @@ static int launch_stream(const AttnArgs &a, uint32_t nchunks, uint32_t n_kv, uin
     return WGB_OK;
 }
 
-// Long contexts with head sizes up to 128 and at most two query heads per KV head.
+// Long contexts with contiguous rows, head sizes up to 128 and at most two query heads per KV head.
 static int launch_stream_any(const AttnArgs &a, uint32_t nchunks, cudaStream_t stream, bool pdl)
 {
     const uint32_t n_kv = a.p.n_heads / a.p.kv_mul;
@@ -853,10 +1109,21 @@ static int launch_split(const AttnArgs &a, uint32_t nchunks, uint32_t nchunks_hi
     // `nchunks_hint`: chunks up to the furthest position this launch is expected to serve (performance only:
     // either kernel is correct for any position inside the cache).
     const bool multi = (uint64_t)nchunks_hint * heads > (uint64_t)per_sm_single * (uint32_t)sm_count();
-    // Up to two query heads per KV head the streaming kernel is bandwidth-bound and wins; with more, the
-    // arithmetic per cache byte grows (8 heads: 4 FMA per byte) and its eight consumer warps per SM hide
-    // less latency than two resident blocks of the chunk-walking split kernel.
-    if (multi && VC == 1 && a.p.kv_mul <= 2) return launch_stream_any(a, nchunks, stream, pdl);
+    // Beyond one wave, contiguous rows and up to two query heads per KV head: the streaming kernel (a decode step of four
+    // 7B layers at 3000 positions: 0.283 ms, with the row-streaming kernel 0.299).
+    if (multi && VC == 1 && a.p.kv_mul <= 2 && (a.row_stride ? a.row_stride : a.p.kv_dim) == a.p.head_size)
+        return launch_stream_any(a, nchunks, stream, pdl);
+    // One, two, four or eight query heads per KV head, head sizes up to 128: the row-streaming kernel, everywhere but in
+    // a decode step (position on the device) with up to two heads and a context of one wave.  Its blocks fill
+    // the shared memory, so the matrix-vector launch behind it cannot start prefetching beside it: tiny f32 decode 15.5
+    // ms with the split kernel, 16.2 with this one, GPT-2 32.1 and 34.2, 7B 77.5 and 78.1; but Qwen2 (four heads)
+    // 20.5 and 19.8.  Stand-alone it is the faster one at every length (32 heads on 32, 512 positions: 10.1 and 8.2 us).
+    if (VC == 1 && (multi || a.p.kv_mul >= 4 || !a.pos)) {
+        if (a.p.kv_mul == 1) return launch_rows<1>(a, nchunks, stream, pdl);
+        if (a.p.kv_mul == 2) return launch_rows<2>(a, nchunks, stream, pdl);
+        if (a.p.kv_mul == 4) return launch_rows<4>(a, nchunks, stream, pdl);
+        if (a.p.kv_mul == 8) return launch_rows<8>(a, nchunks, stream, pdl);
+    }
     uint32_t splits = nchunks;
     if (multi) {
         splits = (uint32_t)per_sm_multi * (uint32_t)sm_count() / heads;
