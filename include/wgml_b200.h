@@ -417,7 +417,9 @@ int wgb_llama2_load_stats(const wgb_llama2 *m, size_t *bytes, double *seconds);
 int wgb_llama2_set_sampler(wgb_llama2 *m, float temperature, float topp, uint64_t seed);
 /* Batched prompt prefill, no counterpart in the reference (its chat loop feeds the prompt one position per
  * Llama2::dispatch, chat_llama2.rs:104-116,169-204, and drops the logits).  Once enabled, wgb_llama2_decode
- * sends every prompt position but the last through passes of eight positions: the Q4_K layer matrices are
+ * sends every prompt position but the last through passes: of up to 640 positions when there are sixteen or more to go,
+ * every layer matrix is Q4_K, Q6_K or Q8_0 with a multiple of 128 rows, the head size is 64 or 128 and there is one rank
+ * (two f16 digits per activation, tcgen05.mma kind::f16); of eight positions otherwise: the Q4_K layer matrices are
  * multiplied on the tensor cores (tcgen05.mma kind::i8 on the same fixed-point image of the activations as the
  * matrix-vector kernels, from tile-major copies of the weights made here, which doubles their memory), the Q6_K
  * and Q8_0 ones by kernels of their own (Q6_K: scales folded into the weight operand; Q8_0: the codes are the operand),
@@ -547,7 +549,7 @@ float *wgb_gpt2_value_cache(wgb_gpt2 *m, uint32_t layer);
 /* As wgb_llama2_set_sampler. */
 int wgb_gpt2_set_sampler(wgb_gpt2 *m, float temperature, float topp, uint64_t seed);
 /* Batched prompt prefill as wgb_llama2_set_prefill, for Gpt2::dispatch (models/gpt2/transformer.rs:265-477): passes of
- * eight positions with LayerNorm, the fused qkv product and its split into cache rows, causal attention, the
+ * up to 640 or of eight positions under the same conditions, with LayerNorm, the fused qkv product and its split into cache rows, causal attention, the
  * projections and GELU computed per pass; Q8_0 / Q4_K / Q6_K matrices on the tensor cores.  The reference's loop
  * (chat_gpt2.rs:43-151) feeds the prompt one position per dispatch. */
 int wgb_gpt2_set_prefill(wgb_gpt2 *m, int enable);

@@ -254,10 +254,11 @@ __device__ __forceinline__ void pw_unpack(uint32_t (&v)[32], uint32_t raw, uint3
 
 // Roles: two producer threads (raw weights and per-unit extras; activation operand), one thread issuing MMAs, two groups
 // of four warps building the weight operand (alternate chunks of 64 columns), eight warps finishing units.
-// What bounds it: unpacking, per weight about 1.3 instructions on top of what the tensor pipe does.  A chunk of
-// weights therefore serves as many positions as tensor memory has room for: the accumulator holds both digits (low
-// digits of the four chunks first, then the high ones over the same weight operands, which stay in tensor memory), so
-// a tile is 128 positions; with an accumulator per digit it was 80 and 400 ns per chunk.  The operand goes from
+// What bounds it: the turnaround of the weight operand at unit boundaries and, with two planes, its unpacking (about 1.3
+// to 3 instructions per weight).  A chunk of weights therefore serves as many positions as tensor memory has room for:
+// the accumulator holds both digits (low digits of the four chunks first, then the high ones over the same weight
+// operands, which stay in tensor memory), so a tile is 128 positions; with an accumulator per digit it was 80.  Q4_K
+// 22016x4096 times 511 positions: 227 us then, 164 us now (1.1 PFLOP/s of two-digit MMA work).  The operand goes from
 // registers to tensor memory: written to and read from shared memory it cost as much of that memory's 128 bytes a
 // clock as everything else together.  Raw weights are free again as soon as they are unpacked, ahead of their MMAs;
 // the rows' scales travel in a small ring of their own.

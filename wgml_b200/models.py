@@ -186,8 +186,8 @@ class Llama2:
         return out[:prompt.size - 1 + n_gen]
 
     def set_prefill(self, enable: bool = True) -> None:
-        """Batched prompt prefill: `decode` sends the prompt through passes of eight positions with the Q4_K
-        products on the tensor cores (the reference feeds it position by position, chat_llama2.rs:104-116)."""
+        """Batched prompt prefill: `decode` sends the prompt through passes of up to 640 positions (eight,
+        where a format or shape has no wide path) with the products on the tensor cores (the reference feeds it position by position, chat_llama2.rs:104-116)."""
         check(_lib.load().wgb_llama2_set_prefill(self._h, 1 if enable else 0))
 
     def prefill_positions(self) -> int:
@@ -333,8 +333,8 @@ class Gpt2:
         check(_lib.load().wgb_gpt2_set_sampler(self._h, temperature, topp, seed))
 
     def set_prefill(self, enable: bool = True) -> None:
-        """Batched prompt prefill: `decode` sends the prompt through passes of eight positions with the matrix
-        products on the tensor cores (the reference feeds it position by position, chat_gpt2.rs:43-151)."""
+        """Batched prompt prefill: `decode` sends the prompt through passes of up to 640 positions (eight,
+        where a format or shape has no wide path) with the products on the tensor cores (the reference feeds it position by position, chat_gpt2.rs:43-151)."""
         check(_lib.load().wgb_gpt2_set_prefill(self._h, 1 if enable else 0))
 
     def prefill_positions(self) -> int:
