@@ -1117,11 +1117,12 @@ static int launch_split(const AttnArgs &a, uint32_t nchunks, uint32_t nchunks_hi
     // a decode step (position on the device) with up to two heads and a context of one wave.  Its blocks fill
     // the shared memory, so the matrix-vector launch behind it cannot start prefetching beside it: tiny f32 decode 15.5
     // ms with the split kernel, 16.2 with this one, GPT-2 32.1 and 34.2, 7B 77.5 and 78.1; but Qwen2 (four heads)
-    // 20.5 and 19.8.  Stand-alone it is the faster one at every length (32 heads on 32, 512 positions: 10.1 and 8.2 us).
-    // With fewer than eight KV heads a context of one wave stays with the split kernel as well (its blocks are one chunk
-    // each; here the merge of up to 37 splits by one block costs more: one such shape of 12.3 us took 14.1), but for
-    // decode steps with four heads per KV head, the Qwen2 figure above (four KV heads).
-    const bool one_wave = a.pos && a.p.kv_mul <= 4 ? a.p.kv_mul == 4 : n_kv >= 8;
+    // 20.5 and 19.8.  Stand-alone it is the faster one with many KV heads (32 heads on 32, 512 positions: 10.1 and 8.2 us).
+    // With fewer than eight KV heads (sixteen, at one or two query heads each) a context of one wave stays with the
+    // split kernel as well: its blocks are one chunk each, and here one block merges up to 37 splits (twelve KV heads,
+    // one query head each, 2200 positions: 9.8 us against 10.8); but for decode steps with four heads per KV head, the
+    // Qwen2 figure above (four KV heads).
+    const bool one_wave = a.pos && a.p.kv_mul <= 4 ? a.p.kv_mul == 4 : n_kv >= (a.p.kv_mul <= 2 ? 16u : 8u);
     if (VC == 1 && (multi || one_wave)) {
         if (a.p.kv_mul == 1) return launch_rows<1>(a, nchunks, stream, pdl);
         if (a.p.kv_mul == 2) return launch_rows<2>(a, nchunks, stream, pdl);
