@@ -76,6 +76,25 @@ def test_repeated_streaming_calls_reuse_the_ticket_counters():
     assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("case", [
+    (512, 32, 128, 1, 300), (512, 32, 64, 2, 300), (512, 32, 128, 4, 300), (4224, 64, 128, 8, 4100),   # row-streaming kernel, each width
+    (512, 8, 64, 1, 300), (512, 12, 64, 3, 130),                                                       # split kernel
+])
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_output_at_any_word(case, offset):
+    """`xb` may start at any float: only q and the caches are read sixteen bytes at a time.  Same bits, nothing beside it."""
+    seq_len, n_heads, hs, kv_mul, pos = case
+    g = torch.Generator(device="cuda").manual_seed(5)
+    kv_dim, n = n_heads // kv_mul * hs, n_heads * hs
+    q, k, v = (torch.randn(*s, device="cuda", generator=g) for s in ((n,), (seq_len, kv_dim), (seq_len, kv_dim)))
+    p, a = ops.BatchedMultiqueryAttentionParams(seq_len, kv_dim, kv_mul, n_heads, hs, pos), ops.BatchedMultiqueryAttention.from_device()
+    exp, buf = torch.empty(n, device="cuda"), torch.full((n + 8,), 7.0, device="cuda")
+    a.dispatch(p, q, k, v, None, exp)
+    a.dispatch(p, q, k, v, None, buf[offset:offset + n])
+    assert torch.equal(buf[offset:offset + n], exp)
+    assert (buf[:offset] == 7.0).all() and (buf[offset + n:] == 7.0).all()
+
+
 def test_parameter_checks():
     a = ops.BatchedMultiqueryAttention.from_device()
     z = torch.zeros(64 * 128, device="cuda")

@@ -1012,7 +1012,15 @@ __global__ void __launch_bounds__(ATT_NT, 1) attn_rows_kernel(const __grid_const
             }
         }
     }
-    if (on) reinterpret_cast<float4 *>(a.xb + (size_t)(kvh * kv_mul + j) * hs)[lane] = make_float4(o.x / Lt, o.y / Lt, o.z / Lt, o.w / Lt);
+    if (on) {
+        const float4 r = make_float4(o.x / Lt, o.y / Lt, o.z / Lt, o.w / Lt);
+        float *dst = a.xb + (size_t)(kvh * kv_mul + j) * hs + 4 * lane;
+        if (((uintptr_t)a.xb & 15) == 0) {   // a caller's output need not be aligned (q, K and V have to be: 16 bytes)
+            *reinterpret_cast<float4 *>(dst) = r;
+        } else {
+            dst[0] = r.x; dst[1] = r.y; dst[2] = r.z; dst[3] = r.w;
+        }
+    }
     if (threadIdx.x == 0) stamp_end(a.stamp);
 }
 
