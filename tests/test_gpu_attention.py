@@ -95,6 +95,27 @@ def test_output_at_any_word(case, offset):
     assert (buf[:offset] == 7.0).all() and (buf[offset + n:] == 7.0).all()
 
 
+@pytest.mark.parametrize("case", [(512, 32, 128, 1, 300), (512, 32, 64, 2, 300), (512, 32, 128, 4, 300), (4224, 64, 128, 8, 1300)])
+@pytest.mark.parametrize("masked", [(0, 8), (0, 23), (0, 130), (8, 16), (40, 290), (1, 297)])
+def test_rows_scored_minus_infinity_weigh_nothing(case, masked):
+    """Cache rows a host has masked with keys of -inf (left padding): whole groups, warps and blocks of the row-streaming
+    kernel see nothing but -inf, and the answer is that of the other rows (RTOL / ATOL as everywhere)."""
+    seq_len, n_heads, hs, kv_mul, pos = case
+    rng = np.random.default_rng(9)
+    n_kv = n_heads // kv_mul
+    q, k, v = (rng.standard_normal(s).astype(np.float32) for s in ((n_heads, hs), (seq_len, n_kv, hs), (seq_len, n_kv, hs)))
+    q[:, 0] = np.abs(q[:, 0]) + 0.5
+    k[masked[0]:masked[1], :, 0] = -np.inf
+    p = ops.BatchedMultiqueryAttentionParams(seq_len, n_kv * hs, kv_mul, n_heads, hs, pos)
+    xb = torch.full((n_heads * hs,), float("nan"), device="cuda")
+    ops.BatchedMultiqueryAttention.from_device().dispatch(p, *(torch.from_numpy(t.reshape(len(t), -1) if t.ndim == 3 else t.ravel()).cuda() for t in (q, k, v)), None, xb)
+    keep = np.r_[0:masked[0], masked[1]:pos + 1]
+    s = np.einsum("ghd,tgd->ght", q.reshape(n_kv, kv_mul, hs).astype(np.float64), k[keep].astype(np.float64)) / np.sqrt(hs)
+    w = np.exp(s - s.max(-1, keepdims=True))
+    exp = np.einsum("ght,tgd->ghd", w / w.sum(-1, keepdims=True), v[keep].astype(np.float64))
+    assert_close(xb.cpu().numpy(), exp.ravel(), RTOL, ATOL, f"rows {masked} masked")
+
+
 def test_parameter_checks():
     a = ops.BatchedMultiqueryAttention.from_device()
     z = torch.zeros(64 * 128, device="cuda")

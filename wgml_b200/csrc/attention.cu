@@ -903,9 +903,10 @@ __global__ void __launch_bounds__(ATT_NT, 1) attn_rows_kernel(const __grid_const
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
-            const float mn = fmaxf(M[j], m);          // finite: position 0 of the group is valid
-            const float rs = expf(M[j] - mn);         // 0 at the warp's first group (M = -inf)
-            const float e = expf(sv - mn);            // 0 for positions past the end
+            const float mn = fmaxf(M[j], m);
+            const float mz = mn == -INFINITY ? 0.0f : mn;   // all of the warp's scores so far are -inf: weights of 0, not of NaN
+            const float rs = expf(M[j] - mz);         // 0 at the warp's first group (M = -inf)
+            const float e = expf(sv - mz);            // 0 for positions past the end
             M[j] = mn;
             float psum = 0.0f;
             acc[j].x *= rs;
@@ -947,10 +948,11 @@ __global__ void __launch_bounds__(ATT_NT, 1) attn_rows_kernel(const __grid_const
         float mb = s_red[j][0];
 #pragma unroll
         for (int w = 1; w < ATT_WARPS; w++) mb = fmaxf(mb, s_red[j][w]);
+        const float mz = mb == -INFINITY ? 0.0f : mb;
         float sv = 0.0f, lb = 0.0f;
 #pragma unroll
         for (int w = 0; w < ATT_WARPS; w++) {
-            const float f = expf(s_red[j][w] - mb);   // 0 for a warp that had no positions
+            const float f = expf(s_red[j][w] - mz);   // 0 for a warp without a score above -inf
             sv = fmaf(s_acc[((size_t)w * QH + j) * astr + i], f, sv);
             lb = fmaf(s_sum[j][w], f, lb);
         }
@@ -983,6 +985,7 @@ __global__ void __launch_bounds__(ATT_NT, 1) attn_rows_kernel(const __grid_const
     float Mj = -INFINITY;
     for (uint32_t sp = lane; sp < nsplit_active; sp += 32) Mj = fmaxf(Mj, __ldcg(base + (size_t)sp * astr + hs));
     Mj = warp_max(Mj);
+    if (Mj == -INFINITY) Mj = 0.0f;   // no score above -inf at all: 0 / 0, as the definition has it
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
     float Lt = 0.0f;
 #pragma unroll 8
