@@ -97,3 +97,30 @@ def test_wide_gpt2_passes_match_sequential_loop(qtype, n_prompt):
         for a, b in ((bat.key_cache(l), seq.key_cache(l)), (bat.value_cache(l), seq.value_cache(l))):
             a, b = a[:n_prompt].cpu().numpy(), b[:n_prompt].cpu().numpy()
             assert_close(a, b, RTOL, ATOL * max(1.0, float(np.abs(b).max())), f"cache {l}")
+
+
+@pytest.mark.parametrize("heads,n_prompt,bad", [(8, 90, (40, 70)), (4, 140, (63, 64, 100)), (8, 40, (38,))])
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+def test_later_positions_reach_no_earlier_one(heads, n_prompt, bad, value):
+    """Positions whose embedding (hence every cache row from them on) is not finite leave the rows of the positions before them
+    as the token loop has them, in every layer: attention is causal also where a weight of zero meets an infinity."""
+    cfg = dict(SMALL_LLAMA, n_layers=3, n_q_heads=heads, n_kv_heads=heads, seq_len=160)
+    t = synth.llama_tensors(cfg, 23, scale=0.002)
+    emb = t["token_embd.weight"]
+    t["token_embd.weight"] = (synth.F32, oracle.dequantize(emb[0], emb[1]).reshape(cfg["vocab_size"], cfg["dim"]).astype(np.float32).copy())
+    t["token_embd.weight"][1][7, ::5] = value
+    t["token_embd.weight"] = (synth.F32, t["token_embd.weight"][1].ravel())
+    prompt = synth.prompt(n_prompt, cfg["vocab_size"], seed=5)
+    prompt[prompt == 7] = 8
+    prompt[list(bad)] = 7
+    seq, _, _ = llama_pair(cfg, tensors=t)
+    wide, _, _ = llama_pair(cfg, tensors=t)
+    wide.set_prefill(True)
+    for m in (seq, wide):
+        m.decode(prompt, 1)
+    assert wide.prefill_positions() > bad[-1]
+    n = bad[0]
+    for l, ((kb, vb), (ks, vs)) in enumerate(zip(_caches(wide, n), _caches(seq, n))):
+        assert np.isfinite(ks).all() and np.isfinite(vs).all()
+        assert_close(kb, ks, RTOL, ATOL * max(1.0, float(np.abs(ks).max())), f"key cache {l}")
+        assert_close(vb, vs, RTOL, ATOL * max(1.0, float(np.abs(vs).max())), f"value cache {l}")

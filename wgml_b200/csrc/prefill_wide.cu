@@ -877,18 +877,18 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
             if (c0 + r <= last) pre[k] = *reinterpret_cast<const float4 *>(base + (size_t)(c0 + r) * row_stride + e);
         }
     };
-    auto place = [&]() {
+    auto place = [&](bool flag) -> int {   // nonzero when any thread passes a flag
         __syncthreads();   // the tile before has been read
 #pragma unroll
         for (uint32_t k = 0; k < NP; k++) {
             const uint32_t i = tid + 256 * k, r = i / (HD / 4), e = 4 * (i % (HD / 4));
             *reinterpret_cast<float4 *>(ks + r * LD + e) = pre[k];
         }
-        __syncthreads();
+        return __syncthreads_or(flag);
     };
     fetch(kh, 0);
     for (uint32_t c0 = 0; c0 <= last; c0 += 64) {
-        place();
+        place(false);
         fetch(vh, c0);
         float s[4][4];
 #pragma unroll
@@ -940,8 +940,34 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
 #pragma unroll
             for (uint32_t c = 0; c < NC; c++) { acc[i][c].x *= rs; acc[i][c].y *= rs; acc[i][c].z *= rs; acc[i][c].w *= rs; }
         }
-        place();
+        // Where the tile holds rows that some of the block's positions do not attend to, their weight of 0 keeps a row out of
+        // the sum only if the row is finite; with an infinity or NaN about, such rows are left out one by one.
+        float z = 0.0f;   // 0 times every element: NaN if one is not finite
+        if (c0 + 63 > pos0 + t0) {
+#pragma unroll
+            for (uint32_t k = 0; k < NP; k++) z = fmaf(pre[k].x, 0.0f, fmaf(pre[k].y, 0.0f, fmaf(pre[k].z, 0.0f, fmaf(pre[k].w, 0.0f, z))));
+        }
+        const bool one_by_one = place(z != 0.0f) != 0;
         if (c0 + 64 <= last) fetch(kh, c0 + 64);
+        if (one_by_one) {
+#pragma unroll 1
+            for (uint32_t j = 0; j < 64; j++) {
+#pragma unroll
+                for (uint32_t c = 0; c < NC; c++) {
+                    const float4 vv = *reinterpret_cast<const float4 *>(vs + j * LD + 64 * c + 4 * tx);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        if (c0 + j > pos0 + t0 + 4 * ty + i) continue;
+                        const float w = ps[(4 * ty + i) * LP + j];
+                        acc[i][c].x = fmaf(w, vv.x, acc[i][c].x);
+                        acc[i][c].y = fmaf(w, vv.y, acc[i][c].y);
+                        acc[i][c].z = fmaf(w, vv.z, acc[i][c].z);
+                        acc[i][c].w = fmaf(w, vv.w, acc[i][c].w);
+                    }
+                }
+            }
+            continue;
+        }
 #pragma unroll 2
         for (uint32_t j = 0; j < 64; j += 4) {
             float4 pv[4];
