@@ -2,6 +2,7 @@
 float64 and against the position-by-position loop, at the edges of the tiles of positions, rows and passes."""
 import numpy as np
 import pytest
+import torch
 
 import oracle
 from conftest import ATOL, RTOL, assert_close
@@ -124,3 +125,43 @@ def test_later_positions_reach_no_earlier_one(heads, n_prompt, bad, value):
         assert np.isfinite(ks).all() and np.isfinite(vs).all()
         assert_close(kb, ks, RTOL, ATOL * max(1.0, float(np.abs(ks).max())), f"key cache {l}")
         assert_close(vb, vs, RTOL, ATOL * max(1.0, float(np.abs(vs).max())), f"value cache {l}")
+
+
+@pytest.mark.parametrize("arch", ["llama", "gpt2"])
+def test_prompt_passes_without_room_for_the_wide_ones(arch):
+    """With device memory for the eight-position passes but not for the buffers of the wide ones, enabling prompt passes
+    succeeds, what was half allocated is given back and prompts go through passes of eight positions."""
+    if arch == "llama":   # the wide buffers are about 0.3 GB here, the others 0.1 GB
+        cfg = dict(SMALL_LLAMA, hidden_dim=28672, n_layers=1, seq_len=700)
+        seq, _, t = llama_pair(cfg, seed=3, scale=0.002)
+        m, _, _ = llama_pair(cfg, tensors=t)
+        vocab = cfg["vocab_size"]
+    else:
+        cfg = dict(SMALL_GPT2, ff_len=28672, n_layer=1, n_seq=700)
+        seq, _, _ = gpt2_pair(cfg, seed=3, scale=0.002)
+        m, _, _ = gpt2_pair(cfg, seed=3, scale=0.002)
+        vocab = cfg["n_vocab"]
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    prompt = synth.prompt(41, vocab, 8)
+    exp = seq.decode(prompt, 4)
+    m.decode(prompt, 4)   # what decode itself allocates is there
+    torch.cuda.empty_cache()
+    before = free()
+    m.set_prefill(True)
+    need = before - free()
+    m.set_prefill(False)
+    short = 120 << 20
+    filler = torch.empty(free() - (need - short), dtype=torch.uint8, device="cuda")
+    try:
+        m.set_prefill(True)
+        assert free() > short // 2, "buffers of the wide passes are kept although they are not complete"
+        got = m.decode(prompt, 4)
+        assert m.prefill_positions() == 40
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert np.array_equal(got, exp)

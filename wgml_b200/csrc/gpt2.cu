@@ -254,6 +254,21 @@ int enqueue_forward(wgb_gpt2 *m, cudaStream_t s, int *nkernels)
     return WGB_OK;
 }
 
+// Gives back what wide passes work in (they are off afterwards).
+void wide_free(wgb_gpt2 *m)
+{
+    wgb_gpt2::Prefill &pf = m->pf;
+    for (uint8_t **b : { &pf.wimg_e, &pf.wimg_h }) {
+        if (*b) cudaFree(*b);
+        *b = nullptr;
+    }
+    for (float **b : { &pf.wx, &pf.wq, &pf.wxb, &pf.wpart[0], &pf.wpart[1] }) {
+        if (*b) cudaFree(*b);
+        *b = nullptr;
+    }
+    pf.wide_cap = 0;
+}
+
 void prefill_free(wgb_gpt2 *m)
 {
     for (uint8_t *t : m->pf.tiles) if (t) cudaFree(t);
@@ -263,10 +278,7 @@ void prefill_free(wgb_gpt2 *m)
     for (float *b : bufs) if (b) cudaFree(b);
     if (m->pf.attn_counters) cudaFree(m->pf.attn_counters);
     if (m->pf.pos) cudaFree(m->pf.pos);
-    if (m->pf.wimg_e) cudaFree(m->pf.wimg_e);
-    if (m->pf.wimg_h) cudaFree(m->pf.wimg_h);
-    float *wbufs[] = { m->pf.wx, m->pf.wq, m->pf.wxb, m->pf.wpart[0], m->pf.wpart[1] };
-    for (float *b : wbufs) if (b) cudaFree(b);
+    wide_free(m);
     m->pf = wgb_gpt2::Prefill();
 }
 
@@ -776,12 +788,14 @@ WGB_EXPORT int wgb_gpt2_set_prefill(wgb_gpt2 *m, int enable)
     if (wide) {
         const size_t cap = std::min<size_t>(PW_CAP, p.n_seq);
         pf.wpart_floats = cap * std::max<size_t>(4 * (size_t)n, ff);
-        if (cudaMalloc((void **)&pf.wimg_e, prefill_wide_image_bytes(n)) != cudaSuccess || cudaMalloc((void **)&pf.wimg_h, prefill_wide_image_bytes(ff)) != cudaSuccess)
-            return bail(fail(WGB_ERR_CUDA, "cudaMalloc(images of a wide prompt pass)"));
-        if ((rc = dalloc(&pf.wx, cap * n)) || (rc = dalloc(&pf.wq, cap * n)) || (rc = dalloc(&pf.wxb, cap * n)) || (rc = dalloc(&pf.wpart[0], pf.wpart_floats)) ||
-            (rc = dalloc(&pf.wpart[1], pf.wpart_floats)))
-            return bail(rc);
-        pf.wide_cap = (uint32_t)cap;
+        // Without room for these the prompt goes through the passes of PF_TOK positions, whose buffers are there already.
+        wide = cudaMalloc((void **)&pf.wimg_e, prefill_wide_image_bytes(n)) == cudaSuccess && cudaMalloc((void **)&pf.wimg_h, prefill_wide_image_bytes(ff)) == cudaSuccess &&
+               !dalloc(&pf.wx, cap * n) && !dalloc(&pf.wq, cap * n) && !dalloc(&pf.wxb, cap * n) && !dalloc(&pf.wpart[0], pf.wpart_floats) &&
+               !dalloc(&pf.wpart[1], pf.wpart_floats);
+        if (!wide) {
+            wide_free(m);
+            cudaGetLastError();   // an allocation that was refused is no error of a later launch
+        } else pf.wide_cap = (uint32_t)cap;
     }
     WGB_CUDA(cudaDeviceSynchronize());
     pf.enabled = true;

@@ -425,6 +425,21 @@ int enqueue_forward(wgb_llama2 *m, cudaStream_t s, int *nkernels)
     return WGB_OK;
 }
 
+// Gives back what wide passes work in (they are off afterwards).
+void wide_free(wgb_llama2 *m)
+{
+    wgb_llama2::Prefill &pf = m->pf;
+    for (uint8_t **b : { &pf.wimg_dim, &pf.wimg_q, &pf.wimg_hidden }) {
+        if (*b) cudaFree(*b);
+        *b = nullptr;
+    }
+    for (float **b : { &pf.wx, &pf.wq, &pf.wxb, &pf.wpart[0], &pf.wpart[1], &pf.wpart[2] }) {
+        if (*b) cudaFree(*b);
+        *b = nullptr;
+    }
+    pf.wide_cap = 0;
+}
+
 void prefill_free(wgb_llama2 *m)
 {
     for (uint8_t *t : m->pf.tiles) if (t) cudaFree(t);
@@ -434,10 +449,7 @@ void prefill_free(wgb_llama2 *m)
     float *bufs[] = { m->pf.x, m->pf.xn, m->pf.q, m->pf.xb, m->pf.h, m->pf.part[0], m->pf.part[1], m->pf.part[2], m->pf.red, m->pf.attn_scratch };
     if (m->pf.attn_counters) cudaFree(m->pf.attn_counters);
     for (float *b : bufs) if (b) cudaFree(b);
-    uint8_t *wimgs[] = { m->pf.wimg_dim, m->pf.wimg_q, m->pf.wimg_hidden };
-    for (uint8_t *b : wimgs) if (b) cudaFree(b);
-    float *wbufs[] = { m->pf.wx, m->pf.wq, m->pf.wxb, m->pf.wpart[0], m->pf.wpart[1], m->pf.wpart[2] };
-    for (float *b : wbufs) if (b) cudaFree(b);
+    wide_free(m);
     m->pf = wgb_llama2::Prefill();
 }
 
@@ -1392,12 +1404,14 @@ WGB_EXPORT int wgb_llama2_set_prefill(wgb_llama2 *m, int enable)
             WGB_CUDA(cudaMalloc((void **)p, prefill_wide_image_bytes(K)));
             return WGB_OK;
         };
-        if ((rc = wimage(&pf.wimg_dim, c.dim)) || (rc = wimage(&pf.wimg_q, m->q_dim)) || (rc = wimage(&pf.wimg_hidden, m->hidden)) ||
-            (rc = dalloc(&pf.wx, cap * c.dim)) || (rc = dalloc(&pf.wq, cap * m->q_dim)) || (rc = dalloc(&pf.wxb, cap * m->q_dim)))
-            return bail(rc);
-        for (int i = 0; i < 3; i++)
-            if ((rc = dalloc(&pf.wpart[i], pf.wpart_floats))) return bail(rc);
-        pf.wide_cap = (uint32_t)cap;
+        // Without room for these the prompt goes through the passes of PF_TOK positions, whose buffers are there already.
+        wide = !wimage(&pf.wimg_dim, c.dim) && !wimage(&pf.wimg_q, m->q_dim) && !wimage(&pf.wimg_hidden, m->hidden) && !dalloc(&pf.wx, cap * c.dim) &&
+               !dalloc(&pf.wq, cap * m->q_dim) && !dalloc(&pf.wxb, cap * m->q_dim);
+        for (int i = 0; i < 3 && wide; i++) wide = !dalloc(&pf.wpart[i], pf.wpart_floats);
+        if (!wide) {
+            wide_free(m);
+            cudaGetLastError();   // an allocation that was refused is no error of a later launch
+        } else pf.wide_cap = (uint32_t)cap;
     }
     WGB_CUDA(cudaDeviceSynchronize());
     pf.enabled = true;
