@@ -104,3 +104,19 @@ def test_binding_excerpt_in_the_integration_notes_matches_the_header():
         r = [p.split(":")[0].strip() for p in _split_params(params)]
         c = [re.findall(r"[A-Za-z_][A-Za-z0-9_]*", p)[-1] for p in c_decls[name]]
         assert r == c, f"{name}: Rust excerpt has {r}, the header {c}"
+
+
+def test_status_codes_name_one_kernel():
+    """The code of an expired wait (the number in the message of ERR_TIMEOUT) stands in one source file only."""
+    src = os.path.join(ROOT, "wgml_b200", "csrc")
+    where = {}
+    for f in sorted(os.listdir(src)):
+        if not f.endswith(".cu"):
+            continue
+        text = open(os.path.join(src, f)).read()
+        codes = re.findall(r"\ba\.err, (\d+)\b", text) + re.findall(r"\bwait\(bar_\w+[^;]*?, (\d+)\)", text)
+        for c in codes:
+            where.setdefault(int(c), set()).add(f)
+    where.pop(0, None)   # atomicCAS(a.err, 0, code)
+    assert len(where) > 30
+    assert {c: fs for c, fs in where.items() if len(fs) > 1} == {}

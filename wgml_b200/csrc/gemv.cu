@@ -797,8 +797,9 @@ bool gemv_fast_supported(const QMat &m)
 }
 
 // Device status word shared by all launches on one device: 0, or the code of the first bounded wait that
-// expired (1 consumer, 2 producer, 3 epilogue, 6 flags of the tensor-parallel peers, 7 / 8 streaming
-// attention, 16+ tensor-memory kernel).  While it is non-zero the kernels do not wait for peers at all.
+// expired (1 consumer, 2 producer, 3 epilogue, 6 flags of the tensor-parallel peers, 7 / 8 streaming attention; tensor-core
+// products: 11.. single vector, 21.. / 31.. / 41.. eight vectors Q4_K / Q6_K / Q8_0, 61.. wide passes).  While it is
+// non-zero the kernels do not wait for peers at all.
 static bool g_trace_plan = false;   // WGML_B200_TRACE_PLAN=1 prints the plan of every launch to stderr
 
 uint32_t *gemv_status_word()

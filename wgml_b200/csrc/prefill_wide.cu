@@ -351,8 +351,8 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                 const uint8_t *wt = a.w[mi] + (size_t)(w.tile - a.tile0[mi]) * a.nkb * F::RAW;
                 for (uint32_t kb = w.kb; kb < w.kb_end; kb++, m++) {
                     const uint32_t u = m % NR, x = m % NX;
-                    if (m >= NR) ok = tc_wait(bar_ue(u), (m / NR - 1) & 1, dead, a.err, 41);
-                    if (ok && m >= NX) ok = tc_wait(bar_xe(x), (m / NX - 1) & 1, dead, a.err, 42);
+                    if (m >= NR) ok = tc_wait(bar_ue(u), (m / NR - 1) & 1, dead, a.err, 61);
+                    if (ok && m >= NX) ok = tc_wait(bar_xe(x), (m / NX - 1) & 1, dead, a.err, 62);
                     if (!ok) break;
                     mbar_expect_tx(bar_u(u), F::RAW);
                     bulk_copy_g2s(sm_raw + u * F::RAW, wt + (size_t)kb * F::RAW, F::RAW, bar_u(u));
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                     const uint8_t *img = a.img + ((size_t)w.pt * a.nkb + kb) * unit_bytes;
                     for (uint32_t st = 0; st < 4 * P; st++, n++) {
                         const uint32_t s = n % NB;
-                        if (n >= NB) ok = tc_wait(bar_be(s), (n / NB - 1) & 1, dead, a.err, 43);
+                        if (n >= NB) ok = tc_wait(bar_be(s), (n / NB - 1) & 1, dead, a.err, 63);
                         if (!ok) break;
                         mbar_expect_tx(bar_b(s), bstep);
                         bulk_copy_g2s(sm_b + s * PW_B_STEP, img + (st & 3) * bstep, bstep, bar_b(s));
@@ -401,13 +401,13 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
             for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++, m++) {
                 const uint32_t u = m & 1, dcol = tmem_base + u * PW_MAXN;
                 // (with mins, the wait for the min sums of unit m - 2 covers this one)
-                if (FMT != WGB_Q4_K && m >= 2) ok = wait(bar_t(u), ((m >> 1) - 1) & 1, 44);
+                if (FMT != WGB_Q4_K && m >= 2) ok = wait(bar_t(u), ((m >> 1) - 1) & 1, 64);
                 for (uint32_t pl = 0; pl < P && ok; pl++, q++) {
 #pragma unroll 1
                     for (uint32_t st = 0; st < 4; st++, n++) {
                         const uint32_t j = st & 1, s = n % NB;   // low digits of the two pairs of chunks, then the high ones
-                        if (st < 2) ok = wait(bar_a(j), q & 1, 46);
-                        if (ok) ok = wait(bar_b(s), (n / NB) & 1, 45);
+                        if (st < 2) ok = wait(bar_a(j), q & 1, 66);
+                        if (ok) ok = wait(bar_b(s), (n / NB) & 1, 65);
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const uint32_t at = tmem_base + PW_TMEM_A + 2 * j * PW_A_COLS;
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                         __syncwarp();
                     }
                 }
-                if (FMT == WGB_Q4_K && ok && m >= 1) ok = wait(bar_m, (m - 1) & 1, 48);
+                if (FMT == WGB_Q4_K && ok && m >= 1) ok = wait(bar_m, (m - 1) & 1, 68);
                 if (!ok) break;
                 if (FMT == WGB_Q4_K) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (tc_elect()) {
@@ -448,9 +448,9 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
             w.set(a, item);
             for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++, m++) {
                 const uint32_t ur = m % NR, raw = sm_raw + ur * F::RAW;
-                ok = tc_wait(bar_u(ur), (m / NR) & 1, dead, a.err, 49);
+                ok = tc_wait(bar_u(ur), (m / NR) & 1, dead, a.err, 69);
                 // (on behalf of the MMA of the mins, which reads the group sums)
-                if (FMT == WGB_Q4_K && grp == 1 && ok) ok = tc_wait(bar_x(m % NX), (m / NX) & 1, dead, a.err, 47);
+                if (FMT == WGB_Q4_K && grp == 1 && ok) ok = tc_wait(bar_x(m % NX), (m / NX) & 1, dead, a.err, 67);
                 ok = __all_sync(0xffffffffu, ok);
 #pragma unroll 1
                 for (uint32_t i = 0; i < 2 * P && ok; i++) {
@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                     // the row is built in registers before its buffer is free: only the store waits for the MMAs
                     uint32_t v[32];
                     pw_unpack<FMT>(v, raw, r, c, P == 2 && i < 2);
-                    if (q) ok = __all_sync(0xffffffffu, tc_wait(bar_ae(j), (q - 1) & 1, dead, a.err, 50));
+                    if (q) ok = __all_sync(0xffffffffu, tc_wait(bar_ae(j), (q - 1) & 1, dead, a.err, 70));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     pw_st32(trow + PW_TMEM_A + c * PW_A_COLS, v);
@@ -526,8 +526,8 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                 for (uint32_t j = 0; j < 4; j++) acc[g][j] = 0ull;
             for (uint32_t kb = w.kb; kb < w.kb_end && ok; kb++, m++) {
                 const uint32_t u = m & 1, x = m % NX, ebase = sm_aux + x * PW_AUX + 32 * np;
-                ok = tc_wait(bar_x(x), (m / NX) & 1, dead, a.err, 52) && tc_wait(bar_r(m & 3), (m >> 2) & 1, dead, a.err, 53) &&
-                     tc_wait(bar_d(u), (m >> 1) & 1, dead, a.err, 54);
+                ok = tc_wait(bar_x(x), (m / NX) & 1, dead, a.err, 72) && tc_wait(bar_r(m & 3), (m >> 2) & 1, dead, a.err, 73) &&
+                     tc_wait(bar_d(u), (m >> 1) & 1, dead, a.err, 74);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 const float2 sc = rowscale[m & 3][r];
