@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
     using F = PwFmt<FMT>;
     constexpr uint32_t NA = PW_A_RING / 2, NB = PW_B_RING, NX = PW_X_RING, NR = F::RAW_RING, P = F::PLANES;
     extern __shared__ uint8_t pw_smem_raw[];
-    __shared__ __align__(8) unsigned long long bars[2 * NA + 2 * NB + 2 * NX + 2 * NR + 9];
+    __shared__ __align__(8) unsigned long long bars[2 * NA + 2 * NB + 2 * NX + 2 * NR + 10];
     __shared__ float2 rowscale[4][TC_TILE_ROWS];
     __shared__ uint32_t tmem_base_slot;
     __shared__ uint32_t dead_flag;
@@ -293,6 +293,7 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
     auto bar_t = [&](uint32_t u) { return bar(B0 + 2 * NR + 2 + u); };     //   and have been read
     auto bar_r = [&](uint32_t i) { return bar(B0 + 2 * NR + 4 + i); };     // its rows' scales are written (i = m % 4)
     const uint32_t bar_m = bar(B0 + 2 * NR + 8);                           // the min sums have been read
+    const uint32_t bar_end = bar(B0 + 2 * NR + 9);                         // after an expired wait: the MMAs in flight are through
     const uint32_t sm_b = tc_uniform(smem_addr(smem)), sm_raw = sm_b + NB * PW_B_STEP, sm_min = sm_raw + NR * F::RAW, sm_aux = sm_min + 2 * F::AMIN;
 
     if (threadIdx.x == 0) {
@@ -319,6 +320,7 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
             mbar_init(bar_t(u), PW_FINISH_WARPS);
         }
         mbar_init(bar_m, PW_FINISH_WARPS);
+        mbar_init(bar_end, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -435,6 +437,11 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                 }
                 __syncwarp();
             }
+        }
+        if (!ok) {   // the MMAs in flight read shared memory and write tensor memory: they end before the block gives these back
+            if (tc_elect()) tc_commit(bar_end);
+            __syncwarp();
+            mbar_wait(bar_end, 0, nullptr, 0, DRAIN_NS);
         }
     } else if (warp < 2 + PW_UNPACK_WARPS) {
         // ------------------------------ weight operand ------------------------------
