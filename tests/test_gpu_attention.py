@@ -44,23 +44,24 @@ def test_split_kernel_shapes(case):
 
 
 @pytest.mark.parametrize("case", [
-    (4224, 32, 128, 1, 4100),    # 7B heads, long context: one query head per block, 15 chunks per block
-    (4224, 32, 128, 1, 4095),    # last chunk exactly full
+    (4224, 32, 128, 1, 4100),    # 7B heads, long context: four blocks per KV head
+    (4224, 32, 128, 1, 4095),    # last group of eight rows exactly full
     (4224, 32, 128, 4, 4100),    # four query heads per KV head
-    (4224, 32, 128, 2, 2049),    # two, last chunk of two positions
-    (4224, 40, 128, 5, 3000),    # five query heads share a block of eight
-    (4224, 96, 128, 12, 1500),   # twelve: two groups of eight (tail masked)
+    (4224, 32, 128, 2, 2049),    # two, last group of two rows
+    (4224, 40, 128, 5, 3000),    # five query heads per KV head: split kernel, two groups of four (tail masked)
+    (4224, 96, 128, 12, 1500),   # twelve: split kernel, three groups of four
     (8256, 64, 64, 8, 8200),     # head size 64: half of the lanes idle
     (8256, 24, 96, 1, 5000),     # head size 96
-    (4224, 64, 128, 8, 2047), (4224, 64, 128, 8, 2048),   # grouped streaming kernel: last chunk full, one position in it
-    (4224, 64, 128, 8, 1300),    # a little more than a chunk per block: runs of one and two chunks
+    (4224, 64, 128, 8, 2047), (4224, 64, 128, 8, 2048),   # last group full, one row in it
+    (4224, 64, 128, 8, 1300),    # nine to ten groups of rows per block: not every warp has a second one
     (8256, 32, 96, 4, 7001),     # four heads per KV head, a quarter of the lanes idle
-    (4224, 64, 128, 8, 0),       # only the first chunk holds anything, and only one position
+    (4224, 64, 128, 8, 0),       # only the first group holds anything, and only one row
     (4224, 64, 128, 8, 63), (4224, 64, 128, 8, 64), (4224, 64, 128, 8, 130),
 ])
 def test_streaming_kernel_shapes(case):
-    """Shapes whose chunks outnumber the resident blocks of the split kernel and take the streaming kernel
-    (head sizes up to 128): the position bound passed with a host-side `pos` is the position itself."""
+    """Stand-alone calls on long contexts or with many query heads per KV head: the row-streaming kernel (one, two, four or
+    eight query heads per KV head) or the split kernel with several chunks per block.  (The streaming kernel proper wants the rows
+    of a head side by side, as the models' caches have them: test_gpu_decode_attention.py.)"""
     run(*case, want_attn=False, seed=3)
 
 
@@ -70,7 +71,7 @@ def test_repeated_calls_reuse_the_ticket_counters():
     assert torch.equal(a, b)
 
 
-def test_repeated_streaming_calls_reuse_the_ticket_counters():
+def test_repeated_streaming_calls_reuse_the_ticket_counters():   # row-streaming kernel
     a = run(4224, 64, 128, 8, 4100, False, seed=4)
     b = run(4224, 64, 128, 8, 4100, False, seed=4)
     assert torch.equal(a, b)

@@ -1,0 +1,56 @@
+"""Attention of the decode step (position on the device, head-major caches, programmatic launches) at contexts and groupings
+that the model tests do not reach: the streaming kernel (one or two query heads per KV head, more chunks of 64 rows than
+the split kernel's blocks fit in one wave) and the row-streaming kernel (four or eight) with and without its requests
+ahead of the wait for the launch before.  The caches are filled on both sides with the same rows, then a few greedy
+steps run against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import ATOL, RTOL, assert_close
+from helpers import SMALL_LLAMA, llama_pair
+from wgml_b200 import _lib, synth
+from wgml_b200.models import _device_view
+
+pytestmark = pytest.mark.gpu
+
+
+def steps(heads, kv_heads, head_size, start, gen, seq_len, seed=3):
+    cfg = dict(SMALL_LLAMA, dim=heads * head_size, hidden_dim=512, n_layers=1, n_q_heads=heads, n_kv_heads=kv_heads, vocab_size=300, seq_len=seq_len)
+    t = synth.llama_tensors(cfg, seed, scale=0.002)
+    rng = np.random.default_rng(seed)
+    # a faint embedding: the residual stream, hence the logits, come from the attention
+    t["token_embd.weight"] = (synth.F32, rng.standard_normal(300 * cfg["dim"]).astype(np.float32) * np.float32(1e-3))
+    gpu, cpu, _ = llama_pair(cfg, tensors=t)
+    kv_dim = kv_heads * head_size
+    caches = [rng.standard_normal((seq_len, kv_dim)).astype(np.float32) for _ in range(2)]
+    lib = _lib.load()
+    for rows, host, ptr in zip(caches, cpu.caches(), (lib.wgb_llama2_key_cache(gpu._h, 0), lib.wgb_llama2_value_cache(gpu._h, 0))):
+        host[0] = rows
+        dev = _device_view(ptr, seq_len * kv_dim).view(kv_heads, seq_len, head_size)
+        dev.copy_(torch.from_numpy(rows).cuda().view(seq_len, kv_heads, head_size).permute(1, 0, 2))
+    tok = np.array([17], np.uint32)
+    exp = cpu.decode(tok, gen, start)[0]
+    got = gpu.decode(tok, gen, start)
+    assert np.array_equal(got, exp)
+    ref = cpu.logits()
+    assert_close(gpu.logits().cpu().numpy(), ref, RTOL, ATOL * max(1.0, float(np.abs(ref).max())), f"logits after position {start + gen - 1}")
+
+
+@pytest.mark.parametrize("shape", [(32, 32, 64), (64, 32, 64), (32, 32, 96)])
+@pytest.mark.parametrize("start", [955, 1022, 2100])   # 955: fifteen chunks; 1022: a chunk fills up and the next one begins
+def test_streaming_kernel_in_decode_steps(shape, start):
+    """Three blocks of the split kernel per SM hold 444 chunks: with 32 KV heads a context of more than 13 chunks is over one wave."""
+    steps(*shape, start, 4, 2176)
+
+
+def test_streaming_kernel_with_several_chunks_per_block():
+    steps(32, 32, 128, 4090, 8, 4160)
+
+
+@pytest.mark.parametrize("shape", [(32, 8, 64), (32, 4, 64), (16, 4, 128), (32, 4, 128), (40, 5, 64)])
+@pytest.mark.parametrize("start", [0, 126, 200, 1001, 3003])
+def test_row_streaming_kernel_in_decode_steps(shape, start):
+    """Ten steps leave every number of rows in the last group of eight.  Up to about 140 positions there are fewer groups
+    than blocks, and no warp requests anything ahead of the wait; from 1001 on most do."""
+    steps(*shape, start, 10, 3072)

@@ -1,5 +1,5 @@
 """Batched prompt prefill: the tensor-core product for up to eight input vectors against the oracle, and the
-token loop with the prompt sent through passes of eight positions against the position-by-position loop and
+token loop with the prompt sent through passes of eight positions (or wide ones, where all formats allow them) against the position-by-position loop and
 against the oracle (cache rows, logits after the prompt, greedy tokens)."""
 import numpy as np
 import pytest
@@ -133,13 +133,16 @@ def _caches(gpu, n):
 
 
 @pytest.mark.parametrize("case", [
-    dict(n_prompt=45, n_kv_heads=8, qwen=False, mixed=False),     # five full passes and a remainder of four (a short pass)
-    dict(n_prompt=20, n_kv_heads=2, qwen=True, mixed=False),      # grouped-query heads, biases, Neox RoPE; remainder 3 stays sequential
-    dict(n_prompt=34, n_kv_heads=8, qwen=False, mixed=True),      # a Q6_K and a Q8_0 matrix among the Q4_K ones
-    # a context of several 256-row chunks: the prompt attention of a (head, pair of positions) is shared by blocks
+    dict(n_prompt=45, n_kv_heads=8, qwen=False, mixed=False),     # 44 positions: one wide pass
+    dict(n_prompt=20, n_kv_heads=2, qwen=True, mixed=False),      # the same with grouped-query heads, biases, Neox RoPE; remainder 3 stays sequential
+    dict(n_prompt=34, n_kv_heads=8, qwen=False, mixed=True),      # passes of eight: Q5_K, Q6_K and Q8_0 matrices among the Q4_K ones
+    # long prompts, all formats with tensor-core copies: wide passes, two and three of them
     dict(n_prompt=700, n_kv_heads=4, qwen=False, mixed=False, seq_len=720, n_layers=2, n_gen=6),
-    # eight chunks and more: eight positions per attention block
     dict(n_prompt=1900, n_kv_heads=8, qwen=False, mixed=False, seq_len=1920, n_layers=1, n_gen=4),
+    # the same two through passes of eight positions, as one matrix has no tensor-core copy.  Several 256-row chunks of
+    # context: blocks share the rows of a (head, group of positions); eight chunks and more: eight positions per block
+    dict(n_prompt=700, n_kv_heads=4, qwen=False, mixed=False, q5=True, seq_len=720, n_layers=2, n_gen=6),
+    dict(n_prompt=1900, n_kv_heads=8, qwen=False, mixed=False, q5=True, seq_len=1920, n_layers=1, n_gen=4),
 ])
 def test_prefill_matches_sequential_loop_and_oracle(case):
     cfg = dict(SMALL_LLAMA, n_layers=case.get("n_layers", 3), n_kv_heads=case["n_kv_heads"], seq_len=case.get("seq_len", SMALL_LLAMA["seq_len"]))
@@ -149,6 +152,8 @@ def test_prefill_matches_sequential_loop_and_oracle(case):
         tensors["blk.1.ffn_down.weight"] = synth.matrix(synth.Q6_K, 512, 1024, 3, "d6", 0.002)
         tensors["blk.2.ffn_up.weight"] = synth.matrix(synth.Q8_0, 1024, 512, 3, "up8", 0.002)
         tensors["blk.1.attn_q.weight"] = synth.matrix(synth.Q5_K, 512, 512, 3, "q5", 0.002)   # no tensor-core path: position by position
+    if case.get("q5"):
+        tensors["blk.0.attn_q.weight"] = synth.matrix(synth.Q5_K, 512, 512, 3, "q5", 0.002)
     seq, cpu, _ = llama_pair(cfg, biases=case["qwen"], qwen=case["qwen"], tensors=tensors)
     bat, _, _ = llama_pair(cfg, biases=case["qwen"], qwen=case["qwen"], tensors=tensors)
     bat.set_prefill(True)
@@ -213,9 +218,11 @@ def test_prefill_with_the_sampler_and_up_to_the_last_cache_row():
 
 
 @pytest.mark.parametrize("case", [
-    dict(cfg=dict(SMALL_GPT2), n_prompt=45, qtype=synth.Q8_0),                                   # five passes and a short one
+    dict(cfg=dict(SMALL_GPT2), n_prompt=45, qtype=synth.Q8_0),                                   # 44 positions: one wide pass
     dict(cfg=dict(SMALL_GPT2), n_prompt=19, qtype=synth.Q5_1),                                   # no tensor-core copy: per position
-    dict(cfg=dict(synth.CONFIGS["gpt2-124m"], n_layer=2), n_prompt=300, qtype=synth.Q8_0),       # 124M widths, two chunks of context
+    dict(cfg=dict(synth.CONFIGS["gpt2-124m"], n_layer=2), n_prompt=300, qtype=synth.Q8_0),       # 124M widths, a wide pass
+    dict(cfg=dict(synth.CONFIGS["gpt2-124m"], n_layer=2, n_head=8), n_prompt=300, qtype=synth.Q8_0),   # head size 96: passes of eight, two chunks of context
+    dict(cfg=dict(synth.CONFIGS["gpt2-124m"], n_layer=1), n_prompt=900, qtype=synth.Q8_0),       # two wide passes
 ])
 def test_gpt2_prefill_matches_sequential_loop_and_oracle(case):
     cfg = dict(case["cfg"], default_qtype=case["qtype"])
