@@ -66,33 +66,19 @@ __device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t *p)
     return v;
 }
 
-// Ring slots are told apart by a count of their releases, not by the parity of an mbarrier.  The lanes of the producer
-// and epilogue warps progress independently, consumer warps take every ncl-th task, and copies land in any order, so a
-// waiter can come to a slot while the slot's previous use is unfinished; a parity is then that of the use before and
-// reads as "done" (a slot taken early is armed twice, which the hardware reports as a launch failure).  Waiting for the
-// exact number of releases first makes the parities of `full` and `done` unambiguous.
-__device__ __forceinline__ void count_set(uint32_t addr, uint32_t v)
-{
-    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
-__device__ __forceinline__ bool count_wait(uint32_t addr, uint32_t want, uint32_t *err, uint32_t code, unsigned long long limit_ns)
-{
-    if (want == 0) return true;
-    unsigned long long t0 = 0;
-#pragma unroll 1
-    for (uint32_t i = 1;; i++) {
-        uint32_t v;
-        asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
-        if (v >= want) return true;
-        if ((i & 1023u) == 0) {
-            const unsigned long long t = global_ns();
-            if (!t0) t0 = t;
-            if (t - t0 > limit_ns) break;
-        }
-    }
-    if (err) atomicCAS(err, 0u, code);
-    return false;
-}
+// Which use of a ring slot a barrier stands at is read from its parity, so a waiter must know that the use before (of that
+// barrier) is through; otherwise the parity is that of the use before and reads as "done" (a slot armed twice ends in a
+// launch failure).
+//   * Producer (`empty`): the lanes of a pass meet before the next pass, and the use before lies in an earlier pass (spb <=
+//     nstage), whose lanes have waited for its release.
+//   * Consumer warp (`full`) and lane group of the epilogue (`done`): they take every ncl-th task and every nb-th stage, so the use
+//     before of a slot may be another's, and unfinished.  Uses take turns on two barriers per slot (round & 1): what has to be
+//     through at stage `it` is the use two back, stage it - 2 nstage.  The waiter's own stage before is at most L = ceil(ncl /
+//     rparts), respectively nb, stages back and has landed; its pass of the producer begins L + spb - 1 stages back or later, and
+//     until then all slots of earlier passes had been released, so every stage up to it - L - spb - nstage is through.  That
+//     covers it - 2 nstage when L + spb <= nstage.  For nb the batches below see to it (nstage = 1: the same lanes take every
+//     stage); for the consumers plan() does, unless a warp takes a task of every use of a slot anyway (ring_safe).
+// (Counting a slot's releases instead, a second word to poll in every wait, cost a 7B decode step 2 % and a tiny one 3 %.)
 
 __device__ __forceinline__ void cons_sync() { asm volatile("bar.sync 1, %0;" ::"n"(GEMV_CONS_THREADS) : "memory"); }
 
@@ -168,7 +154,8 @@ __device__ __forceinline__ float warp_sum_rows(const float (&acc)[R], int lane)
 // reconvergence point until all of them have left their wait, so a pass must be assumed to finish only
 // when every stage in it has: the epilogue pass that frees a slot must never contain a stage whose copy
 // the producer can only issue in a pass that needs that very slot.  epilogue_batch + producer_batch <=
-// nstage + 1 rules the cycle out; the producer also leaves half of the ring queued while it waits.
+// nstage + 1 rules the cycle out; the producer also leaves half of the ring queued while it waits.  (From two stages on
+// the sum stays within nstage, which the waits on `done` need as well.)
 __host__ __device__ inline uint32_t epilogue_batch(uint32_t nstage) { return nstage >= 8 ? 4u : (nstage >= 4 ? 2u : 1u); }
 __host__ __device__ inline uint32_t producer_batch(uint32_t nstage, uint32_t copies_per_stage)
 {
@@ -355,8 +342,7 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
     __shared__ float red[32];
     __shared__ float part[GEMV_MAX_STAGES][GEMV_NCONS][GEMV_MAX_RS];    // [stage][column part][stage row]
     __shared__ __align__(16) float lane_part[GEMV_NCONS][GEMV_TASK_ROWS][32];   // [consumer warp][task row][lane]
-    __shared__ __align__(8) unsigned long long bars[2 * GEMV_MAX_STAGES];
-    __shared__ uint32_t freed[GEMV_MAX_STAGES];    // per ring slot: how often the epilogue warp has released it
+    __shared__ __align__(8) unsigned long long bars[5 * GEMV_MAX_STAGES];
     __shared__ float2 rope_tab[GEMV_ROPE_TAB];     // (cos, sin) per pair index of a head (EPI_QKV_ROPE)
 
     const uint32_t K = a.mat[0].ncols;
@@ -364,14 +350,14 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
     const uint32_t nstage = a.nstage;
     uint8_t *smem = reinterpret_cast<uint8_t *>(smem4);
     const uint32_t ring = smem_addr(smem + a.ring_offset);
-    const uint32_t full0 = smem_addr(&bars[0]), done0 = smem_addr(&bars[GEMV_MAX_STAGES]), freed0 = smem_addr(&freed[0]);
+    // full, done: [round & 1][slot]
+    const uint32_t full0 = smem_addr(&bars[0]), done0 = smem_addr(&bars[2 * GEMV_MAX_STAGES]), empty0 = smem_addr(&bars[4 * GEMV_MAX_STAGES]);
     const uint32_t kp = a.kparts, rparts = a.rparts;
 
     // one thread per barrier: initialising them one after the other would cost a microsecond
-    if (threadIdx.x < 2 * nstage) {
+    if (threadIdx.x < 5 * nstage) {
         const uint32_t kind = threadIdx.x / nstage, s = threadIdx.x - kind * nstage;
-        mbar_init((kind == 0 ? full0 : done0) + 8 * s, kind == 1 ? kp * rparts : 1);
-        if (kind == 0) freed[s] = 0;
+        mbar_init(full0 + 8 * (kind * GEMV_MAX_STAGES + s), (kind >> 1) == 1 ? kp * rparts : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -393,31 +379,34 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
         const uint32_t sb = (uint32_t)lane >> a.cps_log2, ci = (uint32_t)lane & (cps - 1);
         const uint32_t gmask = ((1u << cps) - 1u) << (sb * cps);
         if (sb >= spb) return;
-        uint32_t s = sb % nstage, round = sb / nstage;           // ring slot of stage `it` and its use count
-        for (uint32_t it = sb; it < nst; it += spb) {
-            Part parts[2];
-            uint32_t n = 0;
-            const int nparts = group_parts(a, EPI, blockIdx.x + it * gridDim.x, parts, n);
-            if (ci == 0) {
-                count_wait(freed0 + 4 * s, round, a.err, 2, a.wait_ns);
-                mbar_expect_tx(full0 + 8 * s, nparts * n * row_bytes);
+        const uint32_t pmask = spb * cps >= 32 ? ~0u : (1u << (spb * cps)) - 1u;   // the lanes that stay
+        uint32_t s = sb, round = 0;                              // ring slot of stage `it` and its use count (spb <= nstage)
+        for (uint32_t it = sb; it < nst + sb; it += spb) {       // every lane: as many passes as the first
+            if (it < nst) {
+                Part parts[2];
+                uint32_t n = 0;
+                const int nparts = group_parts(a, EPI, blockIdx.x + it * gridDim.x, parts, n);
+                const uint32_t full = full0 + 8 * ((round & 1) * GEMV_MAX_STAGES + s);
+                if (ci == 0) {
+                    if (round) mbar_wait(empty0 + 8 * s, (round - 1) & 1, a.err, 2, a.wait_ns);
+                    mbar_expect_tx(full, nparts * n * row_bytes);
+                }
+                __syncwarp(gmask);
+                if (ci < (uint32_t)nparts * nplanes) {
+                    const uint32_t pi = ci / nplanes, pl = ci % nplanes;   // nplanes is a compile-time power of two
+                    // a stage holds plane after plane; within a plane, the rows of part 0 then those of part 1
+                    const QMat &m = a.mat[parts[pi].mat];
+                    uint32_t off = pi * n * m.pitch[pl];
+                    for (uint32_t q = 0; q < pl; q++) off += (uint32_t)nparts * n * m.pitch[q];
+                    bulk_copy_g2s(ring + s * a.stage_bytes + off, m.p[pl] + (size_t)parts[pi].row0 * m.pitch[pl], n * m.pitch[pl], full);
+                }
             }
-            __syncwarp(gmask);
-            if (ci < (uint32_t)nparts * nplanes) {
-                const uint32_t pi = ci / nplanes, pl = ci % nplanes;   // nplanes is a compile-time power of two
-                // a stage holds plane after plane; within a plane, the rows of part 0 then those of part 1
-                const QMat &m = a.mat[parts[pi].mat];
-                uint32_t off = pi * n * m.pitch[pl];
-                for (uint32_t q = 0; q < pl; q++) off += (uint32_t)nparts * n * m.pitch[q];
-                bulk_copy_g2s(ring + s * a.stage_bytes + off, m.p[pl] + (size_t)parts[pi].row0 * m.pitch[pl], n * m.pitch[pl],
-                              full0 + 8 * s);
-            }
+            __syncwarp(pmask);
             s += spb;
-            while (s >= nstage) { s -= nstage; round++; }
+            if (s >= nstage) { s -= nstage; round++; }
         }
         return;
     }
-
     if (warp == GEMV_EPILOGUE) {
         // ------------------------------ epilogue ------------------------------
         // Up to four stages per pass: lanes 8k..8k+7 take stage it0 + k, one lane per output unit.
@@ -455,8 +444,7 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
             const EpiCtx c = epi_prepare(a, EPI, parts, nparts, n, ul, nunits, rope_tab);
             uint32_t ra = 0, rb = 0;
             if (c.on) unit_rows(EPI, parts, nparts, n, ul, ra, rb);
-            count_wait(freed0 + 4 * s, round, a.err, 3, a.wait_ns);
-            mbar_wait(done0 + 8 * s, round & 1, a.err, 3, a.wait_ns);
+            mbar_wait(done0 + 8 * ((round & 1) * GEMV_MAX_STAGES + s), (round >> 1) & 1, a.err, 3, a.wait_ns);
             if (PRO == PRO_RMS && !have_scale) {
                 // every consumer warp wrote its sum of squares before its first arrival on a `done` barrier
                 float ss = 0.0f;
@@ -477,7 +465,7 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
                 }
             }
             __syncwarp(gmask);
-            if (ul == 0) count_set(freed0 + 4 * s, round + 1);   // stage and partial sums may be overwritten
+            if (ul == 0) mbar_arrive(empty0 + 8 * s);   // stage and partial sums may be overwritten
             epi_finish(a, EPI, parts, c, ya, yb);
         }
         if ((EPI == EPI_STORE || EPI == EPI_RESIDUAL) && a.peer_out.n) {
@@ -713,8 +701,7 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
         const uint32_t j0 = rp * Rn;
         const uint32_t jn = min(Rn, nrows > j0 ? nrows - j0 : 0u);
         const uint32_t stage = ring + s * a.stage_bytes;
-        count_wait(freed0 + 4 * s, round, a.err, 1, a.wait_ns);
-        mbar_wait(full0 + 8 * s, round & 1, a.err, 1, a.wait_ns);
+        mbar_wait(full0 + 8 * ((round & 1) * GEMV_MAX_STAGES + s), (round >> 1) & 1, a.err, 1, a.wait_ns);
         for (uint32_t ks = kw; ks < nsteps; ks += kp) {
             const uint32_t col0 = ks * step_cols<QT>();
             if (held != ks) {
@@ -745,7 +732,7 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
         v += __shfl_xor_sync(0xffffffffu, v, 1);
         if ((lane & 7) == 0 && (uint32_t)(lane >> 3) < jn) part[s][kw][j0 + (lane >> 3)] = v;
         __syncwarp();
-        if (lane == 0) mbar_arrive(done0 + 8 * s);
+        if (lane == 0) mbar_arrive(done0 + 8 * ((round & 1) * GEMV_MAX_STAGES + s));
     }
 }
 
@@ -861,6 +848,12 @@ void status_poll_destroy(StatusPoll &sp)
     }
 }
 
+// Whether the consumers' waits can tell the uses of a ring of `nstage` slots apart (above cons_sync), with one stage per producer pass.
+static bool ring_safe(uint32_t per_block, uint32_t nstage, uint32_t ncl, uint32_t rparts)
+{
+    return per_block <= nstage || ncl <= rparts || (nstage * rparts) % ncl == 0 || (ncl + rparts - 1) / rparts < nstage;
+}
+
 static uint32_t steps_of(int qt, uint32_t K)
 {
     const uint32_t sc = qt == WGB_Q4_K ? step_cols<WGB_Q4_K>() : qt == WGB_Q6_K ? step_cols<WGB_Q6_K>()
@@ -922,7 +915,7 @@ static bool plan(GemvArgs &a, size_t &smem_bytes, uint32_t &grid)
         for (uint32_t rparts = 1; rparts <= 8; rparts *= 2) {
             if (rs % rparts) continue;
             const uint32_t rrows = rs / rparts;
-            if (rrows > (uint32_t)GEMV_TASK_ROWS) continue;
+            if (rrows > (uint32_t)GEMV_TASK_ROWS || !ring_safe(per, ns, ncl, rparts)) continue;
             const uint32_t in_work = (ncl + rparts - 1) / rparts + 1;   // stages the consumers hold at a time
             double flight;
             if (ns >= per) flight = 1.0;                                // the block's whole share fits in the ring
@@ -965,6 +958,8 @@ static bool plan(GemvArgs &a, size_t &smem_bytes, uint32_t &grid)
     // pass than that needs, so that the ring stays as full as possible.
     a.spb = (24576u + a.stage_bytes - 1) / a.stage_bytes;
     if (a.spb > producer_batch(a.nstage, cps)) a.spb = producer_batch(a.nstage, cps);
+    const uint32_t lag = (ncl + best_rp - 1) / best_rp;   // stages between two tasks of a consumer warp, most
+    if (a.per_block > a.nstage && ncl > best_rp && (a.nstage * best_rp) % ncl != 0 && a.spb > a.nstage - lag) a.spb = a.nstage - lag;
     smem_bytes = image + (size_t)a.nstage * a.stage_bytes;
     return true;
 }
