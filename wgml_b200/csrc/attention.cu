@@ -181,8 +181,11 @@ __device__ __forceinline__ void attn_merge_chunks(const AttnArgs &a, uint32_t kv
 // context of 800 positions are all resident at once.  (Left to itself the kernel takes 85 registers, two blocks per
 // SM, and a launch is 1.2 us shorter while its blocks fit one wave -- 576 positions for 32 heads -- but a second
 // wave costs 2.5 us, more than the streaming kernel.)
+// Four query heads at a time, several chunks per block: two blocks per SM (left to itself the kernel has taken 128 registers
+// in one version of this file and 162, one block, in another: five query heads on 40 KV heads, head size 128, 8192
+// positions 208 and 471 us).
 template <int QH, int VC, bool MULTI>
-__global__ void __launch_bounds__(ATT_NT, (QH == 1 && VC == 1) ? 3 : 0) attn_split_kernel(const __grid_constant__ AttnArgs a)
+__global__ void __launch_bounds__(ATT_NT, (QH == 1 && VC == 1) ? 3 : (QH == 4 && VC == 1 && MULTI) ? 2 : 0) attn_split_kernel(const __grid_constant__ AttnArgs a)
 {
     __shared__ float s_score[QH][ATT_CHUNK];
     __shared__ float s_red[QH][ATT_WARPS];
