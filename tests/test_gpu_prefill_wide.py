@@ -56,6 +56,10 @@ def _caches(gpu, n):
     dict(n_prompt=90, heads=4, kv=4, qwen=False, mixed=True),               # head size 128; three formats in one layer's products
     dict(n_prompt=700, heads=4, kv=2, qwen=False, mixed=False, seq_len=720),   # two passes: the second attends to the first's rows
     dict(n_prompt=530, heads=8, kv=4, qwen=False, mixed=True, seq_len=700, start=150, n_layers=1),   # a pass that starts at a later position
+    # few positions at a later one: blocks of the attention share the cache rows of a head
+    dict(n_prompt=17, heads=8, kv=2, qwen=True, mixed=False, seq_len=1700, start=1630, n_layers=2),  # 26 tiles of rows, the last one short
+    dict(n_prompt=73, heads=4, kv=4, qwen=False, mixed=False, seq_len=900, start=762, n_layers=2),   # head size 128; two tiles of positions, of 12 and 13
+    dict(n_prompt=41, heads=8, kv=8, qwen=False, mixed=False, seq_len=256, start=200, n_layers=2),   # two blocks of two tiles each
 ])
 def test_wide_passes_match_sequential_loop(case):
     cfg = dict(SMALL_LLAMA, n_layers=case.get("n_layers", 3), n_q_heads=case["heads"], n_kv_heads=case["kv"], seq_len=case.get("seq_len", 128))

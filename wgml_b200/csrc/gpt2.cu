@@ -62,6 +62,8 @@ struct wgb_gpt2 {
         float *wx = nullptr, *wq = nullptr, *wxb = nullptr;   // [wide_cap][n_embd]
         float *wpart[2] = {};                // product slices of a wide pass
         size_t wpart_floats = 0;
+        float *wattn_scratch = nullptr;      // blocks of the attention that share cache rows, and their counters
+        uint32_t *wattn_counters = nullptr;
     } pf;
 };
 
@@ -262,10 +264,12 @@ void wide_free(wgb_gpt2 *m)
         if (*b) cudaFree(*b);
         *b = nullptr;
     }
-    for (float **b : { &pf.wx, &pf.wq, &pf.wxb, &pf.wpart[0], &pf.wpart[1] }) {
+    for (float **b : { &pf.wx, &pf.wq, &pf.wxb, &pf.wpart[0], &pf.wpart[1], &pf.wattn_scratch }) {
         if (*b) cudaFree(*b);
         *b = nullptr;
     }
+    if (pf.wattn_counters) cudaFree(pf.wattn_counters);
+    pf.wattn_counters = nullptr;
     pf.wide_cap = 0;
 }
 
@@ -381,7 +385,8 @@ int wide_pass(wgb_gpt2 *m, cudaStream_t s, const uint32_t *d_tokens, uint32_t po
             return rc;
         if ((rc = wide_product(m, l, WGB_G_ATTN_QKV, pf.wimg_e, ntok, t, pf.wpart[0], &ns, s))) return rc;
         if ((rc = launch_prefill_qkv_split(pf.wpart[0], ns, ntok, w.v[WGB_G_ATTN_QKV_B], pf.wq, kc, vc, n, pos0, ntok, s))) return rc;
-        if ((rc = launch_wide_attention(pf.wq, kc, vc, pf.wxb, p.n_head, hs, 1, n, hs, pos0, ntok, s))) return rc;
+        if ((rc = launch_wide_attention(pf.wq, kc, vc, pf.wxb, p.n_head, hs, 1, n, hs, pos0, ntok, pf.wattn_scratch, pf.wattn_counters, s)))
+            return rc;
         if ((rc = launch_wide_norm_image(pf.wxb, nullptr, 0, nullptr, nullptr, nullptr, 0.0f, n, ntok, t, pf.wimg_e, s))) return rc;
         if ((rc = wide_product(m, l, WGB_G_ATTN_PROJ, pf.wimg_e, ntok, t, pf.wpart[1], &ns, s))) return rc;
         if ((rc = launch_wide_norm_image(pf.wx, pf.wpart[1], ns, w.v[WGB_G_ATTN_PROJ_B], w.v[WGB_G_LN_2_G], w.v[WGB_G_LN_2_B], 1.0e-5f, n, ntok, t, pf.wimg_e, s)))
@@ -792,6 +797,9 @@ WGB_EXPORT int wgb_gpt2_set_prefill(wgb_gpt2 *m, int enable)
         wide = cudaMalloc((void **)&pf.wimg_e, prefill_wide_image_bytes(n)) == cudaSuccess && cudaMalloc((void **)&pf.wimg_h, prefill_wide_image_bytes(ff)) == cudaSuccess &&
                !dalloc(&pf.wx, cap * n) && !dalloc(&pf.wq, cap * n) && !dalloc(&pf.wxb, cap * n) && !dalloc(&pf.wpart[0], pf.wpart_floats) &&
                !dalloc(&pf.wpart[1], pf.wpart_floats);
+        const size_t counters = prefill_wide_attention_counters() * sizeof(uint32_t);
+        wide = wide && !dalloc(&pf.wattn_scratch, prefill_wide_attention_scratch_floats(hs)) &&
+               cudaMalloc((void **)&pf.wattn_counters, counters) == cudaSuccess && cudaMemset(pf.wattn_counters, 0, counters) == cudaSuccess;
         if (!wide) {
             wide_free(m);
             cudaGetLastError();   // an allocation that was refused is no error of a later launch

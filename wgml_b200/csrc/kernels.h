@@ -257,8 +257,10 @@ int launch_wide_silu_image(const float *gate, uint32_t gsplit, const float *up, 
                            cudaStream_t stream);
 int launch_wide_gelu_image(const float *part, uint32_t nsplit, const float *bias, uint32_t K, uint32_t ntok, const WideTiling &t, uint8_t *image, cudaStream_t stream);
 bool prefill_wide_attention_supported(uint32_t head_size);
+size_t prefill_wide_attention_scratch_floats(uint32_t head_size);
+size_t prefill_wide_attention_counters();   // words, zeroed once by the caller
 int launch_wide_attention(const float *q, const float *k_cache, const float *v_cache, float *out, uint32_t n_heads, uint32_t head_size, uint32_t kv_mul,
-                          uint32_t row_stride, uint32_t head_stride, uint32_t pos0, uint32_t ntok, cudaStream_t stream);
+                          uint32_t row_stride, uint32_t head_stride, uint32_t pos0, uint32_t ntok, float *scratch, uint32_t *counters, cudaStream_t stream);
 // x[t] = row d_tokens[t] of the embedding (+ row pos0 + t of `pos_embd`).
 int launch_embed_rows(const QMat &embd, const QMat *pos_embd, const uint32_t *d_tokens, uint32_t pos0, uint32_t ntok, float *x, cudaStream_t stream);
 

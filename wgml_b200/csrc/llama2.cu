@@ -101,6 +101,8 @@ struct wgb_llama2 {
         float *wx = nullptr, *wq = nullptr, *wxb = nullptr;   // [wide_cap][dim | q_dim]
         float *wpart[3] = {};                // product slices of a wide pass
         size_t wpart_floats = 0;             //   floats of each
+        float *wattn_scratch = nullptr;      // blocks of the attention that share cache rows, and their counters
+        uint32_t *wattn_counters = nullptr;
     } pf;
 };
 
@@ -433,10 +435,12 @@ void wide_free(wgb_llama2 *m)
         if (*b) cudaFree(*b);
         *b = nullptr;
     }
-    for (float **b : { &pf.wx, &pf.wq, &pf.wxb, &pf.wpart[0], &pf.wpart[1], &pf.wpart[2] }) {
+    for (float **b : { &pf.wx, &pf.wq, &pf.wxb, &pf.wpart[0], &pf.wpart[1], &pf.wpart[2], &pf.wattn_scratch }) {
         if (*b) cudaFree(*b);
         *b = nullptr;
     }
+    if (pf.wattn_counters) cudaFree(pf.wattn_counters);
+    pf.wattn_counters = nullptr;
     pf.wide_cap = 0;
 }
 
@@ -659,7 +663,7 @@ int wide_pass(wgb_llama2 *m, cudaStream_t s, const uint32_t *d_tokens, uint32_t 
         qa.freq = m->rope_freq;
         if ((rc = launch_prefill_rope_append(qa, ntok, s))) return rc;
         if ((rc = launch_wide_attention(pf.wq, qa.k_cache, qa.v_cache, pf.wxb, m->n_q_local, m->head_size, m->kv_mul, m->head_size, c.seq_len * m->head_size, pos0,
-                                        ntok, s)))
+                                        ntok, pf.wattn_scratch, pf.wattn_counters, s)))
             return rc;
         if ((rc = launch_wide_norm_image(pf.wxb, nullptr, 0, nullptr, nullptr, nullptr, 0.0f, q_dim, ntok, t, pf.wimg_q, s))) return rc;
         if ((rc = wide_products(m, l, &wo, 1, pf.wimg_q, ntok, t, pf.wpart, ns, s))) return rc;
@@ -1408,6 +1412,9 @@ WGB_EXPORT int wgb_llama2_set_prefill(wgb_llama2 *m, int enable)
         wide = !wimage(&pf.wimg_dim, c.dim) && !wimage(&pf.wimg_q, m->q_dim) && !wimage(&pf.wimg_hidden, m->hidden) && !dalloc(&pf.wx, cap * c.dim) &&
                !dalloc(&pf.wq, cap * m->q_dim) && !dalloc(&pf.wxb, cap * m->q_dim);
         for (int i = 0; i < 3 && wide; i++) wide = !dalloc(&pf.wpart[i], pf.wpart_floats);
+        const size_t counters = prefill_wide_attention_counters() * sizeof(uint32_t);
+        wide = wide && !dalloc(&pf.wattn_scratch, prefill_wide_attention_scratch_floats(m->head_size)) &&
+               cudaMalloc((void **)&pf.wattn_counters, counters) == cudaSuccess && cudaMemset(pf.wattn_counters, 0, counters) == cudaSuccess;
         if (!wide) {
             wide_free(m);
             cudaGetLastError();   // an allocation that was refused is no error of a later launch

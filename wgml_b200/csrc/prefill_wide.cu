@@ -844,10 +844,16 @@ int launch_wide_gelu_image(const float *part, uint32_t nsplit, const float *bias
 // with a running softmax; everything in f32 on the CUDA cores.  256 threads: thread (ty, tx) owns positions 4 ty .. + 3,
 // scores of rows tx + 16 j, and value columns 4 tx + 64 j.  Rows of the K and Q tiles are padded by four floats so
 // that the sixteen rows a half-warp reads sit in different banks.  Longest tiles first.
-template <uint32_t HD>
+// Few positions on a long context (a second turn of a conversation) are few blocks, each walking all the rows: blockIdx.z then
+// shares the tiles of rows of one (head, tile of positions) among blocks, which leave their unnormalised sums, maxima and
+// denominators in `scratch`; the last to arrive (a counter that wraps back to zero) merges them in the order of blockIdx.z.
+template <uint32_t HD> constexpr uint32_t WA_SLOT = 4 * (HD / 64) * 256 + 32;
+constexpr uint32_t WA_BLOCKS = 2;   // blocks per SM that share rows, most: as many as are resident
+template <uint32_t HD, bool SHARED>   // SHARED: blocks share rows (a kernel of its own: the merge costs the other one registers)
 __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__restrict__ q, const float *__restrict__ k_cache, const float *__restrict__ v_cache,
                                                                 float *__restrict__ out, uint32_t q_dim, uint32_t kv_mul, uint32_t row_stride,
-                                                                uint32_t head_stride, uint32_t pos0, uint32_t ntok)
+                                                                uint32_t head_stride, uint32_t pos0, uint32_t ntok, float4 *__restrict__ scratch,
+                                                                uint32_t *__restrict__ counters)
 {
     constexpr uint32_t LD = HD + 4, LP = 64 + 4, NC = HD / 64, NP = HD / 16;
     extern __shared__ float wa_smem[];
@@ -856,6 +862,11 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
     pdl_wait();
     const uint32_t h = blockIdx.x, t0 = (gridDim.y - 1 - blockIdx.y) * 64, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const uint32_t nq = ntok - t0 < 64 ? ntok - t0 : 64;
+    const uint32_t last = pos0 + t0 + nq - 1;
+    // this block's tiles of rows
+    const uint32_t ntiles = last / 64 + 1, nz = !SHARED ? 1u : gridDim.z < ntiles ? gridDim.z : ntiles, z = SHARED ? blockIdx.z : 0u;
+    if (z >= nz) return;
+    const uint32_t c_begin = SHARED ? 64 * (z * ntiles / nz) : 0u, c_end = SHARED ? 64 * ((z + 1) * ntiles / nz) : last + 1;
     const float *kh = k_cache + (size_t)(h / kv_mul) * head_stride, *vh = v_cache + (size_t)(h / kv_mul) * head_stride;
     const float inv_sqrt = 1.0f / sqrtf((float)HD);
     for (uint32_t i = tid; i < 64 * HD / 4; i += 256) {
@@ -873,7 +884,6 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
 #pragma unroll
         for (uint32_t c = 0; c < NC; c++) acc[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    const uint32_t last = pos0 + t0 + nq - 1;
     // a tile travels through registers, requested one phase before it is needed
     float4 pre[NP];
     auto fetch = [&](const float *base, uint32_t c0) {
@@ -893,8 +903,8 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
         }
         return __syncthreads_or(flag);
     };
-    fetch(kh, 0);
-    for (uint32_t c0 = 0; c0 <= last; c0 += 64) {
+    fetch(kh, c_begin);
+    for (uint32_t c0 = c_begin; c0 < c_end; c0 += 64) {
         place(false);
         fetch(vh, c0);
         float s[4][4];
@@ -931,7 +941,7 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
             }
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            // row 0 is always attended to, so from the first tile on the maximum is finite (or the scores are not)
+            // -inf as long as the block has met no row that the position attends to
             const float rs = mx == -INFINITY ? 1.0f : expf(mrun[i] - mx);
             mrun[i] = mx;
             float sum = 0.0f;
@@ -955,7 +965,7 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
             for (uint32_t k = 0; k < NP; k++) z = fmaf(pre[k].x, 0.0f, fmaf(pre[k].y, 0.0f, fmaf(pre[k].z, 0.0f, fmaf(pre[k].w, 0.0f, z))));
         }
         const bool one_by_one = place(z != 0.0f) != 0;
-        if (c0 + 64 <= last) fetch(kh, c0 + 64);
+        if (c0 + 64 < c_end) fetch(kh, c0 + 64);
         if (one_by_one) {
 #pragma unroll 1
             for (uint32_t j = 0; j < 64; j++) {
@@ -997,6 +1007,47 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
             }
         }
     }
+    if constexpr (SHARED) {
+        __shared__ uint32_t s_last;
+        constexpr uint32_t SLOT = WA_SLOT<HD>;   // float4 per block: sums [register][thread], then (maximum, denominator) [row]
+        const uint32_t pair = blockIdx.x * gridDim.y + blockIdx.y;
+        float4 *all = scratch + (size_t)pair * gridDim.z * SLOT, *mine = all + (size_t)z * SLOT;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+#pragma unroll
+            for (uint32_t c = 0; c < NC; c++) mine[(i * NC + c) * 256 + tid] = acc[i][c];
+            if (tx == 0) reinterpret_cast<float2 *>(mine + 4 * NC * 256)[4 * ty + i] = make_float2(mrun[i], lrun[i]);
+        }
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) s_last = atomicInc(counters + pair, nz - 1) == nz - 1;
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            float mx = -INFINITY;
+            for (uint32_t zz = 0; zz < nz; zz++) mx = fmaxf(mx, __ldcg(reinterpret_cast<const float2 *>(all + zz * SLOT + 4 * NC * 256) + 4 * ty + i).x);
+            lrun[i] = 0.0f;
+#pragma unroll
+            for (uint32_t c = 0; c < NC; c++) acc[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (uint32_t zz = 0; zz < nz; zz++) {
+                const float4 *part = all + zz * SLOT;
+                const float2 ml = __ldcg(reinterpret_cast<const float2 *>(part + 4 * NC * 256) + 4 * ty + i);
+                if (ml.x == -INFINITY && ml.y == 0.0f) continue;   // nothing but rows the position does not attend to
+                const float w = expf(ml.x - mx);
+                lrun[i] = fmaf(ml.y, w, lrun[i]);
+#pragma unroll
+                for (uint32_t c = 0; c < NC; c++) {
+                    const float4 v = __ldcg(part + (i * NC + c) * 256 + tid);
+                    acc[i][c].x = fmaf(v.x, w, acc[i][c].x);
+                    acc[i][c].y = fmaf(v.y, w, acc[i][c].y);
+                    acc[i][c].z = fmaf(v.z, w, acc[i][c].z);
+                    acc[i][c].w = fmaf(v.w, w, acc[i][c].w);
+                }
+            }
+        }
+    }
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         if (4 * ty + i < nq) {
@@ -1011,29 +1062,46 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
 
 template <uint32_t HD>
 static int launch_wide_attention_hd(const float *q, const float *k_cache, const float *v_cache, float *out, uint32_t n_heads, uint32_t kv_mul, uint32_t row_stride,
-                                    uint32_t head_stride, uint32_t pos0, uint32_t ntok, bool *attrs, cudaStream_t stream)
+                                    uint32_t head_stride, uint32_t pos0, uint32_t ntok, float *scratch, uint32_t *counters, bool *attrs, cudaStream_t stream)
 {
     const size_t smem = (size_t)(2 * 64 * (HD + 4) + 64 * 68) * sizeof(float);
     if (!*attrs) {
-        WGB_CUDA(cudaFuncSetAttribute(wide_attention_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        WGB_CUDA(cudaFuncSetAttribute(wide_attention_kernel<HD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        WGB_CUDA(cudaFuncSetAttribute(wide_attention_kernel<HD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         *attrs = true;
     }
-    WGB_CUDA(launch_pdl(wide_attention_kernel<HD>, dim3(n_heads, (ntok + 63) / 64), dim3(256), smem, stream, q, k_cache, v_cache, out, n_heads * HD, kv_mul,
-                        row_stride, head_stride, pos0, ntok));
+    // Blocks for the rows of one (head, tile of positions): as many as are resident at once, with two tiles of rows or more
+    // each.  Sixteen positions of a two-layer model of 7B widths (32 blocks) at position 4000: 2045 us a pass with one block each, 631 with nine (eight-position passes 759); a
+    // pass with more blocks than half of what is resident is as before.
+    const uint32_t pairs = n_heads * ((ntok + 63) / 64), tiles = (pos0 + ntok + 63) / 64;
+    uint32_t nz = scratch && counters ? WA_BLOCKS * (uint32_t)sm_count() / pairs : 1u;
+    if (nz > tiles / 2) nz = tiles / 2;
+    if (nz < 1) nz = 1;
+    void (*kernel)(const float *, const float *, const float *, float *, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, float4 *, uint32_t *) =
+        nz > 1 ? wide_attention_kernel<HD, true> : wide_attention_kernel<HD, false>;
+    WGB_CUDA(launch_pdl(kernel, dim3(n_heads, (ntok + 63) / 64, nz), dim3(256), smem, stream, q, k_cache, v_cache, out, n_heads * HD, kv_mul,
+                        row_stride, head_stride, pos0, ntok, reinterpret_cast<float4 *>(scratch), counters));
     return WGB_OK;
 }
+
+// What blocks that share rows leave for one another; the counters start at zero and return to it.
+size_t prefill_wide_attention_scratch_floats(uint32_t head_size)
+{
+    return (size_t)WA_BLOCKS * sm_count() * 4 * (head_size == 64 ? WA_SLOT<64> : WA_SLOT<128>);
+}
+size_t prefill_wide_attention_counters() { return (size_t)WA_BLOCKS * sm_count(); }
 
 bool prefill_wide_attention_supported(uint32_t head_size) { return head_size == 64 || head_size == 128; }
 
 int launch_wide_attention(const float *q, const float *k_cache, const float *v_cache, float *out, uint32_t n_heads, uint32_t head_size, uint32_t kv_mul,
-                          uint32_t row_stride, uint32_t head_stride, uint32_t pos0, uint32_t ntok, cudaStream_t stream)
+                          uint32_t row_stride, uint32_t head_stride, uint32_t pos0, uint32_t ntok, float *scratch, uint32_t *counters, cudaStream_t stream)
 {
     DeviceState *ds = device_state();
     if (!ds) return WGB_ERR_CUDA;
     if (head_size == 64)
-        return launch_wide_attention_hd<64>(q, k_cache, v_cache, out, n_heads, kv_mul, row_stride, head_stride, pos0, ntok, &ds->wide_attn_attrs[0], stream);
+        return launch_wide_attention_hd<64>(q, k_cache, v_cache, out, n_heads, kv_mul, row_stride, head_stride, pos0, ntok, scratch, counters, &ds->wide_attn_attrs[0], stream);
     WGB_REQUIRE(head_size == 128, "wide prompt attention: head size %u", head_size);
-    return launch_wide_attention_hd<128>(q, k_cache, v_cache, out, n_heads, kv_mul, row_stride, head_stride, pos0, ntok, &ds->wide_attn_attrs[1], stream);
+    return launch_wide_attention_hd<128>(q, k_cache, v_cache, out, n_heads, kv_mul, row_stride, head_stride, pos0, ntok, scratch, counters, &ds->wide_attn_attrs[1], stream);
 }
 
 }  // namespace wgb
