@@ -350,8 +350,15 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
     const uint32_t nstage = a.nstage;
     uint8_t *smem = reinterpret_cast<uint8_t *>(smem4);
     const uint32_t ring = smem_addr(smem + a.ring_offset);
-    // full, done: [round & 1][slot]
-    const uint32_t full0 = smem_addr(&bars[0]), done0 = smem_addr(&bars[2 * GEMV_MAX_STAGES]), empty0 = smem_addr(&bars[4 * GEMV_MAX_STAGES]);
+    // full, done: [round & 1][slot].  Whoever walks the slots keeps the byte offset of the round's half and the parity of the
+    // round's turn on it, and steps them when it passes the end of the ring.
+    constexpr uint32_t HALF = 8 * GEMV_MAX_STAGES, DONE = 2 * HALF, EMPTY = 4 * HALF;
+    const uint32_t full0 = smem_addr(&bars[0]);
+    auto next_round = [&](uint32_t &s, uint32_t &half, uint32_t &turn) {
+        s -= nstage;
+        turn ^= half ? 1u : 0u;
+        half ^= HALF;
+    };
     const uint32_t kp = a.kparts, rparts = a.rparts;
 
     // one thread per barrier: initialising them one after the other would cost a microsecond
@@ -380,15 +387,15 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
         const uint32_t gmask = ((1u << cps) - 1u) << (sb * cps);
         if (sb >= spb) return;
         const uint32_t pmask = spb * cps >= 32 ? ~0u : (1u << (spb * cps)) - 1u;   // the lanes that stay
-        uint32_t s = sb, round = 0;                              // ring slot of stage `it` and its use count (spb <= nstage)
+        uint32_t s = sb, half = 0, turn = 0;                     // ring slot of stage `it` (spb <= nstage)
         for (uint32_t it = sb; it < nst + sb; it += spb) {       // every lane: as many passes as the first
             if (it < nst) {
                 Part parts[2];
                 uint32_t n = 0;
                 const int nparts = group_parts(a, EPI, blockIdx.x + it * gridDim.x, parts, n);
-                const uint32_t full = full0 + 8 * ((round & 1) * GEMV_MAX_STAGES + s);
+                const uint32_t full = full0 + 8 * s + half;
                 if (ci == 0) {
-                    if (round) mbar_wait(empty0 + 8 * s, (round - 1) & 1, a.err, 2, a.wait_ns);
+                    if (it >= nstage) mbar_wait(full0 + EMPTY + 8 * s, half ? 0u : 1u, a.err, 2, a.wait_ns);   // release of the use before
                     mbar_expect_tx(full, nparts * n * row_bytes);
                 }
                 __syncwarp(gmask);
@@ -403,7 +410,7 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
             }
             __syncwarp(pmask);
             s += spb;
-            if (s >= nstage) { s -= nstage; round++; }
+            if (s >= nstage) next_round(s, half, turn);
         }
         return;
     }
@@ -427,14 +434,11 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
         const uint32_t nb = epilogue_batch(nstage);
         const uint32_t sub = (uint32_t)lane >> 3, ul = (uint32_t)lane & 7;
         const uint32_t gmask = 0xffu << (8 * sub);
-        uint32_t s = sub % nstage, round = sub / nstage;   // ring slot and use of stage it0 + sub
+        uint32_t s = sub, half = 0, turn = 0;   // ring slot of stage it0 + sub (nb <= nstage)
         float rms_scale = 1.0f;
         bool have_scale = false;
         for (uint32_t it0 = 0; it0 < nst; it0 += nb, s += nb) {
-            while (s >= nstage) {
-                s -= nstage;
-                round++;
-            }
+            if (s >= nstage) next_round(s, half, turn);
             const uint32_t it = it0 + sub;
             if (sub >= nb || it >= nst) continue;
             Part parts[2];
@@ -444,7 +448,7 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
             const EpiCtx c = epi_prepare(a, EPI, parts, nparts, n, ul, nunits, rope_tab);
             uint32_t ra = 0, rb = 0;
             if (c.on) unit_rows(EPI, parts, nparts, n, ul, ra, rb);
-            mbar_wait(done0 + 8 * ((round & 1) * GEMV_MAX_STAGES + s), (round >> 1) & 1, a.err, 3, a.wait_ns);
+            mbar_wait(full0 + DONE + 8 * s + half, turn, a.err, 3, a.wait_ns);
             if (PRO == PRO_RMS && !have_scale) {
                 // every consumer warp wrote its sum of squares before its first arrival on a `done` barrier
                 float ss = 0.0f;
@@ -465,7 +469,7 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
                 }
             }
             __syncwarp(gmask);
-            if (ul == 0) mbar_arrive(empty0 + 8 * s);   // stage and partial sums may be overwritten
+            if (ul == 0) mbar_arrive(full0 + EMPTY + 8 * s);   // stage and partial sums may be overwritten
             epi_finish(a, EPI, parts, c, ya, yb);
         }
         if ((EPI == EPI_STORE || EPI == EPI_RESIDUAL) && a.peer_out.n) {
@@ -682,15 +686,12 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
     float *my_part = &lane_part[warp][0][0];
     uint32_t held = ~0u;   // column step whose part of the input is in `x`
     int lane_d = lane;
-    uint32_t s = 0, round = 0, it_prev = 0;
+    uint32_t s = 0, half = 0, turn = 0, it_prev = 0;
     for (uint32_t t = cl; t < nst * rparts; t += ncl) {
         const uint32_t it = t >> a.rparts_log2, rp = t & (rparts - 1);
         s += it - it_prev;
         it_prev = it;
-        while (s >= nstage) {
-            s -= nstage;
-            round++;
-        }
+        while (s >= nstage) next_round(s, half, turn);
         uint32_t nrows = a.rs;   // rows in this stage: fewer only in the last group of a matrix
         if (EPI != EPI_QKV_ROPE) {
             Part parts[2];
@@ -701,7 +702,7 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
         const uint32_t j0 = rp * Rn;
         const uint32_t jn = min(Rn, nrows > j0 ? nrows - j0 : 0u);
         const uint32_t stage = ring + s * a.stage_bytes;
-        mbar_wait(full0 + 8 * ((round & 1) * GEMV_MAX_STAGES + s), (round >> 1) & 1, a.err, 1, a.wait_ns);
+        mbar_wait(full0 + 8 * s + half, turn, a.err, 1, a.wait_ns);
         for (uint32_t ks = kw; ks < nsteps; ks += kp) {
             const uint32_t col0 = ks * step_cols<QT>();
             if (held != ks) {
@@ -732,7 +733,7 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
         v += __shfl_xor_sync(0xffffffffu, v, 1);
         if ((lane & 7) == 0 && (uint32_t)(lane >> 3) < jn) part[s][kw][j0 + (lane >> 3)] = v;
         __syncwarp();
-        if (lane == 0) mbar_arrive(done0 + 8 * ((round & 1) * GEMV_MAX_STAGES + s));
+        if (lane == 0) mbar_arrive(full0 + DONE + 8 * s + half);
     }
 }
 
