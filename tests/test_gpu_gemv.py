@@ -129,3 +129,26 @@ def test_gemv_outlier_inputs(qtype):
         _, o64 = oracle.gemv_quant(qtype, raw, nrows, ncols, xv, want_f64=True)
         atol = ATOL * float(np.sqrt(np.mean(o64 ** 2))) if name != "zeros" else 0.0
         assert_close(o, o64, RTOL, atol, f"qtype {qtype}, {name}")
+
+
+@pytest.mark.parametrize("qtype,nrows,ncols", [
+    (ops.F32, 32000, 288),      # five warps a column part, one task a stage, 24 slots: a warp's tasks wander over the slots
+    (ops.F32, 60000, 32),       # sixteen warps a column part: the longest stride
+    (ops.Q8_0, 50257, 768),     # the same with two tasks a stage: always the same slots
+    (ops.Q4_K, 26000, 4096),    # eight warps, two tasks a stage
+    (ops.Q4_K, 26000, 6144),    # five warps, a short ring
+    (ops.Q6_K, 32000, 4096),    # seven slots, an odd number
+])
+def test_ring_slots_used_many_times(qtype, nrows, ncols):
+    """Matrices whose blocks go around the ring several times, in the ways consumer warps can meet a slot's uses; called again and
+    again, every output has the same bits."""
+    raw, x = make(qtype, nrows, ncols, 17)
+    m, xd, op = ops.GpuQuantMatrix(qtype, raw, nrows, ncols), torch.from_numpy(x).cuda(), ops.GemvQuant.from_device()
+    outs = [torch.full((nrows,), float("nan"), device="cuda") for _ in range(16)]
+    for o in outs:
+        op.dispatch(o, m, xd)
+    ops.device_status()
+    for o in outs[1:]:
+        assert torch.equal(o, outs[0])
+    _, o64 = oracle.gemv_quant(qtype, raw, nrows, ncols, x, want_f64=True)
+    assert_close(outs[0].cpu().numpy(), o64, RTOL, ATOL * max(1.0, float(np.sqrt(np.mean(o64 ** 2)))), f"qtype {qtype} {nrows}x{ncols}")
