@@ -96,11 +96,14 @@ def test_output_at_any_word(case, offset):
     assert (buf[:offset] == 7.0).all() and (buf[offset + n:] == 7.0).all()
 
 
-@pytest.mark.parametrize("case", [(512, 32, 128, 1, 300), (512, 32, 64, 2, 300), (512, 32, 128, 4, 300), (4224, 64, 128, 8, 1300)])
+@pytest.mark.parametrize("case", [
+    (512, 32, 128, 1, 300), (512, 32, 64, 2, 300), (512, 32, 128, 4, 300), (4224, 64, 128, 8, 1300),
+    (512, 12, 64, 3, 300), (2112, 32, 128, 1, 2100), (2112, 60, 64, 5, 2100),   # split kernel (one chunk a block, several); rows, one query head
+])
 @pytest.mark.parametrize("masked", [(0, 8), (0, 23), (0, 130), (8, 16), (40, 290), (1, 297)])
 def test_rows_scored_minus_infinity_weigh_nothing(case, masked):
     """Cache rows a host has masked with keys of -inf (left padding): whole groups, warps and blocks of the row-streaming
-    kernel see nothing but -inf, and the answer is that of the other rows (RTOL / ATOL as everywhere)."""
+    kernel and chunks of the split kernel see nothing but -inf, and the answer is that of the other rows (RTOL / ATOL as everywhere)."""
     seq_len, n_heads, hs, kv_mul, pos = case
     rng = np.random.default_rng(9)
     n_kv = n_heads // kv_mul

@@ -35,6 +35,10 @@ size_t attn_scratch_floats(uint32_t n_heads, uint32_t head_size, uint32_t seq_le
     return (size_t)n_heads * attn_num_splits(seq_len) * (head_size + 4);
 }
 
+// Where running maxima start: as good as -inf for every finite score, and rows whose scores are all -inf (keys a host has
+// masked) get weights of exp(-inf) = 0 and not of exp(-inf + inf) = NaN.
+constexpr float ATT_LOWEST = -3.402823466e+38f;
+
 // QH = query heads per KV head handled at once; VC = float4 chunks of a head per lane (1: head
 // sizes up to 128, 2: up to 256).
 // MULTI: a block may get several chunks (long contexts, few heads) and keeps a running softmax over them;
@@ -54,7 +58,7 @@ __device__ __forceinline__ void attn_merge_chunks(const AttnArgs &a, uint32_t kv
         __shared__ float s_M[QH];
 #pragma unroll
         for (int j = 0; j < QH; j++) {
-            float m = -INFINITY;
+            float m = ATT_LOWEST;
             if (hq0 + j < kv_mul) {
                 const float *base = a.scratch + (size_t)(kvh * kv_mul + hq0 + j) * max_splits * (hs + 4);
                 for (uint32_t sp = threadIdx.x; sp < nsplit_active; sp += ATT_NT) m = fmaxf(m, __ldcg(base + (size_t)sp * (hs + 4) + hs));
@@ -127,7 +131,7 @@ __device__ __forceinline__ void attn_merge_chunks(const AttnArgs &a, uint32_t kv
         float4 o[VC];
 #pragma unroll
         for (int c = 0; c < VC; c++) o[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-        float Mw = -INFINITY, Lw = 0.0f;
+        float Mw = ATT_LOWEST, Lw = 0.0f;
         for (uint32_t sp = warp; sp < nsplit_active; sp += ATT_WARPS) {
             const float *row = base + (size_t)sp * (hs + 4);
             const float ms = __ldcg(row + hs), ls = __ldcg(row + hs + 1);
@@ -138,7 +142,7 @@ __device__ __forceinline__ void attn_merge_chunks(const AttnArgs &a, uint32_t kv
                 v[c] = ch < nchunk ? __ldcg(reinterpret_cast<const float4 *>(row) + ch) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
             const float mn = fmaxf(Mw, ms);
-            const float rs = expf(Mw - mn), w = expf(ms - mn);   // rs = 0 at the warp's first chunk (Mw = -inf)
+            const float rs = expf(Mw - mn), w = expf(ms - mn);   // (Lw = 0 at the warp's first chunk)
             Mw = mn;
             Lw = fmaf(Lw, rs, ls * w);
 #pragma unroll
@@ -272,7 +276,7 @@ __global__ void __launch_bounds__(ATT_NT, (QH == 1 && VC == 1) ? 3 : (QH == 4 &&
     float4 acc[QH][VC];
 #pragma unroll
     for (int j = 0; j < QH; j++) {
-        M[j] = -INFINITY;
+        M[j] = ATT_LOWEST;
         L[j] = 0.0f;
 #pragma unroll
         for (int c = 0; c < VC; c++) acc[j][c] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -347,7 +351,7 @@ __global__ void __launch_bounds__(ATT_NT, (QH == 1 && VC == 1) ? 3 : (QH == 4 &&
         // Chunk maximum per query head, then exponentials against the running maximum and their sum.
 #pragma unroll
         for (int j = 0; j < QH; j++) {
-            float m = -INFINITY;
+            float m = ATT_LOWEST;
             for (uint32_t tl = threadIdx.x; tl < nt; tl += ATT_NT) m = fmaxf(m, s_score[j][tl]);
             m = warp_max(m);
             if (lane == 0) s_red[j][warp] = m;
@@ -360,7 +364,7 @@ __global__ void __launch_bounds__(ATT_NT, (QH == 1 && VC == 1) ? 3 : (QH == 4 &&
 #pragma unroll
             for (int w = 1; w < ATT_WARPS; w++) m = fmaxf(m, s_red[j][w]);
             const float mn = MULTI ? fmaxf(M[j], m) : m;
-            rescale[j] = MULTI ? expf(M[j] - mn) : 0.0f;   // 0 for the first chunk (M = -inf)
+            rescale[j] = MULTI ? expf(M[j] - mn) : 0.0f;   // (L = 0 before the first chunk)
             M[j] = mn;
         }
         __syncthreads();
@@ -852,7 +856,7 @@ __global__ void __launch_bounds__(ATT_NT, 1) attn_rows_kernel(const __grid_const
 #pragma unroll
     for (int j = 0; j < QH; j++) {
         q[j] = on ? __ldcg(reinterpret_cast<const float4 *>(a.q + (size_t)(kvh * kv_mul + j) * hs) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-        M[j] = -INFINITY;
+        M[j] = ATT_LOWEST;
         L[j] = 0.0f;
         acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -907,9 +911,8 @@ __global__ void __launch_bounds__(ATT_NT, 1) attn_rows_kernel(const __grid_const
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
             const float mn = fmaxf(M[j], m);
-            const float mz = mn == -INFINITY ? 0.0f : mn;   // all of the warp's scores so far are -inf: weights of 0, not of NaN
-            const float rs = expf(M[j] - mz);         // 0 at the warp's first group (M = -inf)
-            const float e = expf(sv - mz);            // 0 for positions past the end
+            const float rs = expf(M[j] - mn);         // (sums and vector are 0 before the warp's first group)
+            const float e = expf(sv - mn);            // 0 for positions past the end
             M[j] = mn;
             float psum = 0.0f;
             acc[j].x *= rs;
@@ -951,11 +954,10 @@ __global__ void __launch_bounds__(ATT_NT, 1) attn_rows_kernel(const __grid_const
         float mb = s_red[j][0];
 #pragma unroll
         for (int w = 1; w < ATT_WARPS; w++) mb = fmaxf(mb, s_red[j][w]);
-        const float mz = mb == -INFINITY ? 0.0f : mb;
         float sv = 0.0f, lb = 0.0f;
 #pragma unroll
         for (int w = 0; w < ATT_WARPS; w++) {
-            const float f = expf(s_red[j][w] - mz);   // 0 for a warp without a score above -inf
+            const float f = expf(s_red[j][w] - mb);   // (0 or 1 for a warp without positions, whose sums are 0)
             sv = fmaf(s_acc[((size_t)w * QH + j) * astr + i], f, sv);
             lb = fmaf(s_sum[j][w], f, lb);
         }
@@ -985,10 +987,9 @@ __global__ void __launch_bounds__(ATT_NT, 1) attn_rows_kernel(const __grid_const
     constexpr uint32_t WPH = ATT_WARPS / QH;
     const uint32_t j = warp % QH, part = warp / QH;
     const float *base = a.scratch + (size_t)(kvh * kv_mul + j) * max_splits * astr;
-    float Mj = -INFINITY;
+    float Mj = ATT_LOWEST;
     for (uint32_t sp = lane; sp < nsplit_active; sp += 32) Mj = fmaxf(Mj, __ldcg(base + (size_t)sp * astr + hs));
     Mj = warp_max(Mj);
-    if (Mj == -INFINITY) Mj = 0.0f;   // no score above -inf at all: 0 / 0, as the definition has it
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
     float Lt = 0.0f;
 #pragma unroll 8
