@@ -1100,6 +1100,8 @@ static int launch_stream_any(const AttnArgs &a, uint32_t nchunks, cudaStream_t s
     return launch_stream<1>(a, nchunks, n_kv, 1, stream, pdl);
 }
 
+constexpr int ATT_CLASS = 1 << 16;   // answers of a sizing query start here, above every status
+
 template <int QH, int VC>
 static int launch_split(const AttnArgs &a, uint32_t nchunks, uint32_t nchunks_hint, uint32_t n_kv, uint32_t zgroups,
                         cudaStream_t stream, bool pdl)
@@ -1117,36 +1119,44 @@ static int launch_split(const AttnArgs &a, uint32_t nchunks, uint32_t nchunks_hi
         occ_single[dev] = one < 1 ? 1 : one;
     }
     const int per_sm_single = occ_single[dev], per_sm_multi = occ_multi[dev];
-    const uint32_t heads = n_kv * zgroups;
-    if (!a.q) {   // sizing query (attn_sizing_class): no launch
-        return (uint64_t)nchunks_hint * heads > (uint64_t)per_sm_single * (uint32_t)sm_count() ? 1 : 0;
-    }
+    const uint32_t heads = n_kv * zgroups, sms = (uint32_t)sm_count();
     // `nchunks_hint`: chunks up to the furthest position this launch is expected to serve (performance only:
-    // either kernel is correct for any position inside the cache).
-    const bool multi = (uint64_t)nchunks_hint * heads > (uint64_t)per_sm_single * (uint32_t)sm_count();
+    // any kernel is correct for any position inside the cache).
+    const bool multi = (uint64_t)nchunks_hint * heads > (uint64_t)per_sm_single * sms;
     // Beyond one wave, contiguous rows and up to two query heads per KV head: the streaming kernel (a decode step of four
     // 7B layers at 3000 positions: 0.283 ms, with the row-streaming kernel 0.299).
-    if (multi && VC == 1 && a.p.kv_mul <= 2 && (a.row_stride ? a.row_stride : a.p.kv_dim) == a.p.head_size)
-        return launch_stream_any(a, nchunks, stream, pdl);
-    // One, two, four or eight query heads per KV head, head sizes up to 128: the row-streaming kernel, everywhere but in
-    // a decode step (position on the device) with up to two heads and a context of one wave.  Its blocks fill
-    // the shared memory, so the matrix-vector launch behind it cannot start prefetching beside it: tiny f32 decode 15.5
-    // ms with the split kernel, 16.2 with this one, GPT-2 32.1 and 34.2, 7B 77.5 and 78.1; but Qwen2 (four heads)
-    // 20.5 and 19.8.  Stand-alone it is the faster one with many KV heads (32 heads on 32, 512 positions: 10.1 and 8.2 us).
-    // With fewer than eight KV heads (sixteen, at one or two query heads each) a context of one wave stays with the
-    // split kernel as well: its blocks are one chunk each, and here one block merges up to 37 splits (twelve KV heads,
-    // one query head each, 2200 positions: 9.8 us against 10.8); but for decode steps with four heads per KV head, the
-    // Qwen2 figure above (four KV heads).
-    const bool one_wave = a.pos && a.p.kv_mul <= 4 ? a.p.kv_mul == 4 : n_kv >= (a.p.kv_mul <= 2 ? 16u : 8u);
-    if (VC == 1 && (multi || one_wave)) {
+    const bool stream_kernel = multi && VC == 1 && a.p.kv_mul <= 2 && (a.row_stride ? a.row_stride : a.p.kv_dim) == a.p.head_size;
+    // One, two, four or eight query heads per KV head, head sizes up to 128: the row-streaming kernel beyond one wave.  (Microseconds,
+    // split kernel and this one.  Stand-alone calls: replayed graphs over caches beyond the L2, KV heads 1 to 148, contexts
+    // 64 to 8192.  Decode steps: two layers, KV heads 1 to 64.)
+    //   * not where one block per KV head leaves 30 % of the SMs idle, with four query heads per KV head on more than eight chunks:
+    //     75 KV heads of size 128, 1024 positions 37.7 and 40.9, 8192 positions 211 and 282 (200 positions: 18.5 and 14.5); but
+    //     104 KV heads 302 and 282.  (Two blocks each: 50 KV heads 28.3 and 23.8, 137 and 146.  Eight query heads: 75 KV
+    //     heads of size 64, 4096 positions 273 and 189.)
+    //   * one wave, stand-alone: two query heads per KV head from sixteen KV heads on (16 of size 128, 512 positions: 8.7 and
+    //     7.9), four and eight from eight on (8 of four: 11.3 and 9.2; of eight: 11.6 and 10.2); a single query head never
+    //     (32 KV heads, 512 positions: 7.7 and 9.2).
+    //   * one wave, decode step (position on the device): its blocks fill the shared memory, so that the matrix-vector
+    //     launch behind it cannot start prefetching beside it.  Up to two query heads the split kernel (GPT-2 decode
+    //     32.1 and 34.2 ms); four heads this one (8 KV heads, 900 positions: 81.2 and 71.6 a step); eight heads this one from
+    //     eight KV heads of size 64 and 512 positions on (84.0 and 76.1; but 200 positions of 16 KV heads 143.2 and 146.9, and 8
+    //     of size 128 at 500 positions 150.6 and 153.6).
+    const bool idle = a.p.kv_mul == 4 && 2 * n_kv > sms && 10 * n_kv < 7 * sms && nchunks_hint > 8;
+    const bool fits = VC == 1 && (a.p.kv_mul == 1 || a.p.kv_mul == 2 || a.p.kv_mul == 4 || a.p.kv_mul == 8);
+    const bool one_wave = a.pos ? a.p.kv_mul == 4 || (a.p.kv_mul == 8 && n_kv >= 8 && a.p.head_size <= 64 && nchunks_hint > 8)
+                                : a.p.kv_mul > 1 && n_kv >= (a.p.kv_mul == 2 ? 16u : 8u);
+    const bool rows_kernel = !stream_kernel && fits && (multi ? !idle : one_wave);
+    if (!a.q) return ATT_CLASS + (multi ? 1 : 0) + (rows_kernel ? 2 : 0);   // sizing query (attn_sizing_class): no launch
+    if (stream_kernel) return launch_stream_any(a, nchunks, stream, pdl);
+    if (rows_kernel) {
         if (a.p.kv_mul == 1) return launch_rows<1>(a, nchunks, stream, pdl);
         if (a.p.kv_mul == 2) return launch_rows<2>(a, nchunks, stream, pdl);
         if (a.p.kv_mul == 4) return launch_rows<4>(a, nchunks, stream, pdl);
-        if (a.p.kv_mul == 8) return launch_rows<8>(a, nchunks, stream, pdl);
+        return launch_rows<8>(a, nchunks, stream, pdl);
     }
     uint32_t splits = nchunks;
     if (multi) {
-        splits = (uint32_t)per_sm_multi * (uint32_t)sm_count() / heads;
+        splits = (uint32_t)per_sm_multi * sms / heads;
         if (splits < 1) splits = 1;
         if (splits > nchunks) splits = nchunks;
     }
@@ -1186,15 +1196,15 @@ int launch_attention(const AttnArgs &a, cudaStream_t stream, bool pdl)
     return big ? launch_split<1, 2>(a, nchunks, nh, n_kv, zg, stream, pdl) : launch_split<1, 1>(a, nchunks, nh, n_kv, zg, stream, pdl);
 }
 
-// 0 / 1: which of the two launch shapes launch_attention picks for positions up to p.pos (a caller that
-// records launches for later replay re-records when the class changes); negative on error.
+// Which launch launch_attention picks for positions up to p.pos, as a small number (a caller that records launches for
+// later replay re-records when it changes); negative on error.
 int attn_sizing_class(const wgb_attn_params &p)
 {
     AttnArgs a = {};
     a.p = p;
     a.pos = reinterpret_cast<const uint32_t *>(&a);   // "position on the device": p.pos is the bound
     const int r = launch_attention(a, nullptr, false);
-    return r > 1 ? -1 : r;
+    return r >= ATT_CLASS ? r - ATT_CLASS : -1;
 }
 
 }  // namespace wgb
