@@ -9,16 +9,23 @@
 // RmsNorm / LayerNorm / Silu / GELU / BatchedMultiqueryAttention of one position, for many.
 //
 // Arithmetic.  A unit is 256 columns.  Activations: x = X * 2^e with one exponent per position and unit, |X| <= 2048,
-// written as two f16 digits X = hi + lo (hi an integer; |lo| <= 1/2 rounded to eleven bits, so X is good to 2^-13
-// on average: finer than the integers of 2^22 of the other products, which makes up for the exponent being
-// shared by 256 columns instead of 32).  Weights: the part of a weight that varies inside a unit, as one or two f16
-// numbers,
-//   Q4_K  scale * code           <= 945: one plane;  d per row and unit, mins through a product of their own
+// written as two f16 digits X = hi + lo.  hi has eleven bits of the loudest value of its 32 columns, in steps no finer than
+// 2^-PW_QUIET; lo is the rest rounded to eleven bits, so X is good to 2^-13 (loud groups) to 2^-16: 2^-24 to 2^-27 of the
+// unit's loudest value.  Weights: the part of a weight that varies inside a unit, as one or two f16 numbers,
+//   Q4_K  scale * code - centre  <= 520 in magnitude: one plane;  d per row and unit.  What centring takes off (codes are
+//         all of one sign, and inputs of one sign would leave the accumulator's bits) comes back with the mins, which it
+//         all but cancels: the group coefficients d centre - dmin min times the groups' sums of X, an MMA of their own
 //   Q6_K  scale * (code - 32)    <= 4096 in magnitude: 16 a1 + a2, two planes;  d per row and unit
-//   Q8_0  code * d_group / 2^E   18 bits: a1 + a2 (a1 an integer <= 512), two planes;  2^E the row's power of two
-// The products of the large digits are integers below 2^22 and their sum over a unit stays within or near the 24 bits of
-// the f32 accumulator.  One accumulator takes all of a unit's products, the small ones (a2, lo) first: what they add
-// below the final sum's last bit is dropped once, not per product.
+//   Q8_0  code * d_group / 2^E   two planes: a1 the upper nine bits, a2 the rest, exact while the group's scale is no less
+//         than 1/64 of the largest of the row's eight;  2^E the row's power of two
+// On even data the products of the large digits are multiples of one step (16 for Q6_K) and a unit's sum of them stays within
+// about 24 bits, those of the f32 accumulator.  One accumulator takes all of a unit's products, the small ones (a2, lo)
+// first: what they add below the final sum's last bit is dropped once, not per product (and towards zero: with inputs
+// near a constant and codes not centred the error was 2 to 3e-6 of the result, fifteen times the eight-position product's).
+// Error of a product against 64 bits (mean over rows of the 2-norm, 1024 to 11008 columns; the eight-position product in
+// brackets): even data 1.3 to 1.5e-7 (2.7 to 3.4e-7), heavy tails 1.9 to 2.2e-7 (4.2e-7 to 1.3e-6), a column in 256 a hundred
+// times as loud 2.2 to 2.5e-7 (5.7e-7 to 1.6e-6), inputs near a constant 1.0 to 1.2e-7 (1.2 to 1.7e-7), Q8_0 scales spread by e and
+// e^2 1.5 to 1.7e-7 (2.8 to 3.4e-7).
 #include "kernels.h"
 #include "tc_common.cuh"
 
@@ -36,7 +43,7 @@ constexpr uint32_t PW_B_STEP = 2 * PW_MAXN * 128;                  // one digit 
 constexpr uint32_t PW_B_RING = 4;
 constexpr uint32_t PW_AUX = 36 * PW_MAXN;                          // per unit: sums of the mins' product, exponents
 constexpr uint32_t PW_X_RING = 3;
-constexpr uint32_t PW_AMIN = 2 * TC_TILE_ROWS * 16;                // mins as f16, [two K-cores][row], in shared memory
+constexpr uint32_t PW_AMIN = 4 * TC_TILE_ROWS * 16;                // group coefficients as f16, [digit][two K-cores][row], in shared memory
 // Tensor memory: two sets of sums (128 columns), the min sums (128), four weight operands (32).
 constexpr uint32_t PW_TMEM_COLS = 512;
 constexpr uint32_t PW_TMEM_MIN = 2 * PW_MAXN;
@@ -53,6 +60,10 @@ template <int FMT> constexpr uint32_t pw_smem()
 {
     return PW_B_RING * PW_B_STEP + PwFmt<FMT>::RAW_RING * PwFmt<FMT>::RAW + 2 * PwFmt<FMT>::AMIN + PW_X_RING * PW_AUX;
 }
+// A group of 32 columns that is quieter than the loudest of its unit takes a finer large digit, by as many bits as it is
+// quieter, PW_QUIET at most: a digit finer than the accumulator's last bit (2^-2 to 2^0 in the middle of a unit's sums) is cut off
+// at every MMA instead of once, and always towards zero.
+constexpr uint32_t PW_QUIET = 3;
 constexpr uint32_t PW_STATIC = 4 * TC_TILE_ROWS * 8 + 512;         // row scales, barriers
 static_assert(pw_smem<WGB_Q4_K>() + 1024 + PW_STATIC <= 227 * 1024 && pw_smem<WGB_Q6_K>() + 1024 + PW_STATIC <= 227 * 1024 &&
                   pw_smem<WGB_Q8_0>() + 1024 + PW_STATIC <= 227 * 1024,
@@ -149,6 +160,16 @@ __device__ __forceinline__ uint64_t f2fma(uint64_t a, uint64_t b, uint64_t c)
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
+__device__ __forceinline__ uint64_t f2add(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b)
+{
+    asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
 __device__ __forceinline__ uint64_t f2mul(uint64_t a, uint64_t b)
 {
     uint64_t r;
@@ -167,8 +188,23 @@ __device__ __forceinline__ uint32_t pw_q80_exp(uint4 sc)
     return ex < 100u ? 100u : (ex > 142u ? 142u : ex);
 }
 
+// Exponent field of twice the unit in which a Q4_K row's group coefficients d centre - dmin min are written: they stay
+// within 128 max(8 |d|, |dmin|) (centres are at most 8 * 63 + 16), 2^14 units.
+__device__ __forceinline__ uint32_t pw_coef_exp(float2 dm)
+{
+    const uint32_t ex = (__float_as_uint(fmaxf(8.0f * fabsf(dm.x), fabsf(dm.y))) >> 23) & 0xffu;
+    return (ex < 100u ? 100u : (ex > 146u ? 146u : ex)) - 5u;
+}
+
+// Two scales as f16 -> what pw_unpack takes off the low nibbles' scale * code.
+__device__ __forceinline__ __half2 pw_centre(__half2 sc)
+{
+    return __hneg2(__hfma2(sc, __float2half2_rn(1024.0f), __hmul2(sc, __float2half2_rn(-1032.0f))));
+}
+
 // Weight operand of one step for row r: the 64 columns of chunk c of the unit at `raw`, plane 0 = the small one of a
 // two-plane format, as 32 words of two f16.
+// Of every four columns the words hold (0, 2) and (1, 3), which saves Q4_K a byte permutation; so does the activation image.
 template <int FMT>
 __device__ __forceinline__ void pw_unpack(uint32_t (&v)[32], uint32_t raw, uint32_t r, uint32_t c, bool small_plane)
 {
@@ -178,12 +214,12 @@ __device__ __forceinline__ void pw_unpack(uint32_t (&v)[32], uint32_t raw, uint3
         const uint32_t j0 = 2 * c;
         const uint32_t sc_lo = hdr.y & 0x3f3f3f3fu, sc_hi = (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u);
         const uint32_t scw = ((j0 & 4) ? sc_hi : sc_lo) >> (8 * (j0 & 3));
-        // 1024 + code and 1024 + 16 code as f16, times the scale (a sixteenth of it), minus 1024 (64) times the scale:
-        // every intermediate is exact
+        // scale * code - centre, the centre close to 8 * scale.  Low nibbles: 1024 + code as f16, times the scale, minus 1032
+        // times the scale as f16 has it (pw_centre).  High ones: 1024 + 16 code, times a sixteenth of the scale, minus 72 times
+        // the scale.  The results, integers below 2^10, are exact.
         const __half2 s0 = __half2half2(__ushort2half_rn((unsigned short)(scw & 0xffu)));
         const __half2 s1 = __half2half2(__ushort2half_rn((unsigned short)((scw >> 8) & 0xffu)));
-        const __half2 o0 = __hmul2(s0, __float2half2_rn(-1024.0f)), o1 = __hmul2(s1, __float2half2_rn(-64.0f));
-        const __half2 s1s = __hmul2(s1, __float2half2_rn(0.0625f));
+        const __half2 o0 = __hmul2(s0, __float2half2_rn(-1032.0f)), o1 = __hmul2(s1, __float2half2_rn(-72.0f)), s1s = __hmul2(s1, __float2half2_rn(0.0625f));
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const uint4 q = lds128(raw + r * 144 + 16 + 32 * c + 16 * h);
@@ -192,7 +228,7 @@ __device__ __forceinline__ void pw_unpack(uint32_t (&v)[32], uint32_t raw, uint3
             for (int k = 0; k < 4; k++) {
 #pragma unroll
                 for (int p = 0; p < 2; p++) {
-                    const uint32_t t = __byte_perm(qw[k], 0u, p ? 0x4342 : 0x4140);
+                    const uint32_t t = qw[k] >> (8 * p);
                     v[8 * h + 2 * k + p] = h2u(__hfma2(u2h((t & 0x000f000fu) | 0x64006400u), s0, o0));
                     v[16 + 8 * h + 2 * k + p] = h2u(__hfma2(u2h((t & 0x00f000f0u) | 0x64006400u), s1s, o1));
                 }
@@ -217,7 +253,7 @@ __device__ __forceinline__ void pw_unpack(uint32_t (&v)[32], uint32_t raw, uint3
                     const uint32_t q = ((qlw[k] >> (4 * (c & 1))) & 0x0f0f0f0fu) | (((qhw[k] >> (2 * h)) & 0x03030303u) << 4);
 #pragma unroll
                     for (int p = 0; p < 2; p++) {
-                        const __half2 qv = __hsub2(u2h(__byte_perm(q, 0x64646464u, p ? 0x4342 : 0x4140)), c1056);
+                        const __half2 qv = __hsub2(u2h(__byte_perm(q, 0x64646464u, p ? 0x4341 : 0x4240)), c1056);
                         const __half2 a1 = __hsub2(__hfma2(qv, sc, magic), magic);   // multiple of 16
                         v[16 * h + 8 * cc + 2 * k + p] = small_plane ? h2u(__hfma2(qv, sc, __hneg2(a1))) : h2u(a1);
                     }
@@ -226,13 +262,16 @@ __device__ __forceinline__ void pw_unpack(uint32_t (&v)[32], uint32_t raw, uint3
         }
     } else {
         const uint4 scs = lds128(raw + TC_TILE_ROWS * 256 + r * 16);
-        const float norm = __uint_as_float((255u - pw_q80_exp(scs)) << 23);   // 2^(2 - E): d norm < 4
+        const float norm = __uint_as_float((259u - pw_q80_exp(scs)) << 23);   // 2^(6 - E): d norm < 64
         const uint32_t scw = c == 0 ? scs.x : c == 1 ? scs.y : c == 2 ? scs.z : scs.w;
-        const __half2 c1152 = __float2half2_rn(1152.0f), magic = __float2half2_rn(1536.0f);
+        const __half2 c1152 = __float2half2_rn(1152.0f);
         const uint32_t row = raw + (c >> 1) * 16384 + r * 128;
 #pragma unroll
         for (uint32_t h = 0; h < 2; h++) {
             const __half2 ds = __float2half2_rn(__half2float(__ushort_as_half((unsigned short)(h ? (scw >> 16) : (scw & 0xffffu)))) * norm);
+            // 768 times the power of two at or below |ds| (for the largest scale in [32, 64): 768 * 32): adding it leaves the
+            // product's upper nine bits, and what is left is exact in eight (a product has 18 bits)
+            const __half2 magic = __hmul2(__hmax2(u2h(h2u(ds) & 0x7c007c00u), __float2half2_rn(32.0f / (1 << PW_QUIET))), __float2half2_rn(768.0f));
 #pragma unroll
             for (uint32_t cc = 0; cc < 2; cc++) {
                 const uint4 qq = lds128(row + (((4 * (c & 1) + 2 * h + cc) ^ sw) << 4));
@@ -242,8 +281,8 @@ __device__ __forceinline__ void pw_unpack(uint32_t (&v)[32], uint32_t raw, uint3
                     const uint32_t u = qw[k] ^ 0x80808080u;
 #pragma unroll
                     for (int p = 0; p < 2; p++) {
-                        const __half2 qv = __hsub2(u2h(__byte_perm(u, 0x64646464u, p ? 0x4342 : 0x4140)), c1152);
-                        const __half2 a1 = __hsub2(__hfma2(qv, ds, magic), magic);   // an integer
+                        const __half2 qv = __hsub2(u2h(__byte_perm(u, 0x64646464u, p ? 0x4341 : 0x4240)), c1152);
+                        const __half2 a1 = __hsub2(__hfma2(qv, ds, magic), magic);
                         v[16 * h + 8 * cc + 2 * k + p] = small_plane ? h2u(__hfma2(qv, ds, __hneg2(a1))) : h2u(a1);
                     }
                 }
@@ -429,10 +468,14 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                 if (!ok) break;
                 if (FMT == WGB_Q4_K) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (tc_elect()) {
-                    // sum over the eight groups of min x (sum of the group's X), both digits of the sums in one MMA
-                    if (FMT == WGB_Q4_K)
-                        pw_mma_ss(tmem_base + PW_TMEM_MIN, tc_smem_desc(sm_min + u * F::AMIN, TC_TILE_ROWS * 16, 128),
-                                  tc_smem_desc(sm_aux + (m % NX) * PW_AUX, np * 16, 128), idesc, 0u);
+                    // sum over the eight groups of coefficient x (sum of the group's X): both digits of the sums in one MMA, one for
+                    // either digit of the coefficient, the small one first
+                    if (FMT == WGB_Q4_K) {
+                        const uint64_t sums = tc_smem_desc(sm_aux + (m % NX) * PW_AUX, np * 16, 128);
+                        const uint32_t coef = sm_min + u * F::AMIN;
+                        pw_mma_ss(tmem_base + PW_TMEM_MIN, tc_smem_desc(coef + 2 * TC_TILE_ROWS * 16, TC_TILE_ROWS * 16, 128), sums, idesc, 0u);
+                        pw_mma_ss(tmem_base + PW_TMEM_MIN, tc_smem_desc(coef, TC_TILE_ROWS * 16, 128), sums, idesc, 1u);
+                    }
                     tc_commit(bar_d(u));
                 }
                 __syncwarp();
@@ -478,35 +521,56 @@ __global__ void __launch_bounds__(PW_NT, 1) gemm_wide_kernel(const __grid_consta
                         // Once per unit, off the path of its first MMAs.  (The MMAs of two units back are through: a chunk of
                         // the unit before has just been read.)
                         if (grp == 0) {
-                            float d, dmin = 0.0f;
+                            float d, coef = 0.0f;
                             if constexpr (FMT == WGB_Q4_K) {
                                 uint32_t dm;
                                 asm volatile("ld.shared.u32 %0, [%1];" : "=r"(dm) : "r"(raw + r * 144));
                                 const float2 f = __half22float2(u2h(dm));
                                 d = f.x;
-                                dmin = f.y * -2.0f;
+                                coef = __uint_as_float(pw_coef_exp(f) << 23);   // twice the coefficients' unit: the sums are halves
                             } else if constexpr (FMT == WGB_Q6_K) {
                                 uint32_t db;
                                 asm volatile("ld.shared.u16 %0, [%1];" : "=r"(db) : "r"(raw + TC_TILE_ROWS * 208 + r * 2));
                                 d = __half2float(__ushort_as_half((unsigned short)db));
                             } else {
-                                d = __uint_as_float((pw_q80_exp(lds128(raw + TC_TILE_ROWS * 256 + r * 16)) - 1u) << 23);   // 2^(E - 2)
+                                d = __uint_as_float((pw_q80_exp(lds128(raw + TC_TILE_ROWS * 256 + r * 16)) - 5u) << 23);   // 2^(E - 6)
                             }
-                            rowscale[m & 3][r] = make_float2(d, dmin);
+                            rowscale[m & 3][r] = make_float2(d, coef);
                             __syncwarp();
                             if (lane == 0) mbar_arrive(bar_r(m & 3));
-                        } else if (FMT == WGB_Q4_K) {
-                            // the row's eight mins, once per K-core: for either digit of the group sums
+                        }
+                        if constexpr (FMT == WGB_Q4_K) {
+                            // Of the row's eight group coefficients d centre - dmin min (what centring took off the unit's products, and the
+                            // mins) the four of this half, in two digits, each once per K-core: for either digit of the group sums.
                             const uint4 hdr = lds128(raw + r * 144);
-                            const uint32_t m_lo = hdr.z & 0x3f3f3f3fu, m_hi = ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u);
-                            const __half2 k1024 = __float2half2_rn(1024.0f);
-                            const uint32_t v0 = h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4140)), k1024)),
-                                           v1 = h2u(__hsub2(u2h(__byte_perm(m_lo, 0x64646464u, 0x4342)), k1024)),
-                                           v2 = h2u(__hsub2(u2h(__byte_perm(m_hi, 0x64646464u, 0x4140)), k1024)),
-                                           v3 = h2u(__hsub2(u2h(__byte_perm(m_hi, 0x64646464u, 0x4342)), k1024));
-                            const uint32_t at = sm_min + (m & 1) * F::AMIN + r * 16;
-                            sts128(at, v0, v1, v2, v3);
-                            sts128(at + TC_TILE_ROWS * 16, v0, v1, v2, v3);
+                            const float2 f = __half22float2(u2h(hdr.x));
+                            const float inv = __uint_as_float((255u - pw_coef_exp(f)) << 23);   // one over the unit
+                            const float d1 = f.x * inv, dm = -f.y * inv;
+                            const uint64_t d2 = f2pack(d1, 8.0f * d1), dm2 = f2pack(dm, dm), off = f2pack(-8388608.0f, -8388608.0f), one = f2pack(-1.0f, -1.0f);
+                            const uint32_t sc = grp ? (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u) : hdr.y & 0x3f3f3f3fu;
+                            const uint32_t mi = grp ? ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u) : hdr.z & 0x3f3f3f3fu;
+                            auto two = [&](uint32_t w, uint32_t b) {   // bytes b and b + 1 as floats
+                                return f2add(f2pack(__uint_as_float(__byte_perm(w, 0x4b000000u, 0x7550 + b)), __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7551 + b))), off);
+                            };
+                            const float2 even = __half22float2(pw_centre(__hsub2(u2h(__byte_perm(sc, 0x64646464u, 0x4240)), __float2half2_rn(1024.0f))));
+                            uint32_t c1[2], c2[2];
+#pragma unroll
+                            for (uint32_t i = 0; i < 2; i++) {
+                                const float odd = __uint_as_float(__byte_perm(sc, 0x4b000000u, 0x7551 + 2 * i)) - 8388608.0f;
+                                const uint64_t w = f2fma(f2pack(i ? even.y : even.x, odd), d2, f2mul(two(mi, 2 * i), dm2));
+                                float w0, w1;
+                                f2unpack(w, w0, w1);
+                                const __half2 hi = __floats2half2_rn(w0, w1);
+                                const float2 hf = __half22float2(hi);
+                                f2unpack(f2fma(f2pack(hf.x, hf.y), one, w), w0, w1);
+                                c1[i] = h2u(hi);
+                                c2[i] = h2u(__floats2half2_rn(w0, w1));
+                            }
+                            const uint32_t at = sm_min + (m & 1) * F::AMIN + r * 16 + 8 * grp;
+                            sts64(at, c1[0], c1[1]);
+                            sts64(at + TC_TILE_ROWS * 16, c1[0], c1[1]);
+                            sts64(at + 2 * TC_TILE_ROWS * 16, c2[0], c2[1]);
+                            sts64(at + 3 * TC_TILE_ROWS * 16, c2[0], c2[1]);
                             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                         }
                     }
@@ -670,11 +734,17 @@ __device__ __forceinline__ void wide_image_unit(uint8_t *__restrict__ image, uin
     float mx = 0.0f;
 #pragma unroll
     for (int i = 0; i < 8; i++) mx = fmaxf(mx, fabsf(v[i]));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    const uint32_t eg = (__float_as_uint(mx) >> 23) & 0xffu;   // of the lane's group of 32 columns
     mx = warp_max(mx);
     // |v| < 2^(ex - 126), so X = v * 2^(137 - ex) lies within +-2048
     uint32_t ex = (__float_as_uint(mx) >> 23) & 0xffu;
     ex = ex < 24u ? 24u : (ex > 253u ? 253u : ex);
     const float up = __uint_as_float((264u - ex) << 23), down = __uint_as_float((ex - 10u) << 23);
+    // the large digit: eleven bits of the group's largest value (1.5 * 2^23 units, added and taken away, rounds to a unit)
+    const uint32_t quiet = ex > eg ? min(ex - eg, PW_QUIET) : 0u;
+    const float magic = 1.5f * __uint_as_float((150u - quiet) << 23);
     uint32_t hw[4], lw[4];
     float hsum = 0.0f, lsum = 0.0f;
 #pragma unroll
@@ -682,8 +752,8 @@ __device__ __forceinline__ void wide_image_unit(uint8_t *__restrict__ image, uin
         float hi[2], lo[2];
 #pragma unroll
         for (int j = 0; j < 2; j++) {
-            const float X = v[2 * i + j] * up;
-            hi[j] = rintf(X);
+            const float X = v[4 * (i >> 1) + (i & 1) + 2 * j] * up;   // (0, 2), (1, 3): see pw_unpack
+            hi[j] = __fsub_rn(__fadd_rn(X, magic), magic);
             lo[j] = __half2float(__float2half_rn(X - hi[j]));
             hsum += hi[j];
             lsum += lo[j];
