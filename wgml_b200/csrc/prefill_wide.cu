@@ -932,11 +932,15 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
     pdl_wait();
     const uint32_t h = blockIdx.x, t0 = (gridDim.y - 1 - blockIdx.y) * 64, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const uint32_t nq = ntok - t0 < 64 ? ntok - t0 : 64;
-    const uint32_t last = pos0 + t0 + nq - 1;
-    // this block's tiles of rows
-    const uint32_t ntiles = last / 64 + 1, nz = !SHARED ? 1u : gridDim.z < ntiles ? gridDim.z : ntiles, z = SHARED ? blockIdx.z : 0u;
-    if (z >= nz) return;
-    const uint32_t c_begin = SHARED ? 64 * (z * ntiles / nz) : 0u, c_end = SHARED ? 64 * ((z + 1) * ntiles / nz) : last + 1;
+    // the block's tiles of rows (all of them, to the last row that is attended to, where none are shared)
+    uint32_t c_begin = 0, c_end = 0, nz = 1;
+    if constexpr (SHARED) {
+        const uint32_t ntiles = (pos0 + t0 + nq - 1) / 64 + 1;
+        nz = gridDim.z < ntiles ? gridDim.z : ntiles;
+        if (blockIdx.z >= nz) return;
+        c_begin = 64 * (blockIdx.z * ntiles / nz);
+        c_end = 64 * ((blockIdx.z + 1) * ntiles / nz);
+    }
     const float *kh = k_cache + (size_t)(h / kv_mul) * head_stride, *vh = v_cache + (size_t)(h / kv_mul) * head_stride;
     const float inv_sqrt = 1.0f / sqrtf((float)HD);
     for (uint32_t i = tid; i < 64 * HD / 4; i += 256) {
@@ -954,6 +958,7 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
 #pragma unroll
         for (uint32_t c = 0; c < NC; c++) acc[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    const uint32_t last = pos0 + t0 + nq - 1;
     // a tile travels through registers, requested one phase before it is needed
     float4 pre[NP];
     auto fetch = [&](const float *base, uint32_t c0) {
@@ -973,8 +978,9 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
         }
         return __syncthreads_or(flag);
     };
+    auto mine = [&](uint32_t c) { return SHARED ? c < c_end : c <= last; };
     fetch(kh, c_begin);
-    for (uint32_t c0 = c_begin; c0 < c_end; c0 += 64) {
+    for (uint32_t c0 = c_begin; mine(c0); c0 += 64) {
         place(false);
         fetch(vh, c0);
         float s[4][4];
@@ -1035,7 +1041,7 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
             for (uint32_t k = 0; k < NP; k++) z = fmaf(pre[k].x, 0.0f, fmaf(pre[k].y, 0.0f, fmaf(pre[k].z, 0.0f, fmaf(pre[k].w, 0.0f, z))));
         }
         const bool one_by_one = place(z != 0.0f) != 0;
-        if (c0 + 64 < c_end) fetch(kh, c0 + 64);
+        if (mine(c0 + 64)) fetch(kh, c0 + 64);
         if (one_by_one) {
 #pragma unroll 1
             for (uint32_t j = 0; j < 64; j++) {
@@ -1081,12 +1087,12 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
         __shared__ uint32_t s_last;
         constexpr uint32_t SLOT = WA_SLOT<HD>;   // float4 per block: sums [register][thread], then (maximum, denominator) [row]
         const uint32_t pair = blockIdx.x * gridDim.y + blockIdx.y;
-        float4 *all = scratch + (size_t)pair * gridDim.z * SLOT, *mine = all + (size_t)z * SLOT;
+        float4 *all = scratch + (size_t)pair * gridDim.z * SLOT, *part = all + (size_t)blockIdx.z * SLOT;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
 #pragma unroll
-            for (uint32_t c = 0; c < NC; c++) mine[(i * NC + c) * 256 + tid] = acc[i][c];
-            if (tx == 0) reinterpret_cast<float2 *>(mine + 4 * NC * 256)[4 * ty + i] = make_float2(mrun[i], lrun[i]);
+            for (uint32_t c = 0; c < NC; c++) part[(i * NC + c) * 256 + tid] = acc[i][c];
+            if (tx == 0) reinterpret_cast<float2 *>(part + 4 * NC * 256)[4 * ty + i] = make_float2(mrun[i], lrun[i]);
         }
         __threadfence();
         __syncthreads();
@@ -1102,14 +1108,14 @@ __global__ void __launch_bounds__(256, 2) wide_attention_kernel(const float *__r
 #pragma unroll
             for (uint32_t c = 0; c < NC; c++) acc[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
             for (uint32_t zz = 0; zz < nz; zz++) {
-                const float4 *part = all + zz * SLOT;
-                const float2 ml = __ldcg(reinterpret_cast<const float2 *>(part + 4 * NC * 256) + 4 * ty + i);
+                const float4 *other = all + zz * SLOT;
+                const float2 ml = __ldcg(reinterpret_cast<const float2 *>(other + 4 * NC * 256) + 4 * ty + i);
                 if (ml.x == -INFINITY && ml.y == 0.0f) continue;   // nothing but rows the position does not attend to
                 const float w = expf(ml.x - mx);
                 lrun[i] = fmaf(ml.y, w, lrun[i]);
 #pragma unroll
                 for (uint32_t c = 0; c < NC; c++) {
-                    const float4 v = __ldcg(part + (i * NC + c) * 256 + tid);
+                    const float4 v = __ldcg(other + (i * NC + c) * 256 + tid);
                     acc[i][c].x = fmaf(v.x, w, acc[i][c].x);
                     acc[i][c].y = fmaf(v.y, w, acc[i][c].y);
                     acc[i][c].z = fmaf(v.z, w, acc[i][c].z);
@@ -1141,8 +1147,8 @@ static int launch_wide_attention_hd(const float *q, const float *k_cache, const 
         *attrs = true;
     }
     // Blocks for the rows of one (head, tile of positions): as many as are resident at once, with two tiles of rows or more
-    // each.  Sixteen positions of a two-layer model of 7B widths (32 blocks) at position 4000: 2045 us a pass with one block each, 631 with nine (eight-position passes 759); a
-    // pass with more blocks than half of what is resident is as before.
+    // each.  Sixteen positions of a two-layer model of 7B widths (32 blocks) at position 4000: 2045 us a pass with one block
+    // each, 631 with nine (eight-position passes 759); a pass with more blocks than half of what is resident is as before.
     const uint32_t pairs = n_heads * ((ntok + 63) / 64), tiles = (pos0 + ntok + 63) / 64;
     uint32_t nz = scratch && counters ? WA_BLOCKS * (uint32_t)sm_count() / pairs : 1u;
     if (nz > tiles / 2) nz = tiles / 2;
