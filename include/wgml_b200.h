@@ -419,7 +419,8 @@ int wgb_llama2_set_sampler(wgb_llama2 *m, float temperature, float topp, uint64_
  * Llama2::dispatch, chat_llama2.rs:104-116,169-204, and drops the logits).  Once enabled, wgb_llama2_decode
  * sends every prompt position but the last through passes: of up to 640 positions when there are sixteen or more to go,
  * every layer matrix is Q4_K, Q6_K or Q8_0 with a multiple of 128 rows, the head size is 64 or 128 and there is one rank
- * (two f16 digits per activation, tcgen05.mma kind::f16); of eight positions otherwise: the Q4_K layer matrices are
+ * (two f16 digits per activation, tcgen05.mma kind::f16) and the device has room for their buffers when the feature is
+ * enabled; of eight positions otherwise: the Q4_K layer matrices are
  * multiplied on the tensor cores (tcgen05.mma kind::i8 on the same fixed-point image of the activations as the
  * matrix-vector kernels, from tile-major copies of the weights made here, which doubles their memory), the Q6_K
  * and Q8_0 ones by kernels of their own (Q6_K: scales folded into the weight operand; Q8_0: the codes are the operand),

@@ -1,7 +1,7 @@
 // Matrix-vector kernels: the fused, TMA-fed kernel used by the models and by GemvQuant, and the
 // generic per-format fallback.
 //
-// Fused kernel.  One persistent block per SM with three roles: eighteen consumer warps, a producer
+// Fused kernel.  One persistent block per SM with three roles: sixteen consumer warps, a producer
 // warp and an epilogue warp.
 //   * Rows are taken in groups of `rs` (1..8) that lie contiguously in HBM.  The producer streams
 //     group after group into a ring of shared-memory stages with one bulk asynchronous copy
@@ -11,7 +11,7 @@
 //     launch): weights never depend on activations.
 //   * The consumers build the shared image of the (normalised) input vector once.  Consumer warp w
 //     owns column part w % kp of the matrix for the whole kernel, so its share of the input stays in
-//     registers; the warps of one column part form ncl = 18 / kp "lanes" that take the (stage, row
+//     registers; the warps of one column part form ncl = 16 / kp "lanes" that take the (stage, row
 //     part) tasks of the block in turn.  A task is `rrows` rows of one stage: the warp computes the
 //     partial dot products (the loop over rows fully unrolled, so that the loads of later rows overlap
 //     the arithmetic of earlier ones), folds them across its lanes with a transposing butterfly (9
@@ -37,9 +37,9 @@
 namespace wgb {
 
 // Consumer warps per block.  Registers are allocated per scheduler partition (a quarter of the register file
-// each, warps dealt round-robin): 18 consumers + producer + epilogue = 20 warps put five warps on every
-// partition, which leaves 96 registers per thread -- the same as 17 to 19 warps would -- so 18 is the most
-// consumers that budget buys.
+// each, warps dealt round-robin): 16 consumers + producer + epilogue = 18 warps put five warps on two of the
+// partitions, which leaves 96 registers per thread.  18 consumers fit that budget too; a
+// 7B decode step was slower with them.
 #ifndef WGB_GEMV_NCONS
 #define WGB_GEMV_NCONS 16
 #endif
@@ -866,7 +866,7 @@ static uint32_t steps_of(int qt, uint32_t K)
 // false when the shapes do not fit the kernel's assumptions.
 //
 // Candidates are (rs rows per stage, rparts row parts per stage); a consumer task is rrows = rs / rparts
-// rows of one column part, and the ncl = 18 / kparts warps of a column part take the tasks of the block
+// rows of one column part, and the ncl = 16 / kparts warps of a column part take the tasks of the block
 // in turn.  The time of the launch is that of its fullest block: ceil(tasks / ncl) rounds of
 // (rrows + 1/2) row products, the half row standing for the wait, reduction and hand-off of a task.
 // That is divided by how much of the ~80 KB per SM that must be in flight to cover HBM latency at full

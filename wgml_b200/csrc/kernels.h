@@ -240,7 +240,9 @@ int launch_prefill_attention(const float *q, const float *k_cache, const float *
 // ---- wide prompt passes (prefill_wide.cu) ---------------------------------------------------------------
 constexpr uint32_t PW_TILE = 128;            // prompt positions per tile of a wide product, most
 constexpr uint32_t PW_CAP = 5 * PW_TILE;     // prompt positions per wide pass, most
-constexpr uint32_t PW_MIN = 16;              // fewer than this go through the passes of PF_TOK positions
+// Fewer than this go through the passes of PF_TOK positions.  (Two layers of 7B widths, microseconds: 16 positions 363 as a wide
+// pass, 505 as two of eight; 12 positions as two of eight 458, 8 as one 257.  Four layers of GPT-2 124M widths: 286 and 404; 212.)
+constexpr uint32_t PW_MIN = 16;
 // Tiles of positions of a pass: npt tiles of np positions each.
 struct WideTiling { uint32_t np, npt; };
 WideTiling prefill_wide_tiling(uint32_t ntok);
