@@ -78,8 +78,8 @@ def test_repeated_streaming_calls_reuse_the_ticket_counters():   # row-streaming
 
 
 @pytest.mark.parametrize("case", [
-    (512, 32, 128, 1, 300), (512, 32, 64, 2, 300), (512, 32, 128, 4, 300), (4224, 64, 128, 8, 4100),   # row-streaming kernel, each width
-    (512, 8, 64, 1, 300), (512, 12, 64, 3, 130),                                                       # split kernel
+    (2112, 32, 128, 1, 2100), (512, 32, 64, 2, 300), (512, 32, 128, 4, 300), (4224, 64, 128, 8, 4100),   # row-streaming kernel, each width
+    (512, 32, 128, 1, 300), (512, 12, 64, 3, 130),                                                       # split kernel
 ])
 @pytest.mark.parametrize("offset", [1, 2, 3])
 def test_output_at_any_word(case, offset):
@@ -97,8 +97,8 @@ def test_output_at_any_word(case, offset):
 
 
 @pytest.mark.parametrize("case", [
-    (512, 32, 128, 1, 300), (512, 32, 64, 2, 300), (512, 32, 128, 4, 300), (4224, 64, 128, 8, 1300),
-    (512, 12, 64, 3, 300), (2112, 32, 128, 1, 2100), (2112, 60, 64, 5, 2100),   # split kernel (one chunk a block, several); rows, one query head
+    (2112, 32, 128, 1, 2100), (512, 32, 64, 2, 300), (512, 32, 128, 4, 300), (4224, 64, 128, 8, 1300),   # row-streaming kernel, each width
+    (512, 32, 128, 1, 300), (512, 12, 64, 3, 300), (2112, 60, 64, 5, 2100),   # split kernel, one chunk a block and several
 ])
 @pytest.mark.parametrize("masked", [(0, 8), (0, 23), (0, 130), (8, 16), (40, 290), (1, 297)])
 def test_rows_scored_minus_infinity_weigh_nothing(case, masked):

@@ -52,5 +52,6 @@ def test_streaming_kernel_with_several_chunks_per_block():
 @pytest.mark.parametrize("start", [0, 126, 200, 1001, 3003])
 def test_row_streaming_kernel_in_decode_steps(shape, start):
     """Ten steps leave every number of rows in the last group of eight.  Up to about 140 positions there are fewer groups
-    than blocks, and no warp requests anything ahead of the wait; from 1001 on most do."""
+    than blocks, and no warp requests anything ahead of the wait; from 1001 on most do.  (Eight query heads per KV head: the
+    split kernel as long as the context is one wave.)"""
     steps(*shape, start, 10, 3072)
