@@ -131,17 +131,44 @@ def test_gemv_outlier_inputs(qtype):
         assert_close(o, o64, RTOL, atol, f"qtype {qtype}, {name}")
 
 
+@pytest.mark.parametrize("qtype,cols", [(ops.Q4_K, (256, 2048, 2304, 4352, 51200)), (ops.Q6_K, (256, 2048, 2304, 4352, 48640)),
+                                        (ops.Q8_0, (32, 96, 1024, 1056, 2080, 46080)), (ops.F32, (4, 60, 512, 516, 1088, 25600))])
+@pytest.mark.parametrize("nrows", [1, 7, 9, 16, 1184, 1185, 2376])
+def test_gemv_tile_edges(qtype, cols, nrows):
+    """Rows around a tile of eight, of sixteen and the line between the two (148 tiles of eight); columns around a unit, a stage of
+    eight units and two of them, down to one block and up to the longest row the fused kernel has ever taken.
+    The input is held as 23-bit fixed point against the largest of 32 columns (2^-23 of it at most), the sums of a row are f32 in
+    fewer than K / 32 + 64 steps, each within 2^-24 of the sum of magnitudes."""
+    for ncols in cols:
+        if ncols > 20000 and nrows > 16:
+            continue
+        raw, x = make(qtype, nrows, ncols, 29)
+        out = torch.full((nrows,), float("nan"), device="cuda")
+        ops.GemvQuant.from_device().dispatch(out, ops.GpuQuantMatrix(qtype, raw, nrows, ncols), torch.from_numpy(x).cuda())
+        w = np.abs(oracle.dequantize(qtype, raw).reshape(nrows, ncols).astype(np.float64))
+        pad = -ncols % 32
+        top = np.repeat(np.abs(np.pad(x, (0, pad))).reshape(-1, 32).max(axis=1), 32)[:ncols].astype(np.float64)
+        mags = w @ np.abs(x.astype(np.float64))
+        if qtype in (ops.Q4_K, ops.Q6_K):   # codes and mins of a group are summed apart: magnitudes before the two cancel
+            mags = mags + 2.0 * np.abs(w).reshape(nrows, -1, 32).max(axis=2) @ np.abs(x.astype(np.float64)).reshape(-1, 32).sum(axis=1)
+        bound = 2.0 ** -23 * (w @ top) + (ncols / 32 + 64) * 2.0 ** -24 * mags
+        _, o64 = oracle.gemv_quant(qtype, raw, nrows, ncols, x, want_f64=True)
+        err = np.abs(out.cpu().numpy().astype(np.float64) - o64)
+        assert (err <= bound).all(), f"qtype {qtype} {nrows}x{ncols}: {(err / np.maximum(bound, 1e-300)).max()}"
+
+
 @pytest.mark.parametrize("qtype,nrows,ncols", [
-    (ops.F32, 32000, 288),      # five warps a column part, one task a stage, 24 slots: a warp's tasks wander over the slots
-    (ops.F32, 60000, 32),       # sixteen warps a column part: the longest stride
-    (ops.Q8_0, 50257, 768),     # the same with two tasks a stage: always the same slots
-    (ops.Q4_K, 26000, 4096),    # eight warps, two tasks a stage
-    (ops.Q4_K, 26000, 6144),    # five warps, a short ring
-    (ops.Q6_K, 32000, 4096),    # seven slots, an odd number
+    (ops.F32, 32000, 288),      # one stage a tile: the consumer groups take tiles in turn, three epilogue warps
+    (ops.F32, 60000, 32),       # the same with one unit at work
+    (ops.Q8_0, 50257, 768),     # six units of a stage at work
+    (ops.Q4_K, 26000, 4096),    # two stages a tile: a group always has the same columns
+    (ops.Q4_K, 26000, 6144),    # three: they alternate
+    (ops.Q6_K, 32000, 4096),    # a ring of six slots, an odd number would fit
+    (ops.Q4_K, 9000, 28672),    # fourteen stages a tile, a ring of six: one epilogue warp
 ])
 def test_ring_slots_used_many_times(qtype, nrows, ncols):
-    """Matrices whose blocks go around the ring several times, in the ways consumer warps can meet a slot's uses; called again and
-    again, every output has the same bits."""
+    """Matrices whose blocks go around the ring several times, in the ways consumer and epilogue warps can meet a slot's uses;
+    called again and again, every output has the same bits."""
     raw, x = make(qtype, nrows, ncols, 17)
     m, xd, op = ops.GpuQuantMatrix(qtype, raw, nrows, ncols), torch.from_numpy(x).cuda(), ops.GemvQuant.from_device()
     outs = [torch.full((nrows,), float("nan"), device="cuda") for _ in range(16)]

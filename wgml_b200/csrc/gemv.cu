@@ -1,28 +1,25 @@
 // Matrix-vector kernels: the fused, TMA-fed kernel used by the models and by GemvQuant, and the
 // generic per-format fallback.
 //
-// Fused kernel.  One persistent block per SM with three roles: sixteen consumer warps, a producer
-// warp and an epilogue warp.
-//   * Rows are taken in groups of `rs` (1..8) that lie contiguously in HBM.  The producer streams
-//     group after group into a ring of shared-memory stages with one bulk asynchronous copy
-//     (cp.async.bulk, completion on an mbarrier) per plane of the group, running as many stages
-//     ahead as the ring holds and handling several stages per pass, one per group of lanes.  It
-//     starts before the kernel waits for its predecessor in the stream (programmatic dependent
-//     launch): weights never depend on activations.
-//   * The consumers build the shared image of the (normalised) input vector once.  Consumer warp w
-//     owns column part w % kp of the matrix for the whole kernel, so its share of the input stays in
-//     registers; the warps of one column part form ncl = 16 / kp "lanes" that take the (stage, row
-//     part) tasks of the block in turn.  A task is `rrows` rows of one stage: the warp computes the
-//     partial dot products (the loop over rows fully unrolled, so that the loads of later rows overlap
-//     the arithmetic of earlier ones), folds them across its lanes with a transposing butterfly (9
-//     shuffles for up to 8 rows), writes them to shared memory and arrives on the stage's `done`
-//     barrier.  Consumers never wait for each other or for the epilogue.
-//   * The epilogue warp waits for `done`, adds the column parts of every row in a fixed order,
-//     releases the stage to the producer and applies the epilogue (bias, residual, SiLU gate, GELU,
-//     RoPE + KV-cache append), one lane per output unit.  Its global loads (bias, residual, position)
-//     are issued before the wait, so they overlap the consumers' work on the stage.
-//   * Group g belongs to block g % gridDim.x, so every SM gets the same number of groups to within
-//     one; rs and the row split are chosen per launch (see plan()).
+// Fused kernel.  One persistent block per SM with three roles: sixteen consumer warps in two groups, a producer warp and up to
+// three epilogue warps.
+//   * A block takes row tiles -- sixteen rows, or eight where a matrix has too few to go round -- and walks each in stages of eight
+//     units of columns (gemv_core.cuh).  The producer brings stage after stage into a ring in shared memory by tensor copies (TMA,
+//     one per plane and eight rows, completion on an mbarrier), as far ahead as the ring reaches.  It starts before the
+//     kernel waits for its predecessor in the stream (programmatic dependent launch): weights never depend on activations.
+//     (Stages of whole rows, one bulk copy each, fit two or three times into the ring where rows are long.)
+//   * The consumers build the shared image of the (normalised) input vector once.  The groups alternate stages; warp w of a group
+//     takes unit w of its stages: the products of the tile's rows with one unit of columns on the tensor cores, a fold over the
+//     four lanes of a row, and sixteen sums to shared memory.  Consumers never wait for each other or for the epilogue.
+//     (Eight consumer warps and room for the next launch's block beside this one: 19.2 us for Q4_K 32000x4096 where sixteen take
+//     13.8; two warps per scheduler do not cover the latencies of a unit.)
+//   * An epilogue warp waits for the eight units of a stage, adds them in a fixed order to the sums of its tile, releases the
+//     stage to the producer and after the last stage of a tile applies the epilogue (bias, residual, SiLU gate, GELU,
+//     RoPE + KV-cache append), one lane per output unit.  Its global loads (bias, residual) are issued a tile ahead.
+//   * Tile i belongs to block i % gridDim.x.
+// Bound by HBM in long launches (Q4_K 32000x4096, us: 13.8, 5.4 TB/s; Q6_K 21.4, 5.0 TB/s; Q8_0 24.1, 5.8 TB/s; the dp4a kernel
+// before took 16.0, 27.9 and 27.4), in short ones by the hand-over between launches: wait 0.6, input 0.4 (under load 0.8), staging
+// 0.3, first unit 0.3 to 0.7, last sums and exit 0.5.
 // Every wait is bounded in time: a waiter that runs out records an error code in the launch's status word and
 // carries on with whatever is in shared memory, so the kernel always terminates.
 #include "async_copy.cuh"
@@ -36,23 +33,16 @@
 
 namespace wgb {
 
-// Consumer warps per block.  Registers are allocated per scheduler partition (a quarter of the register file
-// each, warps dealt round-robin): 16 consumers + producer + epilogue = 18 warps put five warps on two of the
-// partitions, which leaves 96 registers per thread.  18 consumers fit that budget too; a
-// 7B decode step was slower with them.
-#ifndef WGB_GEMV_NCONS
-#define WGB_GEMV_NCONS 16
-#endif
-constexpr int GEMV_NCONS = WGB_GEMV_NCONS;
+constexpr int GEMV_NCONS = 2 * TILE_UNITS;          // consumer warps: two groups, a warp per unit of a stage
 constexpr int GEMV_CONS_THREADS = GEMV_NCONS * 32;
 constexpr int GEMV_PRODUCER = GEMV_NCONS;           // warp index of the producer
-constexpr int GEMV_EPILOGUE = GEMV_NCONS + 1;       // warp index of the epilogue warp
-constexpr int GEMV_NT = (GEMV_EPILOGUE + 1) * 32;
-constexpr int GEMV_MAX_RS = 8;                      // rows per stage
-constexpr int GEMV_TASK_ROWS = 4;                   // rows per consumer task, at most
-constexpr int GEMV_MAX_STAGES = 24;
+constexpr int GEMV_EPILOGUE = GEMV_NCONS + 1;       // warp index of the first epilogue warp
+constexpr int GEMV_NEPI = 3;                        // epilogue warps (twenty warps: five per scheduler, 96 registers a thread)
+constexpr int GEMV_NT = (GEMV_EPILOGUE + GEMV_NEPI) * 32;
+constexpr uint32_t GEMV_MAX_STAGES = 12;
 constexpr uint32_t GEMV_ROPE_TAB = 128;             // pair indices with a precomputed rotation
-constexpr size_t GEMV_SMEM_BUDGET = 200 * 1024;     // dynamic shared memory per block
+constexpr uint32_t GEMV_PART_BYTES = TILE_UNITS * 16 * 4;   // partial sums of a stage: [unit][row]
+constexpr size_t GEMV_SMEM_BUDGET = 224 * 1024;     // dynamic shared memory per block
 
 __device__ __forceinline__ float4 ld_act4(const float *p)
 {
@@ -66,143 +56,46 @@ __device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t *p)
     return v;
 }
 
-// Which use of a ring slot a barrier stands at is read from its parity, so a waiter must know that the use before (of that
-// barrier) is through; otherwise the parity is that of the use before and reads as "done" (a slot armed twice ends in a
-// launch failure).
-//   * Producer (`empty`): the lanes of a pass meet before the next pass, and the use before lies in an earlier pass (spb <=
-//     nstage), whose lanes have waited for its release.
-//   * Consumer warp (`full`) and lane group of the epilogue (`done`): they take every ncl-th task and every nb-th stage, so the use
-//     before of a slot may be another's, and unfinished.  Uses take turns on two barriers per slot (round & 1): what has to be
-//     through at stage `it` is the use two back, stage it - 2 nstage.  The waiter's own stage before is at most L = ceil(ncl /
-//     rparts), respectively nb, stages back and has landed; its pass of the producer begins L + spb - 1 stages back or later, and
-//     until then all slots of earlier passes had been released, so every stage up to it - L - spb - nstage is through.  That
-//     covers it - 2 nstage when L + spb <= nstage.  For nb the batches below see to it (nstage = 1: the same lanes take every
-//     stage); for the consumers plan() does, unless a warp takes a task of every use of a slot anyway (ring_safe).
-// (Counting a slot's releases instead, a second word to poll in every wait, cost a 7B decode step 2 % and a tiny one 3 %.)
-
 __device__ __forceinline__ void cons_sync() { asm volatile("bar.sync 1, %0;" ::"n"(GEMV_CONS_THREADS) : "memory"); }
 
-// Sum over the consumer threads (named barrier 1); every consumer gets the result.
-__device__ __forceinline__ float cons_sum(float v, float *red)
-{
-    v = warp_sum(v);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    cons_sync();
-    if (lane == 0) red[warp] = v;
-    cons_sync();
-    float t = (lane < GEMV_NCONS) ? red[lane] : 0.0f;
-    static_assert(GEMV_NCONS <= 32, "one partial per consumer warp");
-    return warp_sum(t);
-}
-
-// Sums acc[0..8) over the lanes of the warp.  Lane l returns the total of row
-// 4 * bit4(l) + 2 * bit3(l) + bit2(l); the four lanes that share bits 2..4 hold the same value.
-__device__ __forceinline__ float warp_sum8(const float (&acc)[8], int lane)
-{
-    float a4[4], a2[2];
-    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const float keep = h16 ? acc[i + 4] : acc[i], send = h16 ? acc[i] : acc[i + 4];
-        a4[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-        const float keep = h8 ? a4[i + 2] : a4[i], send = h8 ? a4[i] : a4[i + 2];
-        a2[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-    }
-    const float keep = h4 ? a2[1] : a2[0], send = h4 ? a2[0] : a2[1];
-    float v = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    return v;
-}
-
-// The same for R = 4, 2, 1 rows: the total of row r ends up in the lanes whose top log2(R) bits spell r.
-template <int R>
-__device__ __forceinline__ float warp_sum_rows(const float (&acc)[R], int lane)
-{
-    static_assert(R == 1 || R == 2 || R == 4 || R == 8, "rows per task");
-    if constexpr (R == 8) {
-        return warp_sum8(acc, lane);
-    } else if constexpr (R == 4) {
-        const bool h16 = lane & 16, h8 = lane & 8;
-        float a2[2];
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const float keep = h16 ? acc[i + 2] : acc[i], send = h16 ? acc[i] : acc[i + 2];
-            a2[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-        }
-        const float keep = h8 ? a2[1] : a2[0], send = h8 ? a2[0] : a2[1];
-        float v = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-        v += __shfl_xor_sync(0xffffffffu, v, 4);
-        v += __shfl_xor_sync(0xffffffffu, v, 2);
-        v += __shfl_xor_sync(0xffffffffu, v, 1);
-        return v;
-    } else if constexpr (R == 2) {
-        const bool h16 = lane & 16;
-        float v = (h16 ? acc[1] : acc[0]) + __shfl_xor_sync(0xffffffffu, h16 ? acc[0] : acc[1], 16);
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        return v;
-    } else {
-        return warp_sum(acc[0]);
-    }
-}
-
-// Stages per pass of the epilogue warp and of the producer warp.  The lanes of a warp may be held at a
-// reconvergence point until all of them have left their wait, so a pass must be assumed to finish only
-// when every stage in it has: the epilogue pass that frees a slot must never contain a stage whose copy
-// the producer can only issue in a pass that needs that very slot.  epilogue_batch + producer_batch <=
-// nstage + 1 rules the cycle out; the producer also leaves half of the ring queued while it waits.  (From two stages on
-// the sum stays within nstage, which the waits on `done` need as well.)
-__host__ __device__ inline uint32_t epilogue_batch(uint32_t nstage) { return nstage >= 8 ? 4u : (nstage >= 4 ? 2u : 1u); }
-__host__ __device__ inline uint32_t producer_batch(uint32_t nstage, uint32_t copies_per_stage)
-{
-    uint32_t b = nstage / 2;
-    if (b > 32 / copies_per_stage) b = 32 / copies_per_stage;
-    return b < 1 ? 1 : b;
-}
-
-// ---- groups ------------------------------------------------------------------------------------
+// ---- tiles -------------------------------------------------------------------------------------
 struct Part {
     int mat;
     uint32_t row0;
 };
 
-// Parts (1 or 2 runs of `n` consecutive rows of one matrix) of group gi; returns the number of parts,
-// 0 past the end.
-__device__ __forceinline__ int group_parts(const GemvArgs &a, const int EPI, uint32_t gi, Part (&parts)[2], uint32_t &n)
+// n / d by a multiplication, for n * d < 2^32 and d > 1: magic = ceil(2^32 / d).  (A division is some fifty dependent instructions, and the
+// epilogue warp of a q/k/v launch, which had four per tile, took longer over its tiles than the consumers.)  d = 1: magic = 0.
+__device__ __forceinline__ uint32_t small_div(uint32_t n, uint32_t magic) { return magic ? __umulhi(n, magic) : n; }
+
+// Parts of row tile `ti`: one run of up to tile_rows rows of one matrix, or two of up to eight (gate and up, the two halves of
+// a Neox head) that take rows 0.. and 8.. of the tile.  `n`: rows per part.  Returns the number of parts.
+__device__ __forceinline__ int tile_parts(const GemvArgs &a, const int EPI, uint32_t ti, Part (&parts)[2], uint32_t &n)
 {
-    const uint32_t rs = a.rs;
-    if (gi >= a.ngroups) return 0;
     if (EPI == EPI_SILU_PAIR) {
-        const uint32_t h = rs / 2, r0 = gi * h, nr = a.mat[0].nrows;
-        n = min(h, nr - r0);
+        const uint32_t r0 = ti * TILE_ROWS;
+        n = min(TILE_ROWS, a.mat[0].nrows - r0);
         parts[0] = { 0, r0 };
         parts[1] = { 1, r0 };
         return 2;
-    } else if (EPI == EPI_QKV_ROPE) {
-        const uint32_t gq = a.gq, gk = a.gk;
-        const int s = gi < gq ? 0 : (gi < gq + gk ? 1 : 2);
-        const uint32_t lg = gi - (s == 0 ? 0 : (s == 1 ? gq : gq + gk));
+    }
+    int s = 0;
+    if (EPI == EPI_QKV_ROPE) {
+        s = ti < a.tq ? 0 : (ti < a.tq + a.tk ? 1 : 2);
+        ti -= s == 0 ? 0 : (s == 1 ? a.tq : a.tq + a.tk);
         if (s < 2 && a.rope_variant == WGB_ROPE_NEOX) {
-            const uint32_t h2 = rs / 2, half = a.head_size / 2, lp = lg * h2;
-            const uint32_t r0 = (lp / half) * a.head_size + lp % half;
-            n = h2;
+            const uint32_t half = a.head_size / 2, head = small_div(ti, a.per_head_magic), o = (ti - head * a.per_head) * TILE_ROWS;
+            const uint32_t r0 = head * a.head_size + o;
+            n = min(TILE_ROWS, half - o);
             parts[0] = { s, r0 };
             parts[1] = { s, r0 + half };
             return 2;
         }
-        n = rs;
-        parts[0] = { s, lg * rs };
-        return 1;
-    } else {
-        const uint32_t r0 = gi * rs, nr = a.mat[0].nrows;
-        n = min(rs, nr - r0);
-        parts[0] = { 0, r0 };
-        return 1;
     }
+    const uint32_t r0 = ti * a.tile_rows;
+    n = min(a.tile_rows, a.mat[s].nrows - r0);
+    parts[0] = { s, r0 };
+    return 1;
 }
 
 __device__ __forceinline__ float gelu_f32(float x)
@@ -212,16 +105,16 @@ __device__ __forceinline__ float gelu_f32(float x)
     return 0.5f * x * (1.0f + tanhf(SQRT_2_OVER_PI * x * (1.0f + GELU_COEF_A * x * x)));
 }
 
-// Output units of a group (a unit = the stage rows that make one output: a row, or a pair) and the
-// stage rows of unit u.
-__device__ __forceinline__ uint32_t group_units(const int EPI, const Part (&parts)[2], int nparts, uint32_t n)
+// Output units of a tile (a unit = the tile rows that make one output: a row, or a pair) and the
+// tile rows of unit u.
+__device__ __forceinline__ uint32_t tile_outputs(const int EPI, const Part (&parts)[2], int nparts, uint32_t n)
 {
     if (EPI == EPI_QKV_ROPE && nparts == 1 && parts[0].mat < 2) return n / 2;   // adjacent pairs
     return n;
 }
-__device__ __forceinline__ void unit_rows(const int EPI, const Part (&parts)[2], int nparts, uint32_t n, uint32_t u, uint32_t &ra, uint32_t &rb)
+__device__ __forceinline__ void output_rows(const int EPI, const Part (&parts)[2], int nparts, uint32_t u, uint32_t &ra, uint32_t &rb)
 {
-    if (EPI == EPI_SILU_PAIR || (EPI == EPI_QKV_ROPE && nparts == 2)) { ra = u; rb = n + u; }
+    if (EPI == EPI_SILU_PAIR || (EPI == EPI_QKV_ROPE && nparts == 2)) { ra = u; rb = TILE_ROWS + u; }
     else if (EPI == EPI_QKV_ROPE && parts[0].mat < 2) { ra = 2 * u; rb = 2 * u + 1; }
     else { ra = u; rb = u; }
 }
@@ -230,6 +123,8 @@ __device__ __forceinline__ void unit_rows(const int EPI, const Part (&parts)[2],
 // sums are ready so that the global loads overlap the consumers' work.
 struct EpiCtx {
     bool on;            // the lane has a unit
+    bool v;             // EPI_QKV_ROPE: of the value matrix (no rotation)
+    uint32_t ra, rb;    // tile rows of the unit
     uint32_t r0, r1;    // output rows of the unit (matrix row indices)
     uint32_t d0, d1;    // EPI_QKV_ROPE: their offsets from `dst`
     float b0, b1;       // bias of r0 / r1, or the residual in b1 for EPI_RESIDUAL
@@ -237,12 +132,17 @@ struct EpiCtx {
     float *dst;         // EPI_QKV_*: where the rows of the unit go
 };
 
-__device__ __forceinline__ EpiCtx epi_prepare(const GemvArgs &a, const int EPI, const Part (&parts)[2], int nparts, uint32_t n, uint32_t t,
-                                              uint32_t nunits, const float2 *rope_tab)
+// `pos`: the step's position (EPI_QKV_*).
+__device__ __forceinline__ EpiCtx epi_prepare(const GemvArgs &a, const int EPI, uint32_t ti, uint32_t t, uint32_t pos, const float2 *rope_tab)
 {
     EpiCtx c = {};
-    c.on = t < nunits;
+    Part parts[2];
+    uint32_t n = 0;
+    const int nparts = tile_parts(a, EPI, ti, parts, n);
+    c.on = t < tile_outputs(EPI, parts, nparts, n);
     if (!c.on) return c;
+    output_rows(EPI, parts, nparts, t, c.ra, c.rb);
+    c.v = EPI == EPI_QKV_ROPE && parts[0].mat == 2;
     if (EPI == EPI_STORE || EPI == EPI_RESIDUAL || EPI == EPI_GELU) {
         c.r0 = parts[0].row0 + t;
         if (a.bias) c.b0 = a.bias[c.r0];
@@ -252,7 +152,6 @@ __device__ __forceinline__ EpiCtx epi_prepare(const GemvArgs &a, const int EPI, 
     } else if (EPI == EPI_QKV_ROPE) {
         const int s = parts[0].mat;
         const float *bias = s == 0 ? a.bias : (s == 1 ? a.bias_k : a.bias_v);
-        const uint32_t pos = *a.pos;
         const uint32_t rstr = a.kv_row_stride ? a.kv_row_stride : a.kv_dim;
         c.dst = s == 0 ? a.out : ((s == 1 ? a.k_cache : a.v_cache) + (size_t)pos * rstr);
         if (s == 2) {
@@ -264,31 +163,22 @@ __device__ __forceinline__ EpiCtx epi_prepare(const GemvArgs &a, const int EPI, 
             c.r0 = parts[0].row0 + 2 * t;
             c.r1 = c.r0 + 1;
         }
-        // where rows r0 / r1 land: q as is, k / v by (head, element) in the cache's layout
-        c.d0 = c.r0;
-        c.d1 = c.r1;
-        if (s != 0 && a.kv_row_stride) {
-            c.d0 = (c.r0 / a.head_size) * a.kv_head_stride + c.r0 % a.head_size;
-            c.d1 = (c.r1 / a.head_size) * a.kv_head_stride + c.r1 % a.head_size;
-        }
+        // where rows r0 / r1, two of one head, land: q as is, k / v by (head, element) in the cache's layout
+        const uint32_t head = small_div(c.r0, a.head_magic), e0 = c.r0 - head * a.head_size;
+        c.d0 = s != 0 && a.kv_row_stride ? head * a.kv_head_stride + e0 : c.r0;
+        c.d1 = c.d0 + (c.r1 - c.r0);
         if (bias) {
             c.b0 = bias[c.r0];
             c.b1 = bias[c.r1];
         }
         if (s < 2) {
             // RoPE (ops/rope.wgsl:36-77): angle = pos * base^(-(2i % head_size) / head_size) for pair (r0, r1)
-            const uint32_t half = a.head_size / 2;
-            const uint32_t fi = (a.rope_variant == WGB_ROPE_NEOX) ? (c.r0 % a.head_size) : ((c.r0 / 2) % half);
-            if (half <= GEMV_ROPE_TAB) {
-                const float2 r = rope_tab[fi];
-                c.cs = r.x;
-                c.sn = r.y;
-            } else {
-                sincosf((float)pos * a.rope_freq[fi], &c.sn, &c.cs);
-            }
+            const float2 r = rope_tab[a.rope_variant == WGB_ROPE_NEOX ? e0 : e0 / 2];
+            c.cs = r.x;
+            c.sn = r.y;
         }
     } else if (EPI == EPI_QKV_SPLIT) {
-        const uint32_t row = parts[0].row0 + t, d = a.kv_dim, pos = *a.pos;
+        const uint32_t row = parts[0].row0 + t, d = a.kv_dim;
         c.r0 = row;
         if (a.bias) c.b0 = a.bias[row];
         if (row < d) c.dst = a.out + row;
@@ -298,8 +188,9 @@ __device__ __forceinline__ EpiCtx epi_prepare(const GemvArgs &a, const int EPI, 
     return c;
 }
 
-// ya / yb: finished dot products of the unit's first / second stage row.
-__device__ __forceinline__ void epi_finish(const GemvArgs &a, const int EPI, const Part (&parts)[2], const EpiCtx &c, float ya, float yb)
+// ya / yb: finished dot products of the unit's first / second tile row.
+template <bool PEERS>
+__device__ __forceinline__ void epi_finish(const GemvArgs &a, const int EPI, const EpiCtx &c, float ya, float yb)
 {
     if (!c.on) return;
     if (EPI == EPI_STORE || EPI == EPI_RESIDUAL || EPI == EPI_GELU) {
@@ -307,7 +198,7 @@ __device__ __forceinline__ void epi_finish(const GemvArgs &a, const int EPI, con
         if (a.bias) y += c.b0;
         if (EPI == EPI_RESIDUAL) y = c.b1 + y;
         if (EPI == EPI_GELU) y = gelu_f32(y);
-        if ((EPI == EPI_STORE || EPI == EPI_RESIDUAL) && a.peer_out.n) {
+        if (PEERS && a.peer_out.n) {
             for (uint32_t p = 0; p < a.peer_out.n; p++) a.peer_out.mail[p][c.r0] = y;   // every rank's mailbox, own included
         } else {
             a.out[c.r0] = y;
@@ -315,7 +206,7 @@ __device__ __forceinline__ void epi_finish(const GemvArgs &a, const int EPI, con
     } else if (EPI == EPI_SILU_PAIR) {
         a.out[c.r0] = yb * (ya / (1.0f + expf(-ya)));
     } else if (EPI == EPI_QKV_ROPE) {
-        if (parts[0].mat == 2) {
+        if (c.v) {
             c.dst[c.d0] = ya + c.b0;
         } else {
             const float y0 = ya + c.b0, y1 = yb + c.b1;
@@ -327,152 +218,170 @@ __device__ __forceinline__ void epi_finish(const GemvArgs &a, const int EPI, con
     }
 }
 
+// Weights pass through L2 once per step: they are the first to go, ahead of activations, cache rows and code.
+__device__ __forceinline__ uint64_t streaming_policy()
+{
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ void tile_copy(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t row, uint32_t bar, uint64_t policy)
+{
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;" ::"r"(dst),
+                 "l"(map), "r"(x), "r"(row), "r"(bar), "l"(policy)
+                 : "memory");
+}
+
+// Bytes of planes 0 .. pl - 1 of a tile of eight rows.
+__host__ __device__ constexpr uint32_t tile_offset(int qt, int pl)
+{
+    uint32_t n = 0;
+    for (int i = 0; i < pl; i++) n += TILE_ROWS * tile_box(qt, i);
+    return n;
+}
+__host__ __device__ constexpr uint32_t tile_bytes(int qt) { return tile_offset(qt, tile_planes(qt)); }
+
 // One kernel per block format, prologue and epilogue.  The launches of a decode step alternate between
 // kernels and evict one another's code from the instruction caches (measured: +0.7 us per launch when two
-// kernels alternate, +1.7 us with four), so what matters is how little code one launch executes: a single
-// kernel with the prologue and epilogue chosen at run time shares its hot loop between launches but was
-// measured 13 % slower over a 7B decode step (more code per launch, a worse register allocation).
-template <int QT, int PRO_T, int EPI_T>
+// kernels alternate, +1.7 us with four), so what matters is how little code one launch executes: loops over the input and the tiles
+// are rolled, and the exchange between tensor-parallel ranks (PEERS) is compiled apart (q/k/v of Q4_K: 57 KB of code,
+// 26 without either; 68.2 and 64.4 ms for 48 steps of a 7B model, 13.9 and 12.9 for 136 of a tiny one).
+template <int QT, int PRO_T, int EPI_T, bool PEERS>
 __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant__ GemvArgs a)
 {
-    using S = Step<QT>;
+    using U = Unit<QT>;
     constexpr int PRO = PRO_T, EPI = EPI_T;
-    constexpr int NPL = QT == WGB_Q6_K ? 4 : (QT == WGB_Q8_0 ? 2 : 1);   // planes of the format
+    constexpr int NPL = tile_planes(QT);
     extern __shared__ uint4 smem4[];
-    __shared__ float red[32];
-    __shared__ float part[GEMV_MAX_STAGES][GEMV_NCONS][GEMV_MAX_RS];    // [stage][column part][stage row]
-    __shared__ __align__(16) float lane_part[GEMV_NCONS][GEMV_TASK_ROWS][32];   // [consumer warp][task row][lane]
-    __shared__ __align__(8) unsigned long long bars[5 * GEMV_MAX_STAGES];
+    __shared__ __align__(16) float red[2 * GEMV_NCONS];   // sums over the consumer warps: RMSNorm of squares, LayerNorm of values and of squared deviations
+    __shared__ __align__(8) unsigned long long bars[3 * GEMV_MAX_STAGES];
     __shared__ float2 rope_tab[GEMV_ROPE_TAB];     // (cos, sin) per pair index of a head (EPI_QKV_ROPE)
 
     const uint32_t K = a.mat[0].ncols;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t nstage = a.nstage;
-    uint8_t *smem = reinterpret_cast<uint8_t *>(smem4);
-    const uint32_t ring = smem_addr(smem + a.ring_offset);
-    // full, done: [round & 1][slot].  Whoever walks the slots keeps the byte offset of the round's half and the parity of the
-    // round's turn on it, and steps them when it passes the end of the ring.
-    constexpr uint32_t HALF = 8 * GEMV_MAX_STAGES, DONE = 2 * HALF, EMPTY = 4 * HALF;
-    const uint32_t full0 = smem_addr(&bars[0]);
-    auto next_round = [&](uint32_t &s, uint32_t &half, uint32_t &turn) {
-        s -= nstage;
-        turn ^= half ? 1u : 0u;
-        half ^= HALF;
-    };
-    const uint32_t kp = a.kparts, rparts = a.rparts;
+    const uint32_t nstage = a.nstage, units = a.units, nchunk = a.nchunk;
+    // shared memory: image of the input, partial sums of every slot, the ring (128-byte aligned)
+    const uint32_t smem0 = smem_addr(smem4), skip = ((smem0 + 127) & ~127u) - smem0;
+    uint8_t *image = reinterpret_cast<uint8_t *>(smem4) + skip;
+    float *part = reinterpret_cast<float *>(image + a.part_offset);      // [slot][unit][row]
+    const uint32_t ring = smem0 + skip + a.ring_offset;
+    const uint32_t full0 = smem_addr(&bars[0]), done0 = full0 + 8 * GEMV_MAX_STAGES, empty0 = done0 + 8 * GEMV_MAX_STAGES;
 
     // one thread per barrier: initialising them one after the other would cost a microsecond
-    if (threadIdx.x < 5 * nstage) {
+    if (threadIdx.x < 3 * nstage) {
         const uint32_t kind = threadIdx.x / nstage, s = threadIdx.x - kind * nstage;
-        mbar_init(full0 + 8 * (kind * GEMV_MAX_STAGES + s), (kind >> 1) == 1 ? kp * rparts : 1);
+        mbar_init(full0 + 8 * (kind * GEMV_MAX_STAGES + s), kind == 1 ? TILE_UNITS : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     pdl_launch_dependents();
 
-    const uint32_t row_bytes = a.row_bytes;
-    // stages of this block (the grid never exceeds the number of groups)
-    const uint32_t nst = a.per_block - ((a.rem_blocks != 0 && blockIdx.x >= a.rem_blocks) ? 1u : 0u);
-
+    // Which use of a ring slot a barrier stands at is read from its parity, so a waiter must know that the use before is through.
+    //   Producer (`empty`): it walks all stages.  Consumers (`full`): the slots of a group are its own (the ring is even, or not used
+    //   twice), and it walks them in order.  Epilogue warps (`done`): their own tile before is through, and with it, since the
+    //   groups go in order, everything up to it; plan() has no more of them than the ring allows for.
     if (warp == GEMV_PRODUCER) {
         // ------------------------------ producer ------------------------------
-        // Waiting for a free slot, arming its barrier and issuing a copy is a dependent chain of several
-        // hundred cycles, so the warp runs it for several stages at once: the lanes form groups of `cps`
-        // (copies per stage), one group per stage of a pass; the first lane of a group waits and arms,
-        // every lane issues one copy.
-        const uint32_t nplanes = (uint32_t)NPL;
-        const uint32_t cps = 1u << a.cps_log2;                   // copies per stage: 1, 2, 4 or 8
-        const uint32_t spb = a.spb;                              // stages per pass
-        const uint32_t sb = (uint32_t)lane >> a.cps_log2, ci = (uint32_t)lane & (cps - 1);
-        const uint32_t gmask = ((1u << cps) - 1u) << (sb * cps);
-        if (sb >= spb) return;
-        const uint32_t pmask = spb * cps >= 32 ? ~0u : (1u << (spb * cps)) - 1u;   // the lanes that stay
-        uint32_t s = sb, half = 0, turn = 0;                     // ring slot of stage `it` (spb <= nstage)
-        for (uint32_t it = sb; it < nst + sb; it += spb) {       // every lane: as many passes as the first
-            if (it < nst) {
-                Part parts[2];
-                uint32_t n = 0;
-                const int nparts = group_parts(a, EPI, blockIdx.x + it * gridDim.x, parts, n);
-                const uint32_t full = full0 + 8 * s + half;
-                if (ci == 0) {
-                    if (it >= nstage) mbar_wait(full0 + EMPTY + 8 * s, half ? 0u : 1u, a.err, 2, a.wait_ns);   // release of the use before
-                    mbar_expect_tx(full, nparts * n * row_bytes);
+        const uint32_t oct = a.octets, pl = (uint32_t)lane % NPL, o = (uint32_t)lane / NPL;   // a lane per copy: plane, eight rows
+        if (o >= oct) return;
+        const uint32_t pmask = (1u << (NPL * oct)) - 1u;
+        const uint32_t box = pl == 0 ? tile_box(QT, 0) : pl == 1 ? tile_box(QT, 1) : pl == 2 ? tile_box(QT, 2) : tile_box(QT, 3);
+        const uint32_t step = (pl == 0 ? tile_step(QT, 0) : pl == 1 ? tile_step(QT, 1) : pl == 2 ? tile_step(QT, 2) : tile_step(QT, 3)) / 8;
+        const uint32_t off = pl == 0 ? 0u : pl == 1 ? tile_offset(QT, 1) : pl == 2 ? tile_offset(QT, 2) : tile_offset(QT, 3);
+        const uint32_t dst0 = ring + off * oct + o * TILE_ROWS * box;
+        const uint64_t policy = streaming_policy();
+        uint32_t s = 0, phase = 1, filled = 0;
+        for (uint32_t ti = blockIdx.x; ti < a.ntiles; ti += gridDim.x) {
+            Part parts[2];
+            uint32_t n = 0;
+            const int nparts = tile_parts(a, EPI, ti, parts, n);
+            const uint32_t row = nparts == 2 ? parts[o].row0 : parts[0].row0 + o * TILE_ROWS;
+            const CUtensorMap *map = &a.map[parts[0].mat + (EPI == EPI_SILU_PAIR ? o : 0)][pl];
+            for (uint32_t c = 0; c < nchunk; c++) {
+                if (lane == 0) {
+                    if (filled >= nstage) mbar_wait(empty0 + 8 * s, phase, a.err, 2, a.wait_ns);
+                    mbar_expect_tx(full0 + 8 * s, oct * tile_bytes(QT));
                 }
-                __syncwarp(gmask);
-                if (ci < (uint32_t)nparts * nplanes) {
-                    const uint32_t pi = ci / nplanes, pl = ci % nplanes;   // nplanes is a compile-time power of two
-                    // a stage holds plane after plane; within a plane, the rows of part 0 then those of part 1
-                    const QMat &m = a.mat[parts[pi].mat];
-                    uint32_t off = pi * n * m.pitch[pl];
-                    for (uint32_t q = 0; q < pl; q++) off += (uint32_t)nparts * n * m.pitch[q];
-                    bulk_copy_g2s(ring + s * a.stage_bytes + off, m.p[pl] + (size_t)parts[pi].row0 * m.pitch[pl], n * m.pitch[pl], full);
+                __syncwarp(pmask);
+                tile_copy(dst0 + s * a.stage_bytes, map, c * step, row, full0 + 8 * s, policy);
+                filled++;
+                if (++s == nstage) {
+                    s = 0;
+                    phase ^= 1;
                 }
             }
-            __syncwarp(pmask);
-            s += spb;
-            if (s >= nstage) next_round(s, half, turn);
         }
         return;
     }
-    if (warp == GEMV_EPILOGUE) {
+    if (warp >= GEMV_EPILOGUE) {
         // ------------------------------ epilogue ------------------------------
-        // Up to four stages per pass: lanes 8k..8k+7 take stage it0 + k, one lane per output unit.
+        // The warps take the block's tiles in turn.  (One warp needed 1.2 us per tile of a q/k/v launch, all of it latency, and ended
+        // a launch of five tiles per block a microsecond after the consumers.)
+        const uint32_t nepi = a.nepi, first = (uint32_t)warp - GEMV_EPILOGUE;
+        if (first >= nepi || blockIdx.x + first * gridDim.x >= a.ntiles) return;
         pdl_wait();
+        const uint32_t pos = EPI == EPI_QKV_ROPE || EPI == EPI_QKV_SPLIT ? __ldcg(a.pos) : 0u;
         if (EPI == EPI_QKV_ROPE) {
             // rotation of every pair index of a head at this position (ops/rope.wgsl:36-77)
-            const uint32_t half = a.head_size / 2;
-            if (half <= GEMV_ROPE_TAB) {
-                const float pos = (float)*a.pos;
-                for (uint32_t i = lane; i < half; i += 32) {
-                    float sn, cs;
-                    sincosf(pos * a.rope_freq[i], &sn, &cs);
-                    rope_tab[i] = make_float2(cs, sn);
-                }
+#pragma unroll 1
+            for (uint32_t i = lane; i < a.head_size / 2; i += 32) {
+                float sn, cs;
+                sincosf((float)pos * __ldg(a.rope_freq + i), &sn, &cs);
+                rope_tab[i] = make_float2(cs, sn);
             }
             __syncwarp();
         }
-        const uint32_t nb = epilogue_batch(nstage);
-        const uint32_t sub = (uint32_t)lane >> 3, ul = (uint32_t)lane & 7;
-        const uint32_t gmask = 0xffu << (8 * sub);
-        uint32_t s = sub, half = 0, turn = 0;   // ring slot of stage it0 + sub (nb <= nstage)
+        const uint32_t row = (uint32_t)lane & 15, half = (uint32_t)lane >> 4;   // a lane adds four units of a row
+        uint32_t s = 0, phase = 0;
+        auto skip_stages = [&](uint32_t n) {
+            s += n;
+            while (s >= nstage) {
+                s -= nstage;
+                phase ^= 1;
+            }
+        };
+        skip_stages(first * nchunk);
         float rms_scale = 1.0f;
         bool have_scale = false;
-        for (uint32_t it0 = 0; it0 < nst; it0 += nb, s += nb) {
-            if (s >= nstage) next_round(s, half, turn);
-            const uint32_t it = it0 + sub;
-            if (sub >= nb || it >= nst) continue;
-            Part parts[2];
-            uint32_t n = 0;
-            const int nparts = group_parts(a, EPI, blockIdx.x + it * gridDim.x, parts, n);
-            const uint32_t nunits = group_units(EPI, parts, nparts, n);
-            const EpiCtx c = epi_prepare(a, EPI, parts, nparts, n, ul, nunits, rope_tab);
-            uint32_t ra = 0, rb = 0;
-            if (c.on) unit_rows(EPI, parts, nparts, n, ul, ra, rb);
-            mbar_wait(full0 + DONE + 8 * s + half, turn, a.err, 3, a.wait_ns);
-            if (PRO == PRO_RMS && !have_scale) {
-                // every consumer warp wrote its sum of squares before its first arrival on a `done` barrier
-                float ss = 0.0f;
+        // The next tile's loads are out before this tile's sums are waited for (the first round only issues them).
+        EpiCtx next = {};
+#pragma unroll 1
+        for (uint32_t ti = blockIdx.x + first * gridDim.x, round = 0;; ti += nepi * gridDim.x, round++) {
+            const EpiCtx c = next;
+            if (ti < a.ntiles) next = epi_prepare(a, EPI, ti, lane, pos, rope_tab);
+            if (round == 0) continue;
+            float y = 0.0f;
+#pragma unroll 1
+            for (uint32_t left = units; left; ) {
+                const uint32_t in_stage = min(left, TILE_UNITS);
+                mbar_wait(done0 + 8 * s, phase, a.err, 3, a.wait_ns);
+                const float *p = part + s * (TILE_UNITS * 16) + half * 64 + row;
 #pragma unroll
-                for (int w = 0; w < GEMV_NCONS; w++) ss += red[w];
-                rms_scale = 1.0f / sqrtf(ss / (float)K + a.eps);
-                have_scale = true;
+                for (uint32_t k = 0; k < 4; k++)
+                    if (half * 4 + k < in_stage) y += p[k * 16];
+                __syncwarp();
+                if (lane == 0) mbar_arrive(empty0 + 8 * s);   // stage and partial sums may be overwritten
+                left -= in_stage;
+                skip_stages(1);
             }
-            float ya = 0.0f, yb = 0.0f;
-            if (c.on) {
-                for (uint32_t k = 0; k < kp; k++) {
-                    ya += part[s][k][ra];
-                    yb += part[s][k][rb];
+            skip_stages((nepi - 1) * nchunk);
+            y += __shfl_xor_sync(0xffffffffu, y, 16);
+            if (PRO == PRO_RMS) {
+                if (!have_scale) {
+                    // every consumer warp wrote its sum of squares before its first arrival on a `done` barrier
+                    float ss = 0.0f;
+#pragma unroll
+                    for (int w = 0; w < GEMV_NCONS; w++) ss += red[w];
+                    rms_scale = 1.0f / sqrtf(ss / (float)K + a.eps);
+                    have_scale = true;
                 }
-                if (PRO == PRO_RMS) {
-                    ya *= rms_scale;
-                    yb *= rms_scale;
-                }
+                y *= rms_scale;
             }
-            __syncwarp(gmask);
-            if (ul == 0) mbar_arrive(full0 + EMPTY + 8 * s);   // stage and partial sums may be overwritten
-            epi_finish(a, EPI, parts, c, ya, yb);
+            const float ya = __shfl_sync(0xffffffffu, y, c.ra), yb = __shfl_sync(0xffffffffu, y, c.rb);
+            epi_finish<PEERS>(a, EPI, c, ya, yb);
+            if (ti >= a.ntiles) break;
         }
-        if ((EPI == EPI_STORE || EPI == EPI_RESIDUAL) && a.peer_out.n) {
+        if (PEERS && a.peer_out.n) {
             // The block's partial rows are on their way to the peers; the last block of the launch raises
             // this rank's flag everywhere once every block's stores are visible system-wide.
             __threadfence_system();
@@ -494,37 +403,55 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
     }
 
     // ------------------------------ consumers ------------------------------
-    // What the task loop needs and the input does not decide is worked out while the launch before drains.
-    const uint32_t ncl = GEMV_NCONS / kp;                 // "lanes" of warps per column part
-    const XImage im = ximage_carve(QT, K, smem);
-    const uint32_t kunits = QT == WGB_F32 ? K : a.mat[0].bpr;   // what Step::active() compares against
-    const uint32_t nsteps = (K + step_cols<QT>() - 1) / step_cols<QT>();
-    const uint32_t kw = (uint32_t)warp % kp, cl = (uint32_t)warp / kp;
-    // The norm weights are parameters, not products of the launch before: their (cold, HBM-latency) loads
-    // are issued ahead of the dependency wait and are in registers by the time the input can be read.
-    // A thread owns units of eight consecutive inputs (two float4 chunks), u = threadIdx.x + i * GEMV_CONS_THREADS;
-    // the first XU of them live in registers from one round of loads to the staging: all of them up to 8192
-    // columns, up to 12288 where the kernel has no norm parameters to hold.
-    constexpr uint32_t XU = PRO_T == PRO_NONE ? 3 : 2, WU = PRO_T == PRO_NONE ? 1 : 2;
-    const uint32_t nchunk = K / 4, nunit = (nchunk + 1) / 2;
-    float4 wc[2 * WU], bc[2 * WU];
-    if (PRO != PRO_NONE) {
+    // What the input does not decide is worked out while the launch before drains.
+    // Task loop: the warps of a group take the units of every stage, the two groups alternate stages.  The digits of the inputs of a unit stay in registers as long as the unit does (one or
+    // two stages per tile).  Lane 4g + t has rows g and g + 8 of the tile; in a tile of eight rows, g twice.
+    const XImage<QT> im(smem0 + skip, units);
+    uint32_t held = ~0u, phase = 0;
+    const uint32_t w = (uint32_t)warp % TILE_UNITS, group = (uint32_t)warp / TILE_UNITS, ngroups = nstage > 1 ? 2 : 1;
+    const uint32_t g = (uint32_t)lane >> 2, oct = a.octets;
+    uint32_t row_at[NPL], second[NPL];   // the lane's first row within a stage, from there to the second
 #pragma unroll
-        for (uint32_t i = 0; i < WU; i++) {
-            const uint32_t c = 2 * (threadIdx.x + i * GEMV_CONS_THREADS);
-#pragma unroll
-            for (uint32_t h = 0; h < 2; h++) {
-                if (c + h < nchunk) {
-                    wc[2 * i + h] = __ldg(reinterpret_cast<const float4 *>(a.norm_w) + c + h);
-                    if (PRO == PRO_LN) bc[2 * i + h] = __ldg(reinterpret_cast<const float4 *>(a.norm_b) + c + h);
-                }
-            }
-        }
+    for (int q = 0; q < NPL; q++) {
+        row_at[q] = ring + tile_offset(QT, q) * oct + g * tile_box(QT, q);
+        second[q] = (oct - 1) * TILE_ROWS * tile_box(QT, q);
     }
+    const uint32_t nst = (a.per_block - (a.rem_blocks != 0 && blockIdx.x >= a.rem_blocks ? 1u : 0u)) * nchunk;   // stages of this block
+    uint32_t s = group, chunk = group < nchunk ? group : 0u;
+    // The input, eight consecutive values per thread and round.  The norm weights are parameters, not products of the launch
+    // before: the first round's (cold, HBM-latency) loads are issued ahead of the dependency wait.  A round's loads go out a
+    // round ahead.
+    const uint32_t nvec = K / 4, noct = (nvec + 1) / 2;
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    struct Eight { float4 a, b; };
+    auto load_param = [&](const float *p, uint32_t u) {
+        Eight e = { zero4, zero4 };
+        if (2 * u < nvec) e.a = __ldg(reinterpret_cast<const float4 *>(p) + 2 * u);
+        if (2 * u + 1 < nvec) e.b = __ldg(reinterpret_cast<const float4 *>(p) + 2 * u + 1);
+        return e;
+    };
+    auto load_vec = [&](uint32_t c) {
+        if (!PEERS || !a.peer_in.n) return ld_act4(a.x + 4 * c);
+        float4 v = __ldcg(reinterpret_cast<const float4 *>(a.peer_in.mail) + c);
+        for (uint32_t r = 1; r < a.peer_in.n; r++) {
+            const float4 w = __ldcg(reinterpret_cast<const float4 *>(a.peer_in.mail + (size_t)r * K) + c);
+            v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+        }
+        if (blockIdx.x == 0) reinterpret_cast<float4 *>(a.peer_in.x_out)[c] = v;
+        return v;
+    };
+    auto load_x = [&](uint32_t u) {
+        Eight e = { zero4, zero4 };
+        if (2 * u < nvec) e.a = load_vec(2 * u);
+        if (2 * u + 1 < nvec) e.b = load_vec(2 * u + 1);
+        return e;
+    };
+    const uint32_t u0 = threadIdx.x;
+    Eight gain, bias;
+    if (PRO != PRO_NONE) gain = load_param(a.norm_w, u0);
+    if (PRO == PRO_LN) bias = load_param(a.norm_b, u0);
     pdl_wait();
-    float4 xc[2 * XU];
-    const bool gather = PRO == PRO_RMS && a.peer_in.n != 0;
-    if (gather) {
+    if (PEERS && a.peer_in.n) {
         // Partial products from every rank: wait for the flags, then add in rank order.  The wait is bounded
         // in time (a.peer_wait_ns); a wait that runs out leaves code 6 in the status word, and while the word
         // is non-zero no launch waits at all, so one missing rank costs one limit, not one per exchange.
@@ -548,192 +475,107 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
         }
         cons_sync();
     }
-    auto load_chunk = [&](uint32_t c) {
-        if (!gather) return ld_act4(a.x + 4 * c);
-        float4 v = __ldcg(reinterpret_cast<const float4 *>(a.peer_in.mail) + c);
-        for (uint32_t r = 1; r < a.peer_in.n; r++) {
-            const float4 w = __ldcg(reinterpret_cast<const float4 *>(a.peer_in.mail + (size_t)r * K) + c);
-            v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
-        }
-        if (blockIdx.x == 0) reinterpret_cast<float4 *>(a.peer_in.x_out)[c] = v;
-        return v;
-    };
-    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (uint32_t i = 0; i < XU; i++) {
-        const uint32_t c = 2 * (threadIdx.x + i * GEMV_CONS_THREADS);
-        xc[2 * i] = c < nchunk ? load_chunk(c) : zero4;
-        xc[2 * i + 1] = c + 1 < nchunk ? load_chunk(c + 1) : zero4;
-    }
-    // Units past the ones held in registers (longer rows) are read again where needed.
-    const uint32_t u_tail = threadIdx.x + XU * GEMV_CONS_THREADS;
+    Eight x = load_x(u0);
     float mean = 0.0f, scale = 1.0f;
-    if (PRO == PRO_RMS) {
-        float ss = 0.0f;
+    if (PRO == PRO_LN) {
+        // Two passes, mean and deviations from it; up to 4096 columns a thread's values stay in registers.
+        auto total = [&](const auto &term, float *part_sums) {
+            float v = 0.0f;
+            Eight e = x;
+#pragma unroll 1
+            for (uint32_t u = u0; u < noct;) {
+                v += term(e.a);
+                if (2 * u + 1 < nvec) v += term(e.b);   // (only a dense f32 vector can end in the middle of eight)
+                u += GEMV_CONS_THREADS;
+                if (u < noct) e = load_x(u);
+            }
+            v = warp_sum(v);
+            if (lane == 0) part_sums[warp] = v;
+            cons_sync();
+            const float4 *p = reinterpret_cast<const float4 *>(part_sums);   // every thread adds the sixteen
+            float4 t = p[0];
 #pragma unroll
-        for (uint32_t i = 0; i < 2 * XU; i++) ss += xc[i].x * xc[i].x + xc[i].y * xc[i].y + xc[i].z * xc[i].z + xc[i].w * xc[i].w;
-        for (uint32_t u = u_tail; u < nunit; u += GEMV_CONS_THREADS) {
-            for (uint32_t c = 2 * u; c < min(2 * u + 2, nchunk); c++) {
-                const float4 v = load_chunk(c);
-                ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            }
-        }
-        // The scale is one factor for the whole vector, so it commutes with the dot products: the input is
-        // staged as x * w, the warps' sums of squares go to `red`, and the epilogue warp multiplies every
-        // finished dot product by 1 / sqrt(mean square + eps).  No block-wide reduction ahead of the staging.
-        ss = warp_sum(ss);
-        if (lane == 0) red[warp] = ss;
-    } else if (PRO == PRO_LN) {
-        float sm = 0.0f;
-#pragma unroll
-        for (uint32_t i = 0; i < 2 * XU; i++) sm += (xc[i].x + xc[i].y) + (xc[i].z + xc[i].w);   // chunks past the end are zero
-        for (uint32_t u = u_tail; u < nunit; u += GEMV_CONS_THREADS) {
-            for (uint32_t c = 2 * u; c < min(2 * u + 2, nchunk); c++) {
-                const float4 v = load_chunk(c);
-                sm += (v.x + v.y) + (v.z + v.w);
-            }
-        }
-        mean = cons_sum(sm, red) / (float)K;
-        float ss = 0.0f;
-#pragma unroll
-        for (uint32_t i = 0; i < 2 * XU; i++) {
-            if (2 * (threadIdx.x + (i / 2) * GEMV_CONS_THREADS) + (i & 1) < nchunk) {
-                const float dx = xc[i].x - mean, dy = xc[i].y - mean, dz = xc[i].z - mean, dw = xc[i].w - mean;
-                ss += dx * dx + dy * dy + dz * dz + dw * dw;
-            }
-        }
-        for (uint32_t u = u_tail; u < nunit; u += GEMV_CONS_THREADS) {
-            for (uint32_t c = 2 * u; c < min(2 * u + 2, nchunk); c++) {
-                float4 v = load_chunk(c);
-                v.x -= mean; v.y -= mean; v.z -= mean; v.w -= mean;
-                ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            }
-        }
-        ss = cons_sum(ss, red);
-        scale = 1.0f / sqrtf(ss / (float)K + 1.0e-5f);
+            for (int i = 1; i < GEMV_NCONS / 4; i++) { t.x += p[i].x; t.y += p[i].y; t.z += p[i].z; t.w += p[i].w; }
+            return (t.x + t.y) + (t.z + t.w);
+        };
+        mean = total([](const float4 v) { return (v.x + v.y) + (v.z + v.w); }, red) / (float)K;
+        const float m2 = total([&](const float4 v) {
+            const float p = v.x - mean, q = v.y - mean, r = v.z - mean, t = v.w - mean;
+            return (p * p + q * q) + (r * r + t * t);
+        }, red + GEMV_NCONS);
+        scale = 1.0f / sqrtf(m2 / (float)K + 1.0e-5f);
     }
     {
-        const XWriter<QT> xw(smem, K);
-        auto transform = [&](float4 v, const float4 w, const float4 b) {
+        const XWriter<QT> xw(image, units);
+        xw.pad(K, units, threadIdx.x, GEMV_CONS_THREADS);
+        // RMSNorm: the scale is one factor for the whole vector, so it commutes with the dot products.  The input is staged as x * w,
+        // the warps' sums of squares go to `red`, and the epilogue multiplies every finished dot product by
+        // 1 / sqrt(mean square + eps).  No block-wide reduction ahead of the staging.
+        auto transform = [&](float4 v, const float4 g, const float4 b) {
             if (PRO == PRO_RMS) {
-                v.x *= w.x; v.y *= w.y; v.z *= w.z; v.w *= w.w;
+                v.x *= g.x; v.y *= g.y; v.z *= g.z; v.w *= g.w;
             } else if (PRO == PRO_LN) {
-                v.x = ((v.x - mean) * scale) * w.x + b.x; v.y = ((v.y - mean) * scale) * w.y + b.y;
-                v.z = ((v.z - mean) * scale) * w.z + b.z; v.w = ((v.w - mean) * scale) * w.w + b.w;
+                v.x = ((v.x - mean) * scale) * g.x + b.x; v.y = ((v.y - mean) * scale) * g.y + b.y;
+                v.z = ((v.z - mean) * scale) * g.z + b.z; v.w = ((v.w - mean) * scale) * g.w + b.w;
             }
             return v;
         };
-        auto param = [&](const float *p, uint32_t c, bool in) {
-            return in ? __ldg(reinterpret_cast<const float4 *>(p) + c) : zero4;
-        };
+        float ss = 0.0f;
         // whole warps go round together (the writer shuffles): the bound is per warp, not per lane
-        const uint32_t warp_u0 = (uint32_t)warp * 32;
-#pragma unroll
-        for (uint32_t i = 0; i < XU; i++) {
-            if (warp_u0 + i * GEMV_CONS_THREADS < nunit) {
-                const uint32_t u = threadIdx.x + i * GEMV_CONS_THREADS, c = 2 * u;
-                const bool in = c < nchunk, inb = c + 1 < nchunk;
-                float4 w0 = zero4, w1 = zero4, b0 = zero4, b1 = zero4;
-                if (i < WU) {
-                    w0 = wc[2 * i]; w1 = wc[2 * i + 1];
-                    b0 = bc[2 * i]; b1 = bc[2 * i + 1];
-                } else if (PRO != PRO_NONE) {
-                    w0 = param(a.norm_w, c, in); w1 = param(a.norm_w, c + 1, inb);
-                    if (PRO == PRO_LN) { b0 = param(a.norm_b, c, in); b1 = param(a.norm_b, c + 1, inb); }
-                }
-                xw.put8(u, transform(xc[2 * i], w0, b0), transform(xc[2 * i + 1], w1, b1), in, inb);
+#pragma unroll 1
+        for (uint32_t u = u0; u - lane < noct; u += GEMV_CONS_THREADS) {
+            const Eight xn = x, gn = gain, bn = bias;
+            if (u - lane + GEMV_CONS_THREADS < noct) {
+                x = load_x(u + GEMV_CONS_THREADS);
+                if (PRO != PRO_NONE) gain = load_param(a.norm_w, u + GEMV_CONS_THREADS);
+                if (PRO == PRO_LN) bias = load_param(a.norm_b, u + GEMV_CONS_THREADS);
             }
+            if (PRO == PRO_RMS)
+                ss += ((xn.a.x * xn.a.x + xn.a.y * xn.a.y) + (xn.a.z * xn.a.z + xn.a.w * xn.a.w)) +
+                      ((xn.b.x * xn.b.x + xn.b.y * xn.b.y) + (xn.b.z * xn.b.z + xn.b.w * xn.b.w));
+            xw.put8(u, transform(xn.a, gn.a, bn.a), transform(xn.b, gn.b, bn.b), 2 * u < nvec, 2 * u + 1 < nvec);
         }
-        for (uint32_t u0 = warp_u0 + XU * GEMV_CONS_THREADS; u0 < nunit; u0 += GEMV_CONS_THREADS) {
-            const uint32_t u = u0 + lane, c = 2 * u;
-            const bool in = c < nchunk, inb = c + 1 < nchunk;
-            float4 va = zero4, vb = zero4, w0 = zero4, w1 = zero4, b0 = zero4, b1 = zero4;
-            if (in) va = load_chunk(c);
-            if (inb) vb = load_chunk(c + 1);
-            if (PRO != PRO_NONE) { w0 = param(a.norm_w, c, in); w1 = param(a.norm_w, c + 1, inb); }
-            if (PRO == PRO_LN) { b0 = param(a.norm_b, c, in); b1 = param(a.norm_b, c + 1, inb); }
-            xw.put8(u, transform(va, w0, b0), transform(vb, w1, b1), in, inb);
+        if (PRO == PRO_RMS) {
+            ss = warp_sum(ss);
+            if (lane == 0) red[warp] = ss;
         }
     }
     cons_sync();
 
-    if ((uint32_t)warp >= kp * ncl) return;               // warps left over when kp does not divide the consumers
-    typename S::X x;
-    // prefix[q]: bytes of planes 0..q-1 of one row (a stage holds plane after plane, see the producer)
-    uint32_t prefix[NPL];
-    {
-        uint32_t acc = 0;
-#pragma unroll
-        for (int q = 0; q < NPL; q++) {
-            prefix[q] = acc;
-            acc += a.mat[0].pitch[q];
+    if (group >= ngroups) return;
+    typename U::Digits digits;
+    digits.clear();
+    for (uint32_t it = group; it < nst; it += ngroups) {
+        const uint32_t u = chunk * TILE_UNITS + w;
+        if (u < units && u != held) {
+            digits.load(im, u, lane);
+            held = u;
         }
-    }
-
-    // Task loop.  A task is up to GEMV_TASK_ROWS rows of one stage, taken one at a time by a rolled loop whose
-    // body -- one call of the format's dot product -- is the whole hot path of the kernel: two kilobytes of
-    // code that every warp of the block shares in the instruction caches.  (Unrolled over the rows the loop ran
-    // with "no instruction" as its first stall reason, and the launches of a decode step evict one another's
-    // code, so whatever a launch executes it first has to fetch.)  Nothing in the body depends on the lane:
-    // a lane past the end of the row works on the row's first unit with an all-zero input instead of sitting
-    // out.  Each lane leaves its partial sum of a row in shared memory; after the last row the warp adds the
-    // 32 partials of every row: lane l takes four partials of row l / 8, three butterfly steps do the rest.
-    // For every shape the models use the matrix has no more column steps than there are consumer warps, so the
-    // loop over steps makes one trip and the warp's part of the input is loaded once per kernel.
-    constexpr int R = GEMV_TASK_ROWS;
-    static_assert(R == 4, "the reduction below reads four partials per lane of four rows");
-    const uint32_t Rn = a.rrows;
-    float *my_part = &lane_part[warp][0][0];
-    uint32_t held = ~0u;   // column step whose part of the input is in `x`
-    int lane_d = lane;
-    uint32_t s = 0, half = 0, turn = 0, it_prev = 0;
-    for (uint32_t t = cl; t < nst * rparts; t += ncl) {
-        const uint32_t it = t >> a.rparts_log2, rp = t & (rparts - 1);
-        s += it - it_prev;
-        it_prev = it;
-        while (s >= nstage) next_round(s, half, turn);
-        uint32_t nrows = a.rs;   // rows in this stage: fewer only in the last group of a matrix
-        if (EPI != EPI_QKV_ROPE) {
-            Part parts[2];
-            uint32_t n = 0;
-            const int nparts = group_parts(a, EPI, blockIdx.x + it * gridDim.x, parts, n);
-            nrows = nparts * n;
-        }
-        const uint32_t j0 = rp * Rn;
-        const uint32_t jn = min(Rn, nrows > j0 ? nrows - j0 : 0u);
-        const uint32_t stage = ring + s * a.stage_bytes;
-        mbar_wait(full0 + 8 * s + half, turn, a.err, 1, a.wait_ns);
-        for (uint32_t ks = kw; ks < nsteps; ks += kp) {
-            const uint32_t col0 = ks * step_cols<QT>();
-            if (held != ks) {
-                const bool on = S::active(kunits, col0, lane);
-                lane_d = on ? lane : S::lane0(lane);
-                if (on) S::load_x(x, im, col0, lane);
-                else zero_x(x);
-                held = ks;
-            }
-            uint32_t r[4];
+        mbar_wait(full0 + 8 * s, phase, a.err, 1, a.wait_ns);
+        if (u < units) {
+            uint32_t sa[NPL], sb[NPL];
 #pragma unroll
-            for (int q = 0; q < NPL; q++) r[q] = stage + nrows * prefix[q] + j0 * a.mat[0].pitch[q];
-            const bool first = ks == kw;
-#pragma unroll 1
-            for (uint32_t j = 0; j < jn; j++) {
-                float v = S::dot(r, col0, x, lane_d);
-                if (!first) v += my_part[j * 32 + lane];
-                my_part[j * 32 + lane] = v;
-#pragma unroll
-                for (int q = 0; q < NPL; q++) r[q] += a.mat[0].pitch[q];
+            for (int q = 0; q < NPL; q++) {
+                sa[q] = row_at[q] + s * a.stage_bytes;
+                sb[q] = sa[q] + second[q];
             }
+            float ya, yb;
+            U::eval(sa, sb, w, digits, im, u, lane, ya, yb);
+            // fold over the quad: even lanes keep row g, odd ones row g + 8
+            const float send = lane & 1 ? ya : yb;
+            float y = (lane & 1 ? yb : ya) + __shfl_xor_sync(0xffffffffu, send, 1);
+            y += __shfl_xor_sync(0xffffffffu, y, 2);
+            if ((lane & 2) == 0) part[(s * TILE_UNITS + w) * 16 + g + 8 * (lane & 1)] = y;
         }
         __syncwarp();
-        const float4 p4 = reinterpret_cast<const float4 *>(my_part)[lane];   // partials 4 (l % 8) .. + 3 of row l / 8
-        float v = (p4.x + p4.y) + (p4.z + p4.w);
-        v += __shfl_xor_sync(0xffffffffu, v, 4);
-        v += __shfl_xor_sync(0xffffffffu, v, 2);
-        v += __shfl_xor_sync(0xffffffffu, v, 1);
-        if ((lane & 7) == 0 && (uint32_t)(lane >> 3) < jn) part[s][kw][j0 + (lane >> 3)] = v;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(full0 + DONE + 8 * s + half);
+        if (lane == 0) mbar_arrive(done0 + 8 * s);
+        s += ngroups;
+        if (s >= nstage) {
+            s -= nstage;
+            phase ^= 1;
+        }
+        chunk += ngroups;
+        while (chunk >= nchunk) chunk -= nchunk;
     }
 }
 
@@ -775,7 +617,7 @@ __global__ void __launch_bounds__(256) gemv_generic_kernel(const __grid_constant
 
 bool gemv_fast_supported(const QMat &m)
 {
-    if (!has_fast_path(m.qtype)) return false;
+    if (m.qtype != WGB_Q4_K && m.qtype != WGB_Q6_K && m.qtype != WGB_Q8_0 && m.qtype != WGB_F32) return false;
     for (int i = 0; i < m.nplanes; i++)
         if (((uintptr_t)m.p[i] % 16) != 0 || m.pitch[i] % 16 != 0) return false;
     if (m.qtype == WGB_F32) return m.ncols % 4 == 0;
@@ -849,131 +691,91 @@ void status_poll_destroy(StatusPoll &sp)
     }
 }
 
-// Whether the consumers' waits can tell the uses of a ring of `nstage` slots apart (above cons_sync), with one stage per producer pass.
-static bool ring_safe(uint32_t per_block, uint32_t nstage, uint32_t ncl, uint32_t rparts)
+int make_tile_maps(const QMat &m, TileMaps &out)
 {
-    return per_block <= nstage || ncl <= rparts || (nstage * rparts) % ncl == 0 || (ncl + rparts - 1) / rparts < nstage;
+    using Encode = decltype(&cuTensorMapEncodeTiled);
+    static Encode encode = nullptr;
+    if (!encode) {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        WGB_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found));
+        if (found != cudaDriverEntryPointSuccess || !fn) return fail(WGB_ERR_UNSUPPORTED, "the driver has no tensor maps");
+        encode = reinterpret_cast<Encode>(fn);
+    }
+    for (int i = 0; i < m.nplanes; i++) {
+        // rows of eight-byte elements (rows, boxes and steps are multiples of 16 bytes); past the ends of a matrix zeros are read
+        const cuuint64_t dims[2] = { m.pitch[i] / 8, m.nrows }, strides[1] = { m.pitch[i] };
+        const cuuint32_t box[2] = { tile_box(m.qtype, i) / 8, TILE_ROWS }, ones[2] = { 1, 1 };
+        const CUresult r = encode(&out.map[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<uint8_t *>(m.p[i]), dims, strides, box, ones,
+                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return fail(WGB_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for plane %d of %u x %u", (int)r, i, m.nrows, m.ncols);
+        out.p[i] = m.p[i];
+    }
+    out.nrows = m.nrows;
+    return WGB_OK;
 }
 
-static uint32_t steps_of(int qt, uint32_t K)
-{
-    const uint32_t sc = qt == WGB_Q4_K ? step_cols<WGB_Q4_K>() : qt == WGB_Q6_K ? step_cols<WGB_Q6_K>()
-                      : qt == WGB_Q8_0 ? step_cols<WGB_Q8_0>() : step_cols<WGB_F32>();
-    return (K + sc - 1) / sc;
-}
-
-// Chooses rows per stage, the row split, ring depth and grid; fills the plan fields of `a`.  Returns
-// false when the shapes do not fit the kernel's assumptions.
-//
-// Candidates are (rs rows per stage, rparts row parts per stage); a consumer task is rrows = rs / rparts
-// rows of one column part, and the ncl = 16 / kparts warps of a column part take the tasks of the block
-// in turn.  The time of the launch is that of its fullest block: ceil(tasks / ncl) rounds of
-// (rrows + 1/2) row products, the half row standing for the wait, reduction and hand-off of a task.
-// That is divided by how much of the ~80 KB per SM that must be in flight to cover HBM latency at full
-// bandwidth the ring can hold beyond the stages the consumers are working on, and by a mild preference
-// for larger copies.
+// Chooses rows per tile, ring depth and grid; fills the plan fields of `a`.  Returns false when the image of the input leaves no
+// room for a stage.
 static bool plan(GemvArgs &a, size_t &smem_bytes, uint32_t &grid)
 {
     const QMat &m0 = a.mat[0];
-    uint32_t row_bytes = 0;
-    for (int i = 0; i < m0.nplanes; i++) row_bytes += m0.pitch[i];
+    const int qt = m0.qtype;
     const uint32_t sms = (uint32_t)sm_count();
+    const bool pairs = a.epilogue == EPI_SILU_PAIR || (a.epilogue == EPI_QKV_ROPE && a.rope_variant == WGB_ROPE_NEOX);
     uint32_t total_rows = 0;
-    for (int i = 0; i < a.nmat; i++) total_rows += a.mat[i].nrows;
-    const bool pairs = a.epilogue == EPI_SILU_PAIR || a.epilogue == EPI_QKV_ROPE;
-    const size_t image = (ximage_bytes(m0.qtype, m0.ncols) + 127) & ~(size_t)127;
-    if (image + 256 > GEMV_SMEM_BUDGET) return false;
-    const uint32_t nsteps = steps_of(m0.qtype, m0.ncols);
-    const uint32_t kp = nsteps < (uint32_t)GEMV_NCONS ? nsteps : (uint32_t)GEMV_NCONS;
-    const uint32_t ncl = GEMV_NCONS / kp;
-    const double want_in_flight = 80.0 * 1024;
-
-    auto groups_of = [&](uint32_t rs) -> uint32_t {
-        if (a.epilogue == EPI_SILU_PAIR) return (m0.nrows + rs / 2 - 1) / (rs / 2);
-        if (a.epilogue == EPI_QKV_ROPE) return total_rows / rs;
-        return (m0.nrows + rs - 1) / rs;
+    for (int i = 0; i < (a.epilogue == EPI_SILU_PAIR ? 1 : a.nmat); i++) total_rows += a.mat[i].nrows;
+    a.octets = !pairs && (total_rows + TILE_ROWS - 1) / TILE_ROWS <= sms ? 1 : 2;
+    a.tile_rows = a.octets * TILE_ROWS;
+    auto tiles = [&](const QMat &m) { return (m.nrows + a.tile_rows - 1) / a.tile_rows; };
+    if (a.epilogue == EPI_SILU_PAIR) a.ntiles = (m0.nrows + TILE_ROWS - 1) / TILE_ROWS;
+    else if (a.epilogue == EPI_QKV_ROPE) {
+        auto magic = [](uint32_t d) { return d > 1 ? (uint32_t)((0x100000000ull + d - 1) / d) : 0u; };
+        a.per_head = (a.head_size / 2 + TILE_ROWS - 1) / TILE_ROWS;
+        a.per_head_magic = magic(a.per_head);
+        a.head_magic = magic(a.head_size);
+        if ((uint64_t)total_rows * a.head_size >> 32 || a.head_size / 2 > GEMV_ROPE_TAB) return false;   // small_div, rope_tab
+        a.tq = pairs ? a.mat[0].nrows / a.head_size * a.per_head : tiles(a.mat[0]);
+        a.tk = pairs ? a.mat[1].nrows / a.head_size * a.per_head : tiles(a.mat[1]);
+        a.ntiles = a.tq + a.tk + tiles(a.mat[2]);
+    } else a.ntiles = tiles(m0);
+    grid = a.ntiles < sms ? a.ntiles : sms;
+    a.per_block = (a.ntiles + grid - 1) / grid;
+    a.rem_blocks = a.ntiles % grid;
+    a.units = image_units(qt, m0.ncols);
+    a.nchunk = (a.units + TILE_UNITS - 1) / TILE_UNITS;
+    a.stage_bytes = a.octets * tile_bytes(qt);
+    const uint32_t need = a.per_block * a.nchunk;   // stages of the fullest block
+    a.part_offset = (uint32_t)((ximage_bytes(qt, m0.ncols) + 127) & ~(size_t)127);
+    auto stages_in = [&](size_t budget) -> uint32_t {
+        if (a.part_offset + 128 > budget) return 0;
+        const size_t n = (budget - a.part_offset - 128) / (a.stage_bytes + GEMV_PART_BYTES);
+        return (uint32_t)(n < GEMV_MAX_STAGES ? n : GEMV_MAX_STAGES);
     };
-
-    uint32_t best_rs = 0, best_rp = 0, best_ns = 0;
-    double best_cost = 1e300;
-    for (uint32_t rs = GEMV_MAX_RS; rs >= 1; rs--) {
-        if (pairs && (rs & 1)) continue;
-        const size_t stage = ((size_t)rs * row_bytes + 127) & ~(size_t)127;
-        if (image + 2 * stage > GEMV_SMEM_BUDGET && rs > (pairs ? 2u : 1u)) continue;
-        if (image + stage > GEMV_SMEM_BUDGET) continue;
-        if (a.epilogue == EPI_QKV_ROPE) {
-            bool ok = true;
-            for (int i = 0; i < 3; i++) ok = ok && a.mat[i].nrows % rs == 0;
-            if (a.rope_variant == WGB_ROPE_NEOX) ok = ok && (a.head_size / 2) % (rs / 2) == 0;
-            if (!ok) continue;
-        }
-        const uint32_t groups = groups_of(rs);
-        const uint32_t g = groups < sms ? groups : sms;
-        const uint32_t per = (groups + g - 1) / g;
-        uint32_t ns = (uint32_t)((GEMV_SMEM_BUDGET - image) / stage);
-        if (ns > GEMV_MAX_STAGES) ns = GEMV_MAX_STAGES;
-        if (ns > per) ns = per;
-        for (uint32_t rparts = 1; rparts <= 8; rparts *= 2) {
-            if (rs % rparts) continue;
-            const uint32_t rrows = rs / rparts;
-            if (rrows > (uint32_t)GEMV_TASK_ROWS || !ring_safe(per, ns, ncl, rparts)) continue;
-            const uint32_t in_work = (ncl + rparts - 1) / rparts + 1;   // stages the consumers hold at a time
-            double flight;
-            if (ns >= per) flight = 1.0;                                // the block's whole share fits in the ring
-            else {
-                const double bytes = ns > in_work ? (double)(ns - in_work) * stage : 0.25 * stage;
-                flight = bytes >= want_in_flight ? 1.0 : bytes / want_in_flight;
-            }
-            const uint32_t rounds = (per * rparts + ncl - 1) / ncl;
-            const double copy = (double)stage / ((double)stage + 512.0);
-            const double cost = (double)rounds * ((double)rrows + 0.5) / (flight * copy);
-            if (cost < best_cost - 1e-9) {
-                best_cost = cost;
-                best_rs = rs;
-                best_rp = rparts;
-                best_ns = ns;
-            }
-        }
-    }
-    if (!best_rs) return false;
-    a.rs = best_rs;
-    a.rparts = best_rp;
-    a.rparts_log2 = best_rp == 1 ? 0 : (best_rp == 2 ? 1 : (best_rp == 4 ? 2 : 3));
-    if (a.epilogue == EPI_QKV_ROPE) {
-        a.gq = a.mat[0].nrows / best_rs;
-        a.gk = a.mat[1].nrows / best_rs;
-    }
-    a.rrows = best_rs / best_rp;
-    a.kparts = kp;
-    a.ngroups = groups_of(best_rs);
-    a.stage_bytes = (uint32_t)(((size_t)best_rs * row_bytes + 127) & ~(size_t)127);
-    grid = a.ngroups < sms ? a.ngroups : sms;
-    a.nstage = best_ns < 1 ? 1 : best_ns;
-    a.ring_offset = (uint32_t)image;
-    a.row_bytes = row_bytes;
-    a.per_block = (a.ngroups + grid - 1) / grid;
-    a.rem_blocks = a.ngroups % grid;
-    const uint32_t cps = (uint32_t)m0.nplanes * (pairs ? 2u : 1u);
-    a.cps_log2 = cps == 1 ? 0 : (cps == 2 ? 1 : (cps == 4 ? 2 : 3));
-    // One producer pass takes about as long as 24 KB of streaming at full HBM rate: no more stages per
-    // pass than that needs, so that the ring stays as full as possible.
-    a.spb = (24576u + a.stage_bytes - 1) / a.stage_bytes;
-    if (a.spb > producer_batch(a.nstage, cps)) a.spb = producer_batch(a.nstage, cps);
-    const uint32_t lag = (ncl + best_rp - 1) / best_rp;   // stages between two tasks of a consumer warp, most
-    if (a.per_block > a.nstage && ncl > best_rp && (a.nstage * best_rp) % ncl != 0 && a.spb > a.nstage - lag) a.spb = a.nstage - lag;
-    smem_bytes = image + (size_t)a.nstage * a.stage_bytes;
+    const uint32_t ns = stages_in(GEMV_SMEM_BUDGET);
+    if (!ns) return false;
+    a.nstage = ns < need ? ns : need;
+    if (a.nstage < need && a.nstage > 1) a.nstage &= ~1u;   // a slot is always the same group's
+    a.nepi = 1;
+    while (a.nepi < (uint32_t)GEMV_NEPI && !a.peer_out.n && (a.nstage >= need || a.nstage >= (a.nepi + 1) * (a.nchunk > 1 ? a.nchunk : 2))) a.nepi++;
+    a.ring_offset = a.part_offset + a.nstage * GEMV_PART_BYTES;
+    smem_bytes = 128 + a.ring_offset + (size_t)a.nstage * a.stage_bytes;
     return true;
 }
 
-// The prologue / epilogue combinations the models use, each its own kernel.
-#define WGB_GEMV_VARIANTS(F)                                                                                   \
-    F(PRO_NONE, EPI_STORE) F(PRO_RMS, EPI_STORE) F(PRO_LN, EPI_STORE) F(PRO_NONE, EPI_RESIDUAL) F(PRO_RMS, EPI_SILU_PAIR) \
-    F(PRO_LN, EPI_GELU) F(PRO_RMS, EPI_QKV_ROPE) F(PRO_LN, EPI_QKV_SPLIT)
+// The prologue / epilogue combinations the models use, each its own kernel; the last column: with the exchange between ranks.
+#define WGB_GEMV_VARIANTS(F)                                                                                                        \
+    F(PRO_NONE, EPI_STORE, false) F(PRO_RMS, EPI_STORE, false) F(PRO_LN, EPI_STORE, false) F(PRO_NONE, EPI_RESIDUAL, false)         \
+    F(PRO_RMS, EPI_SILU_PAIR, false) F(PRO_LN, EPI_GELU, false) F(PRO_RMS, EPI_QKV_ROPE, false) F(PRO_LN, EPI_QKV_SPLIT, false)     \
+    F(PRO_NONE, EPI_STORE, true) F(PRO_NONE, EPI_RESIDUAL, true) F(PRO_RMS, EPI_STORE, true) F(PRO_RMS, EPI_SILU_PAIR, true)        \
+    F(PRO_RMS, EPI_QKV_ROPE, true)
 
 template <int QT>
 static int set_smem_attr()
 {
-#define WGB_ATTR(PRO, EPI) WGB_CUDA(cudaFuncSetAttribute(gemv_kernel<QT, PRO, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMV_SMEM_BUDGET));
+#define WGB_ATTR(PRO, EPI, PEERS)                                                                                                      \
+    WGB_CUDA(cudaFuncSetAttribute(gemv_kernel<QT, PRO, EPI, PEERS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMV_SMEM_BUDGET));
     WGB_GEMV_VARIANTS(WGB_ATTR)
 #undef WGB_ATTR
     return WGB_OK;
@@ -1004,7 +806,8 @@ template <int QT>
 static int launch_one(GemvArgs &a, cudaStream_t stream, bool pdl)
 {
     void (*kern)(const GemvArgs) = nullptr;
-#define WGB_PICK(PRO, EPI) if (a.prologue == PRO && a.epilogue == EPI) kern = gemv_kernel<QT, PRO, EPI>;
+const bool peers = a.peer_in.n || a.peer_out.n;
+#define WGB_PICK(PRO, EPI, PEERS) if (a.prologue == PRO && a.epilogue == EPI && peers == PEERS) kern = gemv_kernel<QT, PRO, EPI, PEERS>;
     WGB_GEMV_VARIANTS(WGB_PICK)
 #undef WGB_PICK
     if (!kern) return fail(WGB_ERR_UNSUPPORTED, "no fused kernel for prologue %d / epilogue %d", a.prologue, a.epilogue);
@@ -1013,6 +816,16 @@ static int launch_one(GemvArgs &a, cudaStream_t stream, bool pdl)
     if (!plan(a, smem, grid)) return fail(WGB_ERR_UNSUPPORTED, "matrix shape does not fit the fused kernel");
     int rc = gemv_global_init();
     if (rc) return rc;
+    for (int i = 0; i < a.nmat; i++) {
+        const QMat &m = a.mat[i];
+        TileMaps fresh;
+        const TileMaps *maps = m.maps;
+        if (!maps || maps->nrows != m.nrows || maps->p[0] != m.p[0]) {   // blocks in caller memory, a run of rows of a matrix
+            if ((rc = make_tile_maps(m, fresh))) return rc;
+            maps = &fresh;
+        }
+        for (int p = 0; p < m.nplanes; p++) a.map[i][p] = maps->map[p];
+    }
     a.err = gemv_status_word();
     const WaitLimits wl = wait_limits();
     a.wait_ns = wl.local_ns;
@@ -1030,8 +843,8 @@ static int launch_one(GemvArgs &a, cudaStream_t stream, bool pdl)
         cfg.numAttrs = 1;
     }
     if (g_trace_plan)
-        fprintf(stderr, "gemv plan: qt=%d rows=%u K=%u rs=%u rparts=%u kparts=%u ngroups=%u nstage=%u stage=%u grid=%u smem=%zu\n", QT,
-                a.mat[0].nrows, a.mat[0].ncols, a.rs, a.rparts, a.kparts, a.ngroups, a.nstage, a.stage_bytes, grid, smem);
+        fprintf(stderr, "gemv plan: qt=%d rows=%u K=%u tile rows=%u tiles=%u stages per tile=%u ring=%u x %u grid=%u smem=%zu\n", QT, a.mat[0].nrows,
+                a.mat[0].ncols, a.tile_rows, a.ntiles, a.nchunk, a.nstage, a.stage_bytes, grid, smem);
     WGB_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
     return WGB_OK;
 }

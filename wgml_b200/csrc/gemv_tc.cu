@@ -26,6 +26,10 @@
 
 namespace wgb {
 
+// Integer -> f32 without the conversion unit: adding the integer to the bit pattern of 1.5 * 2^23 yields the float exactly, one
+// FP32 subtraction removes the offset.  Valid for |v| < 2^22.
+__device__ __forceinline__ float i2f(int v) { return __uint_as_float((uint32_t)v + 0x4b400000u) - 12582912.0f; }
+
 constexpr uint32_t TC_MAX_K = 4096;
 constexpr uint32_t TC_RING = 6;
 constexpr uint32_t TC_WPQ = 4;                                // worker warps per quarter of the tile's rows

@@ -64,21 +64,20 @@ struct GemvArgs {
     int rope_variant;
     const float *rope_freq;     // head_size/2 inverse frequencies base^(-2j/head_size)
     // launch plan, filled by launch_gemv
-    uint32_t rs;            // rows per shared-memory stage
-    uint32_t ngroups;       // stages' worth of rows in the launch
-    uint32_t nstage;        // ring depth
-    uint32_t stage_bytes;
-    uint32_t ring_offset;   // of the ring inside dynamic shared memory (after the input image)
-    uint32_t kparts;        // column parts = consumer warps that share one row
-    uint32_t rparts;        // row parts per stage (a power of two)
-    uint32_t rparts_log2;
-    uint32_t gq, gk;        // EPI_QKV_ROPE: groups of the q and of the k matrix
-    uint32_t rrows;         // rows per consumer task = rs / rparts
-    uint32_t row_bytes;     // bytes of one row over all planes
-    uint32_t per_block;     // groups of blocks 0 .. rem_blocks-1; the other blocks have one fewer
+    uint32_t octets;        // eight-row parts of a row tile: 1 or 2
+    uint32_t tile_rows;     // 8 * octets
+    uint32_t ntiles;        // row tiles of the launch
+    uint32_t per_block;     // tiles of blocks 0 .. rem_blocks-1; the other blocks have one fewer
     uint32_t rem_blocks;    //   (0: every block has per_block)
-    uint32_t cps_log2;      // log2 of the copies per stage (planes x parts)
-    uint32_t spb;           // stages per producer pass
+    uint32_t tq, tk;        // EPI_QKV_ROPE: those of q and of k
+    uint32_t per_head, per_head_magic, head_magic;   //   Neox: pairs of tiles per head; for divisions by it and by head_size
+    uint32_t units;         // units of columns
+    uint32_t nchunk;        // stages per tile
+    uint32_t nstage;        // ring depth
+    uint32_t nepi;          // epilogue warps at work
+    uint32_t stage_bytes;
+    uint32_t part_offset, ring_offset;   // of the partial sums and the ring in dynamic shared memory (after the input image)
+    CUtensorMap map[3][4];  // of the planes of mat[i]
     uint32_t *err;          // device status word for expired waits
     unsigned long long wait_ns, peer_wait_ns;   // limits of the waits inside the block / for the peers' flags
     unsigned long long *stamp;   // optional: receives the launch's end time (stamp_end)

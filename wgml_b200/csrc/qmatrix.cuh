@@ -15,7 +15,11 @@
 
 #include "common.cuh"
 
+#include <cuda.h>
+
 namespace wgb {
+
+struct TileMaps;
 
 struct QMat {
     int qtype;
@@ -24,7 +28,32 @@ struct QMat {
     int nplanes;
     uint32_t pitch[4];           // bytes per row of each plane
     const uint8_t *p[4];
+    const TileMaps *maps;        // host only, optional: tensor maps of the planes, made at upload
 };
+
+// Tiles in which the matrix-vector kernel (gemv.cu) copies a matrix: TILE_ROWS rows times TILE_UNITS units of unit_cols()
+// columns.  Per plane, `tile_step` bytes of a row belong to the tile; `tile_box` of them are copied, a few more where that makes
+// neighbouring rows start in different shared-memory banks (they are never used).  All are multiples of 16 bytes, and eight boxes
+// of 128.
+constexpr uint32_t TILE_ROWS = 8, TILE_UNITS = 8;
+__host__ __device__ constexpr uint32_t unit_cols(int qt) { return qt == WGB_Q8_0 ? 128u : qt == WGB_F32 ? 64u : 256u; }
+__host__ __device__ constexpr int tile_planes(int qt) { return qt == WGB_Q6_K ? 4 : qt == WGB_Q8_0 ? 2 : 1; }
+__host__ __device__ constexpr uint32_t tile_step(int qt, int plane)
+{
+    return qt == WGB_Q4_K ? 1152u : qt == WGB_Q6_K ? (plane == 0 ? 1024u : plane == 1 ? 512u : plane == 2 ? 128u : 16u)
+         : qt == WGB_Q8_0 ? (plane == 0 ? 1024u : 64u) : 2048u;
+}
+__host__ __device__ constexpr uint32_t tile_box(int qt, int plane)
+{
+    return tile_step(qt, plane) + (qt == WGB_Q4_K || qt == WGB_Q8_0 ? 16u : qt == WGB_Q6_K ? (plane == 0 ? 32u : plane == 1 ? 64u : plane == 2 ? 16u : 0u) : 0u);
+}
+struct TileMaps {
+    CUtensorMap map[4];
+    const uint8_t *p[4];   // of the planes the maps were made for
+    uint32_t nrows;
+};
+// Tensor maps of the planes of a matrix in a layout of the fused kernels (gemv_fast_supported).
+int make_tile_maps(const QMat &m, TileMaps &out);
 
 // Fills nplanes / pitch for a matrix of `bpr` blocks per row.
 __host__ __device__ inline void qmat_set_pitches(QMat &m)
@@ -53,6 +82,7 @@ struct wgb_quant_matrix {
     wgb::QMat view;
     void *storage;   // one cudaMalloc holding every plane (NULL when the matrix wraps caller memory)
     size_t bytes;
+    wgb::TileMaps maps;   // what view.maps points at once they are made
 };
 
 namespace wgb {

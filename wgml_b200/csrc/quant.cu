@@ -1,4 +1,5 @@
 // Dequantisation kernels and the quantised-matrix object (upload, planar repack, row dequant).
+#include "kernels.h"
 #include "qaccess.cuh"
 
 #include <algorithm>
@@ -128,6 +129,15 @@ static int repack_from_device_raw(int qtype, const uint8_t *d_raw, size_t nb, co
     return WGB_OK;
 }
 
+// The tensor maps of a finished matrix: made here once, not by every product.
+static int attach_maps(wgb_quant_matrix *m)
+{
+    if (!gemv_fast_supported(m->view)) return WGB_OK;
+    const int rc = make_tile_maps(m->view, m->maps);
+    if (rc == WGB_OK) m->view.maps = &m->maps;
+    return rc;
+}
+
 int qmat_create_slice(int qtype, const void *h_blocks, size_t nrows, size_t ncols, size_t row0,
                       size_t nrows_keep, size_t kb0, size_t bpr_keep, cudaStream_t stream,
                       wgb_quant_matrix **out)
@@ -173,6 +183,7 @@ int qmat_create_slice(int qtype, const void *h_blocks, size_t nrows, size_t ncol
         if (rc == WGB_OK && e2 != cudaSuccess) rc = cuda_fail(e2, "repack");
         cudaFree(d_raw);
     }
+    if (rc == WGB_OK) rc = attach_maps(m);
     if (rc != WGB_OK) { cudaFree(m->storage); delete m; return rc; }
     *out = m;
     return WGB_OK;
@@ -311,6 +322,7 @@ int qmat_create_slice_async(Uploader &up, int qtype, const void *h_blocks, size_
     const uint8_t *src = (const uint8_t *)h_blocks + (row0 * bpr + kb0) * bb;
     if (rc == WGB_OK) rc = up.copy_rows(d_raw, src, bpr_keep * bb, bpr * bb, nrows_keep);
     if (rc == WGB_OK && planar) rc = repack_from_device_raw(qtype, d_raw, nrows_keep * bpr_keep, m->view, up.stream);
+    if (rc == WGB_OK) rc = attach_maps(m);
     if (rc != WGB_OK) {
         cudaStreamSynchronize(up.stream);
         cudaFree(m->storage);
@@ -352,6 +364,7 @@ int qmat_create(int qtype, const void *blocks, bool src_on_device, size_t nrows,
         e = cudaMemcpyAsync(m->storage, blocks, nrows * bpr * bb, cudaMemcpyDeviceToDevice, stream);
         if (e != cudaSuccess) rc = cuda_fail(e, "cudaMemcpy(quant matrix)");
     }
+    if (rc == WGB_OK) rc = attach_maps(m);
     if (rc != WGB_OK) { cudaFree(m->storage); delete m; return rc; }
     *out = m;
     return WGB_OK;
