@@ -127,3 +127,20 @@ def test_parameter_checks():
         a.dispatch(ops.BatchedMultiqueryAttentionParams(64, 128, 1, 2, 64, 64), z[:128], z, z, None, z[:128])  # pos == seq_len
     with pytest.raises(ops.WgbError):
         a.dispatch(ops.BatchedMultiqueryAttentionParams(64, 128, 3, 2, 64, 1), z[:128], z, z, None, z[:128])
+
+
+@pytest.mark.parametrize("hs", [4, 20, 32, 36, 64, 80, 96, 100, 128])
+@pytest.mark.parametrize("heads,kv_mul", [(1, 1), (6, 3), (16, 4), (24, 1), (40, 5), (72, 8), (130, 1)])
+def test_cluster_kernel_edges(hs, heads, kv_mul):
+    """Blocks per head 8, 4, 2 and 1 (and none resident: heads of more than 64 elements, 130 of them), head sizes around a lane's
+    four float4, contexts around a group of eight rows, the warps of one block and of eight, what a warp requests ahead, and the
+    lines of the dispatch rule."""
+    for pos in (0, 6, 7, 8, 63, 64, 127, 128, 191, 192, 193, 511, 767, 768, 1023, 1024, 1535, 1536):
+        run(1600, heads, hs, kv_mul, pos, want_attn=False, seed=pos)
+
+
+@pytest.mark.parametrize("case", [(512, 132, 128, 1, 300), (512, 132, 96, 2, 300), (512, 132, 128, 3, 200), (512, 264, 64, 4, 130), (512, 260, 32, 1, 200),
+                                  (512, 132, 80, 12, 77), (2048, 264, 64, 8, 1700)])
+def test_more_heads_than_resident_blocks(case):
+    """One, two, three, four, eight and twelve query heads per KV head where the cluster kernel leaves more than a chunk to the others."""
+    run(*case, want_attn=False, seed=2)

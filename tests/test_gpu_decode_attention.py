@@ -1,5 +1,5 @@
 """Attention of the decode step (position on the device, head-major caches, programmatic launches) at contexts and groupings
-that the model tests do not reach: the streaming kernel (one or two query heads per KV head, more chunks of 64 rows than
+that the model tests do not reach: the cluster kernel (short contexts), the streaming kernel (one or two query heads per KV head, more chunks of 64 rows than
 the split kernel's blocks fit in one wave) and the row-streaming kernel (four or eight) with and without its requests
 ahead of the wait for the launch before.  The caches are filled on both sides with the same rows, then a few greedy
 steps run against the oracle."""
@@ -52,6 +52,14 @@ def test_streaming_kernel_with_several_chunks_per_block():
 @pytest.mark.parametrize("start", [0, 126, 200, 1001, 3003])
 def test_row_streaming_kernel_in_decode_steps(shape, start):
     """Ten steps leave every number of rows in the last group of eight.  Up to about 140 positions there are fewer groups
-    than blocks, and no warp requests anything ahead of the wait; from 1001 on most do.  (Eight query heads per KV head: the
-    split kernel as long as the context is one wave.)"""
+    than blocks, and no warp requests anything ahead of the wait; from 1001 on most do.  (Where all blocks of the cluster kernel are
+    resident, contexts up to 1536 positions are its.)"""
     steps(*shape, start, 10, 3072)
+
+
+@pytest.mark.parametrize("shape", [(12, 12, 64), (16, 4, 128), (40, 40, 64), (36, 12, 128), (66, 33, 128)])
+@pytest.mark.parametrize("start", [0, 60, 186, 250, 1018, 1530])
+def test_cluster_kernel_in_decode_steps(shape, start):
+    """Eight, four and two blocks per head and one; ten steps that leave every number of rows in the last group of eight and cross the
+    lines of the dispatch rule (192, 1024 and 1536 positions; a call's launches are those of its last position)."""
+    steps(*shape, start, 10, 1600)

@@ -4,14 +4,14 @@
 // batched_multiquery_attention.wgsl:38-99): score_t = (q_h . k_t) / sqrt(head_size), softmax with
 // the maximum subtracted, xb_h = sum_t p_t v_t; query head h reads KV head h / kv_mul.
 //
-// Split kernel (the hot path): grid (time chunks of 64, KV heads).  A block computes, for every
+// Split kernel: grid (time chunks of 64, KV heads).  A block computes, for every
 // query head of its KV head, the scores of its chunk, the chunk maximum, the exponentials and the
 // weighted sum of its 64 value rows; (max, sum, vector) go to a scratch buffer.  The block that
 // finishes last for a KV head (an atomic ticket, nobody waits) merges the chunks.  K and V rows
 // are read once for all kv_mul query heads.
 //
 // Streaming kernel and row-streaming kernel, further down: one block per SM walks a run of the cache rows and keeps the
-// running softmax per warp; launch_split says which launch takes which.
+// running softmax per warp; launch_split says which launch takes which.  Cluster kernel: short contexts (cluster_blocks).
 //
 // Full kernel (API path that returns the attention weights): one block per query head, the
 // probabilities are materialised in the caller's [n_heads][seq_len] buffer.
@@ -1062,6 +1062,255 @@ static int launch_rows(const AttnArgs &a, uint32_t nchunks, cudaStream_t stream,
     return WGB_OK;
 }
 
+// Cluster kernel (head sizes up to 128, short contexts).  A cluster of 1, 2, 4 or 8 blocks per query head, eight warps each.  A row
+// of the cache belongs to a quarter of a warp: eight lanes, NC float4 each, which keep a running softmax and value sum of
+// their rows to themselves, so a row costs three shuffles and no barrier; a quarter takes ATC_ROWS rows at a time.  A warp
+// requests ATC_STAGES groups of rows ahead (asynchronous copies), in most cases all that it will read, before it waits for the
+// launch before.  Quarters meet through shuffles, warps through shared memory, blocks through the leader's shared memory.
+// Bound by latency: in decode steps at up to some hundred positions the split and the row-streaming kernel spend most of their
+// time between a block's partial result and the end of the launch (scratch in global memory, fence, ticket, second read) and, with 22
+// to 57 KB of code that a step runs through once per layer, on instruction fetches.  Query heads that share a KV head read its
+// rows from L2 again.  (From the end of the q/k/v launch to that of the wait of the output projection, us: 16 heads on 4 of size 128,
+// 60 positions 8.5 and 2.9; 6 heads of size 48 4.9 and 3.3; 32 heads of size 128, 540 positions, 6.5 and 5.3, where 20 MB of cache take
+// 3.1.  Sixteen warps per block, one or three rows per quarter at a time: no faster.)
+constexpr int ATC_ROWS = 2;                                              // rows per quarter and group
+constexpr int ATC_GROUP = 4 * ATC_ROWS, ATC_STAGES = 24 / ATC_GROUP;
+
+__device__ __forceinline__ void atc_copy16(uint32_t dst, const void *src, uint32_t bytes)   // bytes: 16, or 0 for zeros
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// Eight partial softmaxes, lane l of a warp looks after partial l % 8: (maximum, sum) in, factor out; returns the sum of them all
+// against the common maximum `m`.
+__device__ __forceinline__ float atc_weights(float &m, float l, float &factor)
+{
+    float top = m;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    factor = expf(m - top);
+    m = top;
+    l *= factor;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    return l;
+}
+
+template <int NC>
+__global__ void __launch_bounds__(ATT_NT, 1) attn_cluster_kernel(const __grid_constant__ AttnArgs a)
+{
+    constexpr uint32_t ROW = NC * 128, GROUP = ATC_GROUP * ROW;   // bytes of a row (padded to whole eighths) and of a group's K or V
+    extern __shared__ uint4 ring4[];                      // [warp][stage][K | V][rows of the group]
+    __shared__ __align__(16) float s_acc[ATT_WARPS][NC * 32];
+    __shared__ float s_m[ATT_WARPS], s_l[ATT_WARPS];
+    __shared__ float s_all[8][NC * 32], s_allm[8], s_alll[8];   // leader: the blocks' partial results
+
+    const uint32_t pos = a.pos ? *a.pos : a.p.pos;   // written by an earlier step: readable before the wait
+    const uint32_t hs = a.p.head_size, h = blockIdx.y, kvh = h / a.p.kv_mul;
+    const uint32_t rstr = a.row_stride ? a.row_stride : a.p.kv_dim, hstr = a.row_stride ? a.head_stride : hs;
+    const uint32_t rank = blockIdx.x, nblocks = gridDim.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t slot = (uint32_t)lane >> 3, p = (uint32_t)lane & 7;
+    pdl_launch_dependents();
+    if (nblocks > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // every block of the cluster has started
+
+    const uint32_t ngroups = pos / ATC_GROUP + 1, nwarps = nblocks * ATT_WARPS, g0 = rank * ATT_WARPS + warp;
+    const uint32_t ring = smem_addr(ring4) + warp * (ATC_STAGES * 2 * GROUP) + slot * ROW + p * 16;
+    const float *kh = a.k_cache + (size_t)kvh * hstr + 4 * p, *vh = a.v_cache + (size_t)kvh * hstr + 4 * p;
+    auto request = [&](uint32_t g, uint32_t st) {
+        if (g < ngroups) {
+#pragma unroll 1
+            for (uint32_t r = 0; r < ATC_ROWS; r++) {
+                const uint32_t row = ATC_GROUP * g + 4 * r + slot, dst = ring + st * (2 * GROUP) + r * 4 * ROW;
+                const bool in = row <= pos;
+                const size_t at = (size_t)(in ? row : pos) * rstr;
+#pragma unroll
+                for (int i = 0; i < NC; i++) {
+                    if (4 * (p + 8 * i) < hs) {
+                        atc_copy16(dst + i * 128, kh + at + 32 * i, in ? 16 : 0);
+                        atc_copy16(dst + GROUP + i * 128, vh + at + 32 * i, in ? 16 : 0);
+                    }
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");   // one group per stage and lane, empty or not
+    };
+    // Every row before `pos` was written by an earlier step and is requested before the wait for the preceding launch,
+    // which writes the row of `pos` (in the last group, the last of its warp).
+    bool waited = false;
+#pragma unroll 1
+    for (uint32_t st = 0, g = g0; st < ATC_STAGES; st++, g += nwarps) {
+        if (g == ngroups - 1) {
+            pdl_wait();
+            waited = true;
+        }
+        request(g, st);
+    }
+    if (!waited) pdl_wait();
+
+    const float root = sqrtf((float)hs);
+    float4 q[NC], acc[NC];
+#pragma unroll
+    for (int i = 0; i < NC; i++) {
+        q[i] = 4 * (p + 8 * i) < hs ? __ldcg(reinterpret_cast<const float4 *>(a.q + (size_t)h * hs) + p + 8 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float m = ATT_LOWEST, l = 0.0f;
+    uint32_t st = 0;
+#pragma unroll 1
+    for (uint32_t g = g0; g < ngroups; g += nwarps) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ATC_STAGES - 1) : "memory");   // a lane reads back only what it copied
+        const uint32_t src = ring + st * (2 * GROUP);
+        auto fetch = [&](uint32_t at, int i) {   // (columns past the head are not copied: whatever is there)
+            float4 v;
+            asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at + i * 128) : "memory");
+            return 4 * (p + 8 * i) < hs ? v : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        float s[ATC_ROWS], mn = m;
+#pragma unroll
+        for (int r = 0; r < ATC_ROWS; r++) {
+            s[r] = 0.0f;
+#pragma unroll
+            for (int i = 0; i < NC; i++) {
+                const float4 k = fetch(src + r * 4 * ROW, i);
+                s[r] += (q[i].x * k.x + q[i].y * k.y) + (q[i].z * k.z + q[i].w * k.w);
+            }
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+            for (int r = 0; r < ATC_ROWS; r++) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
+#pragma unroll
+        for (int r = 0; r < ATC_ROWS; r++) {
+            s[r] = ATC_GROUP * g + 4 * r + slot <= pos ? s[r] / root : -INFINITY;   // rows past the end: zeros that weigh 0
+            mn = fmaxf(mn, s[r]);
+        }
+        const float rescale = expf(m - mn);
+        m = mn;
+        l *= rescale;
+#pragma unroll
+        for (int i = 0; i < NC; i++) { acc[i].x *= rescale; acc[i].y *= rescale; acc[i].z *= rescale; acc[i].w *= rescale; }
+#pragma unroll
+        for (int r = 0; r < ATC_ROWS; r++) {
+            const float w = expf(s[r] - mn);
+            l += w;
+#pragma unroll
+            for (int i = 0; i < NC; i++) {
+                const float4 v = fetch(src + GROUP + r * 4 * ROW, i);
+                acc[i].x = fmaf(w, v.x, acc[i].x);
+                acc[i].y = fmaf(w, v.y, acc[i].y);
+                acc[i].z = fmaf(w, v.z, acc[i].z);
+                acc[i].w = fmaf(w, v.w, acc[i].w);
+            }
+        }
+        request(g + ATC_STAGES * nwarps, st);
+        st = st + 1 == ATC_STAGES ? 0 : st + 1;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+
+    // The quarters of the warp.
+    float top = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+    const float f = expf(m - top);
+    auto over_quarters = [&](float v) {
+        v *= f;
+        v += __shfl_xor_sync(0xffffffffu, v, 8);
+        return v + __shfl_xor_sync(0xffffffffu, v, 16);
+    };
+    l = over_quarters(l);
+#pragma unroll
+    for (int i = 0; i < NC; i++) {
+        acc[i].x = over_quarters(acc[i].x);
+        acc[i].y = over_quarters(acc[i].y);
+        acc[i].z = over_quarters(acc[i].z);
+        acc[i].w = over_quarters(acc[i].w);
+        if (slot == 0) reinterpret_cast<float4 *>(s_acc[warp])[p + 8 * i] = acc[i];
+    }
+    if (lane == 0) {
+        s_m[warp] = top;
+        s_l[warp] = l;
+    }
+    __syncthreads();
+    // The warps of the block: a thread per element, all warps work out the eight factors.
+    static_assert(ATT_WARPS == 8, "atc_weights");
+    const uint32_t e = threadIdx.x;
+    float bm = s_m[lane & 7], factor;
+    const float bl = atc_weights(bm, s_l[lane & 7], factor);
+    float o = 0.0f;
+#pragma unroll
+    for (int i = 0; i < ATT_WARPS; i++) {
+        const float fi = __shfl_sync(0xffffffffu, factor, i);
+        if (e < NC * 32) o = fmaf(s_acc[i][e], fi, o);
+    }
+    if (nblocks == 1) {
+        if (e < hs) a.xb[(size_t)h * hs + e] = o / bl;
+    } else {
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        auto to_leader = [&](float *mine, float v) {
+            uint32_t dst;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(dst) : "r"(smem_addr(mine)));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(v) : "memory");
+        };
+        if (e < hs) to_leader(&s_all[rank][e], o);
+        if (e == 0) {
+            to_leader(&s_allm[rank], bm);
+            to_leader(&s_alll[rank], bl);
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (rank == 0) {
+            const uint32_t b = (uint32_t)lane & 7;
+            float tm = b < nblocks ? s_allm[b] : ATT_LOWEST, tf;
+            const float tl = atc_weights(tm, b < nblocks ? s_alll[b] : 0.0f, tf);
+            float t = 0.0f;
+#pragma unroll 1
+            for (uint32_t i = 0; i < nblocks; i++) {
+                const float fi = __shfl_sync(0xffffffffu, tf, i);
+                if (e < hs) t = fmaf(s_all[i][e], fi, t);
+            }
+            if (e < hs) a.xb[(size_t)h * hs + e] = t / tl;
+        }
+    }
+    if (threadIdx.x == 0) stamp_end(a.stamp);
+}
+
+template <int NC>
+static int launch_cluster(const AttnArgs &a, uint32_t nblocks, cudaStream_t stream, bool pdl)
+{
+    const size_t smem = (size_t)ATT_WARPS * ATC_STAGES * 2 * ATC_GROUP * NC * 128;
+    static bool ready[MAX_DEVICES] = {};   // per instantiation and device
+    const int dev = current_device();
+    if (dev < 0) return WGB_ERR_CUDA;
+    if (!ready[dev]) {
+        WGB_CUDA(cudaFuncSetAttribute(attn_cluster_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ready[dev] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nblocks, a.p.n_heads);
+    cfg.blockDim = dim3(ATT_NT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = nblocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 2 : 1;
+    WGB_CUDA(cudaLaunchKernelEx(&cfg, attn_cluster_kernel<NC>, a));
+    return WGB_OK;
+}
+
+static int launch_cluster_any(const AttnArgs &a, uint32_t nblocks, cudaStream_t stream, bool pdl)
+{
+    const uint32_t nc = (a.p.head_size + 31) / 32;
+    if (nc == 1) return launch_cluster<1>(a, nblocks, stream, pdl);
+    if (nc == 2) return launch_cluster<2>(a, nblocks, stream, pdl);
+    if (nc == 3) return launch_cluster<3>(a, nblocks, stream, pdl);
+    return launch_cluster<4>(a, nblocks, stream, pdl);
+}
+
 template <int QH>
 static int launch_stream(const AttnArgs &a, uint32_t nchunks, uint32_t n_kv, uint32_t zgroups, cudaStream_t stream, bool pdl)
 {
@@ -1176,6 +1425,29 @@ static int launch_split(const AttnArgs &a, uint32_t nchunks, uint32_t nchunks_hi
     return WGB_OK;
 }
 
+// Blocks per query head of the cluster kernel for contexts of up to `chunks` times 64 positions; 0: another kernel's.  As many as are
+// resident at once, as clusters of eight only where there is room to spare (fewer than nine in ten SMs can be dealt to those).
+// One is best for little to read: up to two chunks, three where a decode call works up to them.  (Microseconds, the kernel of
+// launch_split and 1 / 2 / 4 / 8 blocks.  Stand-alone calls, 32 heads on 32 of size 128: 63 positions 5.4 and 3.5 / 4.3 / 4.4 / 9.9,
+// 611 positions 8.5 and 10.2 / 8.1 / 7.9 / 14.0; 16 heads on 4: 10.4 and 2.9 / 3.7 / 3.8 / 6.3, 12.4 and 9.8 / 7.2 / 5.9 / 8.6.  A decode
+// step of two layers, 32 heads on 32: 60 positions 68.1 and 64.4 / 65.8 / 66.5 / 76.7, 600 positions 72.0 and 76.8 / 72.5 /
+// 69.5 / 81.1.)
+// Where not even one block per head is resident it pays for one chunk (256 heads on 64 of size 128: 8.0 and 6.2; 200 positions 11.2
+// and 11.3), otherwise up to sixteen chunks, and as far as measured, 1500 positions, with two blocks or more (32 heads
+// on 32: 15.2 and 11.6; 96 on 24, one block: 17.7 and 19.6).  Of 1174 shapes measured one is slower by more than 2 %: 40
+// heads on 40, 400 positions, 7.5 and 7.7.
+static uint32_t cluster_blocks(const wgb_attn_params &p, uint32_t chunks, bool decode)
+{
+    if (p.head_size > 128) return 0;
+    const uint32_t resident = p.head_size <= 64 ? 256 : 128;   // two blocks per SM, or one
+    if (p.n_heads > resident) return chunks == 1 ? 1 : 0;
+    if (chunks <= (decode ? 3u : 2u)) return 1;
+    uint32_t n = 1;
+    while (n < 4 && 2 * n * p.n_heads <= resident) n *= 2;
+    if (n == 4 && 8 * p.n_heads <= (p.head_size <= 64 ? 128u : 96u)) n = 8;
+    return chunks <= (n == 1 ? 16u : 24u) ? n : 0;
+}
+
 // `a.counters` must hold n_kv_heads * ceil(kv_mul / QH) zeroed words (QH as chosen below) and `a.scratch`
 // attn_scratch_floats() floats.
 int launch_attention(const AttnArgs &a, cudaStream_t stream, bool pdl)
@@ -1187,6 +1459,8 @@ int launch_attention(const AttnArgs &a, cudaStream_t stream, bool pdl)
     const uint32_t nchunks = attn_num_splits(p.seq_len);
     // With the position on the device, p.pos is the caller's bound on it (0: unknown, assume a short context).
     const uint32_t nh = std::min(nchunks, p.pos / ATT_CHUNK + 1);
+    const uint32_t nblocks = cluster_blocks(p, nh, a.pos != nullptr);
+    if (nblocks) return a.q ? launch_cluster_any(a, nblocks, stream, pdl) : ATT_CLASS + 8 + (int)nblocks;
     const bool big = p.head_size > 128;
     // query heads per block: the largest of 4 / 2 / 1 that divides nothing away (tail heads masked)
     const uint32_t qh = p.kv_mul >= 4 ? 4 : (p.kv_mul >= 2 ? 2 : 1);

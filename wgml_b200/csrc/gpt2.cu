@@ -43,6 +43,8 @@ struct wgb_gpt2 {
     bool fused = true, use_pdl = true;
     cudaGraphExec_t graph = nullptr;
     uint32_t graph_n_prompt = 0;
+    uint32_t pos_bound = 0;                  // furthest position the launches being recorded will serve
+    int graph_attn_class = 0;                // attention launch shape (attn_sizing_class) the captured graph was built for
     int kernels_per_token = 0;
     // batched prompt prefill (wgb_gpt2_set_prefill): tile-major copies of the layer matrices for the tensor-core
     // products, activation images and the buffers of a pass of PF_TOK positions
@@ -148,6 +150,7 @@ int enqueue_forward(wgb_gpt2 *m, cudaStream_t s, int *nkernels)
     at.p.kv_mul = 1;
     at.p.n_heads = p.n_head;
     at.p.head_size = n / p.n_head;
+    at.p.pos = m->pos_bound;
     at.pos = d_pos;
     at.q = m->memory_q;
     at.xb = m->curr_768;
@@ -625,6 +628,7 @@ WGB_EXPORT int wgb_gpt2_forward(wgb_gpt2 *m, uint32_t token, uint32_t pos, void 
     cudaStream_t s = as_stream(stream);
     set_scalars_kernel<<<1, 1, 0, s>>>(m->scalars, token, pos, 0);
     WGB_LAUNCH_CHECK("set_scalars_kernel");
+    m->pos_bound = pos;
     return enqueue_forward(m, s, &m->kernels_per_token);
 }
 
@@ -699,7 +703,19 @@ WGB_EXPORT int wgb_gpt2_decode(wgb_gpt2 *m, const uint32_t *h_prompt, size_t n_p
     ls.prompt = m->d_prompt;
     ls.n_prompt = (uint32_t)n_prompt;
     ls.out_tokens = m->d_out;
-    if (m->graph && m->graph_n_prompt != (uint32_t)n_prompt) drop_graph(m);
+    // The attention launch is sized for the furthest position of this call; the captured step is kept until
+    // that changes the shape of the launch.
+    m->pos_bound = (uint32_t)((size_t)start_pos + total - 1);
+    wgb_attn_params ap = {};
+    ap.seq_len = m->p.n_seq;
+    ap.kv_dim = m->p.n_embd;
+    ap.kv_mul = 1;
+    ap.n_heads = m->p.n_head;
+    ap.head_size = m->p.n_embd / m->p.n_head;
+    ap.pos = m->pos_bound;
+    const int attn_class = attn_sizing_class(ap);
+    WGB_REQUIRE(attn_class >= 0, "attention sizing failed");
+    if (m->graph && (m->graph_n_prompt != (uint32_t)n_prompt || m->graph_attn_class != attn_class)) drop_graph(m);
     if (!m->graph) {
         cudaStream_t cs;
         WGB_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
@@ -724,6 +740,7 @@ WGB_EXPORT int wgb_gpt2_decode(wgb_gpt2 *m, const uint32_t *h_prompt, size_t n_p
         cudaStreamDestroy(cs);
         if (e != cudaSuccess) { m->graph = nullptr; return cuda_fail(e, "CUDA graph capture of a decode step"); }
         m->graph_n_prompt = (uint32_t)n_prompt;
+        m->graph_attn_class = attn_class;
     }
     if ((rc = replay_with_status(m->graph, total - done, s, m->h_pinned + 1, m->poll))) return rc;
     // One wait for the ids and the kernels' status word, both through pinned memory.
