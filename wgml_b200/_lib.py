@@ -187,7 +187,29 @@ SIGNATURES = {
     "wgb_gpt2_kernels_per_token": (_i, [_vp]),
 }
 
+# Entry points that dispatch.c calls, in its order.
+_DISPATCHED = ("wgb_gemv_quant", "wgb_gemm_q4k_tiles", "wgb_gemm_q6k_tiles", "wgb_gemm_q80_tiles", "wgb_rms_norm", "wgb_rope", "wgb_attention",
+               "wgb_silu", "wgb_op_assign")
+
 _lib = None
+_fast = None
+
+
+def dispatch():
+    """The module with the host path of the per-op calls, its library addresses and classes set."""
+    global _fast
+    if _fast is not None:
+        return _fast
+    lib = load()
+    if not os.path.exists(os.path.join(_HERE, "_dispatch.so")):
+        from . import build as _build
+        _build.build()
+    import torch
+    from . import _dispatch
+    _dispatch.setup(torch.Tensor, torch.float32, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream, WgbError, check,
+                    tuple(C.cast(getattr(lib, name), C.c_void_p).value for name in _DISPATCHED))
+    _fast = _dispatch
+    return _fast
 
 
 def load() -> C.CDLL:

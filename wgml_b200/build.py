@@ -6,11 +6,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "csrc", "build")
 LIB = os.path.join(HERE, "libwgml_b200.so")
+EXT = os.path.join(HERE, "_dispatch.so")   # CPython module: host path of the per-op calls (dispatch.c)
 
 SOURCES = ["api.cpp", "gguf.cpp", "tokenizer.cpp", "quant.cu", "gemv.cu", "gemv_tc.cu", "attention.cu", "ops.cu", "sampler.cu", "prefill.cu", "prefill_q6k.cu", "prefill_q80.cu", "prefill_wide.cu", "llama2.cu", "gpt2.cu", "comm.cpp"]
 
@@ -66,6 +68,14 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
         if r.returncode != 0:
             raise RuntimeError("link failed")
+    src = os.path.join(CSRC, "dispatch.c")
+    if force or _stale(EXT, [src, os.path.abspath(__file__)]):
+        cmd = ["gcc", "-O2", "-Wall", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], src, "-o", EXT]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if verbose or r.returncode != 0:
+            sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+        if r.returncode != 0:
+            raise RuntimeError("gcc failed for dispatch.c")
     return LIB
 
 

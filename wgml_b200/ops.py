@@ -105,9 +105,7 @@ class GemvQuant:
         return cls()
 
     def dispatch(self, out: torch.Tensor, m: GpuQuantMatrix, v: torch.Tensor) -> None:
-        if v.numel() != m.ncols or out.numel() != m.nrows:
-            raise WgbError(_lib.ERR_INVALID, "Gemv: dimension mismatch.")
-        check(_lib.load().wgb_gemv_quant(m._h, _f32(v, "v"), _f32(out, "out"), _stream()))
+        _lib.dispatch().gemv(out, m, v)
 
     def dispatch_raw(self, out: torch.Tensor, qtype: int, blocks: torch.Tensor, nrows: int, ncols: int, v: torch.Tensor) -> None:
         """The same product over raw GGUF blocks resident on the device."""
@@ -135,9 +133,7 @@ class Q4KTiles:
 
     def gemm(self, out: torch.Tensor, v: torch.Tensor) -> None:
         """The product for 1..8 input vectors at once: v [n][ncols] -> out [n][nrows] (the batched prefill's kernel)."""
-        if v.dim() != 2 or out.dim() != 2 or v.shape[1] != self.ncols or out.shape[1] != self.nrows or v.shape[0] != out.shape[0]:
-            raise WgbError(_lib.ERR_INVALID, "Gemm: dimension mismatch.")
-        check(_lib.load().wgb_gemm_q4k_tiles(self._h, _f32(v, "v"), v.shape[0], _f32(out, "out"), _stream()))
+        _lib.dispatch().gemm_q4k(out, self, v)
 
     def __del__(self):
         h, self._h = getattr(self, "_h", None), None
@@ -162,9 +158,7 @@ class Q6KTiles:
 
     def gemm(self, out: torch.Tensor, v: torch.Tensor) -> None:
         """The product for 1..8 input vectors at once: v [n][ncols] -> out [n][nrows]."""
-        if v.dim() != 2 or out.dim() != 2 or v.shape[1] != self.ncols or out.shape[1] != self.nrows or v.shape[0] != out.shape[0]:
-            raise WgbError(_lib.ERR_INVALID, "Gemm: dimension mismatch.")
-        check(_lib.load().wgb_gemm_q6k_tiles(self._h, _f32(v, "v"), v.shape[0], _f32(out, "out"), _stream()))
+        _lib.dispatch().gemm_q6k(out, self, v)
 
     def __del__(self):
         h, self._h = getattr(self, "_h", None), None
@@ -189,9 +183,7 @@ class Q80Tiles:
 
     def gemm(self, out: torch.Tensor, v: torch.Tensor) -> None:
         """The product for 1..8 input vectors at once: v [n][ncols] -> out [n][nrows]."""
-        if v.dim() != 2 or out.dim() != 2 or v.shape[1] != self.ncols or out.shape[1] != self.nrows or v.shape[0] != out.shape[0]:
-            raise WgbError(_lib.ERR_INVALID, "Gemm: dimension mismatch.")
-        check(_lib.load().wgb_gemm_q80_tiles(self._h, _f32(v, "v"), v.shape[0], _f32(out, "out"), _stream()))
+        _lib.dispatch().gemm_q80(out, self, v)
 
     def __del__(self):
         h, self._h = getattr(self, "_h", None), None
@@ -223,11 +215,7 @@ class RmsNorm:
         return cls()
 
     def dispatch(self, config: RmsNormConfig, result: torch.Tensor, value: torch.Tensor, weight: torch.Tensor) -> None:
-        n = value.numel()
-        if weight.numel() != n or result.numel() != n:
-            raise WgbError(_lib.ERR_INVALID, "RmsNorm: dimension mismatch.")
-        check(_lib.load().wgb_rms_norm(_f32(result, "result"), _f32(value, "value"), _f32(weight, "weight"), n,
-                                       config.nudge_factor, _stream()))
+        _lib.dispatch().rms_norm(result, value, weight, config.nudge_factor)
 
 
 class LayerNorm:
@@ -259,8 +247,7 @@ class RoPE:
         return cls()
 
     def dispatch(self, variant: RoPEVariant, shape: RoPEConfig, in_out_q: torch.Tensor, in_out_k: torch.Tensor) -> None:
-        check(_lib.load().wgb_rope(int(variant), C.byref(shape), _f32(in_out_q, "in_out_q"), in_out_q.numel(),
-                                   _f32(in_out_k, "in_out_k"), in_out_k.numel(), _stream()))
+        _lib.dispatch().rope(int(variant), shape, in_out_q, in_out_k)
 
 
 class BatchedMultiqueryAttention:
@@ -273,13 +260,7 @@ class BatchedMultiqueryAttention:
 
     def dispatch(self, params: BatchedMultiqueryAttentionParams, q, key_cache, value_cache, attn, xb) -> None:
         """`attn` ([n_heads][seq_len]) may be None: the split kernel then runs and no weights are stored."""
-        need = params.seq_len * params.kv_dim
-        if key_cache.numel() < need or value_cache.numel() < need or q.numel() != params.n_heads * params.head_size \
-                or xb.numel() != q.numel() or (attn is not None and attn.numel() < params.n_heads * params.seq_len):
-            raise WgbError(_lib.ERR_INVALID, "attention: dimension mismatch.")
-        check(_lib.load().wgb_attention(C.byref(params), _f32(q, "q"), _f32(key_cache, "key_cache"),
-                                        _f32(value_cache, "value_cache"), None if attn is None else _f32(attn, "attn"),
-                                        _f32(xb, "xb"), _stream()))
+        _lib.dispatch().attention(params, q, key_cache, value_cache, attn, xb)
 
     # The reference's four-kernel path has the same contract for xb (its attn layout is private).
     dispatch_multi = dispatch
@@ -310,9 +291,7 @@ class Silu:
         return cls()
 
     def dispatch(self, in_out_h1: torch.Tensor, in_h2: torch.Tensor) -> None:
-        if in_out_h1.numel() != in_h2.numel():
-            raise WgbError(_lib.ERR_INVALID, "Silu: dimension mismatch.")
-        check(_lib.load().wgb_silu(_f32(in_out_h1, "in_out_h1"), _f32(in_h2, "in_h2"), in_out_h1.numel(), _stream()))
+        _lib.dispatch().silu(in_out_h1, in_h2)
 
 
 class UnaryOp(enum.IntEnum):
@@ -392,9 +371,7 @@ class OpAssign:
     new = classmethod(lambda cls, device, variant: cls(device, variant))
 
     def dispatch(self, lhs: torch.Tensor, rhs: torch.Tensor) -> None:
-        if lhs.numel() != rhs.numel():
-            raise WgbError(_lib.ERR_INVALID, "OpAssign: dimension mismatch.")
-        check(_lib.load().wgb_op_assign(int(self.variant), _f32(lhs, "lhs"), _f32(rhs, "rhs"), lhs.numel(), _stream()))
+        _lib.dispatch().op_assign(self.variant, lhs, rhs)
 
 
 def sample_argmax(v: torch.Tensor) -> int:
