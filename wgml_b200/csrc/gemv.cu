@@ -404,8 +404,9 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
 
     // ------------------------------ consumers ------------------------------
     // What the input does not decide is worked out while the launch before drains.
-    // Task loop: the warps of a group take the units of every stage, the two groups alternate stages.  The digits of the inputs of a unit stay in registers as long as the unit does (one or
-    // two stages per tile).  Lane 4g + t has rows g and g + 8 of the tile; in a tile of eight rows, g twice.
+    // Task loop, further down: the warps of a group take the units of a stage, the two groups alternate stages.  The digits of the inputs
+    // of a unit stay in registers as long as the unit does (one or two stages per tile).  Lane 4g + t has rows g and g + 8 of the
+    // tile; in a tile of eight rows, g twice.
     const XImage<QT> im(smem0 + skip, units);
     uint32_t held = ~0u, phase = 0;
     const uint32_t w = (uint32_t)warp % TILE_UNITS, group = (uint32_t)warp / TILE_UNITS, ngroups = nstage > 1 ? 2 : 1;
