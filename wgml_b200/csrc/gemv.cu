@@ -356,9 +356,10 @@ __global__ void __launch_bounds__(GEMV_NT, 1) gemv_kernel(const __grid_constant_
                 const uint32_t in_stage = min(left, TILE_UNITS);
                 mbar_wait(done0 + 8 * s, phase, a.err, 3, a.wait_ns);
                 const float *p = part + s * (TILE_UNITS * 16) + half * 64 + row;
+                float t[4];
 #pragma unroll
-                for (uint32_t k = 0; k < 4; k++)
-                    if (half * 4 + k < in_stage) y += p[k * 16];
+                for (uint32_t k = 0; k < 4; k++) t[k] = half * 4 + k < in_stage ? p[k * 16] : 0.0f;
+                y += (t[0] + t[1]) + (t[2] + t[3]);   // (one after the other: a tenth more rounding error in a layer)
                 __syncwarp();
                 if (lane == 0) mbar_arrive(empty0 + 8 * s);   // stage and partial sums may be overwritten
                 left -= in_stage;

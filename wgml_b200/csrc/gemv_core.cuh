@@ -311,15 +311,17 @@ struct Unit<WGB_F32> {
                                                 const XImage<WGB_F32> &im, uint32_t u, int lane, float &ya, float &yb)
     {
         const uint32_t t = (uint32_t)lane & 3, flip = ((uint32_t)lane >> 2) & 1;
-        ya = yb = 0.0f;
+        float sa4[4], sb4[4];
 #pragma unroll
         for (uint32_t i = 0; i < 4; i++) {
             const uint32_t o = t * 16 + ((i ^ flip) << 6);
             const uint4 a = lds128(sa[0] + w * 256 + o), b = lds128(sb[0] + w * 256 + o), x = lds128(im.pair + u * 256 + o);
             const float x0 = __uint_as_float(x.x), x1 = __uint_as_float(x.y), x2 = __uint_as_float(x.z), x3 = __uint_as_float(x.w);
-            ya += __uint_as_float(a.x) * x0 + __uint_as_float(a.y) * x1 + __uint_as_float(a.z) * x2 + __uint_as_float(a.w) * x3;
-            yb += __uint_as_float(b.x) * x0 + __uint_as_float(b.y) * x1 + __uint_as_float(b.z) * x2 + __uint_as_float(b.w) * x3;
+            sa4[i] = (__uint_as_float(a.x) * x0 + __uint_as_float(a.y) * x1) + (__uint_as_float(a.z) * x2 + __uint_as_float(a.w) * x3);
+            sb4[i] = (__uint_as_float(b.x) * x0 + __uint_as_float(b.y) * x1) + (__uint_as_float(b.z) * x2 + __uint_as_float(b.w) * x3);
         }
+        ya = (sa4[0] + sa4[1]) + (sa4[2] + sa4[3]);
+        yb = (sb4[0] + sb4[1]) + (sb4[2] + sb4[3]);
     }
 };
 
