@@ -1,10 +1,24 @@
-"""Host path of the per-op calls (dispatch.c) without a device: what it refuses, in the order and with the errors that the ops name."""
+"""Host path of the per-op calls (dispatch.c, or the same over ctypes) without a device: what it refuses, in the order and with the
+errors that the ops name, and what an installation without a compiler gets."""
+import os
+import shutil
+import subprocess
+import sys
+
 import pytest
 import torch
 
+from conftest import ROOT
 from wgml_b200 import _lib, ops
 
 CPU = torch.zeros(8)
+
+
+@pytest.fixture(params=["module", "ctypes"], autouse=True)
+def path(request, monkeypatch):
+    fast = _lib._dispatch_module() if request.param == "module" else _lib._dispatch_ctypes()
+    assert fast is not None
+    monkeypatch.setattr(_lib, "_fast", fast)
 
 
 class FakeMatrix:
@@ -44,7 +58,7 @@ def test_tensors_off_the_device_are_refused_by_name(call, name):
 
 
 def test_other_arguments():
-    d = _lib.dispatch()
+    d = _lib._dispatch_module()
     with pytest.raises(TypeError):
         d.gemv(CPU, FakeMatrix())
     with pytest.raises(TypeError):
@@ -55,3 +69,33 @@ def test_other_arguments():
         d.silu(object(), CPU)
     with pytest.raises(AttributeError):
         d.gemv(CPU, object(), CPU)
+
+
+def copied_package(tmp_path):
+    """A copy of the package as another installation has it: sources, no built module."""
+    dst = tmp_path / "wgml_b200"
+    shutil.copytree(os.path.join(ROOT, "wgml_b200"), dst, ignore=shutil.ignore_patterns("*.so", "build", "__pycache__"))
+    return dst
+
+
+def in_copy(tmp_path, code, **env):
+    return subprocess.run([sys.executable, "-c", code], cwd=tmp_path, capture_output=True, text=True, timeout=300,
+                          env=dict(os.environ, PYTHONPATH=str(tmp_path), PYTHONDONTWRITEBYTECODE="1", **env))
+
+
+def test_a_given_library_needs_no_compiler(tmp_path, path):
+    """With the library named by WGML_B200_LIB and neither gcc nor nvcc to be found, the per-op calls reach their own checks."""
+    copied_package(tmp_path)
+    r = in_copy(tmp_path, "import torch\nfrom wgml_b200 import ops\nz = torch.zeros(8)\nops.Silu().dispatch(z, z)", PATH="/nonexistent",
+                CUDA_HOME="/nonexistent", WGML_B200_LIB=_lib.LIB_PATH)
+    assert "TypeError: in_out_h1: expected a contiguous float32 CUDA tensor" in r.stderr, r.stderr
+
+
+def test_the_library_builds_without_python_headers(tmp_path, monkeypatch):
+    """build() makes the library alone; the host module is a step of its own."""
+    from wgml_b200 import build
+    monkeypatch.setattr(build, "EXT", str(tmp_path / "module.so"))
+    build.build()
+    assert not (tmp_path / "module.so").exists()
+    build.build_dispatch()
+    assert (tmp_path / "module.so").exists()

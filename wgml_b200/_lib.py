@@ -196,20 +196,33 @@ _fast = None
 
 
 def dispatch():
-    """The module with the host path of the per-op calls, its library addresses and classes set."""
+    """The host path of the per-op calls: the module built from dispatch.c, its library addresses and classes set; where it is neither
+    there nor can be built (no compiler, no Python headers, a tree that is not writable), the same calls over ctypes."""
     global _fast
-    if _fast is not None:
-        return _fast
+    if _fast is None:
+        _fast = _dispatch_module() or _dispatch_ctypes()
+    return _fast
+
+
+def _dispatch_ctypes():
+    load()
+    from . import dispatch_ctypes
+    return dispatch_ctypes
+
+
+def _dispatch_module():
     lib = load()
     if not os.path.exists(os.path.join(_HERE, "_dispatch.so")):
         from . import build as _build
-        _build.build()
+        try:
+            _build.build_dispatch()
+        except (RuntimeError, OSError):
+            return None
     import torch
     from . import _dispatch
     _dispatch.setup(torch.Tensor, torch.float32, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream, WgbError, check,
                     tuple(C.cast(getattr(lib, name), C.c_void_p).value for name in _DISPATCHED))
-    _fast = _dispatch
-    return _fast
+    return _dispatch
 
 
 def load() -> C.CDLL:

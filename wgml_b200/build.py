@@ -1,4 +1,4 @@
-"""Builds libwgml_b200.so (sm_100a only) in-tree with nvcc.  Usage: python -m wgml_b200.build [-v]"""
+"""Builds libwgml_b200.so (sm_100a only) in-tree with nvcc, and the host module of the per-op calls with gcc.  Usage: python -m wgml_b200.build [-v]"""
 from __future__ import annotations
 
 import concurrent.futures as cf
@@ -68,6 +68,12 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
         if r.returncode != 0:
             raise RuntimeError("link failed")
+    return LIB
+
+
+def build_dispatch(force: bool = False, verbose: bool = False) -> str:
+    """The module with the host path of the per-op calls (dispatch.c): a C compiler and Python's headers, no nvcc.  Apart from build():
+    the library, the models and the C ABI do without it, and the per-op calls have the same path in Python."""
     src = os.path.join(CSRC, "dispatch.c")
     if force or _stale(EXT, [src, os.path.abspath(__file__)]):
         cmd = ["gcc", "-O2", "-Wall", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], src, "-o", EXT]
@@ -76,8 +82,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
         if r.returncode != 0:
             raise RuntimeError("gcc failed for dispatch.c")
-    return LIB
+    return EXT
 
 
 if __name__ == "__main__":
     print(build(force="-f" in sys.argv, verbose="-v" in sys.argv))
+    print(build_dispatch(force="-f" in sys.argv, verbose="-v" in sys.argv))
