@@ -99,3 +99,39 @@ def test_the_library_builds_without_python_headers(tmp_path, monkeypatch):
     assert not (tmp_path / "module.so").exists()
     build.build_dispatch()
     assert (tmp_path / "module.so").exists()
+
+
+def test_a_module_of_another_interpreter_is_left_alone(tmp_path):
+    """A file without this interpreter's tag (here not even a library) is not loaded; this one's is built beside it."""
+    pkg = copied_package(tmp_path)
+    (pkg / "_dispatch.so").write_bytes(b"built for another Python")
+    (pkg / "_dispatch.cpython-399-other.so").write_bytes(b"the same")
+    r = in_copy(tmp_path, "import torch\nfrom wgml_b200 import _lib, build, ops\nprint(_lib._dispatch_module().__file__ == build.EXT)\n"
+                "z = torch.zeros(8)\nops.Silu().dispatch(z, z)", WGML_B200_LIB=_lib.LIB_PATH)
+    assert "True" in r.stdout and "TypeError: in_out_h1: expected a contiguous float32 CUDA tensor" in r.stderr, r.stdout + r.stderr
+
+
+def test_the_module_appears_whole(tmp_path, monkeypatch):
+    """The compiler writes beside the module's name, which a finished file takes and a failed one does not."""
+    from wgml_b200 import build
+    ext = tmp_path / "module.so"
+    monkeypatch.setattr(build, "EXT", str(ext))
+    for rc in (1, 0):
+        def gcc(cmd, **kw):
+            assert not ext.exists()
+            open(cmd[-1], "wb").write(b"half")
+            assert not ext.exists()
+            return subprocess.CompletedProcess(cmd, rc, "", "")
+        monkeypatch.setattr(build.subprocess, "run", gcc)
+        if rc:
+            with pytest.raises(RuntimeError):
+                build.build_dispatch()
+            assert not list(tmp_path.iterdir())
+        else:
+            build.build_dispatch()
+            assert list(tmp_path.iterdir()) == [ext]
+
+
+def test_the_module_names_what_it_calls():
+    """The addresses handed over are those of the module's own list, so a module and a library of different versions cannot disagree on it."""
+    assert set(_lib._dispatch_module().ENTRY_POINTS) <= set(_lib.SIGNATURES)

@@ -6,6 +6,7 @@ and cannot be built, importing this module raises.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -187,10 +188,6 @@ SIGNATURES = {
     "wgb_gpt2_kernels_per_token": (_i, [_vp]),
 }
 
-# Entry points that dispatch.c calls, in its order.
-_DISPATCHED = ("wgb_gemv_quant", "wgb_gemm_q4k_tiles", "wgb_gemm_q6k_tiles", "wgb_gemm_q80_tiles", "wgb_rms_norm", "wgb_rope", "wgb_attention",
-               "wgb_silu", "wgb_op_assign")
-
 _lib = None
 _fast = None
 
@@ -212,17 +209,19 @@ def _dispatch_ctypes():
 
 def _dispatch_module():
     lib = load()
-    if not os.path.exists(os.path.join(_HERE, "_dispatch.so")):
-        from . import build as _build
+    from . import build as _build
+    if not os.path.exists(_build.EXT):
         try:
             _build.build_dispatch()
         except (RuntimeError, OSError):
             return None
     import torch
-    from . import _dispatch
-    _dispatch.setup(torch.Tensor, torch.float32, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream, WgbError, check,
-                    tuple(C.cast(getattr(lib, name), C.c_void_p).value for name in _DISPATCHED))
-    return _dispatch
+    spec = importlib.util.spec_from_file_location("wgml_b200._dispatch", _build.EXT)   # by its path: another interpreter's file is another name
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    mod.setup(torch.Tensor, torch.float32, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream, WgbError, check,
+              tuple(C.cast(getattr(lib, name), C.c_void_p).value for name in mod.ENTRY_POINTS))
+    return mod
 
 
 def load() -> C.CDLL:

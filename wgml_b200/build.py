@@ -12,7 +12,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "csrc", "build")
 LIB = os.path.join(HERE, "libwgml_b200.so")
-EXT = os.path.join(HERE, "_dispatch.so")   # CPython module: host path of the per-op calls (dispatch.c)
+# CPython module, host path of the per-op calls (dispatch.c); named by the interpreter it is built for, whose C API it uses
+EXT = os.path.join(HERE, "_dispatch" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 SOURCES = ["api.cpp", "gguf.cpp", "tokenizer.cpp", "quant.cu", "gemv.cu", "gemv_tc.cu", "attention.cu", "ops.cu", "sampler.cu", "prefill.cu", "prefill_q6k.cu", "prefill_q80.cu", "prefill_wide.cu", "llama2.cu", "gpt2.cu", "comm.cpp"]
 
@@ -76,12 +77,16 @@ def build_dispatch(force: bool = False, verbose: bool = False) -> str:
     the library, the models and the C ABI do without it, and the per-op calls have the same path in Python."""
     src = os.path.join(CSRC, "dispatch.c")
     if force or _stale(EXT, [src, os.path.abspath(__file__)]):
-        cmd = ["gcc", "-O2", "-Wall", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], src, "-o", EXT]
+        tmp = f"{EXT}.{os.getpid()}"   # renamed when whole: processes that start together load no half of it
+        cmd = ["gcc", "-O2", "-Wall", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], src, "-o", tmp]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if verbose or r.returncode != 0:
             sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
         if r.returncode != 0:
+            if os.path.exists(tmp):
+                os.remove(tmp)
             raise RuntimeError("gcc failed for dispatch.c")
+        os.replace(tmp, EXT)
     return EXT
 
 

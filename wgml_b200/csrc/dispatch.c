@@ -12,6 +12,9 @@ static PyObject *tensor_type, *float32, *get_device, *raw_stream, *wgb_error, *c
 
 enum { F_GEMV, F_GEMM_Q4K, F_GEMM_Q6K, F_GEMM_Q80, F_RMS_NORM, F_ROPE, F_ATTENTION, F_SILU, F_OP_ASSIGN, F_COUNT };
 static void *fn[F_COUNT];
+static const char *const entry[F_COUNT] = {   /* ENTRY_POINTS of the module: whose addresses setup() wants, in this order */
+    "wgb_gemv_quant", "wgb_gemm_q4k_tiles", "wgb_gemm_q6k_tiles", "wgb_gemm_q80_tiles", "wgb_rms_norm", "wgb_rope", "wgb_attention", "wgb_silu", "wgb_op_assign",
+};
 
 static const long ERR_INVALID = 1;
 
@@ -263,5 +266,13 @@ PyMODINIT_FUNC PyInit__dispatch(void)
     };
     for (size_t i = 0; i < sizeof(names) / sizeof(names[0]); i++)
         if (!(*names[i].at = PyUnicode_InternFromString(names[i].text))) return NULL;
-    return PyModule_Create(&module);
+    PyObject *m = PyModule_Create(&module), *list = m ? PyTuple_New(F_COUNT) : NULL;
+    for (Py_ssize_t i = 0; list && i < F_COUNT; i++) {
+        PyObject *text = PyUnicode_FromString(entry[i]);
+        if (!text) Py_CLEAR(list);
+        else PyTuple_SET_ITEM(list, i, text);
+    }
+    if (!list || PyModule_AddObjectRef(m, "ENTRY_POINTS", list)) Py_CLEAR(m);
+    Py_XDECREF(list);
+    return m;
 }
