@@ -48,6 +48,8 @@ def test_dimension_mismatches(call, message):
 @pytest.mark.parametrize("call,name", [
     (lambda: ops.Silu().dispatch(CPU, CPU), "in_out_h1"),
     (lambda: ops.Silu().dispatch(CPU.double(), CPU), "in_out_h1"),
+    (lambda: ops.GemvQuant().dispatch(CPU, FakeMatrix(), CPU), "v"),                          # a handle of None is the library's to refuse
+    (lambda: ops.Q4KTiles.gemm(FakeMatrix(), torch.zeros(2, 8), torch.zeros(2, 8)), "v"),
     (lambda: ops.RmsNorm().dispatch(ops.RmsNormConfig(1e-5), CPU, CPU, CPU), "result"),
     (lambda: ops.RoPE().dispatch(ops.RoPEVariant.Neox, ops.RoPEConfig(8, 8, 0, 1e4), CPU, CPU), "in_out_q"),
     (lambda: ops.BatchedMultiqueryAttention().dispatch(ops.BatchedMultiqueryAttentionParams(1, 8, 1, 1, 8, 0), CPU, CPU, CPU, None, CPU), "q"),

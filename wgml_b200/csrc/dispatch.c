@@ -111,12 +111,12 @@ static int current_stream(void **out)
     return *out || !PyErr_Occurred();
 }
 
-/* The library's object behind a Python one (its ctypes handle `_h`). */
+/* The library's object behind a Python one (its ctypes handle `_h`; None once destroyed: the library's error follows). */
 static int handle(PyObject *o, void **out)
 {
     PyObject *h = PyObject_GetAttr(o, s_h);
     if (!h) return 0;
-    PyObject *v = PyObject_GetAttr(h, s_value);
+    PyObject *v = h == Py_None ? Py_NewRef(h) : PyObject_GetAttr(h, s_value);
     Py_DECREF(h);
     if (!v) return 0;
     *out = v == Py_None ? NULL : PyLong_AsVoidPtr(v);
