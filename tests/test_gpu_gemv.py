@@ -157,6 +157,28 @@ def test_gemv_tile_edges(qtype, cols, nrows):
         assert (err <= bound).all(), f"qtype {qtype} {nrows}x{ncols}: {(err / np.maximum(bound, 1e-300)).max()}"
 
 
+@pytest.mark.parametrize("qtype,cols", [(ops.F32, (48960, 48964, 53056, 53060)), (ops.Q4_K, (64768, 67584)), (ops.Q6_K, (57344, 61440)), (ops.Q8_0, (67488, 70304))])
+def test_gemv_rows_around_the_longest(qtype, cols):
+    """More rows than eight-row tiles for every block, rows around the two lines of the fused kernel: the longest that leaves room for a
+    stage of sixteen rows, then stages of eight, then the general kernel.  Bound: 23-bit inputs and f32 sums in fewer than K / 32 + 64
+    steps (general kernel: a chain of K / 32 per lane), as in test_gemv_tile_edges."""
+    nrows = 1185
+    for ncols in cols:
+        raw, x = make(qtype, nrows, ncols, 31)
+        out, xd = torch.full((nrows,), float("nan"), device="cuda"), torch.from_numpy(x).cuda()
+        ops.GemvQuant.from_device().dispatch(out, ops.GpuQuantMatrix(qtype, raw, nrows, ncols), xd)
+        w = torch.from_numpy(oracle.dequantize(qtype, raw).reshape(nrows, ncols)).cuda().double()
+        exp = w @ xd.double()
+        w.abs_()
+        pad = torch.nn.functional.pad(xd.abs(), (0, -ncols % 32)).view(-1, 32)
+        mags = w @ xd.abs().double()
+        if qtype in (ops.Q4_K, ops.Q6_K):
+            mags += 2.0 * w.view(nrows, -1, 32).amax(2) @ pad.sum(1).double()
+        bound = 2.0 ** -23 * (w @ pad.amax(1).repeat_interleave(32)[:ncols].double()) + (ncols / 32 + 64) * 2.0 ** -24 * mags
+        err = (out.double() - exp).abs()
+        assert (err <= bound).all(), f"qtype {qtype} {nrows}x{ncols}: {(err / bound).max()}"
+
+
 @pytest.mark.parametrize("qtype,nrows,ncols", [
     (ops.F32, 32000, 288),      # one stage a tile: the consumer groups take tiles in turn, three epilogue warps
     (ops.F32, 60000, 32),       # the same with one unit at work

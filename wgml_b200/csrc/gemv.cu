@@ -617,11 +617,21 @@ __global__ void __launch_bounds__(256) gemv_generic_kernel(const __grid_constant
 // Launchers
 // ---------------------------------------------------------------------------------------------
 
+// Shared memory in front of the ring (the image of the input) and whether a stage of `octets` times eight rows fits behind it.
+static uint32_t image_bytes(const QMat &m) { return (uint32_t)((ximage_bytes(m.qtype, m.ncols) + 127) & ~(size_t)127); }
+static bool gemv_fits(const QMat &m, uint32_t octets)
+{
+    return (size_t)image_bytes(m) + 128 + octets * tile_bytes(m.qtype) + GEMV_PART_BYTES <= GEMV_SMEM_BUDGET;
+}
+
+bool gemv_pairs_supported(const QMat &m) { return gemv_fast_supported(m) && gemv_fits(m, 2); }
+
 bool gemv_fast_supported(const QMat &m)
 {
     if (m.qtype != WGB_Q4_K && m.qtype != WGB_Q6_K && m.qtype != WGB_Q8_0 && m.qtype != WGB_F32) return false;
     for (int i = 0; i < m.nplanes; i++)
         if (((uintptr_t)m.p[i] % 16) != 0 || m.pitch[i] % 16 != 0) return false;
+    if (!gemv_fits(m, 1)) return false;   // (columns up to 67328 of Q4_K, 61184 of Q6_K, 70272 of Q8_0, 53056 of F32)
     if (m.qtype == WGB_F32) return m.ncols % 4 == 0;
     if (m.ncols % 32 != 0) return false;
     if (m.qtype == WGB_Q8_0 || m.qtype == WGB_Q6_K) return m.planar != 0;
@@ -719,7 +729,7 @@ int make_tile_maps(const QMat &m, TileMaps &out)
 }
 
 // Chooses rows per tile, ring depth and grid; fills the plan fields of `a`.  Returns false when the image of the input leaves no
-// room for a stage.
+// room for a stage (pairs of rows, which take sixteen; anything else falls back to eight where sixteen do not fit).
 static bool plan(GemvArgs &a, size_t &smem_bytes, uint32_t &grid)
 {
     const QMat &m0 = a.mat[0];
@@ -728,7 +738,7 @@ static bool plan(GemvArgs &a, size_t &smem_bytes, uint32_t &grid)
     const bool pairs = a.epilogue == EPI_SILU_PAIR || (a.epilogue == EPI_QKV_ROPE && a.rope_variant == WGB_ROPE_NEOX);
     uint32_t total_rows = 0;
     for (int i = 0; i < (a.epilogue == EPI_SILU_PAIR ? 1 : a.nmat); i++) total_rows += a.mat[i].nrows;
-    a.octets = !pairs && (total_rows + TILE_ROWS - 1) / TILE_ROWS <= sms ? 1 : 2;
+    a.octets = !pairs && ((total_rows + TILE_ROWS - 1) / TILE_ROWS <= sms || !gemv_fits(m0, 2)) ? 1 : 2;
     a.tile_rows = a.octets * TILE_ROWS;
     auto tiles = [&](const QMat &m) { return (m.nrows + a.tile_rows - 1) / a.tile_rows; };
     if (a.epilogue == EPI_SILU_PAIR) a.ntiles = (m0.nrows + TILE_ROWS - 1) / TILE_ROWS;
@@ -749,7 +759,7 @@ static bool plan(GemvArgs &a, size_t &smem_bytes, uint32_t &grid)
     a.nchunk = (a.units + TILE_UNITS - 1) / TILE_UNITS;
     a.stage_bytes = a.octets * tile_bytes(qt);
     const uint32_t need = a.per_block * a.nchunk;   // stages of the fullest block
-    a.part_offset = (uint32_t)((ximage_bytes(qt, m0.ncols) + 127) & ~(size_t)127);
+    a.part_offset = image_bytes(m0);
     auto stages_in = [&](size_t budget) -> uint32_t {
         if (a.part_offset + 128 > budget) return 0;
         const size_t n = (budget - a.part_offset - 128) / (a.stage_bytes + GEMV_PART_BYTES);
@@ -808,7 +818,7 @@ template <int QT>
 static int launch_one(GemvArgs &a, cudaStream_t stream, bool pdl)
 {
     void (*kern)(const GemvArgs) = nullptr;
-const bool peers = a.peer_in.n || a.peer_out.n;
+    const bool peers = a.peer_in.n || a.peer_out.n;
 #define WGB_PICK(PRO, EPI, PEERS) if (a.prologue == PRO && a.epilogue == EPI && peers == PEERS) kern = gemv_kernel<QT, PRO, EPI, PEERS>;
     WGB_GEMV_VARIANTS(WGB_PICK)
 #undef WGB_PICK

@@ -90,7 +90,10 @@ struct GemvArgs {
 // `pdl` launches with programmatic stream serialization (the kernel prefetches its first
 // weights before waiting for its predecessor).
 int launch_gemv(const GemvArgs &a, cudaStream_t stream, bool pdl);
+// Format, alignment and row length have a fused kernel; the second: also in the launches that take rows of two matrices or of the two
+// halves of a head together (q/k/v, gate/up), whose longest row is shorter.
 bool gemv_fast_supported(const QMat &m);
+bool gemv_pairs_supported(const QMat &m);
 // One-time per-process set-up of the fused kernels (call outside stream capture).
 int gemv_global_init();
 // WGB_ERR_TIMEOUT if any bounded wait of a fused kernel expired since the last call (synchronises).

@@ -167,6 +167,7 @@ bool fusable(const wgb_llama2 *m)
             if (!l.m[i] || !gemv_fast_supported(l.m[i]->view)) return false;
         const QMat &q = l.m[WGB_L_ATTN_Q]->view, &k = l.m[WGB_L_ATTN_K]->view, &v = l.m[WGB_L_ATTN_V]->view;
         if (q.qtype != k.qtype || q.qtype != v.qtype) return false;
+        if (!gemv_pairs_supported(q) || !gemv_pairs_supported(l.m[WGB_L_FFN_GATE]->view)) return false;   // (k, v and up are as wide)
         if (l.m[WGB_L_FFN_GATE]->view.qtype != l.m[WGB_L_FFN_UP]->view.qtype) return false;
     }
     const wgb_quant_matrix *out = m->output ? m->output : m->token_embd;
