@@ -179,6 +179,27 @@ def test_gemv_rows_around_the_longest(qtype, cols):
         assert (err <= bound).all(), f"qtype {qtype} {nrows}x{ncols}: {(err / bound).max()}"
 
 
+@pytest.mark.parametrize("qtype,ncols,stage", [(ops.F32, 11008, 512), (ops.F32, 22016, 512), (ops.Q8_0, 28672, 1024), (ops.Q8_0, 46080, 1024)])
+def test_gemv_long_rows_are_not_one_chain(qtype, ncols, stage):
+    """All weights 1, 2^24 in the first stage of columns and a 1 in each later one: an addition to the large sum loses the 1 (a tie, to
+    even).  Stages go to four sums in turn, so a quarter of the additions are to the large one, and a few at the end (three between
+    the sums, one between halves of a row): each within half an ulp, 1."""
+    n = 24
+    w = np.ones((n, ncols), np.float32)
+    if qtype == ops.F32:
+        raw = w.view(np.uint8)
+    else:
+        raw = np.concatenate([np.full((n * ncols // 32, 1), 1.0, np.float16).view(np.uint8).reshape(-1, 2), np.ones((n * ncols // 32, 32), np.uint8)], axis=1)
+    assert np.array_equal(oracle.dequantize(qtype, raw.reshape(-1)).reshape(n, ncols), w)
+    x = np.zeros(ncols, np.float32)
+    x[0], x[stage + 64::stage] = 2.0 ** 24, 1.0
+    stages = -(-ncols // stage)
+    out = torch.zeros(n, device="cuda")
+    ops.GemvQuant.from_device().dispatch(out, ops.GpuQuantMatrix(qtype, raw.reshape(-1), n, ncols), torch.from_numpy(x).cuda())
+    err = np.abs(out.cpu().numpy().astype(np.float64) - x.astype(np.float64).sum()).max()
+    assert err <= stages / 4 + 4, (err, stages)
+
+
 @pytest.mark.parametrize("qtype,nrows,ncols", [
     (ops.F32, 32000, 288),      # one stage a tile: the consumer groups take tiles in turn, three epilogue warps
     (ops.F32, 60000, 32),       # the same with one unit at work
