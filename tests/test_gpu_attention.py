@@ -144,3 +144,8 @@ def test_cluster_kernel_edges(hs, heads, kv_mul):
 def test_more_heads_than_resident_blocks(case):
     """One, two, three, four, eight and twelve query heads per KV head where the cluster kernel leaves more than a chunk to the others."""
     run(*case, want_attn=False, seed=2)
+
+
+def test_more_heads_than_a_grid_has_rows():
+    """Short contexts with more query heads than the second axis of a grid holds (65535), on a quarter as many KV heads."""
+    run(8, 65540, 4, 4, 5, want_attn=False, seed=6)

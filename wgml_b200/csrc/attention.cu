@@ -1440,7 +1440,7 @@ static uint32_t cluster_blocks(const wgb_attn_params &p, uint32_t chunks, bool d
 {
     if (p.head_size > 128) return 0;
     const uint32_t resident = p.head_size <= 64 ? 256 : 128;   // two blocks per SM, or one
-    if (p.n_heads > resident) return chunks == 1 ? 1 : 0;
+    if (p.n_heads > resident) return chunks == 1 && p.n_heads <= 65535 ? 1 : 0;   // (a block per head: the second axis of a grid ends there)
     if (chunks <= (decode ? 3u : 2u)) return 1;
     uint32_t n = 1;
     while (n < 4 && 2 * n * p.n_heads <= resident) n *= 2;
