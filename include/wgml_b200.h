@@ -174,6 +174,10 @@ typedef struct {
 int wgb_attention(const wgb_attn_params *p, const float *d_q, const float *d_key_cache,
                   const float *d_value_cache, float *d_attn, float *d_xb, void *stream);
 
+/* Which kernel serves wgb_attention without weights (decode 0) or the attention of a Llama decode step whose last position is
+ * p->pos (decode 1) on the current device; -1 on error.  No launch: for reports, and for tests that are about one of them. */
+enum { WGB_ATTN_SPLIT, WGB_ATTN_SPLIT_CHUNKS, WGB_ATTN_ROWS, WGB_ATTN_STREAM, WGB_ATTN_CLUSTER };
+int wgb_attention_kernel(const wgb_attn_params *p, int decode);
 /* wgb_attention without any device allocation.  No counterpart in the reference; it exists for hosts
  * that cannot have cudaMalloc / cudaFree on the call path: a server that has given the whole device to
  * its own memory pool, or a latency-critical loop in which the device-wide synchronisation of an

@@ -1,8 +1,10 @@
 """Shared builders for the model parity tests: the same seeded tensors go to the oracle and to the GPU."""
+import ctypes as C
+
 import numpy as np
 
 import oracle
-from wgml_b200 import synth
+from wgml_b200 import _lib, synth
 from wgml_b200.models import Gpt2, Gpt2Params, Llama2, Llama2Config, LlamaModelType
 
 SMALL_LLAMA = dict(arch="llama", dim=512, hidden_dim=1024, n_layers=2, n_q_heads=8, n_kv_heads=8, vocab_size=1000,
@@ -34,3 +36,10 @@ def gpt2_pair(cfg: dict, seed=0, fused=True, scale=0.01):
 def rel_err(a, b):
     a, b = np.asarray(a, np.float64), np.asarray(b, np.float64)
     return float(np.abs(a - b).max() / max(np.abs(b).max(), 1e-30))
+
+
+def attention_kernel(seq_len, n_heads, head_size, kv_mul, pos, decode=False):
+    """The kernel that serves an attention call of these sizes (decode: a decode step up to `pos`)."""
+    p = _lib.AttnParams(seq_len, n_heads // kv_mul * head_size, kv_mul, n_heads, head_size, pos)
+    k = _lib.load().wgb_attention_kernel(C.byref(p), int(decode))
+    return ["split", "split, several chunks a block", "rows", "stream", "cluster"][k] if k >= 0 else None

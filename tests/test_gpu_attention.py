@@ -6,6 +6,7 @@ import torch
 
 import oracle
 from conftest import ATOL, RTOL, assert_close
+from helpers import attention_kernel
 from wgml_b200 import ops
 
 pytestmark = pytest.mark.gpu
@@ -30,6 +31,26 @@ def run(seq_len, n_heads, hs, kv_mul, pos, want_attn, seed=0):
     return xb
 
 
+# Every kernel of the stand-alone call, each width (query heads per KV head) of those that have them.  Short contexts are the
+# cluster kernel's as long as its blocks are resident, so the others' cases have more heads than that, longer contexts or wider heads.
+KERNELS = [
+    ("rows", (2112, 32, 128, 1, 2100)), ("rows", (2112, 32, 64, 2, 1700)), ("rows", (512, 264, 64, 4, 300)), ("rows", (512, 264, 64, 8, 300)),
+    ("rows", (512, 264, 64, 2, 300)), ("rows", (4224, 64, 128, 8, 4100)),
+    ("split", (512, 132, 128, 1, 190)), ("split", (512, 132, 128, 12, 250)), ("split", (512, 12, 256, 1, 300)), ("split", (512, 10, 256, 5, 301)),
+    ("split, several chunks a block", (2112, 60, 64, 5, 2100)), ("split, several chunks a block", (512, 132, 256, 1, 400)),
+    ("cluster", (512, 32, 128, 1, 300)), ("cluster", (512, 12, 64, 3, 300)), ("cluster", (512, 32, 128, 4, 300)),
+]
+
+
+@pytest.mark.parametrize("kernel,case", KERNELS)
+def test_each_kernel(kernel, case):
+    """Against the oracle, and again: tickets and scratch are left as the next call needs them."""
+    assert attention_kernel(*case) == kernel
+    a = run(*case, want_attn=False, seed=7)
+    b = run(*case, want_attn=False, seed=7)
+    assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("want_attn", [True, False])
 def test_reference_test_sizes(want_attn):  # ops/batched_multiquery_attention.rs:210-413
     for pos in list(range(9)):
@@ -39,7 +60,7 @@ def test_reference_test_sizes(want_attn):  # ops/batched_multiquery_attention.rs
 @pytest.mark.parametrize("case", [
     (256, 6, 48, 1, 255), (768, 32, 128, 1, 600), (4224, 64, 128, 8, 4100), (1024, 12, 64, 1, 1023),
     (512, 12, 64, 3, 130), (512, 16, 32, 2, 63), (512, 16, 32, 2, 64), (512, 10, 256, 5, 77), (128, 4, 4, 4, 100)])
-def test_split_kernel_shapes(case):
+def test_split_kernel_shapes(case):   # (most of them short contexts of few heads: now the cluster kernel's)
     run(*case, want_attn=False, seed=1)
 
 
@@ -50,22 +71,24 @@ def test_split_kernel_shapes(case):
     (4224, 32, 128, 2, 2049),    # two, last group of two rows
     (4224, 40, 128, 5, 3000),    # five query heads per KV head: split kernel, two groups of four (tail masked)
     (4224, 96, 128, 12, 1500),   # twelve: split kernel, three groups of four
+    (512, 264, 64, 8, 64), (512, 264, 64, 8, 71),    # row-streaming kernel: nine groups over four blocks a KV head, one row in the last and full
+    (512, 144, 128, 8, 130),     # seventeen groups over eight blocks a KV head
     (8256, 64, 64, 8, 8200),     # head size 64: half of the lanes idle
     (8256, 24, 96, 1, 5000),     # head size 96
     (4224, 64, 128, 8, 2047), (4224, 64, 128, 8, 2048),   # last group full, one row in it
-    (4224, 64, 128, 8, 1300),    # nine to ten groups of rows per block: not every warp has a second one
+    (4224, 64, 128, 8, 1300),    # cluster kernel, as the four below
     (8256, 32, 96, 4, 7001),     # four heads per KV head, a quarter of the lanes idle
-    (4224, 64, 128, 8, 0),       # only the first group holds anything, and only one row
+    (4224, 64, 128, 8, 0),
     (4224, 64, 128, 8, 63), (4224, 64, 128, 8, 64), (4224, 64, 128, 8, 130),
 ])
 def test_streaming_kernel_shapes(case):
     """Stand-alone calls on long contexts or with many query heads per KV head: the row-streaming kernel (one, two, four or
-    eight query heads per KV head) or the split kernel with several chunks per block.  (The streaming kernel proper wants the rows
+    eight query heads per KV head) or the split kernel with several chunks per block, up to 1536 positions also the cluster kernel.  (The streaming kernel proper wants the rows
     of a head side by side, as the models' caches have them: test_gpu_decode_attention.py.)"""
     run(*case, want_attn=False, seed=3)
 
 
-def test_repeated_calls_reuse_the_ticket_counters():
+def test_repeated_calls_reuse_the_ticket_counters():   # (cluster kernel, which has none; the others: test_each_kernel)
     a = run(512, 8, 64, 2, 300, False, seed=2)
     b = run(512, 8, 64, 2, 300, False, seed=2)
     assert torch.equal(a, b)
@@ -78,9 +101,8 @@ def test_repeated_streaming_calls_reuse_the_ticket_counters():   # row-streaming
 
 
 @pytest.mark.parametrize("case", [
-    (2112, 32, 128, 1, 2100), (512, 32, 64, 2, 300), (512, 32, 128, 4, 300), (4224, 64, 128, 8, 4100),   # row-streaming kernel, each width
-    (512, 32, 128, 1, 300), (512, 12, 64, 3, 130),                                                       # split kernel
-])
+    (512, 32, 64, 2, 300), (512, 12, 64, 3, 130),   # cluster kernel
+] + [case for _, case in KERNELS])
 @pytest.mark.parametrize("offset", [1, 2, 3])
 def test_output_at_any_word(case, offset):
     """`xb` may start at any float: only q and the caches are read sixteen bytes at a time.  Same bits, nothing beside it."""
@@ -97,9 +119,8 @@ def test_output_at_any_word(case, offset):
 
 
 @pytest.mark.parametrize("case", [
-    (2112, 32, 128, 1, 2100), (512, 32, 64, 2, 300), (512, 32, 128, 4, 300), (4224, 64, 128, 8, 1300),   # row-streaming kernel, each width
-    (512, 32, 128, 1, 300), (512, 12, 64, 3, 300), (2112, 60, 64, 5, 2100),   # split kernel, one chunk a block and several
-])
+    (512, 32, 64, 2, 300), (4224, 64, 128, 8, 1300),   # cluster kernel
+] + [case for _, case in KERNELS])
 @pytest.mark.parametrize("masked", [(0, 8), (0, 23), (0, 130), (8, 16), (40, 290), (1, 297)])
 def test_rows_scored_minus_infinity_weigh_nothing(case, masked):
     """Cache rows a host has masked with keys of -inf (left padding): whole groups, warps and blocks of the row-streaming

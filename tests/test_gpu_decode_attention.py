@@ -8,14 +8,16 @@ import pytest
 import torch
 
 from conftest import ATOL, RTOL, assert_close
-from helpers import SMALL_LLAMA, llama_pair
+from helpers import SMALL_LLAMA, attention_kernel, llama_pair
 from wgml_b200 import _lib, synth
 from wgml_b200.models import _device_view
 
 pytestmark = pytest.mark.gpu
 
 
-def steps(heads, kv_heads, head_size, start, gen, seq_len, seed=3):
+def steps(heads, kv_heads, head_size, start, gen, seq_len, seed=3, kernel=None):
+    if kernel:
+        assert attention_kernel(seq_len, heads, head_size, heads // kv_heads, start + gen - 1, decode=True) == kernel
     cfg = dict(SMALL_LLAMA, dim=heads * head_size, hidden_dim=512, n_layers=1, n_q_heads=heads, n_kv_heads=kv_heads, vocab_size=300, seq_len=seq_len)
     t = synth.llama_tensors(cfg, seed, scale=0.002)
     rng = np.random.default_rng(seed)
@@ -38,10 +40,22 @@ def steps(heads, kv_heads, head_size, start, gen, seq_len, seed=3):
 
 
 @pytest.mark.parametrize("shape", [(32, 32, 64), (64, 32, 64), (32, 32, 96)])
-@pytest.mark.parametrize("start", [955, 1022, 2100])   # 955: fifteen chunks; 1022: a chunk fills up and the next one begins
+@pytest.mark.parametrize("start", [955, 1022, 2100])
 def test_streaming_kernel_in_decode_steps(shape, start):
-    """Three blocks of the split kernel per SM hold 444 chunks: with 32 KV heads a context of more than 13 chunks is over one wave."""
-    steps(*shape, start, 4, 2176)
+    """Three blocks of the split kernel per SM hold 444 chunks: with 32 KV heads a context of more than 13 chunks is over one wave.
+    (Up to 1536 positions of these few heads: the cluster kernel.)"""
+    steps(*shape, start, 4, 2176, kernel="stream" if start == 2100 else "cluster")
+
+
+@pytest.mark.parametrize("shape,start,gen", [
+    ((320, 320, 8), 0, 140), ((320, 160, 8), 0, 300),                               # from the first position on
+    ((320, 320, 8), 955, 4), ((320, 160, 8), 955, 4), ((288, 144, 16), 955, 4),
+    ((320, 320, 8), 1022, 4), ((320, 160, 8), 1022, 4), ((288, 144, 16), 1022, 4),  # a chunk fills up and the next one begins
+])
+def test_streaming_kernel_of_many_heads_in_decode_steps(shape, start, gen):
+    """More heads than resident blocks of the cluster kernel; from position 0 on, in launches sized for the call's last position: most
+    blocks have no rows at first."""
+    steps(*shape, start, gen, 1100, kernel="stream")
 
 
 def test_streaming_kernel_with_several_chunks_per_block():
@@ -52,9 +66,19 @@ def test_streaming_kernel_with_several_chunks_per_block():
 @pytest.mark.parametrize("start", [0, 126, 200, 1001, 3003])
 def test_row_streaming_kernel_in_decode_steps(shape, start):
     """Ten steps leave every number of rows in the last group of eight.  Up to about 140 positions there are fewer groups
-    than blocks, and no warp requests anything ahead of the wait; from 1001 on most do.  (Where all blocks of the cluster kernel are
-    resident, contexts up to 1536 positions are its.)"""
-    steps(*shape, start, 10, 3072)
+    than blocks, and no warp requests anything ahead of the wait; from 1001 on most do.  (Up to 1536 positions of these few heads: the
+    cluster kernel.)"""
+    steps(*shape, start, 10, 3072, kernel="rows" if start == 3003 else "cluster")
+
+
+@pytest.mark.parametrize("shape,start,gen", [
+    ((288, 72, 16), 0, 70), ((320, 40, 8), 0, 530),                                 # from the first position on
+    ((288, 72, 16), 126, 10), ((288, 72, 16), 1001, 10), ((320, 40, 8), 1001, 10), ((288, 36, 16), 1001, 10),
+])
+def test_row_streaming_kernel_of_many_heads_in_decode_steps(shape, start, gen):
+    """More heads than resident blocks of the cluster kernel: the row-streaming kernel from the first position on, with fewer groups of
+    rows than blocks (nothing is requested ahead of the wait) and with more."""
+    steps(*shape, start, gen, 1100, kernel="rows")
 
 
 @pytest.mark.parametrize("shape", [(12, 12, 64), (16, 4, 128), (40, 40, 64), (36, 12, 128), (66, 33, 128)])

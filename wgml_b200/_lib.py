@@ -92,6 +92,7 @@ SIGNATURES = {
     "wgb_layernorm": (_i, [_vp, _vp, _sz, _vp]),
     "wgb_rope": (_i, [_i, C.POINTER(RopeConfig), _vp, _sz, _vp, _sz, _vp]),
     "wgb_attention": (_i, [C.POINTER(AttnParams), _vp, _vp, _vp, _vp, _vp, _vp]),
+    "wgb_attention_kernel": (_i, [C.POINTER(AttnParams), _i]),
     "wgb_attention_static": (_i, [C.POINTER(AttnParams), _vp, _vp, _vp, _vp, _vp]),
     "wgb_softmax": (_i, [_vp, _sz, _sz, _sz, _vp]),
     "wgb_silu": (_i, [_vp, _vp, _sz, _vp]),

@@ -1395,7 +1395,7 @@ static int launch_split(const AttnArgs &a, uint32_t nchunks, uint32_t nchunks_hi
     const bool one_wave = a.pos ? a.p.kv_mul == 4 || (a.p.kv_mul == 8 && n_kv >= 8 && a.p.head_size <= 64 && nchunks_hint > 8)
                                 : a.p.kv_mul > 1 && n_kv >= (a.p.kv_mul == 2 ? 16u : 8u);
     const bool rows_kernel = !stream_kernel && fits && (multi ? !idle : one_wave);
-    if (!a.q) return ATT_CLASS + (multi ? 1 : 0) + (rows_kernel ? 2 : 0);   // sizing query (attn_sizing_class): no launch
+    if (!a.q) return ATT_CLASS + (multi ? 1 : 0) + (rows_kernel ? 2 : 0) + (stream_kernel ? 4 : 0);   // sizing query (attn_sizing_class): no launch
     if (stream_kernel) return launch_stream_any(a, nchunks, stream, pdl);
     if (rows_kernel) {
         if (a.p.kv_mul == 1) return launch_rows<1>(a, nchunks, stream, pdl);
@@ -1470,20 +1470,31 @@ int launch_attention(const AttnArgs &a, cudaStream_t stream, bool pdl)
     return big ? launch_split<1, 2>(a, nchunks, nh, n_kv, zg, stream, pdl) : launch_split<1, 1>(a, nchunks, nh, n_kv, zg, stream, pdl);
 }
 
-// Which launch launch_attention picks for positions up to p.pos, as a small number (a caller that records launches for
-// later replay re-records when it changes); negative on error.
-int attn_sizing_class(const wgb_attn_params &p)
+static int sizing_query(const wgb_attn_params &p, bool decode, uint32_t row_stride)
 {
     AttnArgs a = {};
     a.p = p;
-    a.pos = reinterpret_cast<const uint32_t *>(&a);   // "position on the device": p.pos is the bound
+    a.row_stride = row_stride;
+    if (decode) a.pos = reinterpret_cast<const uint32_t *>(&a);   // "position on the device": p.pos is the bound
     const int r = launch_attention(a, nullptr, false);
     return r >= ATT_CLASS ? r - ATT_CLASS : -1;
 }
 
+// Which launch launch_attention picks for positions up to p.pos, as a small number (a caller that records launches for
+// later replay re-records when it changes); negative on error.
+int attn_sizing_class(const wgb_attn_params &p) { return sizing_query(p, true, 0); }
+
 }  // namespace wgb
 
 using namespace wgb;
+
+WGB_EXPORT int wgb_attention_kernel(const wgb_attn_params *p, int decode)
+{
+    if (!p) return -1;
+    const int c = sizing_query(*p, decode != 0, decode ? p->head_size : 0);
+    if (c < 0) return -1;
+    return c >= 8 ? WGB_ATTN_CLUSTER : c & 4 ? WGB_ATTN_STREAM : c & 2 ? WGB_ATTN_ROWS : c & 1 ? WGB_ATTN_SPLIT_CHUNKS : WGB_ATTN_SPLIT;
+}
 
 WGB_EXPORT int wgb_attention(const wgb_attn_params *p, const float *d_q, const float *d_key_cache,
                              const float *d_value_cache, float *d_attn, float *d_xb, void *stream)
