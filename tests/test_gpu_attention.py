@@ -170,3 +170,19 @@ def test_more_heads_than_resident_blocks(case):
 def test_more_heads_than_a_grid_has_rows():
     """Short contexts with more query heads than the second axis of a grid holds (65535), on a quarter as many KV heads."""
     run(8, 65540, 4, 4, 5, want_attn=False, seed=6)
+
+
+def test_rows_of_a_group_meet_before_the_running_sum():
+    """Equal weights, a value of 2^24 in the first row and 1 in the others, one block per head: a lane adds sixteen groups of two rows to
+    its running sum, then quarters of a warp (2 additions), warps (8) and the division round; each within half an ulp of 2^24, 1."""
+    heads, hs, kv_mul, pos = 96, 128, 4, 1000
+    assert attention_kernel(1024, heads, hs, kv_mul, pos) == "cluster"
+    kv_dim = heads // kv_mul * hs
+    v = torch.ones(1024, kv_dim, device="cuda")
+    v[0] = 2.0 ** 24
+    xb = torch.zeros(heads * hs, device="cuda")
+    ops.BatchedMultiqueryAttention.from_device().dispatch(ops.BatchedMultiqueryAttentionParams(1024, kv_dim, kv_mul, heads, hs, pos),
+                                                          torch.ones(heads * hs, device="cuda"), torch.zeros(1024, kv_dim, device="cuda"), v, None, xb)
+    n = pos + 1
+    err = (xb.double() - (2.0 ** 24 + pos) / n).abs().max().item() * n
+    assert err <= 16 + 2 + 8 + 1 + 1, err
