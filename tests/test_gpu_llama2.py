@@ -60,6 +60,19 @@ def test_small_quantised_llama(qtype, fused):
     compare_steps(gpu, cpu, synth.prompt(12, cfg["vocab_size"], 2), what=f"qtype {qtype}")
 
 
+@pytest.mark.parametrize("qwen,heads,kv_heads,head_size,hidden", [
+    (True, 3, 1, 20, 1028), (True, 6, 2, 36, 516), (True, 4, 4, 100, 1028),   # Neox: halves of 10, 18 and 50 rows in tiles of eight
+    (False, 3, 1, 20, 1028), (False, 7, 7, 12, 260),                          # adjacent pairs, tiles of eight: 60, 20 and 84 rows
+    (False, 50, 10, 20, 1356),                                                # tiles of sixteen: 1000 and 200 rows
+])
+def test_partial_row_tiles_of_the_fused_launches(qwen, heads, kv_heads, head_size, hidden):
+    """Matrices whose rows do not fill the last tile of a matrix, of a half of a head or of gate and up."""
+    cfg = dict(SMALL_LLAMA, dim=heads * head_size, hidden_dim=hidden, n_q_heads=heads, n_kv_heads=kv_heads, vocab_size=1001, default_qtype=synth.F32)
+    gpu, cpu, _ = llama_pair(cfg, seed=6, biases=qwen, qwen=qwen)
+    compare_steps(gpu, cpu, synth.prompt(9, cfg["vocab_size"], 6), what="partial tiles")
+    assert gpu.kernels_per_token() <= 5 * cfg["n_layers"] + 4   # the fused schedule
+
+
 def test_mixed_formats_in_one_layer_fall_back_to_separate_launches():
     cfg = dict(SMALL_LLAMA)
     t = synth.llama_tensors(cfg, 3, scale=0.002)
