@@ -1187,27 +1187,18 @@ __global__ void __launch_bounds__(ATT_NT, 1) attn_cluster_kernel(const __grid_co
         }
         const float rescale = expf(m - mn);
         m = mn;
-        float w[ATC_ROWS], sum = 0.0f;
-#pragma unroll
-        for (int r = 0; r < ATC_ROWS; r++) sum += w[r] = expf(s[r] - mn);
         // The rows of a group meet before they meet the running sums: one rounding of those per group.  (96 heads of size 128 on 24 at 900
         // positions, a block per head, error over that of the row-streaming kernel: row after row 1.05, so 0.99.)
-        l = fmaf(l, rescale, sum);
+        static_assert(ATC_ROWS == 2, "rows of a group");
+        const float w0 = expf(s[0] - mn), w1 = expf(s[1] - mn);
+        l = fmaf(l, rescale, w0 + w1);
 #pragma unroll
         for (int i = 0; i < NC; i++) {
-            float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int r = 0; r < ATC_ROWS; r++) {
-                const float4 v = fetch(src + GROUP + r * 4 * ROW, i);
-                t.x = fmaf(w[r], v.x, t.x);
-                t.y = fmaf(w[r], v.y, t.y);
-                t.z = fmaf(w[r], v.z, t.z);
-                t.w = fmaf(w[r], v.w, t.w);
-            }
-            acc[i].x = fmaf(acc[i].x, rescale, t.x);
-            acc[i].y = fmaf(acc[i].y, rescale, t.y);
-            acc[i].z = fmaf(acc[i].z, rescale, t.z);
-            acc[i].w = fmaf(acc[i].w, rescale, t.w);
+            const float4 v0 = fetch(src + GROUP, i), v1 = fetch(src + GROUP + 4 * ROW, i);
+            acc[i].x = fmaf(acc[i].x, rescale, fmaf(w1, v1.x, w0 * v0.x));
+            acc[i].y = fmaf(acc[i].y, rescale, fmaf(w1, v1.y, w0 * v0.y));
+            acc[i].z = fmaf(acc[i].z, rescale, fmaf(w1, v1.z, w0 * v0.z));
+            acc[i].w = fmaf(acc[i].w, rescale, fmaf(w1, v1.w, w0 * v0.w));
         }
         request(g + ATC_STAGES * nwarps, st);
         st = st + 1 == ATC_STAGES ? 0 : st + 1;
