@@ -1,5 +1,6 @@
 """Host path of the per-op calls (dispatch.c, or the same over ctypes) without a device: what it refuses, in the order and with the
 errors that the ops name, and what an installation without a compiler gets."""
+import ctypes
 import os
 import shutil
 import subprocess
@@ -71,6 +72,28 @@ def test_other_arguments():
         d.silu(object(), CPU)
     with pytest.raises(AttributeError):
         d.gemv(CPU, object(), CPU)
+
+
+def lookalike(cls, *values):
+    """A structure of the same fields as `cls`, of a class of its own."""
+    return type("Other", (ctypes.Structure,), {"_fields_": cls._fields_})(*values)
+
+
+def test_parameter_structures_are_of_their_class_or_a_derived_one():
+    """Any buffer of the right size is no parameter structure (ctypes takes none either); one of a derived class with more fields is."""
+    d = _lib._dispatch_module()
+    attn, rope = (1, 8, 1, 1, 8, 0), (8, 8, 0, 1e4)
+    for p in (bytes(24), lookalike(ops.BatchedMultiqueryAttentionParams, *attn)):
+        with pytest.raises(TypeError, match="^params: expected BatchedMultiqueryAttentionParams$"):
+            d.attention(p, CPU, CPU, CPU, None, CPU)
+    for p in (bytes(16), lookalike(ops.RoPEConfig, *rope)):
+        with pytest.raises(TypeError, match="^shape: expected a RoPEConfig$"):
+            d.rope(0, p, CPU, CPU)
+    for cls, values, call in ((ops.BatchedMultiqueryAttentionParams, attn, lambda p: d.attention(p, CPU, CPU, CPU, None, CPU)),
+                              (ops.RoPEConfig, rope, lambda p: d.rope(0, p, CPU, CPU))):
+        more = type("More", (cls,), {"_fields_": [("note", ctypes.c_uint32)]})
+        with pytest.raises(TypeError, match="expected a contiguous float32 CUDA tensor$"):
+            call(more(*values, 5))
 
 
 def copied_package(tmp_path):

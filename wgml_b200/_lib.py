@@ -220,7 +220,7 @@ def _dispatch_module():
     spec = importlib.util.spec_from_file_location("wgml_b200._dispatch", _build.EXT)   # by its path: another interpreter's file is another name
     mod = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(mod)
-    mod.setup(torch.Tensor, torch.float32, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream, WgbError, check,
+    mod.setup(torch.Tensor, torch.float32, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream, WgbError, check, RopeConfig, AttnParams,
               tuple(C.cast(getattr(lib, name), C.c_void_p).value for name in mod.ENTRY_POINTS))
     return mod
 

@@ -8,7 +8,7 @@
 #include <stdint.h>
 
 static PyObject *s_is_cuda, *s_dtype, *s_is_contiguous, *s_data_ptr, *s_numel, *s_shape, *s_h, *s_value, *s_nrows, *s_ncols;
-static PyObject *tensor_type, *float32, *get_device, *raw_stream, *wgb_error, *check_status;
+static PyObject *tensor_type, *float32, *get_device, *raw_stream, *wgb_error, *check_status, *rope_config, *attn_params;
 
 enum { F_GEMV, F_GEMM_Q4K, F_GEMM_Q6K, F_GEMM_Q80, F_RMS_NORM, F_ROPE, F_ATTENTION, F_SILU, F_OP_ASSIGN, F_COUNT };
 static void *fn[F_COUNT];
@@ -21,14 +21,15 @@ static const long ERR_INVALID = 1;
 static PyObject *setup(PyObject *self, PyObject *args)
 {
     PyObject *addresses;
-    if (!PyArg_ParseTuple(args, "OOOOOOO!", &tensor_type, &float32, &get_device, &raw_stream, &wgb_error, &check_status, &PyTuple_Type, &addresses))
+    if (!PyArg_ParseTuple(args, "OOOOOOOOO!", &tensor_type, &float32, &get_device, &raw_stream, &wgb_error, &check_status, &rope_config, &attn_params,
+                          &PyTuple_Type, &addresses))
         return NULL;
     if (PyTuple_GET_SIZE(addresses) != F_COUNT) return PyErr_Format(PyExc_ValueError, "expected %d addresses", (int)F_COUNT);
     for (int i = 0; i < F_COUNT; i++) {
         fn[i] = PyLong_AsVoidPtr(PyTuple_GET_ITEM(addresses, i));
         if (!fn[i]) return PyErr_Occurred() ? NULL : PyErr_Format(PyExc_ValueError, "null address");
     }
-    PyObject *keep[] = { tensor_type, float32, get_device, raw_stream, wgb_error, check_status };
+    PyObject *keep[] = { tensor_type, float32, get_device, raw_stream, wgb_error, check_status, rope_config, attn_params };
     for (size_t i = 0; i < sizeof(keep) / sizeof(keep[0]); i++) Py_INCREF(keep[i]);
     Py_RETURN_NONE;
 }
@@ -188,6 +189,24 @@ static PyObject *rms_norm(PyObject *self, PyObject *const *a, Py_ssize_t n)   /*
     CALL(((int (*)(void *, void *, void *, size_t, float, void *))fn[F_RMS_NORM])(r, v, w, nv, (float)eps, s));
 }
 
+/* Copies a parameter structure: of its own ctypes class or a derived one, whose first fields are the same. */
+static int structure(PyObject *o, PyObject *type, const char *what, void *to, Py_ssize_t size)
+{
+    const int is = PyObject_IsInstance(o, type);
+    if (is < 0) return 0;
+    if (!is) {
+        PyErr_SetString(PyExc_TypeError, what);
+        return 0;
+    }
+    Py_buffer b;
+    if (PyObject_GetBuffer(o, &b, PyBUF_SIMPLE)) return 0;
+    const int fits = b.len >= size;
+    if (fits) memcpy(to, b.buf, (size_t)size);
+    PyBuffer_Release(&b);
+    if (!fits) PyErr_SetString(PyExc_TypeError, what);
+    return fits;
+}
+
 static PyObject *rope(PyObject *self, PyObject *const *a, Py_ssize_t n)   /* variant, config structure, q, k */
 {
     size_t nq, nk;
@@ -195,27 +214,17 @@ static PyObject *rope(PyObject *self, PyObject *const *a, Py_ssize_t n)   /* var
     if (!expect(n, 4)) return NULL;
     const long variant = PyLong_AsLong(a[0]);
     if (variant == -1 && PyErr_Occurred()) return NULL;
-    if (!f32(a[2], "in_out_q", &q) || !numel(a[2], &nq) || !f32(a[3], "in_out_k", &k) || !numel(a[3], &nk) || !current_stream(&s)) return NULL;
-    Py_buffer b;
-    if (PyObject_GetBuffer(a[1], &b, PyBUF_SIMPLE)) return NULL;
     struct { uint32_t head_size, kv_dim, pos; float base; } cfg;
-    const int fits = b.len == (Py_ssize_t)sizeof(cfg);
-    if (fits) memcpy(&cfg, b.buf, sizeof(cfg));
-    PyBuffer_Release(&b);
-    if (!fits) return PyErr_Format(PyExc_TypeError, "shape: expected a RoPEConfig");
+    if (!structure(a[1], rope_config, "shape: expected a RoPEConfig", &cfg, sizeof(cfg))) return NULL;
+    if (!f32(a[2], "in_out_q", &q) || !numel(a[2], &nq) || !f32(a[3], "in_out_k", &k) || !numel(a[3], &nk) || !current_stream(&s)) return NULL;
     CALL(((int (*)(int, const void *, void *, size_t, void *, size_t, void *))fn[F_ROPE])((int)variant, &cfg, q, nq, k, nk, s));
 }
 
 static PyObject *attention(PyObject *self, PyObject *const *a, Py_ssize_t n)   /* params structure, q, keys, values, weights or None, xb */
 {
     if (!expect(n, 6)) return NULL;
-    Py_buffer b;
-    if (PyObject_GetBuffer(a[0], &b, PyBUF_SIMPLE)) return NULL;
     struct { uint32_t seq_len, kv_dim, kv_mul, n_heads, head_size, pos; } p;
-    const int fits = b.len == (Py_ssize_t)sizeof(p);
-    if (fits) memcpy(&p, b.buf, sizeof(p));
-    PyBuffer_Release(&b);
-    if (!fits) return PyErr_Format(PyExc_TypeError, "params: expected BatchedMultiqueryAttentionParams");
+    if (!structure(a[0], attn_params, "params: expected BatchedMultiqueryAttentionParams", &p, sizeof(p))) return NULL;
     const size_t need = (size_t)p.seq_len * p.kv_dim;
     size_t nk, nv, nq, nx, na = 0;
     if (!numel(a[2], &nk) || !numel(a[3], &nv) || !numel(a[1], &nq) || !numel(a[5], &nx) || (a[4] != Py_None && !numel(a[4], &na))) return NULL;
