@@ -1383,10 +1383,12 @@ static int launch_split(const AttnArgs &a, uint32_t nchunks, uint32_t nchunks_hi
     //     7.9), four and eight from eight on (8 of four: 11.3 and 9.2; of eight: 11.6 and 10.2); a single query head never
     //     (32 KV heads, 512 positions: 7.7 and 9.2).
     //   * one wave, decode step (position on the device): its blocks fill the shared memory, so that the matrix-vector
-    //     launch behind it cannot start prefetching beside it.  Up to two query heads the split kernel (GPT-2 decode
-    //     32.1 and 34.2 ms); four heads this one (8 KV heads, 900 positions: 81.2 and 71.6 a step); eight heads this one from
-    //     eight KV heads of size 64 and 512 positions on (84.0 and 76.1; but 200 positions of 16 KV heads 143.2 and 146.9, and 8
-    //     of size 128 at 500 positions 150.6 and 153.6).
+    //     launch behind it cannot start prefetching beside it.  Up to two query heads the split kernel (GPT-2's twelve heads of
+    //     size 64, a whole decode: 32.1 and 34.2 ms); four heads this one (8 KV heads, 900 positions: 81.2 and 71.6 a step); eight
+    //     heads this one from eight KV heads of size 64 and 512 positions on (84.0 and 76.1; but 200 positions of 16 KV heads
+    //     143.2 and 146.9, and 8 of size 128 at 500 positions 150.6 and 153.6).
+    // (Measured before the cluster kernel, which now takes most of the decode steps named here: cluster_blocks comes first.  What
+    // still reaches these lines is a context past its own.)
     const bool idle = a.p.kv_mul == 4 && 2 * n_kv > sms && 10 * n_kv < 7 * sms && nchunks_hint > 8;
     const bool fits = VC == 1 && (a.p.kv_mul == 1 || a.p.kv_mul == 2 || a.p.kv_mul == 4 || a.p.kv_mul == 8);
     const bool one_wave = a.pos ? a.p.kv_mul == 4 || (a.p.kv_mul == 8 && n_kv >= 8 && a.p.head_size <= 64 && nchunks_hint > 8)
@@ -1430,9 +1432,9 @@ static int launch_split(const AttnArgs &a, uint32_t nchunks, uint32_t nchunks_hi
 // step of two layers, 32 heads on 32: 60 positions 68.1 and 64.4 / 65.8 / 66.5 / 76.7, 600 positions 72.0 and 76.8 / 72.5 /
 // 69.5 / 81.1.)
 // Where not even one block per head is resident it pays for one chunk (256 heads on 64 of size 128: 8.0 and 6.2; 200 positions 11.2
-// and 11.3), otherwise up to sixteen chunks, and as far as measured, 1500 positions, with two blocks or more (32 heads
-// on 32: 15.2 and 11.6; 96 on 24, one block: 17.7 and 19.6).  Of 1174 shapes measured one is slower by more than 2 %: 40
-// heads on 40, 400 positions, 7.5 and 7.7.
+// and 11.3), otherwise up to sixteen chunks (96 heads on 24, one block, 1500 positions: 17.7 and 19.6).  With two blocks or more
+// the line at 24 chunks is where the measurements end, 1500 positions, not where the kernels cross: 32 heads on 32 are at 15.2
+// and 11.6 there.  Of 1174 shapes measured one is slower by more than 2 %: 40 heads on 40, 400 positions, 7.5 and 7.7.
 static uint32_t cluster_blocks(const wgb_attn_params &p, uint32_t chunks, bool decode)
 {
     if (p.head_size > 128) return 0;

@@ -14,7 +14,7 @@ constexpr uint32_t TC_A_BYTES = TC_TILE_ROWS * 256;           // the same, unpac
 
 // 64-bit shared-memory operand descriptor, no swizzle, K-major operand: start address, the byte distance
 // between core matrices (8 rows x 16 bytes) adjacent along K ("leading" field) and the distance between
-// those adjacent along the rows ("stride" field).  Checked against the dp4a kernel on the device.
+// those adjacent along the rows ("stride" field).  Checked against the matrix-vector kernel on the device.
 __device__ __forceinline__ uint64_t tc_smem_desc(uint32_t addr, uint32_t leading_bytes, uint32_t stride_bytes)
 {
     uint64_t d = 0;
