@@ -61,7 +61,7 @@ def test_tensors_off_the_device_are_refused_by_name(call, name):
 
 
 def test_other_arguments():
-    d = _lib._dispatch_module()
+    d = _lib.dispatch()
     with pytest.raises(TypeError):
         d.gemv(CPU, FakeMatrix())
     with pytest.raises(TypeError):
@@ -80,8 +80,8 @@ def lookalike(cls, *values):
 
 
 def test_parameter_structures_are_of_their_class_or_a_derived_one():
-    """Any buffer of the right size is no parameter structure (ctypes takes none either); one of a derived class with more fields is."""
-    d = _lib._dispatch_module()
+    """Any buffer of the right size is no parameter structure; one of a derived class with more fields is."""
+    d = _lib.dispatch()
     attn, rope = (1, 8, 1, 1, 8, 0), (8, 8, 0, 1e4)
     for p in (bytes(24), lookalike(ops.BatchedMultiqueryAttentionParams, *attn)):
         with pytest.raises(TypeError, match="^params: expected BatchedMultiqueryAttentionParams$"):

@@ -7,7 +7,7 @@ import ctypes as C
 import torch
 
 from . import _lib
-from ._lib import ERR_INVALID, WgbError, check
+from ._lib import AttnParams, ERR_INVALID, RopeConfig, WgbError, check
 
 
 def _f32(t, name):
@@ -52,10 +52,14 @@ def rms_norm(result, value, weight, eps):
 
 
 def rope(variant, config, q, k):
+    if not isinstance(config, RopeConfig):
+        raise TypeError("shape: expected a RoPEConfig")
     check(_lib.load().wgb_rope(int(variant), C.byref(config), _f32(q, "in_out_q"), q.numel(), _f32(k, "in_out_k"), k.numel(), _stream()))
 
 
 def attention(params, q, key_cache, value_cache, attn, xb):
+    if not isinstance(params, AttnParams):
+        raise TypeError("params: expected BatchedMultiqueryAttentionParams")
     need = params.seq_len * params.kv_dim
     if key_cache.numel() < need or value_cache.numel() < need or q.numel() != params.n_heads * params.head_size \
             or xb.numel() != q.numel() or (attn is not None and attn.numel() < params.n_heads * params.seq_len):
